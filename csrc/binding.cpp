@@ -49,7 +49,7 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
           const OptT& sfa, const OptT& sfb, int64_t mc, int64_t pf_tiles, int64_t stages, int64_t free_lag, int64_t out2_ptr,
           // fused MX quantisation of the output / RMSNorm statistics (raw addresses, 0 = off)
           int64_t q_out8, int64_t q_sf, int64_t ld_q, int64_t q_bn, int64_t sumsq_out, int64_t zero_buf, int64_t sumsq,
-          const OptT& gather_ids, int64_t gather_n, int64_t gather_rows) {
+          const OptT& gather_ids, int64_t gather_n, int64_t gather_rows, int64_t wide) {
   const bool fp8 = w.scalar_type() == at::kFloat8_e4m3fn;
   if (fp8) {
     TORCH_CHECK(x.scalar_type() == at::kFloat8_e4m3fn && w.is_cuda() && x.is_cuda() && w.is_contiguous() &&
@@ -140,6 +140,10 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
   if (p.epi == b2b::EPI_RESIDUAL) TORCH_CHECK(p.residual != nullptr, "residual epilogue needs residual");
   if (p.epi == b2b::EPI_GLU) TORCH_CHECK(p.out != nullptr || (p.q_out8 != nullptr && p.sfa != nullptr), "GLU epilogue needs an output");
   if (p.signal_flag || p.bump_epoch) TORCH_CHECK(p.done_counter != nullptr, "handoff needs done_counter");
+  if (wide && b2b::gemm_wide_supported(p)) {      // (wide: 1, or the feature tile to use)
+    check(b2b::launch_gemm_wide(p, w.data_ptr(), x.data_ptr(), static_cast<int>(wide), cur_stream()), "gemm_wide");
+    return;
+  }
   check(b2b::launch_gemm_tc(p, w.data_ptr(), x.data_ptr(), static_cast<int>(bn), cur_stream()), "gemm_tc");
 }
 
@@ -147,6 +151,7 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
 void set_wait_policy(int64_t abort_word, double limit_ms) {
   const auto ns = static_cast<unsigned long long>(limit_ms * 1e6);
   check(b2b::set_wait_policy_gemm(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(gemm)");
+  check(b2b::set_wait_policy_wide(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(wide)");
   check(b2b::set_wait_policy_elementwise(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(elementwise)");
   check(b2b::set_wait_policy_mixed(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(mixed)");
   check(b2b::set_wait_policy_diff(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(diff)");
@@ -990,6 +995,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "bee2bee_b200 native sm_100a kernels + NVLink peer-memory runtime";
   m.def("gemm", &gemm);
   m.def("gemm_max_splitk", &gemm_max_splitk);
+  m.def("gemm_wide_clusters4", &b2b::gemm_wide_clusters4);
+  m.def("gemm_wide_gave_up", &b2b::gemm_wide_gave_up);
   m.def("init_kernels", &init_kernels);
   m.def("set_pdl", &set_pdl);
   m.def("get_pdl", &get_pdl);

@@ -1,0 +1,662 @@
+// Prefill GEMM: many tokens, pairs of CTAs, persistent tiles.
+//
+//   out[t, n] = epilogue( sum_k X[t, k] * W[n, k] )        (the epilogues of gemm_tc.cu, bf16 operands, fp32 accumulators)
+//
+// gemm_tc.cu makes the weights the 128 MMA rows and the tokens the columns, which is what few tokens want.  With hundreds of tokens
+// it is bound by shared memory (a CTA reads 128 + 256 operand rows per 128 x 256 tile) and by its epilogue (a lane owns one feature,
+// so every store of a warp is 64 bytes of one token).  Here the TOKENS are the rows:
+//
+//   * a pair of CTAs (tcgen05 cta_group::2) owns 256 tokens x BN features: each CTA holds its 128 token rows and HALF of the
+//     weight rows, the tensor cores read the other half from the neighbour's shared memory -- 128 + 128 rows per CTA for twice
+//     the work of a 128 x 256 tile;
+//   * one pair per two SMs walks the tiles (persistent); the accumulator is double-buffered in tensor memory, so
+//     the epilogue of a tile runs under the main loop of the next one;
+//   * a lane owns one token and 32 adjacent features per TMEM read: rotary pairs, gate/up pairs and residual rows are in its own
+//     registers or 16-byte accesses away, and the finished 32 x 128-byte block goes through shared memory so that a warp
+//     stores whole 128-byte rows;
+//   * tiles left over after the last full round may be split (clusters of four CTAs then): the two pairs of a cluster take half of K each
+//     and exchange half of the columns through distributed shared memory, which halves the time of that round;
+//   * the piece handoff of gemm_tc.cu is here too (wait for the upstream flag, stores into the peer, release flag), so that pieces on
+//     several GPUs run the same arithmetic as one piece.
+//
+// Order of the tiles: token tiles first, so the pairs of a round share few weight tiles (which come from HBM once) and all of X (L2).
+//
+// Bound: tensor pipe (98 % active while a tile runs) and the power cap.  Measured on B200, Llama-3-8B layer shapes, us (TFLOP/s), back to
+// back with cold weights, gemm_tc.cu -> here:
+//   4096 tokens: QKV 218 (945) -> 131 (1573), O 157 (875) -> 96 (1436), gate/up 1041 (924) -> 595 (1616), down 404 (1191) -> 342 (1405)
+//    512 tokens: QKV 39 (656) -> 22 (1193),   O 27 (633) -> 18 (978),   gate/up 139 (866) -> 91 (1326),   down 59 (1019) -> 50 (1198)
+//    160 tokens: QKV 40 -> 17, O 33 -> 14, gate/up 84 -> 55, down 60 -> 30 (the weights alone: 8, 5, 36, 18)
+// Roles (192 threads): warp 0 = TMA producer (both CTAs), warp 1 = TMEM owner, MMA issuer in the pair's even CTA, warps 2..5 = epilogue.
+#include "gemm_tc.cuh"
+
+#include "common.cuh"
+#include "kernels.h"
+#include "launch.cuh"
+#include "tmem.cuh"
+
+namespace b2b {
+
+int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, int elt_bytes);
+
+namespace {
+
+constexpr int WM = 128;                    // token rows per CTA (256 per pair)
+constexpr int WK = 64;                     // K elements per stage (one 128-byte swizzled row)
+constexpr int WA_BYTES = WM * 128;
+constexpr int WIDE_THREADS = 192;
+constexpr int WIDE_PAIRS = 74;             // of the 148 SMs
+constexpr int EPI_PITCH = 144;             // bytes per staged row of 128: 16-byte accesses of 8 lanes fall into distinct banks
+constexpr int EPI_BYTES = 4 * 32 * EPI_PITCH;
+
+__device__ unsigned int g_wide_gave_up = 0;        // CTAs whose waits ran out since the module was loaded
+
+template <int BN>
+struct WideCfg {
+  static constexpr int kBBytes = BN / 2 * 128;                           // this CTA's half of the weight rows
+  static constexpr int kStageBytes = WA_BYTES + kBBytes;
+  static constexpr int kStages = BN == 256 ? 6 : (BN == 192 ? 7 : 8);
+  static constexpr int kLandPitch = BN / 2 + 4;                          // floats per row of the split-K landing zone
+  static constexpr int kSmem = 1024 + kStages * kStageBytes + EPI_BYTES + 512;
+  static constexpr uint32_t kTmemCols = BN == 128 ? 256 : 512;
+  static_assert(WM * kLandPitch * 4 <= kStages * kStageBytes, "the landing zone reuses the ring");
+};
+
+__device__ __forceinline__ float w_gelu(float x) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
+}
+__device__ __forceinline__ float w_silu(float x) { return x / (1.f + __expf(-x)); }
+__device__ __forceinline__ float w_xielu(float x, float ap, float an) {
+  return x > 0.f ? ap * x * x + 0.5f * x : an * (expm1f(x) - x) + 0.5f * x;
+}
+
+template <uint32_t kCols>
+__device__ __forceinline__ void tmem_alloc2(uint32_t* smem_result) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)), "n"(kCols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+template <uint32_t kCols>
+__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(kCols) : "memory");
+}
+__device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the barrier at this offset in the CTAs of `mask` once the MMAs issued so far have retired
+__device__ __forceinline__ void umma2_commit(uint64_t* bar, uint16_t mask) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask)
+      : "memory");
+}
+// tiled load into this CTA's shared memory whose bytes are counted on a barrier of the pair's even CTA (`bar`: its cluster address)
+__device__ __forceinline__ void tma_load2(void* smem_dst, const CUtensorMap* m, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// one arrival per CTA; the last one releases the payload to the downstream piece and this piece's input slot to the upstream one
+__device__ __forceinline__ void publish_handoff(const GemmParams& p, uint32_t total) {
+  if (atomicAdd(p.done_counter, 1u) != total - 1) return;
+  __threadfence_system();
+  *p.done_counter = 0;
+  if (p.signal_flag != nullptr) {
+    const uint32_t e = *reinterpret_cast<volatile uint32_t*>(p.signal_epoch) + 1;
+    *reinterpret_cast<volatile uint32_t*>(p.signal_epoch) = e;
+    st_release_sys(p.signal_flag, e);
+  }
+  if (p.bump_epoch != nullptr) {
+    const uint32_t e = *reinterpret_cast<volatile uint32_t*>(p.bump_epoch) + 1;
+    *reinterpret_cast<volatile uint32_t*>(p.bump_epoch) = e;
+    if (p.ack_flag != nullptr) st_release_sys(p.ack_flag, e);
+  }
+}
+
+// what a pair works on: tile `t`, k-blocks [kb0, kb1), `split`: the other pair of the cluster has the rest of K
+struct Item {
+  int t, kb0, kb1;
+  bool split;
+};
+struct Plan {
+  int tiles, tok_tiles, nkb, pairs, full, rest;
+  bool split;
+  __device__ __forceinline__ bool get(int i, int pair, Item& it) const {
+    const int t = pair + i * pairs;
+    if (t < full) {
+      it = {t, 0, nkb, false};
+      return true;
+    }
+    if (i != full / pairs) return false;
+    if (split) {
+      if ((pair >> 1) >= rest) return false;
+      const int half = nkb / 2;
+      it = {full + (pair >> 1), (pair & 1) ? half : 0, (pair & 1) ? nkb : half, true};
+      return true;
+    }
+    it = {t, 0, nkb, false};
+    return t < tiles;
+  }
+};
+
+template <int BN, int EPI>
+__global__ void __launch_bounds__(WIDE_THREADS, 1)
+gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const GemmParams p,
+                 const int allow_split) {
+  using Cfg = WideCfg<BN>;
+  constexpr int STAGES = Cfg::kStages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* stage_out = smem + STAGES * Cfg::kStageBytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(stage_out + EPI_BYTES);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* acc_full = empty_bar + STAGES;         // [2]
+  uint64_t* acc_empty = acc_full + 2;              // [2], of the pair's even CTA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile uint32_t* abort = tmem_slot + 1;
+  __shared__ float freq_s[128];                    // rotary frequencies of a head (QKV epilogue)
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t crank = cluster_ctarank();
+  const bool odd = (crank & 1u) != 0u;             // which half of the pair
+  const uint32_t lead = crank & ~1u;
+  const int pair = static_cast<int>(blockIdx.x >> 1);
+
+  Plan plan;
+  plan.tok_tiles = (p.m_tok + 2 * WM - 1) / (2 * WM);
+  plan.tiles = plan.tok_tiles * ((p.n_out + BN - 1) / BN);
+  plan.nkb = p.k / WK;
+  plan.pairs = static_cast<int>(gridDim.x >> 1);
+  plan.full = plan.tiles / plan.pairs * plan.pairs;
+  plan.rest = plan.tiles - plan.full;
+  plan.split = allow_split != 0 && plan.rest > 0 && plan.rest <= plan.pairs / 2;      // (clusters of four)
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 8);                 // the epilogue warps of both CTAs
+    }
+    *abort = 0u;
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc2<Cfg::kTmemCols>(tmem_slot);
+  if constexpr (EPI == EPI_QKV_ROPE) {
+    if (p.rope_theta > 0.f)
+      for (int j = threadIdx.x; j < p.head_dim / 2; j += WIDE_THREADS)
+        freq_s[j] = exp2f(-(2.f * j / static_cast<float>(p.head_dim)) * log2f(p.rope_theta));
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_arrive_release();                        // the other CTAs arrive on these barriers
+  cluster_wait_acquire();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_launch_dependents();
+
+  bool ok = true;
+  Item it;
+  if (warp == 0) {
+    // ------------------------------------------------------------------------------------------------ TMA producer
+    if (elect_one()) {
+      uint32_t n = 0;                              // stages filled so far
+      auto fill = [&](int kb, int n0, int m0, bool w, bool x) {
+        const uint32_t s = n % STAGES;
+        uint8_t* st = smem + s * Cfg::kStageBytes;
+        const uint32_t bar = mapa_smem(smem_u32(&full_bar[s]), lead);
+        if (w) {
+          if (!odd) mbar_arrive_expect_tx(&full_bar[s], 2 * Cfg::kStageBytes);
+          tma_load2(st + WA_BYTES, &tmap_w, bar, kb * WK, n0 + (odd ? BN / 2 : 0));
+        }
+        if (x) tma_load2(st, &tmap_x, bar, kb * WK, m0 + (odd ? WM : 0));
+      };
+      for (int i = 0; ok && plan.get(i, pair, it); ++i) {
+        const int m0 = it.t % plan.tok_tiles * (2 * WM), n0 = it.t / plan.tok_tiles * BN;
+        int kb = it.kb0;
+        if (i == 0) {                              // the weights depend on no earlier kernel: fill the ring with them first
+          const int pre = min(STAGES, it.kb1 - it.kb0);
+          for (int j = 0; j < pre; ++j, ++n) fill(kb + j, n0, m0, true, false);
+          pdl_wait();
+          if (p.wait_flag != nullptr) {            // head of a piece: X is written by the upstream GPU
+            wait_flag_ge(p.wait_flag, *reinterpret_cast<const volatile uint32_t*>(p.wait_epoch) + 1);
+            fence_proxy_async_all();               // peer-written (generic proxy) data -> TMA (async proxy) reads
+          }
+          n = 0;
+          for (int j = 0; j < pre; ++j, ++n) fill(kb + j, n0, m0, false, true);
+          kb += pre;
+        }
+        for (; kb < it.kb1; ++kb, ++n) {
+          if (!(ok = ma_wait(&empty_bar[n % STAGES], (n / STAGES & 1u) ^ 1u, abort))) break;
+          fill(kb, n0, m0, true, true);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // -------------------------------------------------------------------------------------------------- MMA issuer
+    if (!odd && elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(2 * WM, BN);
+      const uint16_t both = static_cast<uint16_t>(3u << lead);
+      uint32_t n = 0;
+      for (int i = 0; ok && plan.get(i, pair, it); ++i) {
+        const uint32_t b = i & 1;
+        if (!(ok = ma_wait(&acc_empty[b], (i >> 1 & 1) ^ 1u, abort))) break;
+        tc_fence_after();
+        for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
+          const uint32_t s = n % STAGES;
+          if (!(ok = ma_wait(&full_bar[s], n / STAGES & 1u, abort))) break;
+          tc_fence_after();
+          const uint64_t a = make_sw128_kmajor_desc(smem_u32(smem + s * Cfg::kStageBytes));
+          const uint64_t w = make_sw128_kmajor_desc(smem_u32(smem + s * Cfg::kStageBytes + WA_BYTES));
+#pragma unroll
+          for (int k = 0; k < WK / 16; ++k) umma2_bf16(tmem + b * BN, a + 2 * k, w + 2 * k, idesc, (kb > it.kb0 || k > 0) ? 1u : 0u);
+          umma2_commit(&empty_bar[s], both);
+        }
+        if (ok) umma2_commit(&acc_full[b], both);
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------------------------------------------- epilogue
+    const int q = warp & 3;
+    const int row = q * 32 + lane;                 // TMEM lane == token row of this CTA
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(q * 32) << 16);
+    uint8_t* sbuf = stage_out + (warp - 2) * 32 * EPI_PITCH;
+    uint8_t* srow = sbuf + lane * EPI_PITCH;       // this lane's staged row
+    const int sr = lane >> 3, sc = (lane & 7) * 16;        // coalesced view: rows sr + 4 i, byte column sc
+    const int q_dim = p.n_q_heads * p.head_dim, kv_dim = p.n_kv_heads * p.head_dim;
+    pdl_wait();
+    if (p.wait_flag != nullptr) wait_flag_ge(p.wait_flag, *reinterpret_cast<const volatile uint32_t*>(p.wait_epoch) + 1);
+    if (p.free_flag != nullptr)                    // back-pressure: the consumer must have drained the previous payload of this slot
+      wait_flag_ge(p.free_flag, *reinterpret_cast<const volatile uint32_t*>(p.signal_epoch) - p.free_lag);
+
+    // the residual values of a 64-column block in the coalesced view, in flight while the accumulators are awaited or worked on
+    uint4 res[EPI == EPI_RESIDUAL ? 8 : 1];
+    auto fetch_res = [&](int m0, int n) {
+      if constexpr (EPI == EPI_RESIDUAL) {
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(p.residual + n) + sc;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int t = m0 + q * 32 + sr + 4 * i;
+          res[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (t < p.m_tok && n < p.n_out) res[i] = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * p.ld_res * 2);
+        }
+      }
+    };
+    // columns [c0, c1) of the tile at (token m0, feature n0); `land`: the other pair's partial sums of this lane's row, from column c0 on
+    auto finish = [&](uint32_t acc, int m0, int n0, int c0, int c1, const float* land) {
+      const int tok = m0 + row;
+      const bool live = tok < p.m_tok;
+      if (m0 + q * 32 >= p.m_tok) return;          // no token of this warp (warp-uniform)
+      const float rs = (p.rstd != nullptr && live) ? p.rstd[tok] : 1.f;
+      int slot = -1;
+      float pos = 0.f;
+      if constexpr (EPI == EPI_QKV_ROPE) {
+        slot = live ? p.slots[tok] : -1;
+        pos = (p.positions != nullptr && live) ? static_cast<float>(p.positions[tok]) : 0.f;
+      }
+      auto load = [&](int c, float* v) {           // 32 accumulator columns, scaled
+        uint32_t r[32];
+        ma_ld32(acc + c, r);
+        ma_ld_fence(r);
+        if (land != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 o = *reinterpret_cast<const float4*>(land + (c - c0) + 4 * j);
+            v[4 * j] = __uint_as_float(r[4 * j]) + o.x;
+            v[4 * j + 1] = __uint_as_float(r[4 * j + 1]) + o.y;
+            v[4 * j + 2] = __uint_as_float(r[4 * j + 2]) + o.z;
+            v[4 * j + 3] = __uint_as_float(r[4 * j + 3]) + o.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] *= rs;
+        if (p.bias != nullptr) {
+          const float4* b4 = reinterpret_cast<const float4*>(p.bias + n0 + c);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 bv = b4[j];
+            v[4 * j] += bv.x; v[4 * j + 1] += bv.y; v[4 * j + 2] += bv.z; v[4 * j + 3] += bv.w;
+          }
+        }
+      };
+      auto put = [&](int half, const float* v) {   // 32 values as bf16 into this lane's staged row
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          *reinterpret_cast<uint4*>(srow + half * 64 + j * 16) = make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
+                                                                            pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
+      };
+      // staged rows -> memory: `base` = address of token m0's row at this block's first column, `ld` in bytes
+      auto flush = [&](uint8_t* base, size_t ld) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = sr + 4 * i, t = q * 32 + r;
+          const uint4 w = *reinterpret_cast<const uint4*>(sbuf + r * EPI_PITCH + sc);
+          if (m0 + t < p.m_tok) *reinterpret_cast<uint4*>(base + static_cast<size_t>(m0 + t) * ld + sc) = w;
+        }
+        __syncwarp();
+      };
+
+      if constexpr (EPI == EPI_GLU) {              // 64 gate columns, then 64 up columns -> 64 outputs
+        for (int c = c0; c < c1 && n0 + c < p.n_out; c += 128) {
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            float g[32], u[32];
+            load(c + half * 32, g);
+            load(c + 64 + half * 32, u);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) g[j] = (p.act_gelu ? w_gelu(g[j]) : w_silu(g[j])) * u[j];
+            put(half, g);
+          }
+          flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>((n0 + c) / 2) * 2, static_cast<size_t>(p.ld_out) * 2);
+        }
+      } else if (EPI == EPI_PLAIN && p.out_fp32) {
+        for (int c = c0; c < c1 && n0 + c < p.n_out; c += 32) {
+          float v[32];
+          load(c, v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<float4*>(srow + j * 16) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(n0 + c) * 4, static_cast<size_t>(p.ld_out) * 4);
+        }
+      } else {
+        for (int c = c0; c < c1 && n0 + c < p.n_out; c += 64) {
+          const int n = n0 + c;
+          if constexpr (EPI == EPI_RESIDUAL) {     // the residual rows of this block, whole rows at a time
+#pragma unroll
+            for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(sbuf + (sr + 4 * i) * EPI_PITCH + sc) = res[i];
+            if (c + 64 < c1) fetch_res(m0, n + 64);
+            __syncwarp();
+          }
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            float v[32];
+            load(c + half * 32, v);
+            if constexpr (EPI == EPI_RESIDUAL) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint4 w = *reinterpret_cast<const uint4*>(srow + half * 64 + j * 16);
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float2 f = __bfloat1622float2(h[e]);
+                  v[8 * j + 2 * e] += f.x;
+                  v[8 * j + 2 * e + 1] += f.y;
+                }
+              }
+            } else if constexpr (EPI == EPI_GELU) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                if (p.act_gelu == 2) {
+                  const float r = fmaxf(v[j], 0.f);
+                  v[j] = r * r;
+                } else {
+                  v[j] = p.act_gelu == 3 ? w_xielu(v[j], p.rope_theta, p.q_scale) : w_gelu(v[j]);
+                }
+              }
+            } else if constexpr (EPI == EPI_QKV_ROPE) {
+              const int f = n + half * 32;
+              const int sect = f < q_dim ? 0 : (f < q_dim + kv_dim ? 1 : 2);
+              if (sect < 2 && p.rope_theta > 0.f) {
+                const int j0 = ((f - (sect ? q_dim : 0)) % p.head_dim) >> 1;      // columns (2j, 2j+1) hold (x_j, x_{j+hd/2})
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  float sn, cs;
+                  sincosf(pos * freq_s[j0 + j], &sn, &cs);
+                  const float a = v[2 * j], b = v[2 * j + 1];
+                  v[2 * j] = a * cs - b * sn;
+                  v[2 * j + 1] = b * cs + a * sn;
+                }
+              }
+              if (sect == 0) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] *= p.q_scale;
+              }
+            }
+            put(half, v);
+          }
+          if constexpr (EPI == EPI_QKV_ROPE) {
+            if (n < q_dim) {
+              flush(reinterpret_cast<uint8_t*>(p.q_out + n), static_cast<size_t>(q_dim) * 2);
+            } else {                               // a cache row per token
+              const bool key = n < q_dim + kv_dim;
+              uint8_t* base = reinterpret_cast<uint8_t*>(key ? p.k_cache + (n - q_dim) : p.v_cache + (n - q_dim - kv_dim));
+              __syncwarp();
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int r = sr + 4 * i;
+                const int sl = __shfl_sync(0xffffffffu, slot, r);
+                const uint4 w = *reinterpret_cast<const uint4*>(sbuf + r * EPI_PITCH + sc);
+                if (sl >= 0) *reinterpret_cast<uint4*>(base + static_cast<size_t>(sl) * kv_dim * 2 + sc) = w;
+              }
+              __syncwarp();
+            }
+          } else {
+            flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(n) * 2, static_cast<size_t>(p.ld_out) * 2);
+            if (EPI == EPI_RESIDUAL && p.out2 != nullptr)
+              flush(reinterpret_cast<uint8_t*>(p.out2) + static_cast<size_t>(n) * 2, static_cast<size_t>(p.ld_out) * 2);
+          }
+        }
+      }
+    };
+
+    int i = 0;
+    bool tail = false;
+    for (; ok && plan.get(i, pair, it); ++i) {
+      const uint32_t b = i & 1;
+      const int m0 = it.t % plan.tok_tiles * (2 * WM) + (odd ? WM : 0), n0 = it.t / plan.tok_tiles * BN;
+      fetch_res(m0, n0 + (it.split && (crank >> 1) ? BN / 2 : 0));
+      ok = __all_sync(0xffffffffu, ma_wait(&acc_full[b], i >> 1 & 1, abort));
+      if (!ok) break;
+      tc_fence_after();
+      if (it.split) {                              // the last item: finished behind the exchange below
+        tail = true;
+        break;
+      }
+      finish(lanes + b * BN, m0, n0, 0, BN, nullptr);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive_cluster(mapa_smem(smem_u32(&acc_empty[b]), lead));
+    }
+    if (plan.split) {
+      // ------------------------------------- exchange of a split tile: pair 0 finishes columns [0, BN/2), pair 1 the others
+      const uint32_t acc = lanes + (i & 1) * BN;
+      const int mine = (crank >> 1) ? BN / 2 : 0, theirs = BN / 2 - mine;
+      cluster_arrive_release();                    // every MMA of the cluster has retired: the rings are free
+      cluster_wait_acquire();
+      if (tail) {
+        const uint32_t zone = mapa_smem(smem_u32(smem), crank ^ 2u) + static_cast<uint32_t>(row * Cfg::kLandPitch * 4);
+#pragma unroll 1
+        for (int c = 0; c < BN / 2; c += 32) {
+          uint32_t r[32];
+          ma_ld32(acc + theirs + c, r);
+          ma_ld_fence(r);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            st_dsmem_v4(zone + (c + 4 * j) * 4, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                            __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
+        }
+      }
+      cluster_arrive_release();
+      cluster_wait_acquire();
+      if (tail)
+        finish(acc, it.t % plan.tok_tiles * (2 * WM) + (odd ? WM : 0), it.t / plan.tok_tiles * BN, mine, mine + BN / 2,
+               reinterpret_cast<const float*>(smem) + row * Cfg::kLandPitch);
+      tc_fence_before();
+    }
+    if (p.signal_flag != nullptr || p.bump_epoch != nullptr) {        // tail of a piece: the last CTA publishes the payload
+      __threadfence_system();                      // my (possibly peer-directed) stores are performed
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (threadIdx.x == 64) publish_handoff(p, gridDim.x);
+    }
+  }
+  if (warp < 2) {
+    __syncwarp();
+    if (plan.split) {
+      for (int k = 0; k < 2; ++k) {
+        cluster_arrive_release();
+        cluster_wait_acquire();
+      }
+    }
+  }
+  if (*abort != 0u) __nanosleep(200000);           // copies in flight land before the shared memory is given back
+  tc_fence_before();
+  __syncthreads();
+  cluster_arrive_release();                        // no CTA leaves while another may still arrive on its barriers or read its operands
+  cluster_wait_acquire();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc2<Cfg::kTmemCols>(tmem);
+  }
+  if (threadIdx.x == 0 && *abort != 0u) atomicAdd(&g_wide_gave_up, 1u);
+}
+
+// One launch: `pairs` pairs of CTAs in clusters of 2, or (split) of 4.
+template <int BN, int EPI>
+int launch_wide_one(const GemmParams& p, const CUtensorMap& tw, const CUtensorMap& tx, int pairs, bool split, cudaStream_t stream) {
+  static bool set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !set[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_wide_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<BN>::kSmem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (dev < 64) set[dev] = true;
+  }
+  return static_cast<int>(launch_kernel_cx(gemm_wide_kernel<BN, EPI>, dim3(2 * pairs), dim3(WIDE_THREADS), WideCfg<BN>::kSmem, stream,
+                                           split ? 4u : 2u, tw, tx, p, split ? 1 : 0));
+}
+
+template <int BN>
+int launch_wide_bn(const GemmParams& p, const CUtensorMap& tw, const CUtensorMap& tx, int pairs, bool split, cudaStream_t stream) {
+  switch (p.epi) {
+    case EPI_PLAIN: return launch_wide_one<BN, EPI_PLAIN>(p, tw, tx, pairs, split, stream);
+    case EPI_RESIDUAL: return launch_wide_one<BN, EPI_RESIDUAL>(p, tw, tx, pairs, split, stream);
+    case EPI_GLU:
+      if constexpr (BN % 128 == 0) return launch_wide_one<BN, EPI_GLU>(p, tw, tx, pairs, split, stream);
+      return -4;
+    case EPI_QKV_ROPE: return launch_wide_one<BN, EPI_QKV_ROPE>(p, tw, tx, pairs, split, stream);
+    case EPI_GELU: return launch_wide_one<BN, EPI_GELU>(p, tw, tx, pairs, split, stream);
+    default: return -4;
+  }
+}
+
+// Clusters of four CTAs that are resident at once: a GPC whose SM count is no multiple of four leaves some idle, so fewer than 37 (a
+// persistent grid of 37 ran its last clusters in a second pass and took twice as long).
+int wide_clusters4() {
+  static int known[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 64 && known[dev] > 0) return known[dev];
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(148);
+  cfg.blockDim = dim3(WIDE_THREADS);
+  cfg.dynamicSmemBytes = WideCfg<256>::kSmem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 4;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(gemm_wide_kernel<256, EPI_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<256>::kSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_wide_kernel<256, EPI_PLAIN>, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = 1;
+  }
+  if (n > 37) n = 37;
+  if (dev < 64) known[dev] = n;
+  return n;
+}
+
+struct WideChoice {
+  int bn, pairs;
+  bool split;
+  double cost;
+};
+
+// Rounds of a choice in units of a 256-wide tile's round (a 192-wide tile costs 0.78 of it, a 128-wide one 0.58: its token rows are reused half as often; a
+// split round 0.6: half of K, and the exchange).
+WideChoice wide_choice(const GemmParams& p, int bn, bool split) {
+  const int tiles = ((p.m_tok + 2 * WM - 1) / (2 * WM)) * ((p.n_out + bn - 1) / bn);
+  WideChoice c{bn, WIDE_PAIRS, split, 0.0};
+  const double unit = bn == 256 ? 1.0 : (bn == 192 ? 0.78 : 0.58);
+  if (!split) {
+    c.cost = unit * ((tiles + WIDE_PAIRS - 1) / WIDE_PAIRS);
+    if (tiles < WIDE_PAIRS) c.pairs = tiles;       // the next kernel of the stream may use the other SMs for its set-up
+    return c;
+  }
+  const int clusters = wide_clusters4(), rest = tiles % (2 * clusters);
+  c.pairs = tiles <= clusters ? 2 * tiles : 2 * clusters;
+  c.cost = unit * (tiles / (2 * clusters) + (rest == 0 ? 0.0 : (rest <= clusters ? 0.6 : 1.0)));
+  return c;
+}
+
+}  // namespace
+
+bool gemm_wide_supported(const GemmParams& p) {
+  const int elt = (p.epi == EPI_PLAIN && p.out_fp32) ? 4 : 2;
+  if (p.fp8 || p.norm_src || p.dbg || p.q_out8 || p.sumsq || p.sumsq_out || p.zero_buf) return false;
+  if (p.n_out % 128 != 0 || p.k % WK != 0 || p.k < 2 * WK || p.m_tok <= 0) return false;
+  if (p.epi == EPI_GELU && p.act_gelu == 4) return false;
+  if (p.bias && (reinterpret_cast<uintptr_t>(p.bias) & 15)) return false;
+  if (p.epi == EPI_QKV_ROPE) {
+    if (p.head_dim > 256 || p.head_dim % 32 || (p.n_q_heads * p.head_dim) % 128 || (p.n_kv_heads * p.head_dim) % 128) return false;
+    return !((reinterpret_cast<uintptr_t>(p.q_out) | reinterpret_cast<uintptr_t>(p.k_cache) | reinterpret_cast<uintptr_t>(p.v_cache)) & 15);
+  }
+  if (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.out2)) & 15) || (static_cast<size_t>(p.ld_out) * elt) % 16) return false;
+  if (p.epi == EPI_RESIDUAL && ((reinterpret_cast<uintptr_t>(p.residual) & 15) || (static_cast<size_t>(p.ld_res) * 2) % 16)) return false;
+  return true;
+}
+
+int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, cudaStream_t stream) {
+  if (!gemm_wide_supported(p)) return -2;
+  const bool can_split = p.k / WK >= 8;
+  WideChoice best{0, 0, false, 1e30};
+  for (int b = 256; b >= 128; b -= 64) {
+    if (bn >= 128 && bn <= 256 && b != bn) continue;
+    if (b == 192 && p.epi == EPI_GLU) continue;                                  // (gate/up pairs are 128 columns wide)
+    for (int s = 0; s < 2; ++s) {
+      if (s && (!can_split || b == 192 || (b == 128 && p.epi == EPI_GLU))) continue;     // halves are whole 64-column blocks
+      const WideChoice c = wide_choice(p, b, s != 0);
+      if (c.cost < best.cost) best = c;
+    }
+  }
+  CUtensorMap tw, tx;
+  int r = make_tmap_shared(&tw, w, p.n_out, p.k, p.k, best.bn / 2, 2);
+  if (r) return r;
+  if ((r = make_tmap_shared(&tx, x, p.m_tok, p.k, p.k, WM, 2))) return r;
+  if (best.bn == 0) return -4;
+  if (best.bn == 192) return launch_wide_bn<192>(p, tw, tx, best.pairs, false, stream);
+  return best.bn == 128 ? launch_wide_bn<128>(p, tw, tx, best.pairs, best.split, stream)
+                        : launch_wide_bn<256>(p, tw, tx, best.pairs, best.split, stream);
+}
+
+int gemm_wide_clusters4() { return wide_clusters4(); }
+
+int set_wait_policy_wide(uint32_t* abort_word, unsigned long long limit_ns) {
+  cudaError_t e = cudaMemcpyToSymbol(g_abort_word, &abort_word, sizeof(abort_word));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_wait_limit_ns, &limit_ns, sizeof(limit_ns));
+  return static_cast<int>(e);
+}
+
+unsigned gemm_wide_gave_up() {
+  unsigned n = 0;
+  return cudaMemcpyFromSymbol(&n, g_wide_gave_up, sizeof(n)) == cudaSuccess ? n : ~0u;
+}
+
+}  // namespace b2b

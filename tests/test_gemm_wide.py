@@ -1,0 +1,96 @@
+"""The CTA-pair GEMM of many tokens (csrc/gemm_wide.cu) against 64-bit products, at the sizes where its tiles can go wrong: one row more or
+less than a 256-token tile, feature counts that leave part of a tile, every tile width and the split last round."""
+import pytest
+import torch
+
+from bee2bee_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+ROUND = 2.0 ** -8        # a bf16 result is within half a unit of 2^-8 of the exact one; fp32 sums of these lengths add less than 2^-14
+
+
+def bf(*shape, scale=1.0, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed + sum(shape))
+    return (torch.randn(*shape, device="cuda", generator=g) * scale).to(torch.bfloat16)
+
+
+def near(a, b, bound=ROUND):
+    assert torch.isfinite(a.float()).all()
+    err = (a.double() - b.double()).norm() / b.double().norm()
+    assert err <= bound, float(err)
+
+
+# 129 / 255 / 256 / 257: around a token tile; 65: half a tile.  Features: 128 (one 128-wide tile), 18944 (74 tiles of 256), 13056 (192-wide
+# tiles with a rest of 0 and 128), 4224 x 700 tokens (a ragged last tile).  k 128: the shortest ring; 576: no multiple of the ring depth.
+@pytest.mark.parametrize("m,n,k", [(65, 128, 128), (129, 384, 576), (255, 1024, 512), (256, 18944, 128), (257, 13056, 192), (700, 4224, 1024),
+                                   (300, 6144, 4096)])
+def test_epilogues(m, n, k):
+    w, x, res = bf(n, k, scale=k ** -0.5), bf(m, k), bf(m, n)
+    bias = torch.randn(n, device="cuda")
+    rstd = torch.rand(m, device="cuda") + 0.5
+    ref = x.double() @ w.double().t()
+    near(ops.gemm(w, x, rstd=rstd, bias=bias), ref * rstd.double()[:, None] + bias.double())
+    near(ops.gemm(w, x, bias=bias, out_fp32=True), ref + bias.double(), 1e-5)
+    near(ops.gemm(w, x, epi=ops.EPI_RESIDUAL, residual=res), ref + res.double())
+    wide = torch.zeros(m, n + 64, device="cuda", dtype=torch.bfloat16)               # rows longer than the result
+    ops.gemm(w, x, out=wide[:, :n], epi=ops.EPI_GELU, act_gelu=ops.ACT_RELU_SQ)
+    near(wide[:, :n], ref.clamp_min(0).pow(2), 2 * ROUND)
+    assert float(wide[:, n:].abs().max()) == 0.0
+    near(ops.gemm(w, x, epi=ops.EPI_GELU, bias=bias), torch.nn.functional.gelu(ref + bias.double(), approximate="tanh"))
+
+
+@pytest.mark.parametrize("f,m", [(64, 129), (12672, 256), (1024, 1000)])             # 12672: 99 tiles, the last round is split
+@pytest.mark.parametrize("gelu", [0, 1])
+def test_gate_up(f, m, gelu):
+    k = 512
+    wg, wu, x = bf(f, k, scale=k ** -0.5, seed=1), bf(f, k, scale=k ** -0.5, seed=2), bf(m, k)
+    rstd = torch.rand(m, device="cuda") + 0.5
+    out = ops.gemm(ops.glu_interleave_rows(wg, wu), x, epi=ops.EPI_GLU, act_gelu=gelu, rstd=rstd)
+    g, u = (x.double() @ w.double().t() * rstd.double()[:, None] for w in (wg, wu))
+    g = torch.nn.functional.gelu(g, approximate="tanh") if gelu else torch.nn.functional.silu(g)
+    near(out, g * u)
+
+
+@pytest.mark.parametrize("hd,nq,nkv,m", [(128, 8, 2, 200), (64, 8, 4, 257), (256, 4, 2, 131)])
+def test_qkv(hd, nq, nkv, m):
+    k, theta = 256, 10000.0
+    n = (nq + 2 * nkv) * hd
+    w, x = bf(n, k, scale=k ** -0.5), bf(m, k)
+    pages = m // ops.PAGE + 2
+    pos = torch.randperm(600, device="cuda")[:m].int()
+    slots = torch.randperm(pages * ops.PAGE, device="cuda")[:m].int()
+    slots[::5] = -1
+    kc = torch.zeros(pages, ops.PAGE, nkv, hd, device="cuda", dtype=torch.bfloat16)
+    vc, q = torch.zeros_like(kc), torch.zeros(m, nq * hd, device="cuda", dtype=torch.bfloat16)
+    ops.gemm(w, x, epi=ops.EPI_QKV_ROPE, q_out=q, k_cache=kc, v_cache=vc, positions=pos, slots=slots, n_q_heads=nq, n_kv_heads=nkv,
+             head_dim=hd, rope_theta=theta, q_scale=0.25)
+    y = (x.double() @ w.double().t()).view(m, -1, hd)
+    ang = pos.double()[:, None] * theta ** (-torch.arange(0, hd, 2, device="cuda", dtype=torch.float64) / hd)
+    cos, sin = ang.cos()[:, None], ang.sin()[:, None]
+    a, b = y[..., 0::2], y[..., 1::2]
+    turned = torch.stack([a * cos - b * sin, b * cos + a * sin], -1).flatten(-2)
+    near(q.view(m, nq, hd), turned[:, :nq] * 0.25)
+    keep = slots >= 0
+    want_k, want_v = torch.zeros(kc.view(-1, nkv, hd).shape, device="cuda", dtype=torch.float64), None
+    want_v = want_k.clone()
+    want_k[slots[keep].long()], want_v[slots[keep].long()] = turned[keep][:, nq:nq + nkv], y[keep][:, nq + nkv:]
+    near(kc.view(-1, nkv, hd), want_k)
+    near(vc.view(-1, nkv, hd), want_v)
+    assert torch.equal(kc.view(-1, nkv, hd)[want_k.flatten(1).norm(dim=1) == 0], torch.zeros_like(kc.view(-1, nkv, hd)[want_k.flatten(1).norm(dim=1) == 0]))
+
+
+def test_handoff_words():
+    """upstream flag already published, consumer slot free: the flag words advance by one payload and both destinations hold the result"""
+    m, n, k = 200, 512, 256
+    w, x, res = bf(n, k, scale=k ** -0.5), bf(m, k), bf(m, n)
+    word = torch.zeros(8, device="cuda", dtype=torch.int32)      # in flag, in epoch, out flag, out epoch, done, ack, (free), unused
+    word[0] = 1
+    at = [word.data_ptr() + 4 * i for i in range(8)]
+    out, out2 = torch.zeros(m, n, device="cuda", dtype=torch.bfloat16), torch.zeros(m, n, device="cuda", dtype=torch.bfloat16)
+    ops.gemm(w, x, out=out, epi=ops.EPI_RESIDUAL, residual=res, wait_flag=at[0], wait_epoch=at[1], signal_flag=at[2], signal_epoch=at[3],
+             done_counter=at[4], bump_epoch=at[1], ack_flag=at[5], free_flag=at[6], out2_ptr=out2.data_ptr())
+    near(out, x.double() @ w.double().t() + res.double())
+    assert torch.equal(out, out2)
+    assert word.tolist() == [1, 1, 1, 1, 0, 1, 0, 0]
+    assert ops.native().gemm_wide_gave_up() == 0

@@ -606,8 +606,9 @@ def lin_scan(mode, qk, off_q, off_k, v, off_v, state, out, q_start, q_len, kv_le
              z=None, off_z=0, zbias=None, hparam=None, beta=None, off_b=0, aux=None, qscale=1.0, inv_tau=1.0, rdims=0):
     """Gated linear recurrence over the spans (``mode`` = SCAN_*); ``max_q`` = longest span of the batch (1: the decode
     variant).  SCAN_RETENTION: ``z`` is the rotary table of the step, the first ``rdims`` channels of q and k turn."""
-    native().lin_scan(mode, qk, off_q, off_k, v, off_v, z, off_z, zbias, hparam, beta, off_b, aux, float(qscale),
-                      float(inv_tau), state, out, q_start, q_len, kv_len, seq_slot, n_seqs, max_q, H, G, dk, dv, int(rdims))
+    n = native().lin_scan(mode, qk, off_q, off_k, v, off_v, z, off_z, zbias, hparam, beta, off_b, aux, float(qscale),
+                          float(inv_tau), state, out, q_start, q_len, kv_len, seq_slot, n_seqs, max_q, H, G, dk, dv, int(rdims))
+    LAUNCHES[0] += n - 1       # spans cut into segments: the local pass and the starts are kernels of their own
 
 
 #: spans from this length on run on ``lin_chunk`` where it has a kernel (its tile is 64 tokens)

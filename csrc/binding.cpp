@@ -682,7 +682,8 @@ void mlstm_gates(const Tensor& proj, int64_t off_q, int64_t off_k, int64_t off_i
         "mlstm_gates");
 }
 
-void lin_scan(int64_t mode, const Tensor& qk, int64_t off_q, int64_t off_k, const Tensor& v, int64_t off_v, const OptT& z,
+// returns the number of kernels it launched
+int64_t lin_scan(int64_t mode, const Tensor& qk, int64_t off_q, int64_t off_k, const Tensor& v, int64_t off_v, const OptT& z,
               int64_t off_z, const OptT& zbias, const OptT& hparam, const OptT& beta, int64_t off_b, const OptT& aux,
               double qscale, double inv_tau, const Tensor& state, const Tensor& out, const Tensor& q_start,
               const Tensor& q_len, const Tensor& kv_len, const Tensor& seq_slot, int64_t n_seqs, int64_t max_q, int64_t H,
@@ -695,6 +696,23 @@ void lin_scan(int64_t mode, const Tensor& qk, int64_t off_q, int64_t off_k, cons
                           : fp_or_null(z) != nullptr && fp_or_null(zbias) != nullptr,
               "lin_scan: missing gate inputs for this mode");
   TORCH_CHECK(mode != 1 || (fp_or_null(hparam) != nullptr && fp_or_null(beta) != nullptr), "lin_scan: delta rule inputs");
+  const int iv = static_cast<int>(n_seqs), mq = static_cast<int>(max_q), d = static_cast<int>(dk);
+  const int seg = b2b::lin_span_supported(static_cast<int>(mode), fp(v), static_cast<int>(v.stride(0)), static_cast<int>(off_v), fp(state), fp(out),
+                                          static_cast<int>(out.stride(0)), mq, d, static_cast<int>(dv))
+                      ? b2b::span_plan(iv, mq, static_cast<int>(H), d) : -1;
+  if (seg >= 0) {
+    Tensor ws;
+    if (seg > 0) ws = torch::empty({n_seqs * ((max_q + seg - 1) / seg) * H * (dk * dv + dk)}, state.options().dtype(at::kFloat));
+    check(b2b::launch_lin_span(static_cast<int>(mode), fp(qk), static_cast<int>(qk.stride(0)), static_cast<int>(off_q), static_cast<int>(off_k),
+                               fp(v), static_cast<int>(v.stride(0)), static_cast<int>(off_v), fp_or_null(z), ld(z), static_cast<int>(off_z),
+                               fp_or_null(zbias), fp_or_null(hparam), fp_or_null(beta), ld(beta), static_cast<int>(off_b), fp_or_null(aux),
+                               static_cast<float>(qscale), static_cast<float>(inv_tau), const_cast<float*>(fp(state)),
+                               const_cast<float*>(fp(out)), static_cast<int>(out.stride(0)), ip(q_start), ip(q_len), ip(kv_len), ip(seq_slot),
+                               iv, mq, static_cast<int>(H), static_cast<int>(G), d, seg,
+                               seg > 0 ? ws.data_ptr<float>() : nullptr, cur_stream()),
+          "lin_span");
+    return seg > 0 ? 3 : 1;
+  }
   check(b2b::launch_lin_scan(static_cast<int>(mode), fp(qk), static_cast<int>(qk.stride(0)), static_cast<int>(off_q),
                              static_cast<int>(off_k), fp(v), static_cast<int>(v.stride(0)), static_cast<int>(off_v),
                              fp_or_null(z), ld(z), static_cast<int>(off_z), fp_or_null(zbias), fp_or_null(hparam),
@@ -705,6 +723,7 @@ void lin_scan(int64_t mode, const Tensor& qk, int64_t off_q, int64_t off_k, cons
                              static_cast<int>(H), static_cast<int>(G), static_cast<int>(dk), static_cast<int>(dv),
                              static_cast<int>(rdims), cur_stream()),
         "lin_scan");
+  return 1;
 }
 
 void scan_post(const Tensor& o, const Tensor& gate, int64_t off_g, const Tensor& weight, int64_t act, const OptT& aux,

@@ -130,6 +130,15 @@ int launch_mlstm_gates(const float* proj, int ld, int off_q, int off_k, int off_
 // lower bound, its complement is the write strength; hparam = the bound [H * dk], z = the gate projection, no keys), 4
 // state-space recurrence (hparam = A_log [H], zbias = bias of the step size [H], beta = its projection), 5 retention (hparam =
 // decay [H], z = rotary table [T, rdims] of (cos, sin) pairs)
+// spans of the modes with a diagonal transition, a whole head per block (lin_span.cu); span_plan: tokens per segment when the spans are
+// cut into segments that run side by side (then `ws` holds n_seqs * segments * H * (dk * dk + dk) floats and three kernels are launched), 0: whole
+// spans, -1: lin_scan is the faster one
+bool lin_span_supported(int mode, const float* v, int ld_v, int off_v, const float* state, const float* out, int ld_out, int max_q, int dk, int dv);
+int span_plan(int n_seqs, int max_q, int H, int dk);
+int launch_lin_span(int mode, const float* qk, int ld_qk, int off_q, int off_k, const float* v, int ld_v, int off_v, const float* z, int ld_z,
+                    int off_z, const float* zbias, const float* hparam, const float* beta, int ld_b, int off_b, const float* aux, float qscale,
+                    float inv_tau, float* state, float* out, int ld_out, const int* q_start, const int* q_len, const int* kv_len,
+                    const int* seq_slot, int n_seqs, int max_q, int H, int G, int dk, int seg, float* ws, cudaStream_t s);
 int launch_lin_scan(int mode, const float* qk, int ld_qk, int off_q, int off_k, const float* v, int ld_v, int off_v,
                     const float* z, int ld_z, int off_z, const float* zbias, const float* hparam, const float* beta,
                     int ld_b, int off_b, const float* aux, float qscale, float inv_tau, float* state, float* out,

@@ -419,19 +419,16 @@ def add(a, b, out=None):
 # -------------------------------------------------------------------- attention
 def attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, *, max_q, n_q, n_kv, head_dim,
               window=0, softcap=0.0, splits=1, ws=None, use_tc=-1, fq_out=None, fq_sf=None, fq_bn=0):
-    """Paged-KV attention.  Prefill chunks (max_q >= 2) run on the tcgen05 flash kernel.  Decode (max_q == 1) also does
-    when the batch fills the machine (sequences x kv heads >= 128 CTAs) or no split-KV was asked for: measured on B200
-    (profiles/decode_attention.md) it streams the KV pages at 0.66 of the HBM peak at 8k context against 0.49 for the
-    CUDA-core split-KV kernel, and is faster even at 64 tokens (7.9 vs 10.1 us); few sequences with a long context
-    keep the split-KV kernel (more CTAs than (sequence, kv head) pairs)."""
+    """Paged-KV attention.  Prefill chunks (max_q >= 2) run on the tcgen05 flash kernel (csrc/attention_tc.cu).  Decode steps (max_q == 1) of
+    128- and 256-wide heads run on csrc/attn_decode.cu, which spreads the keys of few sequences over clusters by itself (``splits`` and
+    ``ws`` are not used; 32 sequences x 8.1 k keys: 160 us against 252 on the flash kernel, one sequence x 700 keys: 7.6 against 17.6).
+    64-wide heads: the flash kernel with one-token query blocks, ``splits`` parts of the keys merged by a second kernel.  ``use_tc`` 0: the
+    CUDA-core kernel."""
     if use_tc < 0 and max_q == 1:
-        # split-KV (few sequences x long context) also runs on the tensor-core kernel: every (sequence, kv head, split) CTA
-        # streams its share of the pages, the shared merge pass combines the partials
         use_tc = 1
-    native().attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, ws, max_q, n_q, n_kv, head_dim,
-                       window, softcap, splits, use_tc, _ptr(fq_out), _ptr(fq_sf), fq_bn)
-    if splits > 1:
-        LAUNCHES[0] += 1           # split-KV: the merge pass is a second kernel
+    n = native().attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, ws, max_q, n_q, n_kv, head_dim,
+                           window, softcap, splits, use_tc, _ptr(fq_out), _ptr(fq_sf), fq_bn)
+    LAUNCHES[0] += n - 1           # split-KV: the merge pass is a second kernel
     return out
 
 

@@ -282,7 +282,8 @@ static int64_t g_attn_tc_min_q = [] {
 void set_attn_tc_min_q(int64_t v) { g_attn_tc_min_q = v; }
 int64_t get_attn_tc_min_q() { return g_attn_tc_min_q; }
 
-void attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& out,
+// returns the number of kernels it launched
+int64_t attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, const Tensor& out,
                const Tensor& block_table, const Tensor& q_start, const Tensor& q_len, const Tensor& kv_len,
                const OptT& ws, int64_t max_q, int64_t n_q, int64_t n_kv, int64_t head_dim, int64_t window,
                double softcap, int64_t splits, int64_t use_tc, int64_t fq_out, int64_t fq_sf, int64_t fq_bn) {
@@ -298,6 +299,17 @@ void attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, co
     const int64_t R = b2b::attn_rows(static_cast<int>(n_q / n_kv), 1);
     TORCH_CHECK(ws->numel() >= seqs * n_kv * splits * R * (head_dim + 2), "attention workspace too small");
   }
+  if (want_tc && max_q == 1 && b2b::attn_decode_supported(static_cast<int>(n_q), static_cast<int>(n_kv), static_cast<int>(head_dim))) {
+    check(b2b::launch_attn_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
+                                  reinterpret_cast<const int*>(block_table.data_ptr()), reinterpret_cast<const int*>(q_start.data_ptr()),
+                                  reinterpret_cast<const int*>(q_len.data_ptr()), reinterpret_cast<const int*>(kv_len.data_ptr()), seqs,
+                                  static_cast<int>(block_table.size(1)), static_cast<int>(q.size(0)), static_cast<int>(k_cache.size(0)),
+                                  static_cast<int>(n_q), static_cast<int>(n_kv), static_cast<int>(head_dim), static_cast<int>(window),
+                                  static_cast<float>(softcap), as_ptr<void>(fq_out), as_ptr<void>(fq_sf), static_cast<int>(fq_bn),
+                                  cur_stream()),
+          "attn_decode");
+    return 1;
+  }
   if (want_tc &&
       b2b::attention_tc_supported(static_cast<int>(n_q), static_cast<int>(n_kv), static_cast<int>(head_dim))) {
     // prefill chunk: tcgen05 flash attention
@@ -312,7 +324,7 @@ void attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, co
                                    static_cast<int>(splits), ptr_or_null<float>(ws), as_ptr<void>(fq_out), as_ptr<void>(fq_sf),
                                    static_cast<int>(fq_bn), cur_stream()),
           "attention_tc");
-    return;
+    return max_q == 1 && splits > 1 ? 2 : 1;      // (split keys: the merge pass is a second kernel)
   }
   TORCH_CHECK(fq_out == 0, "fused output quantisation needs the tcgen05 attention kernel");
   if (splits > 1) {
@@ -329,6 +341,7 @@ void attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache, co
                               static_cast<int>(n_kv), static_cast<int>(head_dim), static_cast<int>(window),
                               static_cast<float>(softcap), static_cast<int>(splits), cur_stream()),
         "attention");
+  return max_q == 1 && splits > 1 ? 2 : 1;
 }
 
 // ---------------------------------------------------------------------- sampler
@@ -1013,6 +1026,7 @@ void side_gate(const Tensor& z, const Tensor& ids, const Tensor& table, int64_t 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "bee2bee_b200 native sm_100a kernels + NVLink peer-memory runtime";
   m.def("gemm", &gemm);
+  m.def("attn_decode_gave_up", &b2b::attn_decode_gave_up);
   m.def("gemm_max_splitk", &gemm_max_splitk);
   m.def("gemm_wide_clusters4", &b2b::gemm_wide_clusters4);
   m.def("gemm_wide_gave_up", &b2b::gemm_wide_gave_up);

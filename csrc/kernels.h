@@ -40,6 +40,12 @@ int launch_attention_tc(const void* q, const void* k_cache, const void* v_cache,
                         int n_tokens, int n_pages, int n_q, int n_kv, int head_dim, int window, float softcap,
                         int splits, float* ws, void* q_out8, void* q_sf, int q_bn, cudaStream_t s);
 // merge pass of split-KV decode (shared by the CUDA-core and the tcgen05 kernels)
+// one new token per sequence, keys as MMA rows (attn_decode.cu); _gave_up: CTAs whose bounded waits ran out so far, 0 unless there is a bug
+bool attn_decode_supported(int n_q, int n_kv, int head_dim);
+unsigned attn_decode_gave_up();
+int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table, const int* q_start,
+                       const int* q_len, const int* kv_len, int seqs, int max_pages, int n_tokens, int n_pages, int n_q, int n_kv,
+                       int head_dim, int window, float softcap, void* q_out8, void* q_sf, int q_bn, cudaStream_t s);
 int launch_attention_merge(void* out, const int* q_start, const float* ws, int seqs, int n_q, int n_kv, int head_dim,
                            int splits, cudaStream_t s);
 int attention_init();

@@ -1,0 +1,90 @@
+"""Decode attention with the keys as MMA rows (csrc/attn_decode.cu) against 64-bit sums: lengths around a tile (128 keys) and a page (64), one key,
+clusters that share the keys (few sequences, wide block tables), every head group size, windows, capped scores, idle rows, the e4m3 copy."""
+import pytest
+import torch
+
+from bee2bee_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+# probabilities are rounded to bf16 (2^-9 each, independent) as operands of the second product and the result once more: 2^-8 covers both
+BOUND = 2.0 ** -8
+
+
+def i32(v):
+    return torch.tensor(v, dtype=torch.int32, device="cuda")
+
+
+def setup(lens, nq, nkv, D, spare=0):
+    g = torch.Generator(device="cuda").manual_seed(nq * D + len(lens))
+    need = [(n + 63) // 64 for n in lens]
+    order = (torch.randperm(sum(need), generator=torch.Generator().manual_seed(1)) + 1).tolist()
+    table, at = [], 0
+    for n in need:
+        table.append(order[at:at + n] + [0] * (max(need) + spare - n))
+        at += n
+    k = torch.randn(sum(need) + 1, 64, nkv, D, generator=g, device="cuda").bfloat16()
+    v = torch.randn(sum(need) + 1, 64, nkv, D, generator=g, device="cuda").bfloat16()
+    q = (torch.randn(len(lens), nq * D, generator=g, device="cuda") * 2 * D ** -0.5).bfloat16()
+    return q, k, v, i32(table)
+
+
+def reference(q, k, v, table, lens, nq, nkv, D, window, cap):
+    out = torch.zeros(q.shape, device="cuda", dtype=torch.float64)
+    for s, n in enumerate(lens):
+        at = torch.arange(n, device="cuda")
+        at = (table[s].long()[at // 64] * 64 + at % 64)[max(0, n - window) if window else 0:]
+        kk, vv = (c.view(-1, nkv, D)[at].double().repeat_interleave(nq // nkv, 1) for c in (k, v))
+        sc = torch.einsum("hd,khd->hk", q[s].double().view(nq, D), kk)
+        if cap:
+            sc = cap * torch.tanh(sc / cap)
+        out[s] = torch.einsum("hk,khd->hd", sc.softmax(-1), vv).flatten()
+    return out
+
+
+@pytest.mark.parametrize("nq,nkv,D", [(32, 8, 128), (6, 1, 128), (16, 1, 128), (4, 2, 256), (12, 1, 256), (3, 3, 128)])
+@pytest.mark.parametrize("lens,spare", [([1], 0), ([700], 5), ([128, 129, 127, 64, 63, 65], 0), ([1, 3000, 250, 17], 40), ([90 * i + 1 for i in range(40)], 0)])
+@pytest.mark.parametrize("window,cap", [(0, 0.0), (100, 50.0), (0, 50.0), (128, 0.0)])
+def test_decode(nq, nkv, D, lens, spare, window, cap):
+    q, k, v, table = setup(lens, nq, nkv, D, spare)
+    S = len(lens)
+    idle = S // 2 if S > 2 else -1
+    on = [0 if s == idle else 1 for s in range(S)]
+    out = torch.full_like(q, 7.0)
+    ops.attention(q, k, v, out, table, i32(list(range(S))), i32(on), i32(lens), max_q=1, n_q=nq, n_kv=nkv, head_dim=D, window=window, softcap=cap)
+    keep = [s for s in range(S) if on[s]]
+    ref = reference(q, k, v, table, lens, nq, nkv, D, window, cap)[keep]
+    err = (out[keep].double() - ref).norm(dim=1) / ref.norm(dim=1)
+    assert float(err.max()) < BOUND
+    if idle >= 0:
+        assert bool((out[idle] == 7.0).all())
+    assert ops.native().attn_decode_gave_up() == 0
+
+
+def test_large_scores_move_the_reference():
+    """every later tile outgrows the reference maximum of the tiles before it"""
+    lens, nq, nkv, D = [1000], 8, 2, 128
+    q, k, v, table = setup(lens, nq, nkv, D)
+    at = torch.arange(1000, device="cuda")
+    rows = table[0].long()[at // 64] * 64 + at % 64
+    k.view(-1, nkv, D)[rows] = (k.view(-1, nkv, D)[rows].float() * (1 + at.float()[:, None, None] / 60)).bfloat16()
+    out = torch.zeros_like(q)
+    ops.attention(q, k, v, out, table, i32([0]), i32([1]), i32(lens), max_q=1, n_q=nq, n_kv=nkv, head_dim=D)
+    ref = reference(q, k, v, table, lens, nq, nkv, D, 0, 0.0)
+    assert float((out.double() - ref).norm() / ref.norm()) < BOUND
+
+
+@pytest.mark.parametrize("S", [3, 40])
+def test_quantised_copy(S):
+    nq, nkv, D = 8, 2, 128
+    lens = [100 + 37 * i for i in range(S)]
+    q, k, v, table = setup(lens, nq, nkv, D)
+    args = (table, i32(list(range(S))), i32([1] * S), i32(lens))
+    kw = dict(max_q=1, n_q=nq, n_kv=nkv, head_dim=D)
+    plain = ops.attention(q, k, v, torch.zeros_like(q), *args, **kw)
+    bn = ops.pick_bn_mx(S)
+    want_q, want_sf = ops.quant_mxfp8_rows(plain, bn)
+    fq, sf = torch.zeros(S, nq * D, device="cuda", dtype=torch.float8_e4m3fn), torch.full_like(want_sf, 127)
+    ops.attention(q, k, v, torch.zeros_like(q), *args, **kw, fq_out=fq, fq_sf=sf, fq_bn=bn)
+    assert torch.equal(fq.view(torch.uint8), want_q.view(torch.uint8))
+    assert torch.equal(ops.mx_unchunk(sf, S, nq * D, bn), ops.mx_unchunk(want_sf, S, nq * D, bn))

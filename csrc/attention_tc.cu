@@ -11,6 +11,11 @@
 // Warp roles: 0 = TMA producer, 1 = TMEM owner + MMA issuer, 2..5 = softmax / correction / epilogue.
 // q is pre-scaled by 1/sqrt(d) and rotated by the QKV GEMM epilogue; K is rotated when appended.
 //
+// Bound: the softmax warps' issue slots and latencies beside the hardware exponential (64 per row and tile, 47 % of its rate at T = 4096).
+// Measured on B200, causal, 32 / 8 heads of 128: 4096 tokens 169 -> 135 us (1019 TFLOP/s) with the query blocks of all heads in one
+// longest-first order, packed multiply-adds for the exponents and sums, and four chains instead of one for the row maximum; 8 / 4 heads of 256 with
+// capped scores 110 -> 80 us.
+//
 // Layouts: q/out [tokens, n_q, D]; K/V cache [pages, 64, n_kv, D]; block_table [seqs, max_pages].
 // Reference parity: torch SDPA under `transformers.generate` (bee2bee/hf.py:42-43).
 #include "kernels.h"
@@ -23,6 +28,7 @@
 
 #include "common.cuh"
 #include "launch.cuh"
+#include "tmem.cuh"
 
 namespace b2b {
 
@@ -54,7 +60,37 @@ struct AttnTcParams {
   uint8_t* q_out8;
   uint8_t* q_sf;
   int q_bn;
+  // hybrid graphs: fp32 query rows [token, heads, D] (times `scale`, rounded to bf16 here), the first keep_first keys stay visible
+  // whatever the window, exp(sink[head]) joins the denominator
+  const float* q32;
+  int ld_out;                    // elements between output rows
+  float scale;
+  int keep_first;
+  const float* sink;
 };
+
+typedef unsigned long long apair;            // two fp32 values: the same IEEE results at half the issue slots
+__device__ __forceinline__ apair apack(float lo, float hi) {
+  apair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void aunpack(apair v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ apair afma2(apair a, apair b, apair c) {
+  apair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ apair aadd2(apair a, apair b) {
+  apair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// through exp2: relative error of a few 2^-22 (the hardware tanh: 2^-11)
+__device__ __forceinline__ float tanh_exp(float x) {
+  const float e = ex2(fminf(fabsf(x), 15.f) * (2.f * LOG2E));
+  return copysignf(1.f - __fdividef(2.f, e + 1.f), x);
+}
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t r[32];
@@ -152,19 +188,6 @@ __device__ __forceinline__ void tmem_ld_fence(uint32_t* r) {
                : "memory");
 }
 
-// 2^x on the FMA/ALU pipes (Cody-Waite split + degree-3 minimax polynomial, rel. error 8.8e-5 << bf16 eps).
-// Kept for experiments: moving every other exponential here was SLOWER (660 vs 750 TFLOP/s at T=4096): the
-// softmax warps are issue/latency bound, not MUFU bound (profiles/attention_tc.md).
-__device__ __forceinline__ float exp2_poly(float x) {
-  x = fmaxf(x, -125.f);
-  const float t = __fadd_rd(x, 12582912.f);        // 1.5 * 2^23: floor(x) lands in the low mantissa bits
-  const float f = x - (t - 12582912.f);            // fractional part in [0, 1)
-  float p = fmaf(0.077119089663f, f, 0.227564394474f);
-  p = fmaf(p, f, 0.695146143436f);
-  p = fmaf(p, f, 1.0f);
-  return __uint_as_float(__float_as_uint(p) + (__float_as_uint(t) << 23));
-}
-
 template <int D>
 struct AtcCfg {
   static constexpr int BKV = 64;                                  // keys per tile == one KV page
@@ -178,7 +201,8 @@ struct AtcCfg {
 
 // P_TMEM (EXPERIMENTAL, default false): P stays in tensor memory (written over the first BKV/2 columns of the S buffer
 // it was computed from) and feeds the PV MMA as a TMEM A operand; no P tile in shared memory, no fence.proxy.async.
-template <int D, bool SOFTCAP, bool P_TMEM = false>
+// Q32: the options of the hybrid graphs (see AttnTcParams); P_TMEM only.
+template <int D, bool SOFTCAP, bool P_TMEM, bool Q32>
 __global__ void __launch_bounds__(ATC_THREADS, AtcCfg<D>::kMinCtas)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                        const __grid_constant__ CUtensorMap tm_v, const AttnTcParams p, const int G, const int QB) {
@@ -209,7 +233,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
+    mbar_init(q_full, Q32 ? 4 : 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
@@ -229,9 +253,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   // so an early O-proj CTA that takes TMEM columns and then waits for this grid can never starve one of its CTAs
   pdl_launch_dependents();
   pdl_wait();                                               // q / K / V and the metadata below come from earlier kernels
-  const int seq = blockIdx.z, kvh = blockIdx.y;
+  const int seq = blockIdx.z;
   const bool split_mode = p.splits > 1;
-  const int qblk = split_mode ? 0 : gridDim.x - 1 - blockIdx.x;   // longest (latest) query blocks first
+  // longest (latest) query blocks first, of all key/value heads (with the heads outside, the last head's long blocks started when little
+  // else was left: 23 % of the SM time of a causal 4096-token span was idle)
+  const int kvh = split_mode ? blockIdx.y : blockIdx.x, qblk = split_mode ? 0 : gridDim.y - 1 - blockIdx.y;
   const int qlen = p.q_len[seq], kvlen = p.kv_len[seq];
   const int q0 = qblk * QB;
   bool active = q0 < qlen;                                  // CTA-uniform; an idle CTA only runs the tear-down below
@@ -257,22 +283,27 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       active = false;
     }
   }
-  const int nt = t_hi - t_lo;
+  // tiles of kept first keys in front of the window
+  const int n_keep = (Q32 && p.window > 0 && p.keep_first > 0) ? min(t_lo, (p.keep_first + BKV - 1) / BKV) : 0;
+  const int nt = t_hi - t_lo + n_keep;
+  auto tile_of = [&](int n) { return n < n_keep ? n : t_lo + n - n_keep; };
 
   if (!active) {
     // nothing to compute (inactive row / empty split share)
   } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      mbar_arrive_expect_tx(q_full, Cfg::kQBytes);
-      for (int g = 0; g < G; ++g)
-        for (int c = 0; c < DB; ++c)
-          tma_load_2d(q_s + c * (128 * 128) + g * QB * 128, &tm_q, q_full, (kvh * G + g) * D + c * 64, qtok0);
+      if constexpr (!Q32) {
+        mbar_arrive_expect_tx(q_full, Cfg::kQBytes);
+        for (int g = 0; g < G; ++g)
+          for (int c = 0; c < DB; ++c)
+            tma_load_2d(q_s + c * (128 * 128) + g * QB * 128, &tm_q, q_full, (kvh * G + g) * D + c * 64, qtok0);
+      }
       const int* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
       for (int n = 0; n < nt; ++n) {
         const int s = n & 1;
         const uint32_t ph = static_cast<uint32_t>((n >> 1) & 1);
-        const int page = bt[t_lo + n];
+        const int page = bt[tile_of(n)];
         mbar_wait(&k_empty[s], ph ^ 1u);
         mbar_arrive_expect_tx(&k_full[s], Cfg::kKVBytes);
 #pragma unroll
@@ -342,10 +373,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const float cap = p.softcap;
     const float inv_cap = SOFTCAP ? 1.f / cap : 0.f;
+    const float unit = SOFTCAP ? 1.f : LOG2E;      // scores -> exponents of two
     float m_ref = -INFINITY, l = 0.f;
+    if constexpr (Q32) {                           // this warp's 32 query rows: scaled, fp32 -> bf16, swizzled; rows that do not exist are zero
+      constexpr int LPR = D / 4;                   // lanes per row of 16-byte pieces
+#pragma unroll 4
+      for (int j = lane / LPR; j < 32; j += 32 / LPR) {
+        const int r = quarter * 32 + j, gr = r / QB, ir = r % QB, e = (lane % LPR) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (gr < G && ir < nq_here)
+          x = *reinterpret_cast<const float4*>(p.q32 + (static_cast<size_t>(qtok0 + ir) * p.n_q + kvh * G + gr) * D + e);
+        *reinterpret_cast<uint2*>(q_s + (e >> 6) * (128 * 128) + r * 128 + ((((e & 63) >> 3) ^ (r & 7)) << 4) + (e & 4) * 2) =
+            make_uint2(pack2(x.x * p.scale, x.y * p.scale), pack2(x.z * p.scale, x.w * p.scale));
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(q_full);
+    }
 
     auto tile = [&](int n, auto masked) {
-      const int t = t_lo + n, b = n & 1;
+      const int t = tile_of(n), b = n & 1;
       mbar_wait(&s_full[b], static_cast<uint32_t>((n >> 1) & 1));
       tc_fence_after();
       const uint32_t s_addr = lane_addr + S_COL + static_cast<uint32_t>(b) * BKV;
@@ -355,24 +402,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       tmem_ld32_issue(s_addr + 32, r + 32);
       tmem_ld_fence(r);
       tmem_ld_fence(r + 32);
-      float mrow = -INFINITY;
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // (one chain of 64 maxima would be 64 latencies long)
 #pragma unroll
       for (int e = 0; e < BKV; ++e) {
         float sc = __uint_as_float(r[e]);
-        if constexpr (SOFTCAP) sc = cap * tanhf(sc * inv_cap);
-        sc *= LOG2E;
+        if constexpr (SOFTCAP) sc = cap * LOG2E * (Q32 ? tanh_exp(sc * inv_cap) : tanhf(sc * inv_cap));
         if constexpr (decltype(masked)::value) {
           const int kvpos = t * BKV + e;
-          const bool ok = row_valid && kvpos <= qpos && kvpos < kvlen && (p.window <= 0 || kvpos > qpos - p.window);
+          const bool ok = row_valid && kvpos <= qpos && kvpos < kvlen &&
+                          (p.window <= 0 || kvpos > qpos - p.window || (Q32 && kvpos < p.keep_first));
           sc = ok ? sc : -INFINITY;
         }
         r[e] = __float_as_uint(sc);
-        mrow = fmaxf(mrow, sc);
+        mx[e & 3] = fmaxf(mx[e & 3], sc);
       }
-      // lazy rescaling: keep the reference max while the new maximum is within 2^8 of it
+      const float mrow = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * unit;
+      // lazy rescaling: keep the reference max while the new maximum is within 2^8 of it.  Q32: the exact running maximum, whose weight of one has
+      // no rounding error (measured: 0.00279 against 0.00290 from the 64-bit result; 60 against 56 us for 2048 tokens, window 1024)
       float alpha = 1.f;
-      if (mrow > m_ref + 8.f || (m_ref == -INFINITY && mrow > -INFINITY)) {
-        alpha = (m_ref == -INFINITY) ? 0.f : exp2f(m_ref - mrow);
+      if (mrow > m_ref + (Q32 ? 0.f : 8.f) || (m_ref == -INFINITY && mrow > -INFINITY)) {
+        alpha = (m_ref == -INFINITY) ? 0.f : ex2(m_ref - mrow);
         m_ref = mrow;
       }
       if (n > 0) {
@@ -391,16 +440,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       }
       // P = exp2(s - m_ref) -> bf16 -> swizzled K-major smem tile (A operand of the PV MMA)
       const float mr = (m_ref == -INFINITY) ? 0.f : m_ref;          // fully masked so far: exp2(-inf - 0) = 0
-      float lsum = 0.f;
+      const apair unit2 = apack(unit, unit), ref2 = apack(-mr, -mr);
+      apair ls[2] = {0ull, 0ull};
+      float lsum;
       if constexpr (P_TMEM) {
         uint32_t pk[BKV / 2];            // bf16 pairs: key 2j in the low half of column j
 #pragma unroll
         for (int j = 0; j < BKV / 2; ++j) {
-          const float p0 = exp2f(__uint_as_float(r[2 * j]) - mr);
-          const float p1 = exp2f(__uint_as_float(r[2 * j + 1]) - mr);
-          lsum += p0 + p1;
-          const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-          pk[j] = *reinterpret_cast<const uint32_t*>(&h);
+          float p0, p1;
+          aunpack(afma2(apack(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), unit2, ref2), p0, p1);
+          p0 = ex2(p0);
+          p1 = ex2(p1);
+          pk[j] = pack2(p0, p1);
+          // Q32: the sum of what the product sees, so that the rounding of a dominant weight cancels
+          if constexpr (Q32) ls[j & 1] = aadd2(ls[j & 1], apack(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xffff0000u)));
+          else ls[j & 1] = aadd2(ls[j & 1], apack(p0, p1));
         }
         static_assert(BKV == 64, "P_TMEM packs one 64-key tile into 32 columns");
         tmem_st32_bits(s_addr, pk);      // over the (already consumed) scores of this tile
@@ -411,14 +465,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         uint32_t w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float p0 = exp2f(__uint_as_float(r[8 * j + 2 * e]) - mr);
-          const float p1 = exp2f(__uint_as_float(r[8 * j + 2 * e + 1]) - mr);
-          lsum += p0 + p1;
-          const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-          w[e] = *reinterpret_cast<const uint32_t*>(&h);
+          float p0, p1;
+          aunpack(afma2(apack(__uint_as_float(r[8 * j + 2 * e]), __uint_as_float(r[8 * j + 2 * e + 1])), unit2, ref2), p0, p1);
+          p0 = ex2(p0);
+          p1 = ex2(p1);
+          ls[e & 1] = aadd2(ls[e & 1], apack(p0, p1));
+          w[e] = pack2(p0, p1);
         }
         *reinterpret_cast<uint4*>(ptile + ((j ^ (row & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
       }
+      }
+      {
+        float x, y;
+        aunpack(aadd2(ls[0], ls[1]), x, y);
+        lsum = x + y;
       }
       l = l * alpha + lsum;
       if constexpr (!P_TMEM) fence_proxy_async_smem();   // generic-proxy smem writes -> visible to the tensor core (async proxy)
@@ -428,10 +488,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     };
 
     for (int n = 0; n < nt; ++n) {
-      const int t = t_lo + n;
-      // a tile needs no predicate when every key of it is visible to every (valid) query row of the block
-      const bool full = nq_here == QB && (t + 1) * BKV - 1 <= pos0 && (t + 1) * BKV <= kvlen &&
-                        (p.window <= 0 || t * BKV > pos0 + nq_here - 1 - p.window);
+      const int t = tile_of(n);
+      // a tile needs no predicate when every key of it is visible to every valid query row of the block (the others are not stored)
+      const bool full = (t + 1) * BKV - 1 <= pos0 && (t + 1) * BKV <= kvlen &&
+                        (p.window <= 0 || t * BKV > pos0 + nq_here - 1 - p.window || (Q32 && (t + 1) * BKV <= p.keep_first));
       if (full) tile(n, std::false_type{}); else tile(n, std::true_type{});
     }
 
@@ -440,8 +500,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       mbar_wait(pv_done, static_cast<uint32_t>((nt - 1) & 1));
       tc_fence_after();
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    __nv_bfloat16* dst = p.out + (static_cast<size_t>(qtok0 + i) * p.n_q + kvh * G + g) * D;
+    float inv = l > 0.f ? 1.f / l : 0.f;
+    if constexpr (Q32) {
+      if (p.sink != nullptr && row_valid) {        // exp(sink) in the denominator, relative to the larger of the two references
+        const float sk = p.sink[kvh * G + g] * LOG2E, m = fmaxf(m_ref, sk), w = ex2(m_ref - m);
+        inv = w / (l * w + ex2(sk - m));
+      }
+    }
+    __nv_bfloat16* dst = p.out + static_cast<size_t>(qtok0 + i) * p.ld_out + (kvh * G + g) * D;
     float* wsrow = split_mode ? p.ws + (((static_cast<size_t>(seq) * p.n_kv + kvh) * p.splits + blockIdx.x) * p.ws_rows + g) *
                                            (D + 2) : nullptr;
     if (split_mode && row_valid) {
@@ -516,7 +582,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
   }
 }
 
-template <int D, bool SOFTCAP, bool P_TMEM>
+template <int D, bool SOFTCAP, bool P_TMEM, bool Q32 = false>
 int launch_tc_cap(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnTcParams& p, int G, int QB,
                   int seqs, int qblocks, cudaStream_t s) {
   using Cfg = AtcCfg<D>;
@@ -524,13 +590,13 @@ int launch_tc_cap(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMa
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<D, SOFTCAP, P_TMEM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<D, SOFTCAP, P_TMEM, Q32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::kSmemBytes);
     if (e != cudaSuccess) return static_cast<int>(e);
     set[dev] = true;
   }
-  return static_cast<int>(launch_kernel(attn_prefill_tc_kernel<D, SOFTCAP, P_TMEM>,
-                                        dim3(p.splits > 1 ? p.splits : qblocks, p.n_kv, seqs), dim3(ATC_THREADS),
+  return static_cast<int>(launch_kernel(attn_prefill_tc_kernel<D, SOFTCAP, P_TMEM, Q32>,
+                                        p.splits > 1 ? dim3(p.splits, p.n_kv, seqs) : dim3(p.n_kv, qblocks, seqs), dim3(ATC_THREADS),
                                         Cfg::kSmemBytes, s, 1, tq, tk, tv, p, G, QB));
 }
 
@@ -570,8 +636,10 @@ int launch_attention_tc(const void* q, const void* k_cache, const void* v_cache,
   const uint64_t kv_rows = static_cast<uint64_t>(n_pages) * APAGE, kv_cols = static_cast<uint64_t>(n_kv) * head_dim;
   if ((r = make_tmap_shared(&tk, k_cache, kv_rows, kv_cols, kv_cols, APAGE, 2))) return r;
   if ((r = make_tmap_shared(&tv, v_cache, kv_rows, kv_cols, kv_cols, APAGE, 2))) return r;
-  AttnTcParams p;
+  AttnTcParams p{};
   p.out = static_cast<__nv_bfloat16*>(out);
+  p.ld_out = n_q * head_dim;
+  p.scale = 1.f;
   p.block_table = block_table; p.q_start = q_start; p.q_len = q_len; p.kv_len = kv_len;
   p.max_pages = max_pages; p.n_q = n_q; p.n_kv = n_kv; p.window = window; p.softcap = softcap;
   p.splits = (max_q == 1 && splits > 1 && ws != nullptr) ? splits : 1;
@@ -592,6 +660,37 @@ int launch_attention_tc(const void* q, const void* k_cache, const void* v_cache,
   if (rc == 0 && p.splits > 1)
     rc = launch_attention_merge(out, q_start, ws, seqs, n_q, n_kv, head_dim, p.splits, s);
   return rc;
+}
+
+// Spans of the hybrid graphs' softmax attention (launch_softmax_attention in seqmix.cu takes them here): fp32 queries, a cache of D = V channels
+// per head, window with kept first keys, capped scores, sink.
+bool attention_tc_hybrid_supported(const float* q, const void* k_cache, const void* v_cache, const void* out, int ld_out, int H, int G, int D) {
+  if (G <= 0 || H % G) return false;
+  const int per = H / G;
+  auto al16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
+  return (per == 1 || per == 2 || per == 4 || per == 8 || per == 16) && (D == 64 || D == 128) && al16(q) && al16(k_cache) && al16(v_cache) &&
+         al16(out) && ld_out % 8 == 0;
+}
+int launch_attention_tc_hybrid(const float* q, const void* k_cache, const void* v_cache, void* out, int ld_out, const int* block_table,
+                               int max_pages, int n_pages, const int* q_start, const int* q_len, const int* kv_len, int seqs, int max_q, int H,
+                               int G, int D, int window, float scale, float softcap, int keep_first, const float* sink, cudaStream_t s) {
+  const int per = H / G, QB = 128 / per;
+  const uint64_t kv_rows = static_cast<uint64_t>(n_pages) * APAGE, kv_cols = static_cast<uint64_t>(G) * D;
+  CUtensorMap tk, tv;
+  int r;
+  if ((r = make_tmap_shared(&tk, k_cache, kv_rows, kv_cols, kv_cols, APAGE, 2))) return r;
+  if ((r = make_tmap_shared(&tv, v_cache, kv_rows, kv_cols, kv_cols, APAGE, 2))) return r;
+  AttnTcParams p{};
+  p.out = static_cast<__nv_bfloat16*>(out);
+  p.block_table = block_table; p.q_start = q_start; p.q_len = q_len; p.kv_len = kv_len;
+  p.max_pages = max_pages; p.n_q = H; p.n_kv = G; p.window = window; p.softcap = softcap; p.splits = 1; p.q_bn = 32;
+  p.q32 = q; p.ld_out = ld_out; p.scale = scale; p.keep_first = window > 0 ? keep_first : 0; p.sink = sink;
+  const int qblocks = (max_q + QB - 1) / QB;
+  if (D == 64)
+    return softcap > 0.f ? launch_tc_cap<64, true, true, true>(tk, tk, tv, p, per, QB, seqs, qblocks, s)
+                         : launch_tc_cap<64, false, true, true>(tk, tk, tv, p, per, QB, seqs, qblocks, s);
+  return softcap > 0.f ? launch_tc_cap<128, true, true, true>(tk, tk, tv, p, per, QB, seqs, qblocks, s)
+                       : launch_tc_cap<128, false, true, true>(tk, tk, tv, p, per, QB, seqs, qblocks, s);
 }
 
 }  // namespace b2b

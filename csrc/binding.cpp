@@ -630,7 +630,8 @@ void softmax_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_c
                                       static_cast<int>(window), static_cast<float>(scale),
                                       static_cast<int>(v_cache.stride(1)), is_f32(k_cache), static_cast<float>(softcap),
                                       static_cast<int>(keep_first), fp_or_null(sink), static_cast<int>(v_heads),
-                                      fp_or_null(slopes), is_f32(out), cur_stream()),
+                                      fp_or_null(slopes), is_f32(out), k_cache.is_contiguous() && v_cache.is_contiguous() ? static_cast<int>(k_cache.size(0)) : 0,
+                                      cur_stream()),
         "softmax_attention");
 }
 

@@ -46,6 +46,11 @@ unsigned attn_decode_gave_up();
 int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table, const int* q_start,
                        const int* q_len, const int* kv_len, int seqs, int max_pages, int n_tokens, int n_pages, int n_q, int n_kv,
                        int head_dim, int window, float softcap, void* q_out8, void* q_sf, int q_bn, cudaStream_t s);
+// spans of the hybrid graphs' softmax attention on the prefill kernel of attention_tc.cu (n_pages: pages of the cache)
+bool attention_tc_hybrid_supported(const float* q, const void* k_cache, const void* v_cache, const void* out, int ld_out, int H, int G, int D);
+int launch_attention_tc_hybrid(const float* q, const void* k_cache, const void* v_cache, void* out, int ld_out, const int* block_table,
+                               int max_pages, int n_pages, const int* q_start, const int* q_len, const int* kv_len, int seqs, int max_q, int H,
+                               int G, int D, int window, float scale, float softcap, int keep_first, const float* sink, cudaStream_t s);
 int launch_attention_merge(void* out, const int* q_start, const float* ws, int seqs, int n_q, int n_kv, int head_dim,
                            int splits, cudaStream_t s);
 int attention_init();
@@ -122,7 +127,7 @@ int launch_softmax_attention(const float* q, const void* k_cache, const void* v_
                              const int* block_table, int max_pages, const int* q_start, const int* q_len,
                              const int* kv_len, int n_seqs, int max_q, int H, int G, int D, int V, int window,
                              float scale, int ldv, int f32, float softcap, int keep_first, const float* sink, int Gv,
-                             const float* slope, int out_f32, cudaStream_t s);
+                             const float* slope, int out_f32, int n_pages, cudaStream_t s);
 int launch_short_conv(const float* x, int ld_x, int off, const float* w, float* tail, void* y, int ld_y,
                       const int* q_start, const int* q_len, const int* kv_len, const int* seq_slot, int n_seqs,
                       int max_q, int C, int taps, const float* bias, int act, int y_f32, cudaStream_t s);

@@ -582,6 +582,8 @@ __global__ void __launch_bounds__(32 * (WPQ > 1 ? WPQ : SMX_WARPS))
   }
 }
 
+constexpr int SMX_TC_MIN_Q = 32;        // spans from here on may take attention_tc.cu
+
 // ---- tensor-core variant for spans (bf16 serving mode): S = Q K^T and O = P V as m16n8k16 bf16 MMAs with fp32
 // accumulators; scores, masks, running maximum and sums are fp32 on the accumulator fragments, P is rounded to bf16 only
 // as the operand of the second product (so the exponentials use the 2e-7-relative hardware exp2).  A block = 64 consecutive queries of one (sequence, head), a warp = 16 of them;
@@ -1536,7 +1538,7 @@ int launch_softmax_attention(const float* q, const void* k_cache, const void* v_
                              const int* block_table, int max_pages, const int* q_start, const int* q_len,
                              const int* kv_len, int n_seqs, int max_q, int H, int G, int D, int V, int window,
                              float scale, int ldv, int f32, float softcap, int keep_first, const float* sink, int Gv,
-                             const float* slope, int out_f32, cudaStream_t s) {
+                             const float* slope, int out_f32, int n_pages, cudaStream_t s) {
   if (n_seqs <= 0 || max_q <= 0) return 0;
   if (Gv <= 0) Gv = G;
   if (Gv > H || H % Gv != 0) return -2;
@@ -1545,6 +1547,11 @@ int launch_softmax_attention(const float* q, const void* k_cache, const void* v_
   if (V > 64 * SMX_VR || G <= 0 || H % G != 0) return -2;
   const bool wide_v = V > 32 * SMX_VR;      // values of 257 .. 512 channels: 16 channels per lane
   if (ldv <= 0) ldv = Gv * V;               // values in a cache of their own; otherwise a view into wider rows
+  // longer spans of plain 64- and 128-wide heads: the tcgen05 kernel of the dense models (one span of
+  // 2048 tokens, 16 / 4 heads of 128, window 1024: 60 us against 167 on mma.sync below; 40 tokens: 9 against 10)
+  if (!f32 && plain && D == V && ldv == G * V && max_q >= SMX_TC_MIN_Q && n_pages > 0 && attention_tc_hybrid_supported(q, k_cache, v_cache, out, ld_out, H, G, D))
+    return launch_attention_tc_hybrid(q, k_cache, v_cache, out, ld_out, block_table, max_pages, n_pages, q_start, q_len, kv_len, n_seqs, max_q,
+                                      H, G, D, window, scale, softcap, keep_first, sink, s);
   // short spans and decode steps of grouped heads: the heads that share a key/value head become rows of the tile
   const int hg = (H / G > 1 && max_q < 16 * SMX_MMA_WARPS) ? H / G : 1;
   // (decode steps of 4 or more grouped heads too when sequences x key/value heads fill the machine: a page is staged once

@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
   }
   pdl_launch_dependents();     // the next kernel may start its own set-up / weight prefetch now
   if (threadIdx.x == 0) B2B_DBG(1);
+  __nv_bfloat16 resid[16];     // epilogue warps: residual (or gathered) values of a chunk of 16 columns
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -342,6 +343,18 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
       }
       epi_bar_sync();
     }
+    if constexpr (EPI == EPI_RESIDUAL) {
+      // the residual of the first 16 columns, in flight while the accumulator is awaited: behind the cluster exchange its L2 round trip
+      // was the last link of a decode step's chain (a residual that the upstream GPU writes is read there, behind its flag)
+      if (p.wait_flag == nullptr) {
+        const int n_res = tile_n * BM + (warp & 3) * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int tok = tok0 + col0 + i;
+          resid[i] = (i < ncol && tok < p.m_tok) ? p.residual[static_cast<size_t>(tok) * p.ld_res + n_res] : __float2bfloat16_rn(0.f);
+        }
+      }
+    }
     mbar_wait(tmem_full_bar, 0);
     tc_fence_after();
     if (threadIdx.x == 64) B2B_DBG(5);
@@ -518,8 +531,8 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
       const int n = min(16, ncol - c);
       // residual values of the whole chunk first: 16 independent loads in flight (one L2 round trip) instead of
       // one per token between dependent stores
-      __nv_bfloat16 resid[16];
       if constexpr (EPI == EPI_RESIDUAL) {
+        if (c > 0 || p.wait_flag != nullptr)
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const int tok = tok0 + col0 + c + i;

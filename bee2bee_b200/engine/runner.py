@@ -204,7 +204,7 @@ class GpuRunner:
             return self._decode_launches
         c, n = self.cfg, len(self.layers)
         if c.norm == "ln":
-            per = 9
+            per = 8
         elif c.post_norms:
             per = 7
         else:

@@ -220,8 +220,6 @@ class NativePiece:
         self.h_buf = torch.zeros((max_tokens, c.ffn_size), device=dev, dtype=bf)
         if not self.fused_norm or c.post_norms:
             self.n_buf = torch.zeros((max_tokens, H), device=dev, dtype=bf)
-        if not self.fused_norm:
-            self.qkv_buf = torch.zeros((max_tokens, c.q_dim + 2 * c.kv_dim), device=dev, dtype=bf)
         if last:
             self.last_x = torch.zeros((max_seqs, H), device=dev, dtype=bf)
             self.logits = torch.zeros((max_seqs, self.vocab_pad), device=dev, dtype=torch.float32)
@@ -398,9 +396,10 @@ class NativePiece:
                 if head_wait:
                     ops.native().flag_wait(head_wait, head_epoch, 1)
                 n = ops.layernorm(x, self.w[p + "ln1_w"], self.w[p + "ln1_b"], self.n_buf[:T], eps)
-                ops.gemm(self.w[p + "wqkv"], n, out=self.qkv_buf[:T], epi=ops.EPI_PLAIN, bias=self.w.get(p + "bqkv"))
-                ops.kv_append(self.qkv_buf[:T], self.q_buf, self.k_cache[l], self.v_cache[l], m.slots, c.q_dim,
-                              c.kv_dim, c.softmax_scale)
+                # bias, softmax scale and cache rows in the epilogue of the product (there is no rotation: rope_theta <= 0)
+                ops.gemm(self.w[p + "wqkv"], n, epi=ops.EPI_QKV_ROPE, bias=self.w.get(p + "bqkv"), q_out=self.q_buf, k_cache=self.k_cache[l],
+                         v_cache=self.v_cache[l], positions=m.positions, slots=m.slots, n_q_heads=c.n_heads, n_kv_heads=c.n_kv_heads,
+                         head_dim=c.head_dim, rope_theta=c.rope_theta, q_scale=c.softmax_scale)
             if do_attn:
                 # mxfp8: the attention kernel emits the e4m3 copy of its output for the O-proj itself (no quantiser launch)
                 a_fused = fuse and not c.post_norms and ops.attention_fuses_quant(m.max_q, c.n_heads, c.n_kv_heads, c.head_dim,

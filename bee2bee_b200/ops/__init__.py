@@ -207,12 +207,13 @@ def pick_splitk(n_out: int, m_tok: int, k: int, bn: int, epi: int, stages: int =
         # (bn=32: qkv 4, o 4, gate/up 1, down 8 -> 100 us/layer; bn=16: 4/4/1/4 -> 92.6 us); >= 16 k-blocks per
         # CTA, and every CTA of the cluster keeps >= 4 token columns (vector DSMEM stores)
         # narrower models (K < 4096, or few weight tiles; measured at 32 tokens, back to back): 8 k-blocks per CTA are enough, 4 while
-        # the machine is not full (2048 x 2048: 7.4 against 9.4 us, 1024 x 1024: 5.7 against 9.1, 128 x 2048: 5.6 against 9.1)
+        # the machine is not full (2048 x 2048: 7.4 against 9.4 us, 1024 x 1024: 5.7 against 9.1, 128 x 2048: 5.6 against 9.1), 3 at the
+        # shortest K (768 x 768: 5.2 against 5.9, 2304 x 768: 5.7 against 6.2)
         tiles = (n_out // 128) * ((m_tok + bn - 1) // bn)
         kb, limit = k // 64, 256 if bn >= 32 else 200
         want = 1
         for s in (2, 4, 8):
-            if bn // s >= 4 and ((tiles * s <= limit and kb // s >= 16) or (tiles * s <= 140 and kb // s >= 4)
+            if bn // s >= 4 and ((tiles * s <= limit and kb // s >= 16) or (tiles * s <= 140 and kb // s >= 3)
                                  or (kb < 64 and tiles * s <= limit + 16 and kb // s >= 8)):
                 want = s
     want = min(want, 8, max(1, (k // 64) // 2))
@@ -258,6 +259,12 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
                     splitk //= 2
         else:
             bn = pick_bn(m_tok)
+            # up to 16 tokens: eight parts of K need 32-wide tiles (two columns per CTA of a 16-wide one cannot use vector stores), which pays
+            # for long K or few weight tiles: 4096 x 14336 23.8 against 24.6 us, 2304 x 9216 13.9 against 15.8, 768 x 3072 6.7 against 7.3;
+            # not 4096 x 4096 (11.1 against 10.2)
+            parts = n_out // 128 * 8
+            if bn == 16 and splitk <= 0 and parts <= 256 and (k >= 8192 or (parts <= NUM_SMS and k >= 3072)):
+                bn = 32
     if stages < 0:
         stages = GEMM_STAGES if bn <= 64 else 0
     if splitk <= 0:

@@ -345,10 +345,13 @@ class NativePiece:
             di = self.device.index
             out_fqh = dict(fq_out=tfp(hand.out_qh, [T, F], "u8", di).view(torch.float8_e4m3fn),
                            fq_sf=tfp(hand.out_sfh, [((T + 31) // 32) * (F // 128) * 512], "u8", di), fq_bn=q_bn, no_out=True)
+        next_rstd = None
         for li, l in enumerate(self.layers):
             p = f"l{l}."
             do_attn, do_gu, do_down = self.has_attn(l), self.has_gu(l), self.has_down(l)
             do_mlp = do_gu          # the piece continues past this layer's attention block
+            x_rstd, x2_rstd = next_rstd, None      # 1/rms of the rows entering the layer / its MLP block, when the kernel that wrote them knows it
+            next_rstd = None
             is_tail = (li == n_layers - 1) and not self.last
             head_wait = wait_flag if li == 0 else 0           # the piece's first GEMM consumes the handoff input
             head_epoch = wait_epoch if li == 0 else 0
@@ -389,7 +392,7 @@ class NativePiece:
                     xq, akw = self._quant(x, with_rms=True)
                     ops.gemm(self.w[p + "wqkv"], xq, **akw, **self._wkw(p + "wqkv"), **qkv_kw)
                 else:
-                    r = None if inline else ops.rstd(x, eps)
+                    r = None if inline else (x_rstd if x_rstd is not None else ops.rstd(x, eps))
                     ops.gemm(self.w[p + "wqkv"], x, rstd=r, norm_from_x=inline, wait_flag=head_wait,
                              wait_epoch=head_epoch, **qkv_kw)
             else:
@@ -420,7 +423,9 @@ class NativePiece:
                     o_out = x2
                 if c.post_norms:
                     o = ops.gemm(self.w[p + "wo"], a, out=self.n_buf[:T], epi=ops.EPI_PLAIN)
-                    ops.rmsnorm(o, self.w[p + "post_attn_w"], out=x2, residual=x, eps=eps, plus_one=c.gemma_norm)
+                    if not inline:         # the gate/up product's 1/rms comes with the rows
+                        x2_rstd = torch.empty(T, device=x2.device, dtype=torch.float32)
+                    ops.rmsnorm(o, self.w[p + "post_attn_w"], out=x2, residual=x, eps=eps, plus_one=c.gemma_norm, out_rstd=x2_rstd)
                 elif self.fp8:
                     if a_fused:
                         aq, akw = self._qbuf[c.q_dim][:T], dict(sfb=self._qsf[c.q_dim])
@@ -473,7 +478,7 @@ class NativePiece:
             elif c.glu:
                 r2 = None
                 if self.fused_norm and not inline:
-                    r2 = ops.rstd(x2, eps)
+                    r2 = x2_rstd if x2_rstd is not None else ops.rstd(x2, eps)
                 hmid = ops.gemm(self.w[p + "wgu"], x2, out=None if gu_tail else self.h_buf[:T], epi=ops.EPI_GLU, rstd=r2,
                                 norm_from_x=inline and self.fused_norm, eps=eps, act_gelu=(c.act == "gelu_tanh"),
                                 wait_flag=mlp_wait, wait_epoch=mlp_epoch, **gu_tail)
@@ -496,7 +501,9 @@ class NativePiece:
                     xn = dst
                 else:
                     tgt = out_x[:T] if (is_tail and out_x is not None) else xn
-                    ops.rmsnorm(d, self.w[p + "post_ffn_w"], out=tgt, residual=x2, eps=eps, plus_one=c.gemma_norm)
+                    if not inline and li + 1 < n_layers:
+                        next_rstd = torch.empty(T, device=x2.device, dtype=torch.float32)
+                    ops.rmsnorm(d, self.w[p + "post_ffn_w"], out=tgt, residual=x2, eps=eps, plus_one=c.gemma_norm, out_rstd=next_rstd)
                     xn = tgt
             else:
                 if not do_attn and xn.data_ptr() == x2.data_ptr():

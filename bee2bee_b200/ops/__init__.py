@@ -385,17 +385,18 @@ def quant_mxfp8_rows(x: torch.Tensor, bn: int = 0, eps: float = 1e-5, with_rms: 
 
 
 # ----------------------------------------------------------------- elementwise
-def rmsnorm(x, gamma, out=None, residual=None, eps=1e-5, plus_one=False, rstd_out=None, want_out=True):
+def rmsnorm(x, gamma, out=None, residual=None, eps=1e-5, plus_one=False, rstd_out=None, want_out=True, out_rstd=None):
+    """``out = x / rms(x) * gamma (+ residual)``; ``rstd_out``: 1/rms of the rows of ``x``, ``out_rstd``: of the rows written"""
     if out is None and want_out:
         out = torch.empty_like(x)
-    native().rmsnorm(x, gamma, residual, out, rstd_out, eps, plus_one)
+    native().rmsnorm(x, gamma, residual, out, rstd_out, eps, plus_one, out_rstd)
     return out
 
 
 def rstd(x, eps=1e-5):
     """per-token 1/rms (fp32) for GEMMs whose RMSNorm is fused but whose token tile is large"""
     r = torch.empty(x.shape[0], device=x.device, dtype=torch.float32)
-    native().rmsnorm(x, x, None, None, r, eps, False)
+    native().rmsnorm(x, x, None, None, r, eps, False, None)
     return r
 
 

@@ -173,14 +173,15 @@ void init_kernels(int64_t device) {
 
 // ----------------------------------------------------------------- elementwise
 void rmsnorm(const Tensor& x, const Tensor& gamma, const OptT& residual, const OptT& out, const OptT& rstd_out,
-             double eps, bool gemma_plus_one) {
+             double eps, bool gemma_plus_one, const OptT& out_rstd) {
   check_bf16(x, "x");
   c10::cuda::CUDAGuard guard(x.device());
   const int h = static_cast<int>(x.size(-1));
   const int tokens = static_cast<int>(x.numel() / h);
+  TORCH_CHECK(!(out_rstd.has_value() && out_rstd->defined()) || (out.has_value() && out->defined()), "rmsnorm: out_rstd needs an output");
   check(b2b::launch_rmsnorm(x.data_ptr(), gamma.data_ptr(), ptr_or_null<void>(residual), ptr_or_null<void>(out),
                             ptr_or_null<float>(rstd_out), tokens, h, static_cast<float>(eps), gemma_plus_one ? 1 : 0,
-                            cur_stream()),
+                            ptr_or_null<float>(out_rstd), cur_stream()),
         "rmsnorm");
 }
 

@@ -75,6 +75,88 @@ __global__ void rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
   }
 }
 
+// 1/rms of many rows: a warp per row, all of its loads in flight (NV 16-byte pieces per lane), no block barrier.  Bound: memory.  Measured on
+// B200, 4096 rows of 4096: 13.0 -> 8.1 us.  From about four rows per SM on; below that a block per row has more loads in flight.
+constexpr int NORM_ROWS_MIN = 592;
+template <int NV>
+__global__ void __launch_bounds__(128) rstd_rows_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ rstd_out, int tokens, int h,
+                                                        float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, n = h / 8;
+  if (t >= tokens) return;
+  const uint4* row = reinterpret_cast<const uint4*>(x + static_cast<size_t>(t) * h);
+  uint4 v[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) v[i] = lane + 32 * i < n ? row[lane + 32 * i] : make_uint4(0, 0, 0, 0);
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v[i]);
+    float a = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(p[j]);
+      a += f.x * f.x + f.y * f.y;
+    }
+    ss += a;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (lane == 0) rstd_out[t] = rsqrtf(ss / h + eps);
+}
+
+// Norm with output, rows of up to 4096 channels: a block per row, one 16-byte piece per thread; row, gains and residual are all loaded
+// before the reduction.  out_rstd: 1/rms of the rows WRITTEN, as the next RMSNorm-fused product wants it -- a pass of its own over
+// them cost a read of the stream.  Bound: memory.  Measured on B200, 4096 rows of 2304 with residual: 13.9 us (+ 7.4 for the 1/rms of the
+// output) -> 11.5 with it.
+__global__ void __launch_bounds__(512) rmsnorm_block_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
+                                                            const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out,
+                                                            float* __restrict__ rstd_out, float* __restrict__ out_rstd, int h, float eps,
+                                                            int gemma_plus_one) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float sh[32];
+  const int t = blockIdx.x, n = h / 8;
+  const uint4* row = reinterpret_cast<const uint4*>(x + static_cast<size_t>(t) * h);
+  const uint4* grow = reinterpret_cast<const uint4*>(gamma);
+  const uint4* rrow = reinterpret_cast<const uint4*>(residual + static_cast<size_t>(t) * h);
+  const int c = threadIdx.x;
+  uint4 v = make_uint4(0, 0, 0, 0), g = v, r = v, o;
+  if (c < n) {
+    v = row[c];
+    g = grow[c];
+    if (residual != nullptr) r = rrow[c];
+  }
+  const __nv_bfloat162* pv = reinterpret_cast<const __nv_bfloat162*>(&v);
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 f = __bfloat1622float2(pv[j]);
+    ss += f.x * f.x + f.y * f.y;
+  }
+  ss = block_sum(ss, sh);
+  const float rs = rsqrtf(ss / h + eps);
+  if (rstd_out != nullptr && threadIdx.x == 0) rstd_out[t] = rs;
+  const __nv_bfloat162* pg = reinterpret_cast<const __nv_bfloat162*>(&g);
+  const __nv_bfloat162* pr = reinterpret_cast<const __nv_bfloat162*>(&r);
+  __nv_bfloat162* po = reinterpret_cast<__nv_bfloat162*>(&o);
+  float so = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float2 f = __bfloat1622float2(pv[j]), gg = __bfloat1622float2(pg[j]), rr = __bfloat1622float2(pr[j]);
+    if (gemma_plus_one) { gg.x += 1.f; gg.y += 1.f; }
+    po[j] = __floats2bfloat162_rn(f.x * rs * gg.x + rr.x, f.y * rs * gg.y + rr.y);
+    const float2 w = __bfloat1622float2(po[j]);
+    so += w.x * w.x + w.y * w.y;
+  }
+  if (c < n) reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * h)[c] = o;
+  if (out_rstd == nullptr) return;
+  __syncthreads();
+  so = block_sum(so, sh);
+  if (threadIdx.x == 0) out_rstd[t] = rsqrtf(so / h + eps);
+}
+
 __global__ void layernorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                                  const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ out, int h,
                                  float eps) {
@@ -392,12 +474,33 @@ int launch_decode_advance(int* positions, int* kv_len, int* slots, const int* q_
   return static_cast<int>(cudaGetLastError());
 }
 int launch_rmsnorm(const void* x, const void* gamma, const void* residual, void* out, float* rstd_out, int tokens,
-                   int h, float eps, int gemma_plus_one, cudaStream_t s) {
+                   int h, float eps, int gemma_plus_one, float* out_rstd, cudaStream_t s) {
   if (h % 8) return -2;
+  auto bp = [](const void* q) { return static_cast<const __nv_bfloat16*>(q); };
+  if (out == nullptr && h <= 4096 && tokens >= NORM_ROWS_MIN) {
+    const dim3 grid((tokens + 3) / 4), block(128);
+#define B2B_RSTD(NV) launch_kernel(rstd_rows_kernel<NV>, grid, block, 0, s, 1, bp(x), rstd_out, tokens, h, eps)
+    if (h <= 1024) B2B_RSTD(4);
+    else if (h <= 2048) B2B_RSTD(8);
+    else if (h <= 3072) B2B_RSTD(12);
+    else B2B_RSTD(16);
+#undef B2B_RSTD
+    return static_cast<int>(cudaGetLastError());
+  }
+  // (rows of 4096 x 4096: 19.8 us against 26 when the row is read again behind the reduction; 8192 channels, two pieces per thread: 42 against 38)
+  if (out != nullptr && h <= 4096) {
+    const dim3 block(h >= 4096 ? 512 : (h / 8 + 31) / 32 * 32);
+    launch_kernel(rmsnorm_block_kernel, dim3(tokens), block, 0, s, 1, bp(x), bp(gamma), bp(residual), static_cast<__nv_bfloat16*>(out), rstd_out,
+                  out_rstd, h, eps, gemma_plus_one);
+    return static_cast<int>(cudaGetLastError());
+  }
   const int threads = h >= 4096 ? 512 : 256;
-  launch_kernel(rmsnorm_kernel, dim3(tokens), dim3(threads), 0, s, 1, static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(gamma),
-                                            static_cast<const __nv_bfloat16*>(residual), static_cast<__nv_bfloat16*>(out),
-                                            rstd_out, h, eps, gemma_plus_one);
+  launch_kernel(rmsnorm_kernel, dim3(tokens), dim3(threads), 0, s, 1, bp(x), bp(gamma), bp(residual), static_cast<__nv_bfloat16*>(out),
+                rstd_out, h, eps, gemma_plus_one);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || out_rstd == nullptr) return static_cast<int>(e);
+  launch_kernel(rmsnorm_kernel, dim3(tokens), dim3(threads), 0, s, 1, bp(out), bp(gamma), static_cast<const __nv_bfloat16*>(nullptr),
+                static_cast<__nv_bfloat16*>(nullptr), out_rstd, h, eps, 0);
   return static_cast<int>(cudaGetLastError());
 }
 int launch_layernorm(const void* x, const void* gamma, const void* beta, void* out, int tokens, int h, float eps,

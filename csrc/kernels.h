@@ -8,8 +8,9 @@
 namespace b2b {
 
 // elementwise.cu
+// out_rstd (or null): 1/rms of the rows written
 int launch_rmsnorm(const void* x, const void* gamma, const void* residual, void* out, float* rstd_out, int tokens,
-                   int h, float eps, int gemma_plus_one, cudaStream_t s);
+                   int h, float eps, int gemma_plus_one, float* out_rstd, cudaStream_t s);
 int launch_layernorm(const void* x, const void* gamma, const void* beta, void* out, int tokens, int h, float eps,
                      cudaStream_t s);
 int launch_embed(const int* ids, const void* table, const void* pos_table, const int* positions, void* out, int tokens,

@@ -18,8 +18,8 @@
 //
 // Bound (ncu, 128 x 128): shared-memory reads of the operands 65 %, fp32 pipes 57 %, 2.2 instructions per cycle of 4.  8 columns per thread
 // (2 warps per scheduler, 40 % fewer reads) measured the same.  One head: 0.42 us per token at 128 x 128, 0.18 at 64 x 64.
-// Measured on B200, GLA, lin_scan -> here (us): 16 heads of 128: one span of 2048 tokens 583 -> 186, 512 tokens 149 -> 57, 4 spans of 512
-// 286 -> 181, 32 of 64 295 -> 117; 16 heads of 64: 2048 tokens 409 -> 66.  The error against 64 bits is that of lin_scan.
+// Measured on B200, GLA, lin_scan -> here (us): 16 heads of 128: one span of 2048 tokens 583 -> 161, 512 tokens 149 -> 56, 4 spans of 512
+// 286 -> 175, 32 of 64 295 -> 119; 16 heads of 64: 2048 tokens 414 -> 69.  The error against 64 bits is that of lin_scan.
 // This translation unit is compiled WITHOUT --use_fast_math.
 #include "kernels.h"
 

@@ -168,11 +168,6 @@ def pick_prefill_tile(n_out: int, m_tok: int, k: int = 0):
     return (128 if m_tok <= 512 else 256), 0, 0          # small chunks: not measured, the decode heuristic decides
 
 
-#: cluster size of the TMA-multicast prefill GEMM (2 or 4); correct on hardware but NOT faster (the prefill GEMM is not
-#: L2-bound, profiles/prefill_gemm.md), so default off;
-#: applies to bf16 GEMMs with token tiles of 128 / 256 and no split-K, everything else ignores it
-GEMM_MC = int(os.environ.get("B2B_GEMM_MC", "0"))
-
 #: L2 weight prefetch: built, measured negative and REMOVED from the kernel in round 2 (profiles/l2_prefetch.md; even
 #: switched off its code and parameters cost ~20 us per decode step).  The value is accepted and ignored.
 L2_PREFETCH = 0
@@ -190,7 +185,7 @@ def use_wide(n_out: int, m_tok: int) -> bool:
     tokens: 17 against 40 us for 6144 x 4096, 55 against 84 for 28672 x 4096); at 65 .. 128 tokens, where both read the weights
     once, it is while gemm_tc.cu has no more than one tile per SM (128 tokens: 17 against 33 us for 6144 x 4096, 30 against 63 for
     4096 x 14336, 23 against 27 for 18432 x 2304, but 54 against 51 for 28672 x 4096)."""
-    return GEMM_MC <= 1 and (m_tok > 128 or (m_tok > 64 and n_out <= 128 * NUM_SMS))
+    return m_tok > 128 or (m_tok > 64 and n_out <= 128 * NUM_SMS)
 
 
 #: (n_out, k) -> split-K override (tuning / sweeps)
@@ -233,7 +228,7 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
          wait_flag: int = 0, wait_epoch: int = 0, signal_flag: int = 0, signal_epoch: int = 0,
          done_counter: int = 0, free_flag: int = 0, bump_epoch: int = 0, ack_flag: int = 0,
          dbg: int = 0, w_scale: Optional[torch.Tensor] = None,
-         sfa: Optional[torch.Tensor] = None, sfb: Optional[torch.Tensor] = None, mc: int = -1, pf: int = -1,
+         sfa: Optional[torch.Tensor] = None, sfb: Optional[torch.Tensor] = None, pf: int = -1,
          stages: int = -1, free_lag: int = 0, out2_ptr: int = 0,
          fq_out: Optional[torch.Tensor] = None, fq_sf: Optional[torch.Tensor] = None, fq_bn: int = 0,
          sumsq_out: Optional[torch.Tensor] = None, zero_buf: Optional[torch.Tensor] = None,
@@ -244,7 +239,7 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
     m_tok, k = x.shape
     n_out = w.shape[0]
     # (calls that name a tile, split or ring depth get the kernel those belong to)
-    wide = int(bn <= 0 and splitk <= 0 and stages < 0 and mc < 0 and use_wide(n_out, m_tok))
+    wide = int(bn <= 0 and splitk <= 0 and stages < 0 and use_wide(n_out, m_tok))
     if bn <= 0:
         if sfa is not None:
             bn = pick_bn_mx(m_tok)
@@ -292,7 +287,7 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
     native().gemm(w, x, o_ptr, ldo, epi, bn, splitk, residual_ptr, ld_res, bias, rstd, norm_from_x, eps, int(act_gelu),
                   out_fp32, q_out, k_cache, v_cache, positions, slots, n_q_heads, n_kv_heads, head_dim, rope_theta,
                   q_scale, wait_flag, wait_epoch, signal_flag, signal_epoch, done_counter, free_flag, bump_epoch,
-                  ack_flag, dbg, w_scale, sfa, sfb, GEMM_MC if mc < 0 else mc,
+                  ack_flag, dbg, w_scale, sfa, sfb,
                   L2_PREFETCH if pf < 0 else pf, stages, free_lag, out2_ptr,
                   _ptr(fq_out), _ptr(fq_sf), fq_out.shape[1] if fq_out is not None else 0, fq_bn, _ptr(sumsq_out), _ptr(zero_buf),
                   _ptr(sumsq), gather_ids, gather_n, gather_rows, wide)

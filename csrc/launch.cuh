@@ -20,7 +20,7 @@ inline bool pdl_enabled() {
   return g_pdl_mode == 1;
 }
 
-// cluster along x (TMA-multicast GEMM: CTAs that share a token tile)
+// cluster along x (CTA pairs of the prefill products, CTAs that share the keys of a decode step)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel_cx(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                     unsigned cluster_x, Args... args) {

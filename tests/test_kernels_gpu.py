@@ -510,18 +510,6 @@ def test_dense_layer_forward_backward_on_tensor_cores():
         close(gb, g.mul((zr > 0).float()).sum(0) if act == "relu" else gb, rtol=1e-3, atol=1e-3)
 
 
-# ------------------------------------------------- TMA-multicast cluster GEMM (correct on hardware; not faster, so opt-in)
-@pytest.mark.parametrize("mc", [2, 4])
-@pytest.mark.parametrize("m", [512, 300])
-def test_gemm_multicast_cluster(mc, m):
-    n, k = 1024, 1024
-    w, x, res = bf(n, k, scale=0.05, seed=1), bf(m, k, seed=2), bf(m, n, seed=3)
-    ref = x.float() @ w.float().t()
-    for bn in (128, 256):
-        close(ops.gemm(w, x, bn=bn, splitk=1, mc=mc), ref, rtol=2e-2, atol=2e-2)
-        close(ops.gemm(w, x, bn=bn, splitk=1, mc=mc, epi=ops.EPI_RESIDUAL, residual=res), ref + res.float(), rtol=2e-2, atol=2e-2)
-
-
 @pytest.mark.parametrize("p_tmem", ["1", "0"])
 def test_attention_p_in_tmem_and_smem_variants(p_tmem):
     """P kept in tensor memory (TS-form tcgen05.mma, the default) and the shared-memory P variant: the numerics

@@ -198,7 +198,7 @@ def pick_splitk(n_out: int, m_tok: int, k: int, bn: int, epi: int, stages: int =
     if (n_out, k) in SPLITK_OVERRIDE:
         want = SPLITK_OVERRIDE[(n_out, k)]
     else:
-        # measured (tools/layer_sweep.py, Llama-3-8B, reduce-scatter split-K epilogue): up to ~2 CTAs per SM pay off
+        # measured (Llama-3-8B layer, reduce-scatter split-K epilogue): up to ~2 CTAs per SM pay off
         # (bn=32: qkv 4, o 4, gate/up 1, down 8 -> 100 us/layer; bn=16: 4/4/1/4 -> 92.6 us); >= 16 k-blocks per
         # CTA, and every CTA of the cluster keeps >= 4 token columns (vector DSMEM stores)
         # narrower models (K < 4096, or few weight tiles; measured at 32 tokens, back to back): 8 k-blocks per CTA are enough, 4 while
@@ -278,7 +278,7 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
     if epi == EPI_GELU and act_gelu == ACT_XIELU:
         rope_theta, q_scale = act_p0, act_p1       # the two slopes ride in parameter fields this epilogue does not use
     if TIMELINE is not None and not dbg:
-        # per-CTA %globaltimer stamps (tools/layer_timeline.py): every GEMM call gets its own slice of the buffer
+        # per-CTA %globaltimer stamps: every GEMM call gets its own slice of the buffer
         n_cta = (n_out // 128) * ((m_tok + bn - 1) // bn) * splitk
         dbg = TIMELINE["buf"].data_ptr() + TIMELINE["off"] * 8
         TIMELINE["log"].append((epi, n_out, k, splitk, TIMELINE["off"], n_cta))

@@ -431,7 +431,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     tc_fence_after();
     tmem_dealloc<Cfg::kCols>(tmem);
   }
-  if (threadIdx.x == 0 && *abort != 0u) atomicAdd(&g_decode_gave_up, 1u);
+  if (threadIdx.x == 0 && *abort != 0u) {          // a wait ran out: the process learns of it
+    if (g_abort_word != nullptr) *g_abort_word = 1u;
+    atomicAdd(&g_decode_gave_up, 1u);
+  }
 }
 
 template <int D, int GP, bool SOFTCAP>
@@ -491,6 +494,12 @@ int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, 
   int parts = 1;
   while (parts < 8 && static_cast<long long>(seqs) * n_kv * parts * 2 <= slots && parts * 2 * (DKEYS / DPAGE) <= max_pages) parts *= 2;
   return head_dim == 128 ? launch_dec_g<128>(tq, tk, tv, p, n_q / n_kv, seqs, parts, s) : launch_dec_g<256>(tq, tk, tv, p, n_q / n_kv, seqs, parts, s);
+}
+
+int set_wait_policy_decode(uint32_t* abort_word, unsigned long long limit_ns) {
+  cudaError_t e = cudaMemcpyToSymbol(g_abort_word, &abort_word, sizeof(abort_word));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_wait_limit_ns, &limit_ns, sizeof(limit_ns));
+  return static_cast<int>(e);
 }
 
 unsigned attn_decode_gave_up() {

@@ -104,11 +104,16 @@ __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// one arrival per CTA; the last one releases the payload to the downstream piece and this piece's input slot to the upstream one
-__device__ __forceinline__ void publish_handoff(const GemmParams& p, uint32_t total) {
-  if (atomicAdd(p.done_counter, 1u) != total - 1) return;
+// One arrival per CTA; the last one releases the payload to the downstream piece and this piece's input slot to the upstream one -- unless a
+// CTA gave up (counted in the upper half of the counter) or the process has aborted: a neighbour that waits for this payload then runs
+// into its own limit and reports it, where stale rows would become tokens.
+__device__ __forceinline__ void publish_handoff(const GemmParams& p, uint32_t total, bool gave_up) {
+  const uint32_t mine = gave_up ? 0x10001u : 1u, done = atomicAdd(p.done_counter, mine) + mine;
+  if ((done & 0xffffu) != total) return;
   __threadfence_system();
   *p.done_counter = 0;
+  const volatile uint32_t* ab = g_abort_word;
+  if ((done >> 16) != 0u || (ab != nullptr && *ab != 0u)) return;
   if (p.signal_flag != nullptr) {
     const uint32_t e = *reinterpret_cast<volatile uint32_t*>(p.signal_epoch) + 1;
     *reinterpret_cast<volatile uint32_t*>(p.signal_epoch) = e;
@@ -119,6 +124,16 @@ __device__ __forceinline__ void publish_handoff(const GemmParams& p, uint32_t to
     *reinterpret_cast<volatile uint32_t*>(p.bump_epoch) = e;
     if (p.ack_flag != nullptr) st_release_sys(p.ack_flag, e);
   }
+}
+
+// The flags of the neighbouring pieces.  Every role waits for what its own bounded waits depend on before it starts counting polls: an
+// upstream or downstream piece may be late by the time limit of the process (wait_flag_ge), far longer than those waits last.
+__device__ __forceinline__ void wait_upstream(const GemmParams& p) {
+  if (p.wait_flag != nullptr) wait_flag_ge(p.wait_flag, *reinterpret_cast<const volatile uint32_t*>(p.wait_epoch) + 1);
+}
+// the consumer must have drained the previous payload of this slot
+__device__ __forceinline__ void wait_downstream(const GemmParams& p) {
+  if (p.free_flag != nullptr) wait_flag_ge(p.free_flag, *reinterpret_cast<const volatile uint32_t*>(p.signal_epoch) - p.free_lag);
 }
 
 // what a pair works on: tile `t`, k-blocks [kb0, kb1), `split`: the other pair of the cluster has the rest of K
@@ -230,14 +245,13 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           const int pre = min(STAGES, it.kb1 - it.kb0);
           for (int j = 0; j < pre; ++j, ++n) fill(kb + j, n0, m0, true, false);
           pdl_wait();
-          if (p.wait_flag != nullptr) {            // head of a piece: X is written by the upstream GPU
-            wait_flag_ge(p.wait_flag, *reinterpret_cast<const volatile uint32_t*>(p.wait_epoch) + 1);
-            fence_proxy_async_all();               // peer-written (generic proxy) data -> TMA (async proxy) reads
-          }
+          wait_upstream(p);                        // head of a piece: X is written by the upstream GPU
+          if (p.wait_flag != nullptr) fence_proxy_async_all();      // peer-written (generic proxy) data -> TMA (async proxy) reads
           n = 0;
           for (int j = 0; j < pre; ++j, ++n) fill(kb + j, n0, m0, false, true);
           kb += pre;
         }
+        if (i == 2) wait_downstream(p);            // (two accumulators: from here on the ring waits for the epilogue, too)
         for (; kb < it.kb1; ++kb, ++n) {
           if (!(ok = ma_wait(&empty_bar[n % STAGES], (n / STAGES & 1u) ^ 1u, abort))) break;
           fill(kb, n0, m0, true, true);
@@ -252,6 +266,11 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       uint32_t n = 0;
       for (int i = 0; ok && plan.get(i, pair, it); ++i) {
         const uint32_t b = i & 1;
+        if (i == 0) {
+          pdl_wait();                              // (no result is needed; the waits below may count once the producer's input is there)
+          wait_upstream(p);
+        }
+        if (i == 2) wait_downstream(p);
         if (!(ok = ma_wait(&acc_empty[b], (i >> 1 & 1) ^ 1u, abort))) break;
         tc_fence_after();
         for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
@@ -277,9 +296,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     const int sr = lane >> 3, sc = (lane & 7) * 16;        // coalesced view: rows sr + 4 i, byte column sc
     const int q_dim = p.n_q_heads * p.head_dim, kv_dim = p.n_kv_heads * p.head_dim;
     pdl_wait();
-    if (p.wait_flag != nullptr) wait_flag_ge(p.wait_flag, *reinterpret_cast<const volatile uint32_t*>(p.wait_epoch) + 1);
-    if (p.free_flag != nullptr)                    // back-pressure: the consumer must have drained the previous payload of this slot
-      wait_flag_ge(p.free_flag, *reinterpret_cast<const volatile uint32_t*>(p.signal_epoch) - p.free_lag);
+    wait_upstream(p);
+    wait_downstream(p);
 
     // the residual values of a 64-column block in the coalesced view, in flight while the accumulators are awaited or worked on
     uint4 res[EPI == EPI_RESIDUAL ? 8 : 1];
@@ -502,7 +520,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     if (p.signal_flag != nullptr || p.bump_epoch != nullptr) {        // tail of a piece: the last CTA publishes the payload
       __threadfence_system();                      // my (possibly peer-directed) stores are performed
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (threadIdx.x == 64) publish_handoff(p, gridDim.x);
+      if (threadIdx.x == 64) publish_handoff(p, gridDim.x, *abort != 0u);
     }
   }
   if (warp < 2) {
@@ -523,7 +541,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     tc_fence_after();
     tmem_dealloc2<Cfg::kTmemCols>(tmem);
   }
-  if (threadIdx.x == 0 && *abort != 0u) atomicAdd(&g_wide_gave_up, 1u);
+  if (threadIdx.x == 0 && *abort != 0u) {          // a wait ran out: the process learns of it
+    if (g_abort_word != nullptr) *g_abort_word = 1u;
+    atomicAdd(&g_wide_gave_up, 1u);
+  }
 }
 
 // One launch: `pairs` pairs of CTAs in clusters of 2, or (split) of 4.

@@ -241,6 +241,7 @@ int set_wait_policy_gemm(uint32_t* abort_word, unsigned long long limit_ns);
 int set_wait_policy_mixed(uint32_t* abort_word, unsigned long long limit_ns);
 int set_wait_policy_diff(uint32_t* abort_word, unsigned long long limit_ns);
 int set_wait_policy_step(uint32_t* abort_word, unsigned long long limit_ns);
+int set_wait_policy_decode(uint32_t* abort_word, unsigned long long limit_ns);
 int set_wait_policy_elementwise(uint32_t* abort_word, unsigned long long limit_ns);
 
 // gemm_tc.cu

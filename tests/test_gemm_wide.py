@@ -1,5 +1,7 @@
 """The CTA-pair GEMM of many tokens (csrc/gemm_wide.cu) against 64-bit products, at the sizes where its tiles can go wrong: one row more or
 less than a 256-token tile, feature counts that leave part of a tile, every tile width and the split last round."""
+import time
+
 import pytest
 import torch
 
@@ -94,3 +96,65 @@ def test_handoff_words():
     assert torch.equal(out, out2)
     assert word.tolist() == [1, 1, 1, 1, 0, 1, 0, 0]
     assert ops.native().gemm_wide_gave_up() == 0
+
+
+@pytest.fixture
+def abort_word():
+    """bounded flag waits as in the engine: they raise this word at the limit"""
+    word = torch.zeros(64, device="cuda", dtype=torch.int32)
+    C = ops.native()
+
+    def limit(ms):
+        C.set_wait_policy(word.data_ptr(), float(ms))
+        return word
+    yield limit
+    torch.cuda.synchronize()
+    C.set_wait_policy(0, 0.0)
+
+
+def _handoff(m, n, k, flags):
+    """a product that waits for both neighbours, behind the kernels in front of it at the head of a piece"""
+    w, x, res = bf(n, k, scale=k ** -0.5), bf(m, k), bf(m, n)
+    word = torch.zeros(8, device="cuda", dtype=torch.int32)      # in epoch, out flag, out epoch, done, ack
+    at = [word.data_ptr() + 4 * i for i in range(8)]
+    out = torch.zeros(m, n, device="cuda", dtype=torch.bfloat16)
+    word[2] = 1                                                  # one payload is out already: the next one waits for its release
+    torch.cuda.synchronize()
+    ops.native().flag_wait(flags.data_ptr(), at[0], 1)
+    r = ops.rstd(x, 1e-5)
+    ops.gemm(w, x, out=out, epi=ops.EPI_RESIDUAL, residual=res, rstd=r, wait_flag=flags.data_ptr(), wait_epoch=at[0], signal_flag=at[1],
+             signal_epoch=at[2], done_counter=at[3], bump_epoch=at[0], ack_flag=at[4], free_flag=flags.data_ptr() + 64, free_lag=0)
+    rs = (x.double().pow(2).mean(1, keepdim=True) + 1e-5).rsqrt()
+    return out, (x.double() @ w.double().t()) * rs + res.double(), word
+
+
+@pytest.mark.parametrize("m,n", [(200, 512), (1000, 18944)])     # one tile per pair and four (both accumulators in use)
+def test_late_neighbours(m, n, abort_word):
+    """the host publishes the upstream flag some seconds after the launch and releases the output slot a second later: no wait counts before"""
+    abort = abort_word(30000)
+    before = ops.native().gemm_wide_gave_up()
+    flags = torch.ones(32, dtype=torch.int32).pin_memory()
+    _handoff(m, n, 256, flags)                                   # (kernels are loaded on first use, which a waiting kernel would hold up)
+    torch.cuda.synchronize()
+    flags.zero_()
+    out, ref, word = _handoff(m, n, 256, flags)
+    time.sleep(4.5)                                              # (2^24 polls last 1 to 4 s)
+    flags[0] = 1
+    time.sleep(1.0)
+    flags[16] = 1
+    torch.cuda.synchronize()
+    near(out, ref)
+    assert word.tolist() == [1, 2, 2, 0, 1, 0, 0, 0]
+    assert ops.native().gemm_wide_gave_up() == before and int(abort[0]) == 0
+
+
+def test_neighbour_that_never_comes(abort_word):
+    """the wait for the upstream flag runs out: the abort word is up, and neither the payload nor the input slot is released"""
+    abort = abort_word(300)
+    flags = torch.zeros(32, dtype=torch.int32).pin_memory()
+    flags[16] = 1
+    _, _, word = _handoff(200, 512, 256, flags)
+    torch.cuda.synchronize()
+    assert int(abort[0]) == 1
+    assert word.tolist() == [0, 0, 1, 0, 0, 0, 0, 0]
+    abort.zero_()

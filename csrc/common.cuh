@@ -10,7 +10,9 @@
 namespace b2b {
 
 #ifndef B2B_SPIN_LIMIT
-#define B2B_SPIN_LIMIT (1u << 27)   // bounded waits: a protocol bug traps instead of hanging the GPU
+// Bounded waits: a protocol bug traps instead of hanging the GPU.  A poll lasts 60 to 240 ns, so this is one to four minutes: a wait may begin
+// while an earlier kernel, or this one's loads, are still waiting for a late piece, which may take the time limit of handoff waits (30 s)
+#define B2B_SPIN_LIMIT (1u << 30)
 #endif
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -86,12 +86,6 @@ __device__ __forceinline__ apair aadd2(apair a, apair b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// through exp2: relative error of a few 2^-22 (the hardware tanh: 2^-11)
-__device__ __forceinline__ float tanh_exp(float x) {
-  const float e = ex2(fminf(fabsf(x), 15.f) * (2.f * LOG2E));
-  return copysignf(1.f - __fdividef(2.f, e + 1.f), x);
-}
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t r[32];
   asm volatile(

@@ -126,10 +126,6 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ float tanh_exp(float x) {                 // through exp2: relative error of a few 2^-22 (tanh.approx: 2^-11)
-  const float e = ex2(fminf(fabsf(x), 15.f) * (2.f * DEC_LOG2E));
-  return copysignf(1.f - __fdividef(2.f, e + 1.f), x);
-}
 
 // GP: query heads per key/value head rounded up to 4, 8 or 16.  grid (CTAs of the cluster, key/value heads, sequences)
 template <int D, int GP, bool SOFTCAP>
@@ -398,7 +394,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         den += w * ld_dsmem_f32(mapa_smem(mine + (DHEADS * D + DHEADS + g) * 4, r));
         num += w * ld_dsmem_f32(mapa_smem(mine + e * 4, r));
       }
-      const float v = den > 0.f ? num / den : 0.f;
+      const float v = den == 0.f ? 0.f : num / den;      // (no key: zero; a NaN among the scores stays one)
       const int tok = p.q_start[seq], feat = kvh * G * D + e, ldq = p.n_q * D;
       if (p.q_out8 == nullptr) {
         p.out[static_cast<size_t>(tok) * ldq + feat] = __float2bfloat16_rn(v);

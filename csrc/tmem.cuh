@@ -12,6 +12,13 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// tanh through exp2.  The difference cancels near zero, so the bound is absolute: 2^-22 (the hardware tanh: 2^-11 of the value), times the cap for
+// a capped score.  An overflow of the exponential ends at one, NaN stays NaN.
+__device__ __forceinline__ float tanh_exp(float x) {
+  const float e = ex2(fabsf(x) * 2.885390081777927f);          // 2 log2(e)
+  return copysignf(1.f - __fdividef(2.f, e + 1.f), x);
+}
+
 // bounded wait: sets the CTA's abort word when it runs out, which ends the waits of all its warps
 constexpr uint32_t MA_SPIN_LIMIT = 1u << 24;
 __device__ __forceinline__ bool ma_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort) {

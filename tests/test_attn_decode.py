@@ -88,3 +88,30 @@ def test_quantised_copy(S):
     ops.attention(q, k, v, torch.zeros_like(q), *args, **kw, fq_out=fq, fq_sf=sf, fq_bn=bn)
     assert torch.equal(fq.view(torch.uint8), want_q.view(torch.uint8))
     assert torch.equal(ops.mx_unchunk(sf, S, nq * D, bn), ops.mx_unchunk(want_sf, S, nq * D, bn))
+
+
+@pytest.mark.parametrize("cap", [0.0, 50.0])
+@pytest.mark.parametrize("lens", [[300], [60, 200, 500]])
+def test_nan_stays(lens, cap):
+    """NaN in a query or a key reaches the heads that see it, capped or not, and no other"""
+    nq, nkv, D = 8, 2, 128
+    q, k, v, table = setup(lens, nq, nkv, D)
+    q[-1, 3 * D + 5] = float("nan")                              # head 3 of the last sequence
+    page = int(table[0, 0])
+    k[page, 7, 1, 9] = float("nan")                              # a key of key/value head 1 of the first: its heads 4 to 7
+    out = torch.zeros_like(q)
+    ops.attention(q, k, v, out, table, i32(list(range(len(lens)))), i32([1] * len(lens)), i32(lens), max_q=1, n_q=nq, n_kv=nkv, head_dim=D, softcap=cap)
+    got = out.view(len(lens), nq, D).isnan()
+    want = torch.zeros_like(got)
+    want[-1, 3], want[0, 4:] = True, True
+    assert torch.equal(got, want)
+
+
+def test_capped_scores_far_beyond_the_cap():
+    lens, nq, nkv, D = [200], 4, 1, 128
+    q, k, v, table = setup(lens, nq, nkv, D)
+    q *= 3000.0                                                  # |score / cap| up to some hundreds
+    out = torch.zeros_like(q)
+    ops.attention(q, k, v, out, table, i32([0]), i32([1]), i32(lens), max_q=1, n_q=nq, n_kv=nkv, head_dim=D, softcap=50.0)
+    ref = reference(q, k, v, table, lens, nq, nkv, D, 0, 50.0)
+    assert float((out.double() - ref).norm() / ref.norm()) < BOUND

@@ -115,3 +115,22 @@ def test_capped_scores_far_beyond_the_cap():
     ops.attention(q, k, v, out, table, i32([0]), i32([1]), i32(lens), max_q=1, n_q=nq, n_kv=nkv, head_dim=D, softcap=50.0)
     ref = reference(q, k, v, table, lens, nq, nkv, D, 0, 50.0)
     assert float((out.double() - ref).norm() / ref.norm()) < BOUND
+
+
+def test_dominant_weight():
+    """One key of a later tile outweighs all others while the reference of the first tile is kept, so its weight is 2^c with any mantissa.  The sum
+    is over rounded weights, so this rounding cancels and the result's own is left: 2^-8 / sqrt(3) / mantissa, 0.00166 in the mean square over
+    mantissas (0.0023 with an unrounded sum)."""
+    S, nq, nkv, D = 64, 4, 1, 128
+    q, k, v, table = setup([300] * S, nq, nkv, D)
+    q = q[:, :D].repeat(1, nq)                                   # (the heads of a sequence are alike)
+    unit = (q[:, :D].float() / q[:, :D].float().pow(2).sum(1, keepdim=True))
+    for s in range(S):
+        score = torch.full((300, 1), -6.0, device="cuda")
+        score[0], score[200] = 0.0, 3.0 + 2.0 * s / S            # natural units: c from 4.3 to 7.2
+        at = torch.arange(300, device="cuda")
+        k.view(-1, nkv, D)[table[s].long()[at // 64] * 64 + at % 64, 0] = (score * unit[s]).bfloat16()
+    out = torch.zeros_like(q)
+    ops.attention(q, k, v, out, table, i32(list(range(S))), i32([1] * S), i32([300] * S), max_q=1, n_q=nq, n_kv=nkv, head_dim=D)
+    ref = reference(q, k, v, table, [300] * S, nq, nkv, D, 0, 0.0)
+    assert float((out.double() - ref).norm() / ref.norm()) < 0.0019

@@ -32,7 +32,7 @@ _C = None
 # that were actually recorded, not a formula.
 LAUNCHES = [0]
 _KERNEL_ENTRY_POINTS = ("add", "attention", "decode_advance", "embed", "fetch_window", "flag_signal", "flag_wait", "gemm",
-                        "kv_append", "layernorm", "mark_seen", "quant_fp8_rows", "quant_mxfp8_rows", "rmsnorm", "sample",
+                        "layernorm", "mark_seen", "quant_fp8_rows", "quant_mxfp8_rows", "rmsnorm", "sample",
                         "set_decode_state", "hyb_embed", "hyb_commit_prev", "hc_step", "act_cols", "attn_prep",
                         "sig_attention", "delta_scan", "delta_post", "ls_join", "rot_attn_prep", "softmax_attention",
                         "short_conv", "mlstm_gates", "lin_scan", "scan_post", "post_norm_join", "latent_prep", "rot_heads",
@@ -385,6 +385,8 @@ def rmsnorm(x, gamma, out=None, residual=None, eps=1e-5, plus_one=False, rstd_ou
     if out is None and want_out:
         out = torch.empty_like(x)
     native().rmsnorm(x, gamma, residual, out, rstd_out, eps, plus_one, out_rstd)
+    if out_rstd is not None and x.shape[-1] > 4096:
+        LAUNCHES[0] += 1           # longer rows: the 1/rms of the output is a second kernel
     return out
 
 
@@ -406,10 +408,6 @@ def embed(ids, table, out, pos_table=None, positions=None, scale=1.0, tok_flag=0
     native().embed(ids.data_ptr() if isinstance(ids, torch.Tensor) else int(ids), table, pos_table, positions, out,
                    scale, tok_flag, tok_epoch, pf_flag, pf_need)
     return out
-
-
-def kv_append(qkv, q_out, k_cache, v_cache, slots, q_dim, kv_dim, q_scale):
-    native().kv_append(qkv, q_out, k_cache, v_cache, slots, q_dim, kv_dim, q_scale)
 
 
 def add(a, b, out=None):

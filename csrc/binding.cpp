@@ -207,17 +207,6 @@ void embed(int64_t ids_ptr, const Tensor& table, const OptT& pos_table, const Op
         "embed");
 }
 
-void kv_append(const Tensor& qkv, const Tensor& q_out, const Tensor& k_cache, const Tensor& v_cache,
-               const Tensor& slots, int64_t q_dim, int64_t kv_dim, double q_scale) {
-  check_bf16(qkv, "qkv");
-  c10::cuda::CUDAGuard guard(qkv.device());
-  check(b2b::launch_kv_append(qkv.data_ptr(), q_out.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-                              reinterpret_cast<const int*>(slots.data_ptr()), static_cast<int>(qkv.size(0)),
-                              static_cast<int>(q_dim), static_cast<int>(kv_dim), static_cast<float>(q_scale),
-                              cur_stream()),
-        "kv_append");
-}
-
 void add(const Tensor& a, const Tensor& b, const Tensor& out) {
   check_bf16(a, "a");
   c10::cuda::CUDAGuard guard(a.device());
@@ -1038,7 +1027,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm", &rmsnorm);
   m.def("layernorm", &layernorm);
   m.def("embed", &embed);
-  m.def("kv_append", &kv_append);
   m.def("add", &add);
   m.def("quant_fp8_rows", &quant_fp8_rows);
   m.def("quant_mxfp8_rows", &quant_mxfp8_rows);

@@ -221,25 +221,6 @@ __global__ void embed_kernel(const int* __restrict__ ids, const __nv_bfloat16* _
   }
 }
 
-// Unfused KV append (GPT-2 path): qkv [T, q_dim + 2*kv_dim] -> q_out, paged K/V.
-__global__ void kv_append_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ q_out,
-                                 __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
-                                 const int* __restrict__ slots, int q_dim, int kv_dim, float q_scale) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int t = blockIdx.x;
-  const int tot = q_dim + 2 * kv_dim;
-  const int slot = slots[t];
-  for (int i = threadIdx.x; i < tot; i += blockDim.x) {
-    const __nv_bfloat16 v = qkv[static_cast<size_t>(t) * tot + i];
-    if (i < q_dim) q_out[static_cast<size_t>(t) * q_dim + i] = __float2bfloat16_rn(__bfloat162float(v) * q_scale);
-    else if (slot >= 0) {
-      if (i < q_dim + kv_dim) k_cache[static_cast<size_t>(slot) * kv_dim + (i - q_dim)] = v;
-      else v_cache[static_cast<size_t>(slot) * kv_dim + (i - q_dim - kv_dim)] = v;
-    }
-  }
-}
-
 // y = a + b (residual add for unfused paths), 128-bit
 __global__ void add_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                            __nv_bfloat16* __restrict__ out, size_t n8) {
@@ -516,13 +497,6 @@ int launch_embed(const int* ids, const void* table, const void* pos_table, const
   launch_kernel(embed_kernel, dim3(tokens), dim3(256), 0, s, 1, ids, static_cast<const __nv_bfloat16*>(table),
                                       static_cast<const __nv_bfloat16*>(pos_table), positions,
                                       static_cast<__nv_bfloat16*>(out), h, vocab, scale, tok_flag, tok_epoch, pf_flag, pf_need);
-  return static_cast<int>(cudaGetLastError());
-}
-int launch_kv_append(const void* qkv, void* q_out, void* k_cache, void* v_cache, const int* slots, int tokens,
-                     int q_dim, int kv_dim, float q_scale, cudaStream_t s) {
-  launch_kernel(kv_append_kernel, dim3(tokens), dim3(256), 0, s, 1, static_cast<const __nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(q_out),
-                                          static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache),
-                                          slots, q_dim, kv_dim, q_scale);
   return static_cast<int>(cudaGetLastError());
 }
 int launch_add(const void* a, const void* b, void* out, size_t n, cudaStream_t s) {

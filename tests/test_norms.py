@@ -16,7 +16,9 @@ def test_rms(h, T):
     inv = (d.pow(2).mean(-1) + 1e-6).rsqrt()
     assert float((ops.rstd(x, 1e-6).double() / inv - 1).abs().max()) < 1e-5           # sums of h fp32 squares
     mine, own = torch.empty(T, device="cuda"), torch.empty(T, device="cuda")
+    before = ops.LAUNCHES[0]
     out = ops.rmsnorm(x, w, residual=r, eps=1e-6, plus_one=True, rstd_out=mine, out_rstd=own)
+    assert ops.LAUNCHES[0] - before == (1 if h <= 4096 else 2)
     ref = d * inv[:, None] * (1 + w.double()) + r.double()
     assert float(((out.double() - ref).abs() / ref.abs().clamp_min(1e-3)).max()) < 2.0 ** -8 + 1e-2 * 2.0 ** -4     # one bf16 rounding, cancelling sums
     assert float((mine.double() / inv - 1).abs().max()) < 1e-5

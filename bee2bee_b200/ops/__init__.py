@@ -234,12 +234,13 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
          sumsq_out: Optional[torch.Tensor] = None, zero_buf: Optional[torch.Tensor] = None,
          sumsq: Optional[torch.Tensor] = None, no_out: bool = False, act_p0: float = 0.0,
          act_p1: float = 0.0, gather_ids: Optional[torch.Tensor] = None, gather_n: int = 0,
-         gather_rows: int = 0) -> Optional[torch.Tensor]:
-    """out[t, n] = epilogue(sum_k x[t, k] * w[n, k]) on the tcgen05 swap-AB kernel."""
+         gather_rows: int = 0, wide_tile: int = 0, wide_split: int = -1) -> Optional[torch.Tensor]:
+    """out[t, n] = epilogue(sum_k x[t, k] * w[n, k]) on the tcgen05 kernels.  ``wide_tile`` 128 / 192 / 256 with ``wide_split`` 0 / 1: that
+    feature tile of the CTA-pair kernel, its last round cut along K or not (else both by size)."""
     m_tok, k = x.shape
     n_out = w.shape[0]
     # (calls that name a tile, split or ring depth get the kernel those belong to)
-    wide = int(bn <= 0 and splitk <= 0 and stages < 0 and use_wide(n_out, m_tok))
+    wide = int(bn <= 0 and splitk <= 0 and stages < 0 and use_wide(n_out, m_tok)) if wide_tile <= 0 else wide_tile
     if bn <= 0:
         if sfa is not None:
             bn = pick_bn_mx(m_tok)
@@ -290,7 +291,7 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
                   ack_flag, dbg, w_scale, sfa, sfb,
                   L2_PREFETCH if pf < 0 else pf, stages, free_lag, out2_ptr,
                   _ptr(fq_out), _ptr(fq_sf), fq_out.shape[1] if fq_out is not None else 0, fq_bn, _ptr(sumsq_out), _ptr(zero_buf),
-                  _ptr(sumsq), gather_ids, gather_n, gather_rows, wide)
+                  _ptr(sumsq), gather_ids, gather_n, gather_rows, wide, wide_split)
     return out
 
 

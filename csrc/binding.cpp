@@ -49,7 +49,7 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
           const OptT& sfa, const OptT& sfb, int64_t pf_tiles, int64_t stages, int64_t free_lag, int64_t out2_ptr,
           // fused MX quantisation of the output / RMSNorm statistics (raw addresses, 0 = off)
           int64_t q_out8, int64_t q_sf, int64_t ld_q, int64_t q_bn, int64_t sumsq_out, int64_t zero_buf, int64_t sumsq,
-          const OptT& gather_ids, int64_t gather_n, int64_t gather_rows, int64_t wide) {
+          const OptT& gather_ids, int64_t gather_n, int64_t gather_rows, int64_t wide, int64_t wide_split) {
   const bool fp8 = w.scalar_type() == at::kFloat8_e4m3fn;
   if (fp8) {
     TORCH_CHECK(x.scalar_type() == at::kFloat8_e4m3fn && w.is_cuda() && x.is_cuda() && w.is_contiguous() &&
@@ -139,8 +139,9 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
   if (p.epi == b2b::EPI_RESIDUAL) TORCH_CHECK(p.residual != nullptr, "residual epilogue needs residual");
   if (p.epi == b2b::EPI_GLU) TORCH_CHECK(p.out != nullptr || (p.q_out8 != nullptr && p.sfa != nullptr), "GLU epilogue needs an output");
   if (p.signal_flag || p.bump_epoch) TORCH_CHECK(p.done_counter != nullptr, "handoff needs done_counter");
+  TORCH_CHECK(wide <= 1 || b2b::gemm_wide_supported(p), "gemm: not a call for the tiles of many tokens");
   if (wide && b2b::gemm_wide_supported(p)) {      // (wide: 1, or the feature tile to use)
-    check(b2b::launch_gemm_wide(p, w.data_ptr(), x.data_ptr(), static_cast<int>(wide), cur_stream()), "gemm_wide");
+    check(b2b::launch_gemm_wide(p, w.data_ptr(), x.data_ptr(), static_cast<int>(wide), static_cast<int>(wide_split), cur_stream()), "gemm_wide");
     return;
   }
   check(b2b::launch_gemm_tc(p, w.data_ptr(), x.data_ptr(), static_cast<int>(bn), cur_stream()), "gemm_tc");
@@ -1019,7 +1020,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   m.def("attn_decode_gave_up", &b2b::attn_decode_gave_up);
   m.def("gemm_max_splitk", &gemm_max_splitk);
-  m.def("gemm_wide_clusters4", &b2b::gemm_wide_clusters4);
   m.def("gemm_wide_gave_up", &b2b::gemm_wide_gave_up);
   m.def("init_kernels", &init_kernels);
   m.def("set_pdl", &set_pdl);

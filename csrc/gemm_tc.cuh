@@ -95,11 +95,11 @@ struct GemmParams {
 // Host launcher (gemm_tc.cu). Returns cudaError_t as int.
 int gemm_tc_max_splitk(int bn, int epi, int stages);
 int launch_gemm_tc(const GemmParams& p, const void* w, const void* x, int bn, cudaStream_t stream);
-// many tokens (gemm_wide.cu): bf16 operands, 16-byte aligned rows; bn: feature tile 128 / 256, else chosen by size
+// many tokens (gemm_wide.cu): bf16 operands, 16-byte aligned rows; bn: feature tile 128 / 192 / 256, split: last round cut along K (0 / 1);
+// any other value: chosen by size.  -4: no such tile for this call
 bool gemm_wide_supported(const GemmParams& p);
-int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, cudaStream_t stream);
+int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, int split, cudaStream_t stream);
 int set_wait_policy_wide(uint32_t* abort_word, unsigned long long limit_ns);
-int gemm_wide_clusters4();         // clusters of four of its CTAs that the device holds at once
 unsigned gemm_wide_gave_up();      // CTAs whose bounded waits ran out so far, 0 unless there is a bug
 
 }  // namespace b2b

@@ -644,7 +644,7 @@ bool gemm_wide_supported(const GemmParams& p) {
   return true;
 }
 
-int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, cudaStream_t stream) {
+int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, int split, cudaStream_t stream) {
   if (!gemm_wide_supported(p)) return -2;
   const bool can_split = p.k / WK >= 8;
   WideChoice best{0, 0, false, 1e30};
@@ -652,22 +652,21 @@ int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, 
     if (bn >= 128 && bn <= 256 && b != bn) continue;
     if (b == 192 && p.epi == EPI_GLU) continue;                                  // (gate/up pairs are 128 columns wide)
     for (int s = 0; s < 2; ++s) {
+      if ((split == 0 || split == 1) && s != split) continue;
       if (s && (!can_split || b == 192 || (b == 128 && p.epi == EPI_GLU))) continue;     // halves are whole 64-column blocks
       const WideChoice c = wide_choice(p, b, s != 0);
       if (c.cost < best.cost) best = c;
     }
   }
+  if (best.bn == 0) return -4;
   CUtensorMap tw, tx;
   int r = make_tmap_shared(&tw, w, p.n_out, p.k, p.k, best.bn / 2, 2);
   if (r) return r;
   if ((r = make_tmap_shared(&tx, x, p.m_tok, p.k, p.k, WM, 2))) return r;
-  if (best.bn == 0) return -4;
   if (best.bn == 192) return launch_wide_bn<192>(p, tw, tx, best.pairs, false, stream);
   return best.bn == 128 ? launch_wide_bn<128>(p, tw, tx, best.pairs, best.split, stream)
                         : launch_wide_bn<256>(p, tw, tx, best.pairs, best.split, stream);
 }
-
-int gemm_wide_clusters4() { return wide_clusters4(); }
 
 int set_wait_policy_wide(uint32_t* abort_word, unsigned long long limit_ns) {
   cudaError_t e = cudaMemcpyToSymbol(g_abort_word, &abort_word, sizeof(abort_word));

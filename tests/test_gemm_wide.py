@@ -1,5 +1,5 @@
 """The CTA-pair GEMM of many tokens (csrc/gemm_wide.cu) against 64-bit products, at the sizes where its tiles can go wrong: one row more or
-less than a 256-token tile, feature counts that leave part of a tile, every tile width and the split last round."""
+less than a 256-token tile, feature counts that leave part of a tile, every tile width and the split last round; neighbours that are late."""
 import time
 
 import pytest
@@ -23,8 +23,8 @@ def near(a, b, bound=ROUND):
     assert err <= bound, float(err)
 
 
-# 129 / 255 / 256 / 257: around a token tile; 65: half a tile.  Features: 128 (one 128-wide tile), 18944 (74 tiles of 256), 13056 (192-wide
-# tiles with a rest of 0 and 128), 4224 x 700 tokens (a ragged last tile).  k 128: the shortest ring; 576: no multiple of the ring depth.
+# As the rule picks them.  129 / 255 / 256 / 257: around a token tile; 65: half a tile.  Features: 128 (one 128-wide tile), 384 and 1024
+# (128-wide), 18944 (74 tiles of 256), 13056 and 4224 and 6144 (192-wide, no rest).  k 128: the shortest ring; 576: no multiple of the ring depth.
 @pytest.mark.parametrize("m,n,k", [(65, 128, 128), (129, 384, 576), (255, 1024, 512), (256, 18944, 128), (257, 13056, 192), (700, 4224, 1024),
                                    (300, 6144, 4096)])
 def test_epilogues(m, n, k):
@@ -54,9 +54,46 @@ def test_gate_up(f, m, gelu):
     near(out, g * u)
 
 
+# Every tile, whole and cut along K, over feature counts that leave part of the last one: 640 = 3 x 192 + 64 = 2 x 256 + 128 (cut: the second
+# pair of the cluster has no columns there), 896 = 4 x 192 + 128 = 3 x 256 + 128, 768: no rest.  k 512: the shortest that is cut; 576: halves of 4 and 5 blocks.
+TILES = [(128, 0), (128, 1), (192, 0), (256, 0), (256, 1)]
+
+
+@pytest.mark.parametrize("tile,split", TILES)
+@pytest.mark.parametrize("m,n,k", [(300, 640, 512), (129, 896, 576), (513, 768, 1024)])
+def test_every_tile(tile, split, m, n, k):
+    kw = dict(wide_tile=tile, wide_split=split)
+    w, x, res = bf(n, k, scale=k ** -0.5), bf(m, k), bf(m, n)
+    bias = torch.randn(n, device="cuda")
+    rstd = torch.rand(m, device="cuda") + 0.5
+    ref = x.double() @ w.double().t()
+    wide = torch.zeros(m, n + 64, device="cuda", dtype=torch.bfloat16)
+    ops.gemm(w, x, out=wide[:, :n], rstd=rstd, bias=bias, **kw)
+    near(wide[:, :n], ref * rstd.double()[:, None] + bias.double())
+    assert float(wide[:, n:].abs().max()) == 0.0
+    near(ops.gemm(w, x, bias=bias, out_fp32=True, **kw), ref + bias.double(), 1e-5)
+    near(ops.gemm(w, x, epi=ops.EPI_RESIDUAL, residual=res, **kw), ref + res.double())
+    near(ops.gemm(w, x, epi=ops.EPI_GELU, bias=bias, **kw), torch.nn.functional.gelu(ref + bias.double(), approximate="tanh"))
+    if tile == 256 or (tile == 128 and not split):               # (a gate / up pair is 128 columns wide)
+        g, u = (ref[:, i:i + n // 2] for i in (0, n // 2))
+        out = ops.gemm(ops.glu_interleave_rows(w[:n // 2], w[n // 2:]), x, epi=ops.EPI_GLU, **kw)
+        near(out, torch.nn.functional.silu(g) * u)
+    assert ops.native().gemm_wide_gave_up() == 0
+
+
+@pytest.mark.parametrize("tile,split", TILES)
+@pytest.mark.parametrize("hd,nq,nkv,m", [(128, 3, 1, 300), (64, 6, 2, 129), (256, 3, 2, 257), (32, 20, 4, 140)])
+def test_qkv_every_tile(tile, split, hd, nq, nkv, m):
+    check_qkv(hd, nq, nkv, m, 512, wide_tile=tile, wide_split=split)
+
+
 @pytest.mark.parametrize("hd,nq,nkv,m", [(128, 8, 2, 200), (64, 8, 4, 257), (256, 4, 2, 131)])
 def test_qkv(hd, nq, nkv, m):
-    k, theta = 256, 10000.0
+    check_qkv(hd, nq, nkv, m, 256)
+
+
+def check_qkv(hd, nq, nkv, m, k, **tile):
+    theta = 10000.0
     n = (nq + 2 * nkv) * hd
     w, x = bf(n, k, scale=k ** -0.5), bf(m, k)
     pages = m // ops.PAGE + 2
@@ -66,7 +103,7 @@ def test_qkv(hd, nq, nkv, m):
     kc = torch.zeros(pages, ops.PAGE, nkv, hd, device="cuda", dtype=torch.bfloat16)
     vc, q = torch.zeros_like(kc), torch.zeros(m, nq * hd, device="cuda", dtype=torch.bfloat16)
     ops.gemm(w, x, epi=ops.EPI_QKV_ROPE, q_out=q, k_cache=kc, v_cache=vc, positions=pos, slots=slots, n_q_heads=nq, n_kv_heads=nkv,
-             head_dim=hd, rope_theta=theta, q_scale=0.25)
+             head_dim=hd, rope_theta=theta, q_scale=0.25, **tile)
     y = (x.double() @ w.double().t()).view(m, -1, hd)
     ang = pos.double()[:, None] * theta ** (-torch.arange(0, hd, 2, device="cuda", dtype=torch.float64) / hd)
     cos, sin = ang.cos()[:, None], ang.sin()[:, None]

@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "fp32x2.cuh"
 #include "launch.cuh"
 #include "tmem.cuh"
 
@@ -69,23 +70,6 @@ struct AttnTcParams {
   const float* sink;
 };
 
-typedef unsigned long long apair;            // two fp32 values: the same IEEE results at half the issue slots
-__device__ __forceinline__ apair apack(float lo, float hi) {
-  apair r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void aunpack(apair v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ apair afma2(apair a, apair b, apair c) {
-  apair r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ apair aadd2(apair a, apair b) {
-  apair r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t r[32];
   asm volatile(
@@ -434,21 +418,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       }
       // P = exp2(s - m_ref) -> bf16 -> swizzled K-major smem tile (A operand of the PV MMA)
       const float mr = (m_ref == -INFINITY) ? 0.f : m_ref;          // fully masked so far: exp2(-inf - 0) = 0
-      const apair unit2 = apack(unit, unit), ref2 = apack(-mr, -mr);
-      apair ls[2] = {0ull, 0ull};
+      const pair32 unit2 = pack32(unit, unit), ref2 = pack32(-mr, -mr);
+      pair32 ls[2] = {0ull, 0ull};
       float lsum;
       if constexpr (P_TMEM) {
         uint32_t pk[BKV / 2];            // bf16 pairs: key 2j in the low half of column j
 #pragma unroll
         for (int j = 0; j < BKV / 2; ++j) {
           float p0, p1;
-          aunpack(afma2(apack(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), unit2, ref2), p0, p1);
+          unpack32(fma2(pack32(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), unit2, ref2), p0, p1);
           p0 = ex2(p0);
           p1 = ex2(p1);
           pk[j] = pack2(p0, p1);
           // Q32: the sum of what the product sees, so that the rounding of a dominant weight cancels
-          if constexpr (Q32) ls[j & 1] = aadd2(ls[j & 1], apack(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xffff0000u)));
-          else ls[j & 1] = aadd2(ls[j & 1], apack(p0, p1));
+          if constexpr (Q32) ls[j & 1] = add2(ls[j & 1], pack32(__uint_as_float(pk[j] << 16), __uint_as_float(pk[j] & 0xffff0000u)));
+          else ls[j & 1] = add2(ls[j & 1], pack32(p0, p1));
         }
         static_assert(BKV == 64, "P_TMEM packs one 64-key tile into 32 columns");
         tmem_st32_bits(s_addr, pk);      // over the (already consumed) scores of this tile
@@ -460,10 +444,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           float p0, p1;
-          aunpack(afma2(apack(__uint_as_float(r[8 * j + 2 * e]), __uint_as_float(r[8 * j + 2 * e + 1])), unit2, ref2), p0, p1);
+          unpack32(fma2(pack32(__uint_as_float(r[8 * j + 2 * e]), __uint_as_float(r[8 * j + 2 * e + 1])), unit2, ref2), p0, p1);
           p0 = ex2(p0);
           p1 = ex2(p1);
-          ls[e & 1] = aadd2(ls[e & 1], apack(p0, p1));
+          ls[e & 1] = add2(ls[e & 1], pack32(p0, p1));
           w[e] = pack2(p0, p1);
         }
         *reinterpret_cast<uint4*>(ptile + ((j ^ (row & 7)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -471,7 +455,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
       }
       {
         float x, y;
-        aunpack(aadd2(ls[0], ls[1]), x, y);
+        unpack32(add2(ls[0], ls[1]), x, y);
         lsum = x + y;
       }
       l = l * alpha + lsum;

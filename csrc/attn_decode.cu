@@ -13,7 +13,9 @@
 // K0, K1, V0, K2, V1, ..  The reference maximum of a head is kept while no score exceeds it by 2^8; one barrier with a vote per
 // tile tells all threads.  The weights are summed as they are rounded for the second product.  Relative error against 64-bit sums, means of 8
 // inputs, attention_tc.cu / here with unrounded sums / here: 32 x 8100 keys 0.002277 / 0.002304 / 0.002239, 32 x 500 0.00225 / 0.00217 / 0.00203,
-// 8 x 3000 of 256 channels 0.00223 / 0.00220 / 0.00214 (exact running maxima: 0.0019, and 0.3 % on a decode step).  Few sequences: a cluster of up to eight CTAs shares the keys of one (sequence, key/value head) and merges
+// 8 x 3000 of 256 channels 0.00223 / 0.00220 / 0.00214 (exact running maxima: 0.0019, and 0.3 % on a decode step).
+//
+// Few sequences: a cluster of up to eight CTAs shares the keys of one (sequence, key/value head) and merges
 // the partial sums through distributed shared memory -- no workspace and no second kernel.
 //
 // Bound: the cache stream.  Measured on B200 (attention_tc.cu -> here), 32 query / 8 key/value heads of 128, us: 32 sequences x 8100 keys
@@ -35,7 +37,7 @@ int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t co
 namespace {
 
 constexpr int DPAGE = 64;
-constexpr int DKEYS = 128;                         // keys per tile == MMA rows
+constexpr int DKEYS = 128;                         // keys per tile == MMA rows (ma_value_desc has 128 x 128 bytes between channel blocks)
 constexpr int DHEADS = 16;                         // MMA columns: query heads of a key/value head, padded
 constexpr int DSLOTS = 3;
 constexpr int DEC_THREADS = 192;
@@ -66,17 +68,6 @@ struct DecCfg {
   static constexpr uint32_t kCols = 64;                            // S twice, O for every 128 channels
   static constexpr uint32_t kOCol = 2 * DHEADS;
 };
-
-// A operand whose rows are the contiguous dimension: 128-byte rows of 64 channels per key, `lbo` bytes between the 64-channel blocks
-__device__ __forceinline__ uint64_t dec_value_desc(uint32_t smem_addr, uint32_t lbo) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
-  d |= static_cast<uint64_t>((lbo >> 4) & 0x3FFF) << 16;
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;
-  return d;
-}
 
 template <int GP>
 __device__ __forceinline__ void dec_ld(uint32_t taddr, float* v) {   // GP columns of this thread's lane
@@ -254,7 +245,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int m = 0; m < MB; ++m)
 #pragma unroll
           for (int kk = 0; kk < DKEYS / 16; ++kk) {
-            const uint64_t a = dec_value_desc(smem_u32(smem + s * Cfg::kTile + m * 2 * (DKEYS * 128) + kk * (16 * 128)), DKEYS * 128);
+            const uint64_t a = ma_value_desc(smem_u32(smem + s * Cfg::kTile + m * 2 * (DKEYS * 128) + kk * (16 * 128)));
             const uint64_t b = make_sw128_kmajor_desc(smem_u32(p_s + (n & 1) * Cfg::kP + (kk / 4) * (DHEADS * 128))) + static_cast<uint64_t>((kk % 4) * 2);
             umma_bf16(tmem + Cfg::kOCol + m * DHEADS, a, b, idesc_o, (n > 0 || kk > 0) ? 1u : 0u);
           }

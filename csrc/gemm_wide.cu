@@ -29,6 +29,7 @@
 // Roles (192 threads): warp 0 = TMA producer (both CTAs), warp 1 = TMEM owner, MMA issuer in the pair's even CTA, warps 2..5 = epilogue.
 #include "gemm_tc.cuh"
 
+#include "activations.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.cuh"
@@ -60,15 +61,6 @@ struct WideCfg {
   static constexpr uint32_t kTmemCols = BN == 128 ? 256 : 512;
   static_assert(WM * kLandPitch * 4 <= kStages * kStageBytes, "the landing zone reuses the ring");
 };
-
-__device__ __forceinline__ float w_gelu(float x) {
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
-}
-__device__ __forceinline__ float w_silu(float x) { return x / (1.f + __expf(-x)); }
-__device__ __forceinline__ float w_xielu(float x, float ap, float an) {
-  return x > 0.f ? ap * x * x + 0.5f * x : an * (expm1f(x) - x) + 0.5f * x;
-}
 
 template <uint32_t kCols>
 __device__ __forceinline__ void tmem_alloc2(uint32_t* smem_result) {
@@ -378,7 +370,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             load(c + half * 32, g);
             load(c + 64 + half * 32, u);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) g[j] = (p.act_gelu ? w_gelu(g[j]) : w_silu(g[j])) * u[j];
+            for (int j = 0; j < 32; ++j) g[j] = (p.act_gelu ? gelu_tanh(g[j]) : silu(g[j])) * u[j];
             put(half, g);
           }
           flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>((n0 + c) / 2) * 2, static_cast<size_t>(p.ld_out) * 2);
@@ -421,10 +413,9 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 if (p.act_gelu == 2) {
-                  const float r = fmaxf(v[j], 0.f);
-                  v[j] = r * r;
+                  v[j] = relu_sq(v[j]);
                 } else {
-                  v[j] = p.act_gelu == 3 ? w_xielu(v[j], p.rope_theta, p.q_scale) : w_gelu(v[j]);
+                  v[j] = p.act_gelu == 3 ? xielu(v[j], p.rope_theta, p.q_scale) : gelu_tanh(v[j]);
                 }
               }
             } else if constexpr (EPI == EPI_QKV_ROPE) {

@@ -25,6 +25,7 @@
 
 #include <cstdint>
 
+#include "fp32x2.cuh"
 #include "launch.cuh"
 
 namespace b2b {
@@ -66,24 +67,6 @@ struct SpanCfg {
 
 // state rows of lane ti: ti*4 .. +3 and, for 128 rows, 64 + ti*4 .. +3
 __device__ __forceinline__ int state_row(int ti, int r) { return (r >> 2) * 64 + ti * 4 + (r & 3); }
-
-typedef unsigned long long pair32;                            // two fp32 values
-__device__ __forceinline__ pair32 pack32(float lo, float hi) {
-  pair32 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack32(pair32 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ pair32 mul2(pair32 a, pair32 b) {
-  pair32 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ pair32 fma2(pair32 a, pair32 b, pair32 c) {
-  pair32 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 
 // (p + e) <- (p + e) d, e the rounding error of p: a constant decay rounds the same way every time, so a plain product drifts
 __device__ __forceinline__ void chain(float& p, float& e, float d) {

@@ -1,6 +1,6 @@
 """bee2bee_b200 -- Blackwell-native peer-mesh inference engine with the Bee2Bee surface.
 
-Public exports mirror the reference package (/root/reference/bee2bee/__init__.py:1-11):
+Public exports mirror the reference package (bee2bee/__init__.py:1-11):
 ``P2PNode``, ``run_p2p_node``, ``api_server`` (the FastAPI module) and ``__version__``.
 Heavy sub-modules are imported lazily so ``import bee2bee_b200`` stays cheap."""
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""``bee2bee`` command line (parity: /root/reference/bee2bee/__main__.py:30-123).
+"""``bee2bee`` command line (parity: bee2bee/__main__.py:30-123).
 
 Same verbs and options (``serve-ollama``, ``serve-hf``, ``serve-hf-remote``, ``register``)
 plus what a B200 deployment needs: ``--pieces`` (layer pieces = GPUs), ``config``,

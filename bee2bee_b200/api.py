@@ -1,4 +1,4 @@
-"""HTTP sidecar (parity: /root/reference/bee2bee/api.py): ``/``, ``/peers``, ``/providers``,
+"""HTTP sidecar (parity: bee2bee/api.py): ``/``, ``/peers``, ``/providers``,
 ``/connect``, ``/chat`` == ``/generate`` with the reference's JSON shapes, ``X-API-KEY`` auth
 iff ``BEE2BEE_API_KEY`` is set, CORS from ``CORS_ORIGINS``.
 

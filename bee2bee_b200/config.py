@@ -1,5 +1,5 @@
 """Three-tier configuration: CLI flag > environment > ``$BEE2BEE_HOME/config.json`` > defaults
-(parity: /root/reference/bee2bee/config.py:11-47), extended with validated engine settings
+(parity: bee2bee/config.py:11-47), extended with validated engine settings
 (pieces, dtype, batch, KV budget) that the reference has no notion of."""
 from __future__ import annotations
 

@@ -1,4 +1,4 @@
-"""Dataset helper shims (parity: /root/reference/bee2bee/datasets.py:5-24)."""
+"""Dataset helper shims (parity: bee2bee/datasets.py:5-24)."""
 from __future__ import annotations
 
 from typing import Any, Dict

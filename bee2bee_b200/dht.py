@@ -1,4 +1,4 @@
-"""Provider discovery table (parity: /root/reference/bee2bee/dht.py:6-64).
+"""Provider discovery table (parity: bee2bee/dht.py:6-64).
 
 Same async surface (``DHTNode.start/set/get``, ``announce_piece``, ``find_providers``).
 Backends: Kademlia over UDP when the optional ``kademlia`` package exists and the node is

@@ -1,7 +1,7 @@
 """Inference engine: request queue, continuous batching over fixed batch slots, paged-KV
 admission control, token streaming.  The reference runs one blocking
 ``model.generate`` per request inside the event loop (no batching, no KV management,
-/root/reference/bee2bee/services.py:85-116, api.py:229); here requests are only *enqueued*
+bee2bee/services.py:85-116, api.py:229); here requests are only *enqueued*
 by the asyncio side and a scheduler thread drives the GPU:
 
     admit (pages available?) -> prefill burst -> decode burst of N graph replays -> read tokens
@@ -233,7 +233,7 @@ class Engine:
         r = Request(next(self._ids), ids, params, on_token, t_submit=time.time())
         if self.broken:
             # reference semantics for a lost peer: the provider disappears and the caller is told at once
-            # (/root/reference/bee2bee/p2p_runtime.py:396-410) -- no request may queue behind a dead mesh
+            # (bee2bee/p2p_runtime.py:396-410) -- no request may queue behind a dead mesh
             r.error = self.broken
             r.finish_reason = "error"
             r.t_done = time.time()
@@ -307,7 +307,7 @@ class Engine:
         """Abandon a request (client disconnected, stop word hit, wait timed out): it stops occupying its batch slot
         and KV pages at the next burst boundary instead of decoding to ``max_new_tokens``.  Thread-safe; on a serving
         mesh the cancellation travels to the follower ranks with the next plan broadcast.  The reference leaks its
-        generate thread in the same situation (/root/reference/bee2bee/hf.py:107-136)."""
+        generate thread in the same situation (bee2bee/hf.py:107-136)."""
         if req.done.is_set():
             return
         req.cancelled = True          # retired (finish_reason "cancelled") at the next burst boundary, on every rank

@@ -1,10 +1,10 @@
 """Paged KV-cache bookkeeping (host side).  Pages hold 64 tokens (``ops.PAGE``); page 0 is a
 scratch page that inactive batch rows point at, so it is never handed out.  The reference
 has no KV management at all (HF ``DynamicCache`` grows by concatenation per request and is
-dropped afterwards, /root/reference/bee2bee/hf.py:42-43) and re-sends the whole chat transcript
-every turn with no reuse (SURVEY 5.7).
+dropped afterwards, bee2bee/hf.py:42-43) and re-sends the whole chat transcript
+every turn with no reuse.
 
-**Prefix cache** (round 2): full prompt pages are content-addressed (hash chain over 64-token blocks).  A new request
+**Prefix cache**: full prompt pages are content-addressed (hash chain over 64-token blocks).  A new request
 whose prompt starts with blocks that are still resident shares those physical pages (reference-counted) and only its
 suffix is prefilled -- every piece of the mesh keeps the same page ids, so the decision is replicated on all ranks.
 Sequences that share a prefix therefore read the SAME KV pages in attention (one copy in HBM / L2 for the whole batch).

@@ -1,11 +1,11 @@
 """Tokenizers.  There is no network, hence no vocab files for the named checkpoints: the
 default is a deterministic byte-level tokenizer that works with any vocab >= 260.  A real
 Hugging Face tokenizer is used when the model directory ships one (same call the
-reference makes, /root/reference/bee2bee/hf.py:24).
+reference makes, bee2bee/hf.py:24).
 
 Also hosts the prompt helpers of the reference's streaming path: parsing
 ``user: / assistant:`` transcripts into chat messages and cutting generated text at stop
-words (/root/reference/bee2bee/hf.py:54-71,112-133).
+words (bee2bee/hf.py:54-71,112-133).
 """
 from __future__ import annotations
 

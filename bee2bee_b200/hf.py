@@ -1,5 +1,5 @@
 """Model-backend helpers with the reference's L2 surface
-(/root/reference/bee2bee/hf.py:7-205) on top of this framework's engine instead of
+(bee2bee/hf.py:7-205) on top of this framework's engine instead of
 ``transformers.generate``:
 
     load_model_and_tokenizer -> (LoadedModel, tokenizer, device)

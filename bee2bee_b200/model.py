@@ -1,5 +1,5 @@
 """Dense-layer MLP used by the legacy worker tasks (parity:
-/root/reference/bee2bee/model.py:7-71 and the manual backprop in node.py:99-182).
+bee2bee/model.py:7-71 and the manual backprop in node.py:99-182).
 
 Weights are (in_dim, out_dim) like the reference.  ``layer_backward`` returns the same
 ``dX, gW, gb`` triple the reference's ``layer_backward`` task ships back as JSON.  With a GPU

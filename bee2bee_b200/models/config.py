@@ -1,7 +1,7 @@
 """Model architecture descriptions for the decoder families the mesh serves.
 
 The reference ships no model configs (it defers to ``transformers``,
-/root/reference/bee2bee/hf.py:23-32); these presets are the public architectures named in
+bee2bee/hf.py:23-32); these presets are the public architectures named in
 BASELINE.json (distilgpt2, Llama-3-8B, Zephyr-7B-beta = Mistral-7B, gemma-2-2b) plus tiny
 variants of each family for tests.  A config can also be read from a Hugging Face
 ``config.json`` (``ModelConfig.from_hf_dict``) so ``serve-hf --model <local dir>`` works.
@@ -760,7 +760,7 @@ class ModelConfig:
                 norm_eps=d.get("layer_norm_epsilon", 1e-5), act="gelu_tanh", glu=False, rope_theta=0.0,
                 tie_embeddings=True, bias=True, eos_token_id=d.get("eos_token_id", 50256),
                 bos_token_id=d.get("bos_token_id", 50256))
-        # checkpoints the loader would map wrongly are rejected instead of loading "successfully" 
+        # checkpoints the loader would map wrongly are rejected instead of loading "successfully"
         if d.get("attention_bias") or d.get("mlp_bias"):
             raise ValueError(f"{name or mt}: attention_bias / mlp_bias checkpoints (Qwen-style) are not supported: "
                              "the weight map carries no bias tensors for this family")
@@ -1144,7 +1144,7 @@ def piece_units(cfg: "ModelConfig", pieces: int, bounds: Optional[List[int]] = N
     its head.  Returns ``pieces`` contiguous ``(u0, u1)`` ranges that minimise the heaviest stage of the wavefront under
     a bytes-plus-launch-latency cost model (a decode step is weight-bandwidth bound with a few us of fixed cost per
     kernel); the last piece also carries the lm_head and the sampler.  Llama-3-8B over 8 GPUs: whole layers give
-    5/4/4/4/4/4/4/3 (+head) = 0.81 of the ideal stage time, half layers (round 1) 0.92, thirds 0.97.  ``bounds``
+    5/4/4/4/4/4/4/3 (+head) = 0.81 of the ideal stage time, half layers 0.92, thirds 0.97.  ``bounds``
     overrides the search (tests).  Graphs without the fused RMSNorm / GLU epilogues are cut at whole layers."""
     UPL = UNITS_PER_LAYER
     U = UPL * cfg.n_layers

@@ -4,7 +4,7 @@ Two jobs: (1) the numerical oracle every CUDA kernel / fused path is tested agai
 (2) the execution backend on machines without a B200 (CPU plumbing config of
 distilgpt2 split in two pieces over the loopback mesh).  Semantics follow
 the Hugging Face modelling code the reference delegates to
-(/root/reference/bee2bee/hf.py:23-44).
+(bee2bee/hf.py:23-44).
 """
 from __future__ import annotations
 
@@ -138,7 +138,7 @@ class TorchPiece:
 def sample_reference(logits: torch.Tensor, seen: Optional[torch.Tensor], temperature: float, top_p: float,
                      rep_penalty: float, generator: Optional[torch.Generator] = None) -> torch.Tensor:
     """HF-processor semantics (repetition penalty -> temperature -> top-p -> multinomial /
-    greedy when temperature <= 0), cf. /root/reference/bee2bee/hf.py:91-105.
+    greedy when temperature <= 0), cf. bee2bee/hf.py:91-105.
     logits [B, V] fp32; seen [B, V] bool of ids already in the context."""
     l = logits.float().clone()
     if seen is not None and rep_penalty != 1.0:

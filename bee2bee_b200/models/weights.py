@@ -2,7 +2,7 @@
 Face directory load/save (safetensors, HF tensor names) and the per-piece slicing that
 gives the reference's "piece" its north-star meaning: a contiguous layer range resident on
 one GPU (the reference prototype re-loads the *whole* model on every worker and runs a
-slice, /root/reference/bee2bee/hf.py:180-205 — here only the slice is ever materialised).
+slice, bee2bee/hf.py:180-205 — here only the slice is ever materialised).
 """
 from __future__ import annotations
 
@@ -515,10 +515,10 @@ WEIGHT_SOURCE: Dict[str, str] = {}
 
 
 def random_weights_allowed(model: str) -> bool:
-    """Random initialisation is OPT-IN (ADVICE r1): the synthetic test presets, or ``B2B_ALLOW_RANDOM_WEIGHTS=1``
+    """Random initialisation is OPT-IN: the synthetic test presets, or ``B2B_ALLOW_RANDOM_WEIGHTS=1``
     (benchmarks, smoke runs, CI -- there is no network in the build environment, hence no checkpoints).  Without it a
     node must not announce ``llama-3-8b`` to the mesh and serve noise; the reference would fail to load instead
-    (/root/reference/bee2bee/hf.py:23-32)."""
+    (bee2bee/hf.py:23-32)."""
     name = os.path.basename(os.path.normpath(model)).lower() if model else ""
     return name.startswith(("tiny-", "mini-")) or os.environ.get("B2B_ALLOW_RANDOM_WEIGHTS", "0") == "1"
 

@@ -1,4 +1,4 @@
-"""NAT traversal (parity: /root/reference/bee2bee/nat.py:19-609): UPnP -> NAT-PMP -> PCP ->
+"""NAT traversal (parity: bee2bee/nat.py:19-609): UPnP -> NAT-PMP -> PCP ->
 STUN, public-IP discovery with a 5-minute cache, status/manual-instruction helpers and the
 legacy wrappers (``try_upnp_map``, ``try_stun``, ``auto_port_forward``, ``get_public_ip``).
 

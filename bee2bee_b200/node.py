@@ -1,4 +1,4 @@
-"""Legacy coordinator/worker protocol (parity: /root/reference/bee2bee/node.py:38-294,
+"""Legacy coordinator/worker protocol (parity: bee2bee/node.py:38-294,
 constants in protocol.py).  The reference ships only the *worker* half -- its coordinator no
 longer exists, so nothing can drive it.  Here:
 

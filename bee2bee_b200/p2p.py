@@ -1,8 +1,8 @@
-"""Join links and content hashing (parity: /root/reference/bee2bee/p2p.py:8-52).
+"""Join links and content hashing (parity: bee2bee/p2p.py:8-52).
 
 ``coithub.org://join?network=<n>&model=<m>&hash=<sha256>&bootstrap=<urlsafe-b64, unpadded>...``
 The parser also accepts ``coithub://`` and ``p2pnet://`` (the reference's runtime routes
-``p2pnet://`` links to a parser that rejects them -- SURVEY.md section 8)."""
+``p2pnet://`` links to a parser that rejects them)."""
 from __future__ import annotations
 
 import base64

@@ -1,15 +1,15 @@
-"""Mesh runtime: ``P2PNode`` + ``run_p2p_node`` (parity: /root/reference/bee2bee/p2p_runtime.py).
+"""Mesh runtime: ``P2PNode`` + ``run_p2p_node`` (parity: bee2bee/p2p_runtime.py).
 
 Same public surface and wire messages as the reference (hello / peer_list / ping / pong /
 service_announce / gen_request / gen_chunk / gen_success / gen_error / gen_result /
-piece_request / piece_data, section 2.5 of SURVEY.md), re-designed:
+piece_request / piece_data), re-designed:
 
 * transports are pluggable (``ws://`` wire-compatible sockets, ``inproc://`` hub) and carry
   only the *control plane*; activations between layer pieces move GPU->GPU (``parallel.mesh``)
   or, on CPU-only hosts, as binary ``hidden_forward`` frames -- never JSON number lists;
 * handlers never block the loop: services run through ``aexecute`` / ``aexecute_stream``;
 * a requester resolves on ``gen_success | gen_error | gen_result`` and streams ``gen_chunk``
-  (the reference only resolves ``gen_result`` and times out, SURVEY R8);
+  (the reference only resolves ``gen_result`` and times out);
 * failure detection: missed pongs mark a peer unreachable and drop it; bootstrap peers are
   re-dialled with back-off; byte-piece exchange and the DHT are actually wired.
 """
@@ -320,7 +320,7 @@ class P2PNode:
 
     async def _send(self, conn: Optional[Connection], message: Dict[str, Any]) -> bool:
         """Returns False on failure (the reference swallows send errors, which makes its
-        "unreachable" health state unreachable -- SURVEY section 8)."""
+        "unreachable" health state unreachable)."""
         if conn is None:
             return False
         try:

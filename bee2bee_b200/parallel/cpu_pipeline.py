@@ -1,7 +1,7 @@
 """Layer-piece pipeline over the *control-plane* mesh, for hosts without NVLink (CPU plumbing
 configuration of BASELINE.json: distilgpt2 split in two pieces over the loopback
 ``p2p_runtime``).  This is the generalisation of the reference's orphaned
-``hf_part_load`` / ``hf_part_forward`` worker tasks (/root/reference/bee2bee/node.py:236-277)
+``hf_part_load`` / ``hf_part_forward`` worker tasks (bee2bee/node.py:236-277)
 to decoder LMs with a KV cache:
 
 * ``PieceHost``           one layer range + per-session KV caches on a peer,

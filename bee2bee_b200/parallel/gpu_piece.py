@@ -1,5 +1,5 @@
 """Layer range [start, end) of a decoder LM resident on ONE B200 for the legacy coordinator / worker protocol
-(``hf_part_load`` / ``hf_part_forward``, /root/reference/bee2bee/node.py:236-277), executed by the hand-written
+(``hf_part_load`` / ``hf_part_forward``, bee2bee/node.py:236-277), executed by the hand-written
 kernels (``NativePiece``) with a paged KV cache per session.
 
 The reference ships the hidden state of every hop as a JSON list of fp32 (D2H -> ``.tolist()`` -> WebSocket ->

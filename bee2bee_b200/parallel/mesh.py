@@ -2,7 +2,7 @@
 
 ``peer = one B200 hosting one piece``.  What the reference does with bootstrap links,
 hello/peer_list gossip, DHT lookups, STUN/UPnP and one WebSocket per peer pair
-(/root/reference/bee2bee/p2p_runtime.py:308-372,478-523; dht.py; nat.py) collapses into
+(bee2bee/p2p_runtime.py:308-372,478-523; dht.py; nat.py) collapses into
 
   * a topology table  rank <-> cuda device <-> piece (layer range), canAccessPeer matrix,
   * symmetric staging buffers + flags whose CUDA IPC handles are exchanged ONCE through

@@ -4,7 +4,7 @@ process per GPU piece, or one CPU worker -- runs as a child process group that c
 Why: a GPU rank that *stalls* is survivable in-process (bounded flag waits -> ``MeshStalled`` -> the engine marks itself
 broken, ``engine/runner.py``), but a rank that *dies* takes its NVLink neighbours' CUDA contexts with it (they store into
 its freed memory), and a broken CUDA context cannot be repaired from inside the process that owns it.  The reference's
-semantics for a lost peer are "drop it, the next ``pick_provider`` skips it" (/root/reference/bee2bee/p2p_runtime.py:396-410)
+semantics for a lost peer are "drop it, the next ``pick_provider`` skips it" (bee2bee/p2p_runtime.py:396-410)
 and a human restarts the node; here the supervisor does both: while the group is down the service reports unhealthy (the
 mesh routes around it), in-flight requests fail at once, a fresh group is spawned (new rendezvous port, fresh IPC
 buffers) and the provider becomes healthy again without the front process ever touching a GPU.

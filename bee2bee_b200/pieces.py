@@ -1,7 +1,7 @@
 """Pieces, in both senses.
 
 1. *Byte pieces* -- fixed-size chunks of a blob with SHA-256 hashes, verify + reassemble,
-   ``<hash>_<idx:08d>.part`` files (parity: /root/reference/bee2bee/pieces.py:7-32; the
+   ``<hash>_<idx:08d>.part`` files (parity: bee2bee/pieces.py:7-32; the
    reference's piece_request/piece_data handlers are empty stubs, p2p_runtime.py:675-683 --
    here they are served, see ``p2p_runtime``).
 2. *Layer pieces* -- the north-star meaning: a contiguous layer range of a model resident

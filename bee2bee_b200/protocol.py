@@ -1,8 +1,8 @@
 """Wire protocol catalogue.
 
 Live mesh protocol (JSON frames with a ``type`` key, parity with the dispatch table at
-/root/reference/bee2bee/p2p_runtime.py:460-470) as small typed builders, plus the legacy
-coordinator/worker constants of /root/reference/bee2bee/protocol.py:17-53 that ``node.py``
+bee2bee/p2p_runtime.py:460-470) as small typed builders, plus the legacy
+coordinator/worker constants of bee2bee/protocol.py:17-53 that ``node.py``
 still speaks.  Builders only *construct* dicts -- transports decide how they travel
 (WebSocket text frame, in-process queue, ...), and never on the token path.
 """
@@ -42,7 +42,7 @@ HIDDEN_RESULT = "hidden_result"
 
 LIVE_TYPES = (HELLO, PEER_LIST, PING, PONG, SERVICE_ANNOUNCE, GEN_REQUEST, GEN_CHUNK, GEN_SUCCESS, GEN_ERROR,
               GEN_RESULT, PIECE_REQUEST, PIECE_DATA, PIECE_ANNOUNCE, HIDDEN_FORWARD, HIDDEN_RESULT)
-#: terminal replies a requester must resolve on (the reference only resolves ``gen_result``, SURVEY R8)
+#: terminal replies a requester must resolve on (the reference only resolves ``gen_result``)
 GEN_TERMINAL = (GEN_SUCCESS, GEN_ERROR, GEN_RESULT)
 
 

@@ -1,4 +1,4 @@
-"""Node registry client (parity: /root/reference/bee2bee/registry.py:7-69).
+"""Node registry client (parity: bee2bee/registry.py:7-69).
 
 Same env contract (``SUPABASE_URL|VITE_SUPABASE_URL`` + ``SUPABASE_ANON_KEY|VITE_...`` or
 ``BEE2BEE_ENTRYPOINT``), same upsert payload and headers, same offline mode when no

@@ -1,5 +1,5 @@
 """Service abstraction: what a peer *offers* to the mesh (parity:
-/root/reference/bee2bee/services.py:10-308).
+bee2bee/services.py:10-308).
 
     BaseService(name).get_metadata() / execute(params) -> dict / execute_stream(params) -> iterator
 
@@ -8,7 +8,7 @@ lines + ``{"done": true}`` for HF, raw text chunks for Ollama).  What differs is
 behind them: ``HFService`` enqueues into this framework's continuous-batching engine
 (hand-written sm_100a kernels, pieces across GPUs) instead of calling
 ``transformers.generate`` inline, and every service exposes ``aexecute`` /
-``aexecute_stream`` so asyncio callers never block their loop (SURVEY section 8).
+``aexecute_stream`` so asyncio callers never block their loop.
 """
 from __future__ import annotations
 
@@ -229,7 +229,7 @@ class OllamaService(BaseService):
                  **engine_kw):
         super().__init__("ollama")
         self.model_name = model_name
-        # OLLAMA_HOST is honoured (the reference sets it but never reads it, SURVEY section 8)
+        # OLLAMA_HOST is honoured (the reference sets it but never reads it)
         self.host = host or os.environ.get("OLLAMA_HOST") or "http://localhost:11434"
         if not self.host.startswith("http") and self.host != "embedded":
             self.host = "http://" + self.host

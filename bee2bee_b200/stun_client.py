@@ -1,4 +1,4 @@
-"""RFC 5389 STUN binding client (parity: /root/reference/bee2bee/stun_client.py:10-180 -- dead
+"""RFC 5389 STUN binding client (parity: bee2bee/stun_client.py:10-180 -- dead
 code there, wired into ``nat`` here).  Pure sockets, asyncio datagram endpoints; every
 network call is skipped when ``BEE2BEE_OFFLINE`` is set."""
 from __future__ import annotations

@@ -1,4 +1,4 @@
-"""Identifiers, clocks and hashing helpers (parity: /root/reference/bee2bee/utils.py:43-64)."""
+"""Identifiers, clocks and hashing helpers (parity: bee2bee/utils.py:43-64)."""
 from __future__ import annotations
 
 import hashlib

@@ -1,5 +1,5 @@
 """Node metrics with the reference's JSON keys (``throughput``, ``memory_percent``,
-``gpu_percent``, ``trust_score``; /root/reference/bee2bee/utils.py:102-135) -- but
+``gpu_percent``, ``trust_score``; bee2bee/utils.py:102-135) -- but
 ``throughput`` is the engine's *measured* decode tokens/s when an engine is attached
 (the reference reports ``cpu% x 0.85``), and multi-GPU ``nvidia-smi`` output is averaged
 instead of failing to parse."""

@@ -1,4 +1,4 @@
-"""Home directory and atomic JSON persistence (parity: /root/reference/bee2bee/utils.py:11-40)."""
+"""Home directory and atomic JSON persistence (parity: bee2bee/utils.py:11-40)."""
 from __future__ import annotations
 
 import json

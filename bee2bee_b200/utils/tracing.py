@@ -1,5 +1,4 @@
-"""Tracing / profiling hooks (the reference has none beyond two wall-clock deltas,
-SURVEY section 5.1).  ``BEE2BEE_TRACE=1`` turns on
+"""Tracing / profiling hooks (the reference has none beyond two wall-clock deltas).  ``BEE2BEE_TRACE=1`` turns on
 
 * NVTX ranges around engine phases (visible in Nsight Systems / ncu --nvtx),
 * CUDA-event timing of the same ranges on the launching stream (device time, not wall clock),

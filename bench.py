@@ -272,7 +272,7 @@ def run_ours(args):
                "h2d_bytes_per_step": (eng.h2d_bytes + runner.h2d_bytes - h0) / K,
                "d2h_bytes_per_step": eng.d2h_bytes / K, "includes": "prefill+decode, scheduler, token readback",
                "host_ms": dict(eng.host_ms)}
-        # rank-count independence (VERDICT r1 #8): greedy continuation of the same prompts through the same public call;
+        # rank-count independence: greedy continuation of the same prompts through the same public call;
         # the checksum over the first 32 sequences must be identical at every N (the pieces only change the transport:
         # same kernels, same tiles, same split-K -- tests/test_multigpu.py asserts it token for token on 2 / 4 / 8 GPUs)
         try:
@@ -420,7 +420,7 @@ def run_nccl(args):
 def run_reference(args):
     """Unmodified reference (baseline/_ref): HFService -> transformers.generate on one GPU per rank
     (the reference has no multi-GPU path; N ranks = N independent replica providers, which is its own
-    "load balancing" story, /root/reference/bee2bee/p2p_runtime.py:723-757)."""
+    "load balancing" story, bee2bee/p2p_runtime.py:723-757)."""
     ref = os.path.join(ROOT, "baseline", "_ref")
     if not os.path.isdir(os.path.join(ref, "bee2bee")):
         print(json.dumps({"impl": "reference", "unavailable": "baseline/_ref not installed"}))

@@ -287,7 +287,7 @@ __device__ __forceinline__ void red_release_sys_add(uint32_t* p, uint32_t v) {
   asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // Mesh abort word (device memory, one per process / GPU; set through set_wait_policy() of every translation unit that
-// waits on handoff flags).  A wait that exceeds the time bound does NOT trap the GPU (round 1: a late or dead peer took
+// waits on handoff flags).  A wait that exceeds the time bound does NOT trap the GPU (a late or dead peer once took
 // all 8 contexts down): it raises the abort word and returns; every later wait of this process returns at once, so the
 // pipeline drains with garbage in microseconds, the token read-back kernel reports the word to the host and the engine
 // fails the in-flight requests with a clean error while the process (and its control plane) stays alive.

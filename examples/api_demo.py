@@ -1,4 +1,4 @@
-"""HTTP sidecar walk-through in one process (parity: /root/reference/examples/api_demo.py, extended to the routes that
+"""HTTP sidecar walk-through in one process (parity: examples/api_demo.py, extended to the routes that
 actually generate): starts the FastAPI app with an embedded tiny model, then calls `/`, `/peers`, `/providers`,
 `/generate` (buffered and streamed) and `/metrics` through the test client — no ports, no network.
 

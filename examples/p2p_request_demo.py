@@ -1,4 +1,4 @@
-"""Client-side demo (parity: /root/reference/examples/p2p_request_demo.py): join a mesh, list
+"""Client-side demo (parity: examples/p2p_request_demo.py): join a mesh, list
 providers, pick the cheapest one for a model and stream a generation from it.
 
     python -m bee2bee_b200 serve-hf --model tiny-llama --api-port 8000      # terminal 1 (prints its ws:// address)

@@ -1,5 +1,5 @@
 """Manual probe: a client-side P2PNode joins a mesh, lists providers, picks one by (price, latency) and requests a
-generation through `request_generation` (parity: /root/reference/scripts/debug_p2p_request.py, debug_generation.py).
+generation through `request_generation` (parity: scripts/debug_p2p_request.py, debug_generation.py).
 
     python scripts/debug_p2p_request.py ws://127.0.0.1:4334 --model tiny-llama --prompt "user: hi"
 """

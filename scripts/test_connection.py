@@ -1,4 +1,4 @@
-"""Manual probe (parity: /root/reference/scripts/test_connection.py): hello -> peer_list ->
+"""Manual probe (parity: scripts/test_connection.py): hello -> peer_list ->
 ping/pong against a live node.    python scripts/test_connection.py ws://127.0.0.1:4334"""
 import asyncio
 import json

@@ -1,5 +1,5 @@
 """Manual probe: raw-WebSocket `gen_request` against a live node, buffered or streamed
-(parity: /root/reference/scripts/test_generation.py and test_full_request.py).
+(parity: scripts/test_generation.py and test_full_request.py).
 
     python -m bee2bee_b200 serve-hf --model tiny-llama --port 4334 --api-port 0 &
     python scripts/test_generation.py ws://127.0.0.1:4334 --prompt "user: hi" --stream

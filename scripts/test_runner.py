@@ -1,4 +1,4 @@
-"""Run the CPU test-suite and keep a log under $BEE2BEE_HOME (parity: /root/reference/scripts/test_runner.py, which only
+"""Run the CPU test-suite and keep a log under $BEE2BEE_HOME (parity: scripts/test_runner.py, which only
 import-smokes its test modules; this one actually runs them through pytest).
 
     python scripts/test_runner.py            # -m "not gpu"

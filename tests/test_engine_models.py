@@ -177,7 +177,7 @@ def test_engine_eos_stop_and_streaming_thread():
 
 
 def test_engine_cancel_frees_slot_and_pages():
-    """ADVICE r1: an abandoned request (stop word / disconnect / timeout) must not decode to max_new_tokens"""
+    """an abandoned request (stop word / disconnect / timeout) must not decode to max_new_tokens"""
     eng = Engine("tiny-llama", device="cpu", max_batch=1, max_seq_len=256, decode_burst=2)
     sp = SamplingParams(max_new_tokens=200, temperature=0.0, ignore_eos=True)
     a = eng.submit([1, 2, 3], sp)
@@ -212,7 +212,7 @@ def test_engine_cancel_frees_slot_and_pages():
 
 
 def test_engine_prefill_failure_does_not_leak_requests():
-    """ADVICE r1: admitted requests were lost (waiters hung, slot + pages leaked) when runner.prefill raised"""
+    """admitted requests were lost (waiters hung, slot + pages leaked) when runner.prefill raised"""
     eng = Engine("tiny-llama", device="cpu", max_batch=2, max_seq_len=64)
     boom = {"n": 1}
     real = eng.runner.prefill
@@ -315,7 +315,7 @@ def test_split_k_heuristic_matches_the_measured_optimum():
 
 
 def test_weights_policy_random_init_is_opt_in(monkeypatch, tmp_path):
-    """ADVICE r1: `serve-hf --model llama-3-8b` must not silently serve noise"""
+    """`serve-hf --model llama-3-8b` must not silently serve noise"""
     from bee2bee_b200.models.weights import WEIGHT_SOURCE, WeightsUnavailable, load_or_init
     from bee2bee_b200.services import HFService, ServiceError
 
@@ -341,7 +341,7 @@ def test_weights_policy_random_init_is_opt_in(monkeypatch, tmp_path):
 
 
 def test_engine_marks_itself_broken_when_the_mesh_stalls():
-    """SURVEY 5.3: a peer piece that stops answering must fail the in-flight requests and take the provider out of
+    """a peer piece that stops answering must fail the in-flight requests and take the provider out of
     service (the reference drops the peer, p2p_runtime.py:396-410) -- not hang or kill the node."""
     from bee2bee_b200.engine.runner import MeshStalled
 
@@ -401,7 +401,7 @@ def test_prefix_cache_allocator_shares_pins_and_evicts():
 
 
 def test_request_deadline_frees_slot_and_pages():
-    """VERDICT r1 #9: 'timeout -> slot + pages freed at the next burst boundary'.  A request past its ``timeout_s`` is
+    """'timeout -> slot + pages freed at the next burst boundary'.  A request past its ``timeout_s`` is
     retired with finish_reason "timeout" whether it is still queued or already decoding; the others are unaffected."""
     import time
     eng = Engine("tiny-llama", device="cpu", max_batch=1, max_seq_len=256, decode_burst=2)

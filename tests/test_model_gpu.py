@@ -161,9 +161,9 @@ def test_graph_prefill_matches_eager_prefill():
 
 
 def test_legacy_worker_hf_part_on_the_gpu_data_plane():
-    """C16 / VERDICT r1: hf_part_load / hf_part_forward run the layer range on NativePiece and the hop payload stays in
+    """hf_part_load / hf_part_forward run the layer range on NativePiece and the hop payload stays in
     device memory (hidden_ref: cudaMemcpyPeerAsync of a cudaMalloc buffer, exportable as a CUDA IPC handle) instead of
-    the reference's JSON list of fp32 (/root/reference/bee2bee/node.py:270-277).  Result == whole-model oracle."""
+    the reference's JSON list of fp32 (bee2bee/node.py:270-277).  Result == whole-model oracle."""
     import asyncio
     import json
 
@@ -203,9 +203,9 @@ def test_legacy_worker_hf_part_on_the_gpu_data_plane():
 
 
 def test_prefix_cache_shares_kv_pages_and_skips_prefill():
-    """Round 2: content-addressed prompt pages.  A second request with the same 150-token prefix re-uses the resident KV
+    """Content-addressed prompt pages.  A second request with the same 150-token prefix re-uses the resident KV
     pages (same physical pages in its block table) and prefills only its suffix; greedy output equals the engine without
-    the cache.  The reference re-sends and re-computes the whole transcript every turn (SURVEY 5.7)."""
+    the cache.  The reference re-sends and re-computes the whole transcript every turn."""
     V = resolve_config("tiny-llama").vocab_size
     sys_prompt = [(11 * i + 3) % (V - 8) + 4 for i in range(150)]
     prompts = [sys_prompt + [5, 6, 7], sys_prompt + [9, 10, 11, 12], sys_prompt[:70] + [1, 2]]

@@ -64,7 +64,7 @@ def test_two_gpu_sub_layer_piece_boundary(bounds):
 @pytest.mark.parametrize("bounds", ["0,1,12", "0,10,12", "0,6,12", "0,5,12"])
 @pytest.mark.parametrize("prompts", ["bigsmall", "long"])
 def test_two_gpu_multichunk_prefill_backpressure(bounds, prompts):
-    """VERDICT r1 #9 / ADVICE high: >= 16 prefill chunks of very different cost through deliberately unbalanced
+    """>= 16 prefill chunks of very different cost through deliberately unbalanced
     pieces (a 1-unit producer in front of an 11-unit consumer, the reverse, and a cut inside an MLP block).  Without the device-side
     back-pressure (release / ack flags, double-buffered staging) the fast producer overwrites the staging slot
     while the consumer still reads the previous chunk (QKV input + O-proj residual) and the KV / first tokens
@@ -110,7 +110,7 @@ def _agree(a, b):
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs >= 2 GPUs")
 @pytest.mark.parametrize("bounds", ["0,6,12", "0,4,12", "0,9,12", "0,5,12"])
 def test_two_gpu_mxfp8_quantised_hop(bounds):
-    """VERDICT r1 missing #4: fp8 across the handoff.  The tail GEMM of piece 0 (down projection at a layer boundary,
+    """fp8 across the handoff.  The tail GEMM of piece 0 (down projection at a layer boundary,
     O-proj after an attention block) stores the e4m3 copy of the residual stream, its UE8M0 scale-factor chunks and
     the per-token sum of squares into piece 1's memory next to the bf16 stream; piece 1's head GEMM (QKV / gate-up)
     acquires the flag and TMA-loads them -- no quantiser launch at the piece head.  A cut between gate/up and down
@@ -140,9 +140,9 @@ def test_two_gpu_mxfp8_quantised_hop_multichunk_prefill():
 
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs >= 2 GPUs")
 def test_two_gpu_stalled_rank_aborts_cleanly_instead_of_trapping():
-    """Fault injection (SURVEY 5.3 / VERDICT r1 #5): rank 1 is 4 s late, the wait bound is 1 s.  Rank 0's kernels give
+    """Fault injection: rank 1 is 4 s late, the wait bound is 1 s.  Rank 0's kernels give
     up on the flag, raise the device abort word, drain, and the host gets a MeshStalled error within ~1 s; nobody
-    traps, both processes keep a working CUDA context (round 1: every GPU of the mesh trapped)."""
+    traps, both processes keep a working CUDA context."""
     out = _run(2, "tiny-llama", 2, 4, 29629, B2B_FAULT_STALL_S="4", B2B_FAULT_STALL_RANK="1", B2B_WAIT_TIMEOUT_MS="1000")
     r0, r1 = out
     assert r0["stalled"] and r0["after_s"] < 3.5 and r0["cuda_ok"], out

@@ -1,6 +1,6 @@
 """Property-based tests (hypothesis) of the host-side machinery every GPU path depends on: the piece planner, the
-prefix-caching page allocator and the scheduler.  The reference has no equivalent (its tests are example-based,
-SURVEY 4); these guard the invariants the device code silently assumes -- contiguous piece cover, pages never owned
+prefix-caching page allocator and the scheduler.  The reference has no equivalent (its tests are example-based);
+these guard the invariants the device code silently assumes -- contiguous piece cover, pages never owned
 twice unless shared through the prefix cache, every slot and page returned whatever the arrival / cancel pattern."""
 import random
 

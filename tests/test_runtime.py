@@ -87,7 +87,7 @@ def test_generation_local_stream_relay_and_errors():
             await a.connect_bootstrap(b.addr)
             await c.connect_bootstrap(a.addr)
             await settle(lambda: b.peer_id in a.providers and b.peer_id in c.providers and len(c.peers) == 2)
-            # python requester resolves on gen_success (reference never does: SURVEY R8)
+            # python requester resolves on gen_success (the reference never does)
             res = await a.request_generation(b.peer_id, "hello", 7, "echo-model", timeout=5)
             assert res["text"] == "olleh" and res["max_new"] == 7
             # streaming: gen_chunk per delta
@@ -236,7 +236,7 @@ def test_websocket_transport_wire_compat():
 
 
 def test_unhealthy_service_is_announced_and_sorted_last():
-    """a provider whose GPU mesh aborted (engine.broken -> service metadata healthy = False) tells the mesh at
+    """A provider whose GPU mesh aborted (engine.broken -> service metadata healthy = False) tells the mesh at
     the next health tick; every node's pick_provider then prefers the healthy replica even if it is more expensive
     (the reference can only drop peers whose socket closed, p2p_runtime.py:396-410)."""
     async def go():

@@ -1,4 +1,4 @@
-"""Dead-worker recovery (SURVEY 5.3, VERDICT r1 missing #5): the serving front keeps running in its own process, the engine
+"""Dead-worker recovery: the serving front keeps running in its own process, the engine
 group is a child that can be killed; in-flight requests fail at once, the provider reports unhealthy while the group is
 down, a fresh group comes up and serves again.  CPU worker here; on a B200 box the same supervisor spawns one worker
 per GPU piece (a dead rank cannot be repaired inside the process that shares its CUDA context)."""

@@ -340,7 +340,7 @@ class GpuRunner:
                 h_in = self.C.tensor_from_ptr(hand.in_h, [tb, self.cfg.ffn_size], "bf16", dev.index)
         meta = BatchMeta(ids=v["ids"], positions=v["pos"], slots=v["slots"], q_start=v["q_start"], q_len=v["q_len"],
                          kv_len=v["kv_len"], block_table=v["bt"], n_tokens=tb, n_seqs=sb, max_q=mq,
-                         last_idx=v["last_idx"], seq_slot=v["seq_slot"], n_out=ob)
+                         last_idx=v["last_idx"], seq_slot=v["seq_slot"], n_out=ob, bucket=True)
         st["meta"] = meta       # captured kernels address these views by raw pointer: keep them alive
 
         def body():

@@ -782,7 +782,7 @@ class HybridPiece:
         o = self._buf("o0", torch.float32, H * dv)[:T]
         ops.lin_scan(ops.SCAN_HGRN2, proj, mx.off["q"], mx.off["q"], proj, mx.off["v"], self.state[self._key(mx)], o, m.q_start,
                      m.q_len, m.kv_len, m.seq_slot, m.n_seqs, m.max_q, H, H, dk, dv, z=proj, off_z=mx.off["f"],
-                     zbias=mx.f["f.b"], hparam=mx.f["lower"])
+                     zbias=mx.f["f.b"], hparam=mx.f["lower"], ragged=m.bucket)
         do = self._buf(f"mix0.{H * dv}", self.dtype, mx.w_o.shape[1])[:T]
         ops.scan_post(o, o, 0, mx.f["norm"], ops.POST_NONE, None, do, T, H, dv, self.cfg.norm_eps)
         return ops.linear(mx.w_o, do, y)
@@ -895,7 +895,7 @@ class HybridPiece:
                         H, dk)
         o = self._buf(f"o{mx.idx}", torch.float32, H * dv)[:T]
         ops.lin_scan(ops.SCAN_MLSTM, proj, mx.off["q"], mx.off["k"], proj, mx.off["v"], self.state[self._key(mx)], o, m.q_start,
-                     m.q_len, m.kv_len, m.seq_slot, m.n_seqs, m.max_q, H, H, dk, dv, aux=aux, qscale=qs)
+                     m.q_len, m.kv_len, m.seq_slot, m.n_seqs, m.max_q, H, H, dk, dv, aux=aux, qscale=qs, ragged=m.bucket)
         return self._scan_out(mx, o, proj, mx.off["g"], 0, aux, m, y)
 
     def _low_rank(self, mx: _Mix, proj: torch.Tensor, off: int, T: int) -> torch.Tensor:
@@ -911,7 +911,7 @@ class HybridPiece:
         o = self._buf(f"o{mx.idx}", torch.float32, H * dv)[:T]
         ops.lin_scan(ops.SCAN_GLA, proj, mx.off["q"], mx.off["k"], proj, mx.off["v"], self.state[self._key(mx)], o, m.q_start,
                      m.q_len, m.kv_len, m.seq_slot, m.n_seqs, m.max_q, H, H, dk, dv, z=z, zbias=mx.f["zbias"],
-                     qscale=dk ** -0.5, inv_tau=1.0 / sp.tau)
+                     qscale=dk ** -0.5, inv_tau=1.0 / sp.tau, ragged=m.bucket)
         return self._scan_out(mx, o, proj, mx.off["g"], 1, None, m, y)
 
     def _mix_channel_delta(self, mx: _Mix, proj: torch.Tensor, m, y: torch.Tensor) -> torch.Tensor:
@@ -925,7 +925,7 @@ class HybridPiece:
         o = self._buf(f"o{mx.idx}", torch.float32, H * dv)[:T]
         ops.lin_scan(ops.SCAN_DELTA, conv, 0, G * dk, conv, 2 * G * dk, self.state[self._key(mx)], o, m.q_start, m.q_len,
                      m.kv_len, m.seq_slot, m.n_seqs, m.max_q, H, G, dk, dv, z=z, zbias=mx.f["zbias"], hparam=mx.f["A_log"],
-                     beta=proj, off_b=mx.off["b"], qscale=dk ** -0.5)
+                     beta=proj, off_b=mx.off["b"], qscale=dk ** -0.5, ragged=m.bucket)
         return self._scan_out(mx, o, z, H * dk, 0, None, m, y)
 
     def _debug_sum(self, st: torch.Tensor, pend, T: int) -> torch.Tensor:
@@ -1141,7 +1141,7 @@ class HybridPiece:
         else:
             ops.lin_scan(ops.SCAN_SSD, xbc, inner + G * N, inner, xbc, 0, self.state[key], o, m.q_start, m.q_len, m.kv_len,
                          m.seq_slot, m.n_seqs, m.max_q, H, G, N, V, zbias=mx.f["dt_bias"], hparam=mx.f["A_log"], beta=proj,
-                         off_b=mx.off["dt"])
+                         off_b=mx.off["dt"], ragged=m.bucket)
         go = self._buf(f"mix{mx.idx}.{inner}", self.dtype, mx.w_o.shape[1])[:T]
         ops.ssd_post(o, xbc, 0, proj, mx.off["z"], mx.f["D"], mx.f["norm"], go, T, H, V, sp.norm_groups, self.cfg.norm_eps)
         return ops.linear(mx.w_o, go, y)
@@ -1167,5 +1167,5 @@ class HybridPiece:
                          m.seq_slot, m.n_seqs, H, H, D, V, hparam=mx.f["decay"], tab=tab, rdims=rd, qscale=D ** -0.5)
         else:
             ops.lin_scan(ops.SCAN_RETENTION, proj, mx.off["q"], mx.off["k"], proj, mx.off["v"], st, o, m.q_start, m.q_len, m.kv_len,
-                         m.seq_slot, m.n_seqs, m.max_q, H, H, D, V, z=tab, hparam=mx.f["decay"], qscale=D ** -0.5, rdims=rd)
+                         m.seq_slot, m.n_seqs, m.max_q, H, H, D, V, z=tab, hparam=mx.f["decay"], qscale=D ** -0.5, rdims=rd, ragged=m.bucket)
         return self._scan_out(mx, o, proj, mx.off["g"], ops.POST_SILU, None, m, y)

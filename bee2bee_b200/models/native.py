@@ -85,6 +85,7 @@ class BatchMeta:
     splits: int = 1
     seq_slot: Optional[torch.Tensor] = None   # [S] int32 batch slot of each sequence (per-sequence recurrent state)
     n_out: int = 0                            # rows of logits wanted (0 = one per sequence)
+    bucket: bool = False                      # the sizes are a bucket's: fewer sequences and tokens may be live (q_len says which)
 
 
 class NativePiece:

@@ -602,11 +602,12 @@ def mlstm_gates(proj, off_q, off_k, off_i, off_f, bi, bf, cap, qscale, nstate, m
 
 
 def lin_scan(mode, qk, off_q, off_k, v, off_v, state, out, q_start, q_len, kv_len, seq_slot, n_seqs, max_q, H, G, dk, dv, *,
-             z=None, off_z=0, zbias=None, hparam=None, beta=None, off_b=0, aux=None, qscale=1.0, inv_tau=1.0, rdims=0):
+             z=None, off_z=0, zbias=None, hparam=None, beta=None, off_b=0, aux=None, qscale=1.0, inv_tau=1.0, rdims=0, ragged=False):
     """Gated linear recurrence over the spans (``mode`` = SCAN_*); ``max_q`` = longest span of the batch (1: the decode
-    variant).  SCAN_RETENTION: ``z`` is the rotary table of the step, the first ``rdims`` channels of q and k turn."""
+    variant).  ``ragged``: ``n_seqs`` and ``max_q`` are upper bounds (a bucket of a captured graph, a long span beside short ones), so how the
+    spans are run is decided on the device from ``q_len``.  SCAN_RETENTION: ``z`` is the rotary table of the step, the first ``rdims`` channels of q and k turn."""
     n = native().lin_scan(mode, qk, off_q, off_k, v, off_v, z, off_z, zbias, hparam, beta, off_b, aux, float(qscale),
-                          float(inv_tau), state, out, q_start, q_len, kv_len, seq_slot, n_seqs, max_q, H, G, dk, dv, int(rdims))
+                          float(inv_tau), state, out, q_start, q_len, kv_len, seq_slot, n_seqs, max_q, H, G, dk, dv, int(rdims), bool(ragged))
     LAUNCHES[0] += n - 1       # spans cut into segments: the local pass and the starts are kernels of their own
 
 

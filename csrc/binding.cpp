@@ -692,7 +692,7 @@ int64_t lin_scan(int64_t mode, const Tensor& qk, int64_t off_q, int64_t off_k, c
               int64_t off_z, const OptT& zbias, const OptT& hparam, const OptT& beta, int64_t off_b, const OptT& aux,
               double qscale, double inv_tau, const Tensor& state, const Tensor& out, const Tensor& q_start,
               const Tensor& q_len, const Tensor& kv_len, const Tensor& seq_slot, int64_t n_seqs, int64_t max_q, int64_t H,
-              int64_t G, int64_t dk, int64_t dv, int64_t rdims) {
+              int64_t G, int64_t dk, int64_t dv, int64_t rdims, bool ragged) {
   c10::cuda::CUDAGuard guard(qk.device());
   auto ld = [](const OptT& t) { return (t.has_value() && t->defined()) ? static_cast<int>(t->stride(0)) : 0; };
   TORCH_CHECK(mode == 2   ? fp_or_null(aux) != nullptr
@@ -702,22 +702,23 @@ int64_t lin_scan(int64_t mode, const Tensor& qk, int64_t off_q, int64_t off_k, c
               "lin_scan: missing gate inputs for this mode");
   TORCH_CHECK(mode != 1 || (fp_or_null(hparam) != nullptr && fp_or_null(beta) != nullptr), "lin_scan: delta rule inputs");
   const int iv = static_cast<int>(n_seqs), mq = static_cast<int>(max_q), d = static_cast<int>(dk);
-  const int seg = b2b::lin_span_supported(static_cast<int>(mode), fp(v), static_cast<int>(v.stride(0)), static_cast<int>(off_v), fp(state), fp(out),
-                                          static_cast<int>(out.stride(0)), mq, d, static_cast<int>(dv))
-                      ? b2b::span_plan(iv, mq, static_cast<int>(H), d) : -1;
-  if (seg >= 0) {
+  b2b::SpanLaunch r{false, true, false, 0, 0};
+  if (b2b::lin_span_supported(static_cast<int>(mode), fp(v), static_cast<int>(v.stride(0)), static_cast<int>(off_v), fp(state), fp(out),
+                              static_cast<int>(out.stride(0)), mq, d, static_cast<int>(dv)))
+    r = b2b::span_launch(iv, mq, static_cast<int>(H), d, ragged);
+  if (r.span) {
     Tensor ws;
-    if (seg > 0) ws = torch::empty({n_seqs * ((max_q + seg - 1) / seg) * H * (dk * dv + dk)}, state.options().dtype(at::kFloat));
+    if (r.slots > 0) ws = torch::empty({b2b::span_workspace(r.slots, static_cast<int>(H), d)}, state.options().dtype(at::kFloat));
     check(b2b::launch_lin_span(static_cast<int>(mode), fp(qk), static_cast<int>(qk.stride(0)), static_cast<int>(off_q), static_cast<int>(off_k),
                                fp(v), static_cast<int>(v.stride(0)), static_cast<int>(off_v), fp_or_null(z), ld(z), static_cast<int>(off_z),
                                fp_or_null(zbias), fp_or_null(hparam), fp_or_null(beta), ld(beta), static_cast<int>(off_b), fp_or_null(aux),
                                static_cast<float>(qscale), static_cast<float>(inv_tau), const_cast<float*>(fp(state)),
                                const_cast<float*>(fp(out)), static_cast<int>(out.stride(0)), ip(q_start), ip(q_len), ip(kv_len), ip(seq_slot),
-                               iv, mq, static_cast<int>(H), static_cast<int>(G), d, seg,
-                               seg > 0 ? ws.data_ptr<float>() : nullptr, cur_stream()),
+                               iv, static_cast<int>(H), static_cast<int>(G), d, r, r.slots > 0 ? ws.data_ptr<float>() : nullptr, cur_stream()),
           "lin_span");
-    return seg > 0 ? 3 : 1;
   }
+  const int64_t launched = r.span ? (r.slots > 0 ? 3 : 1) : 0;
+  if (!r.scan) return launched;
   check(b2b::launch_lin_scan(static_cast<int>(mode), fp(qk), static_cast<int>(qk.stride(0)), static_cast<int>(off_q),
                              static_cast<int>(off_k), fp(v), static_cast<int>(v.stride(0)), static_cast<int>(off_v),
                              fp_or_null(z), ld(z), static_cast<int>(off_z), fp_or_null(zbias), fp_or_null(hparam),
@@ -726,9 +727,9 @@ int64_t lin_scan(int64_t mode, const Tensor& qk, int64_t off_q, int64_t off_k, c
                              const_cast<float*>(fp(out)), static_cast<int>(out.stride(0)), ip(q_start), ip(q_len),
                              ip(kv_len), ip(seq_slot), static_cast<int>(n_seqs), static_cast<int>(max_q),
                              static_cast<int>(H), static_cast<int>(G), static_cast<int>(dk), static_cast<int>(dv),
-                             static_cast<int>(rdims), cur_stream()),
+                             static_cast<int>(rdims), r.span && r.scan ? 1 : 0, cur_stream()),
         "lin_scan");
-  return 1;
+  return launched + 1;
 }
 
 void scan_post(const Tensor& o, const Tensor& gate, int64_t off_g, const Tensor& weight, int64_t act, const OptT& aux,
@@ -1069,6 +1070,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mixed_attention_gave_up", &b2b::mixed_attention_gave_up);
   m.def("short_conv", &short_conv);
   m.def("mlstm_gates", &mlstm_gates);
+  m.def("span_plan", [](const std::vector<int>& lens, int n_seqs, int max_q, int H, int dk) {      // (sequences behind `lens` are idle)
+    std::vector<int> all(lens);
+    all.resize(n_seqs, 0);
+    return b2b::span_plan(all.data(), n_seqs, max_q, H, dk);
+  });
   m.def("lin_scan", &lin_scan);
   m.def("scan_post", &scan_post);
   m.def("post_norm_join", &post_norm_join);

@@ -140,20 +140,27 @@ int launch_mlstm_gates(const float* proj, int ld, int off_q, int off_k, int off_
 // lower bound, its complement is the write strength; hparam = the bound [H * dk], z = the gate projection, no keys), 4
 // state-space recurrence (hparam = A_log [H], zbias = bias of the step size [H], beta = its projection), 5 retention (hparam =
 // decay [H], z = rotary table [T, rdims] of (cos, sin) pairs)
-// spans of the modes with a diagonal transition, a whole head per block (lin_span.cu); span_plan: tokens per segment when the spans are
-// cut into segments that run side by side (then `ws` holds n_seqs * segments * H * (dk * dk + dk) floats and three kernels are launched), 0: whole
-// spans, -1: lin_scan is the faster one
+// spans of the modes with a diagonal transition, a whole head per block (lin_span.cu).  SpanLaunch: the kernels of a call -- scan: lin_scan (together with
+// span: choose = 1, one of the two leaves at once), span: launch_lin_span, which runs a pass over whole spans or (slots > 0) three kernels over
+// segments of seg tokens, or of as many as q_len makes best (ragged: the sizes of the call are upper bounds), with span_workspace floats of
+// workspace.  span_plan: what a ragged call does with the lengths `lens` (host): -1 lin_scan, 0 whole spans, else tokens per segment
+struct SpanLaunch {
+  bool span, scan, ragged;
+  int seg, slots;
+};
 bool lin_span_supported(int mode, const float* v, int ld_v, int off_v, const float* state, const float* out, int ld_out, int max_q, int dk, int dv);
-int span_plan(int n_seqs, int max_q, int H, int dk);
+SpanLaunch span_launch(int n_seqs, int max_q, int H, int dk, bool ragged);
+long long span_workspace(int slots, int H, int dk);
+int span_plan(const int* lens, int n_seqs, int max_q, int H, int dk);
 int launch_lin_span(int mode, const float* qk, int ld_qk, int off_q, int off_k, const float* v, int ld_v, int off_v, const float* z, int ld_z,
                     int off_z, const float* zbias, const float* hparam, const float* beta, int ld_b, int off_b, const float* aux, float qscale,
                     float inv_tau, float* state, float* out, int ld_out, const int* q_start, const int* q_len, const int* kv_len,
-                    const int* seq_slot, int n_seqs, int max_q, int H, int G, int dk, int seg, float* ws, cudaStream_t s);
+                    const int* seq_slot, int n_seqs, int H, int G, int dk, const SpanLaunch& r, float* ws, cudaStream_t s);
 int launch_lin_scan(int mode, const float* qk, int ld_qk, int off_q, int off_k, const float* v, int ld_v, int off_v,
                     const float* z, int ld_z, int off_z, const float* zbias, const float* hparam, const float* beta,
                     int ld_b, int off_b, const float* aux, float qscale, float inv_tau, float* state, float* out,
                     int ld_out, const int* q_start, const int* q_len, const int* kv_len, const int* seq_slot, int n_seqs,
-                    int max_q, int H, int G, int dk, int dv, int rdims, cudaStream_t s);
+                    int max_q, int H, int G, int dk, int dv, int rdims, int choose, cudaStream_t s);
 int launch_scan_post(const float* o, int ld_o, const float* gate, int ld_g, int off_g, const float* weight, int wshared,
                      int act, const float* aux, void* out, int ld_out, int T, int H, int dv, float eps, int f32,
                      cudaStream_t s);

@@ -32,6 +32,7 @@
 #include <cstdint>
 
 #include "launch.cuh"
+#include "span_plan.cuh"
 
 namespace b2b {
 namespace {
@@ -1105,6 +1106,7 @@ struct ScanArgs {
   const int* q_start; const int* q_len; const int* kv_len; const int* seq_slot;
   int H, G, dk, dv;
   int rdims;                                      // RET: rotated channels
+  int n_seqs, choose;                             // choose: lin_span.cu is launched, too: leave the spans to it where it is faster
 };
 
 template <int MODE, int R, int LN, bool DEC, int CB>
@@ -1124,6 +1126,7 @@ __global__ void __launch_bounds__(LN* CB / ls_cols(DEC) + (DEC ? 0 : ls_stage_th
   __shared__ __align__(16) float ds[NBUF * TT * DKP];
   __shared__ __align__(16) float vs[NBUF * TT * CB];
   __shared__ float bs[NBUF * TT];
+  if (!DEC && a.choose && span_whole_wins(span_work(a.q_len, a.n_seqs), a.H, a.dk)) return;
   const int s = blockIdx.z, hd = blockIdx.y;
   const int n = a.q_len[s];
   if (n <= 0) return;                               // (block-uniform)
@@ -1712,11 +1715,11 @@ int launch_lin_scan(int mode, const float* qk, int ld_qk, int off_q, int off_k, 
                     const float* z, int ld_z, int off_z, const float* zbias, const float* hparam, const float* beta,
                     int ld_b, int off_b, const float* aux, float qscale, float inv_tau, float* state, float* out,
                     int ld_out, const int* q_start, const int* q_len, const int* kv_len, const int* seq_slot, int n_seqs,
-                    int max_q, int H, int G, int dk, int dv, int rdims, cudaStream_t s) {
+                    int max_q, int H, int G, int dk, int dv, int rdims, int choose, cudaStream_t s) {
   if (n_seqs <= 0) return 0;
   if (G <= 0 || H % G != 0) return -2;
   ScanArgs a{qk, ld_qk, off_q, off_k, v, ld_v, off_v, z, ld_z, off_z, zbias, hparam, beta, ld_b, off_b, aux, qscale,
-             inv_tau, state, out, ld_out, q_start, q_len, kv_len, seq_slot, H, G, dk, dv, rdims};
+             inv_tau, state, out, ld_out, q_start, q_len, kv_len, seq_slot, H, G, dk, dv, rdims, n_seqs, choose};
   if (mode == LS_GLA) return launch_scan_mode<LS_GLA>(a, n_seqs, max_q, s);
   if (mode == LS_DELTA) return launch_scan_mode<LS_DELTA>(a, n_seqs, max_q, s);
   if (mode == LS_MLSTM) return launch_scan_mode<LS_MLSTM>(a, n_seqs, max_q, s);

@@ -14,8 +14,8 @@ device-driven (all ranks enqueue the same plan):
                               for follower ranks) and gathers the new tokens into mapped pinned host memory
 
 All flags are monotonic epochs that are never reset, so no burst needs a host barrier, a flag reset or an
-NCCL broadcast (round 1 paid two barriers + a reset per burst and a broadcast per read-back).
-Replaces the per-hop JSON transport of /root/reference/bee2bee/node.py:249-277.
+NCCL broadcast (two barriers + a reset per burst and a broadcast per read-back otherwise).
+Replaces the per-hop JSON transport of bee2bee/node.py:249-277.
 """
 from __future__ import annotations
 
@@ -566,7 +566,7 @@ class GpuRunner:
         torch.cuda.synchronize(self.device)
 
     def prepare_burst(self) -> None:
-        """Kept for callers of the round-1 API: bursts need no preparation any more (monotonic epochs)."""
+        """Kept for callers of the earlier API: bursts need no preparation any more (monotonic epochs)."""
         self._ensure_graphs()
 
     def decode(self, n_steps: int, prepared: bool = False) -> None:

@@ -56,7 +56,7 @@ logits for the rows named by ``last_idx``.  What is new here and lives next to t
   matrix products and what the KV cache holds (bf16 on the tcgen05 GEMM, or float32 through cuBLAS for bit-faithful runs).
 
 Launches per layer (kepovik): attention 5 (+3 with a feed-forward), delta rule 7.  The reference has no counterpart
-(it delegates every architecture to ``transformers``, /root/reference/bee2bee/hf.py:23-44).
+(it delegates every architecture to ``transformers``, bee2bee/hf.py:23-44).
 """
 from __future__ import annotations
 

@@ -14,7 +14,7 @@ Per decoder layer (Llama / Mistral) exactly five launches, all on one stream:
 and the first GEMM of the next piece acquires that flag after prefetching its weights.
 Gemma-2 adds its post-norms as residual-fused RMSNorm kernels; GPT-2 uses LayerNorm +
 bias/GELU epilogues.  Replaces ``build_distilbert_partial`` + the JSON hidden-state hop
-of the reference (/root/reference/bee2bee/hf.py:180-205, bee2bee/node.py:249-277).
+of the reference (bee2bee/hf.py:180-205, bee2bee/node.py:249-277).
 """
 from __future__ import annotations
 
@@ -284,7 +284,7 @@ class NativePiece:
 
     def streamed_weight_bytes(self) -> int:
         """Bytes a decode step actually streams from this piece's weights: everything except the embedding tables,
-        of which a step only gathers one row per sequence (weight_bytes() overstated the roofline)."""
+        of which a step only gathers one row per sequence (``weight_bytes()`` would overstate the roofline)."""
         skip = {"embed", "pos_embed"}
         n = sum(v.numel() * v.element_size() for k, v in self.w.items() if k not in skip)
         return n + sum(v.numel() * v.element_size() for v in self.wscale.values())

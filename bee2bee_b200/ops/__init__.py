@@ -130,7 +130,7 @@ def pick_bn(m_tok: int) -> int:
     return 256 if m_tok > 512 else 128
 
 
-#: 0 restores the round-2 mid-term rule for under-filled prefill GEMMs (128-wide tiles, deep ring, decode split-K heuristic)
+#: 0 restores an earlier rule for under-filled prefill GEMMs (128-wide tiles, deep ring, decode split-K heuristic)
 PREFILL_SPLITK = os.environ.get("B2B_PREFILL_SPLITK", "1") == "1"
 
 
@@ -168,7 +168,7 @@ def pick_prefill_tile(n_out: int, m_tok: int, k: int = 0):
     return (128 if m_tok <= 512 else 256), 0, 0          # small chunks: not measured, the decode heuristic decides
 
 
-#: L2 weight prefetch: built, measured negative and REMOVED from the kernel in round 2 (profiles/l2_prefetch.md; even
+#: L2 weight prefetch: built, measured negative and REMOVED from the kernel (profiles/l2_prefetch.md; even
 #: switched off its code and parameters cost ~20 us per decode step).  The value is accepted and ignored.
 L2_PREFETCH = 0
 

@@ -1,8 +1,8 @@
 """Model architecture descriptions for the decoder families the mesh serves.
 
 The reference ships no model configs (it defers to ``transformers``,
-bee2bee/hf.py:23-32); these presets are the public architectures named in
-BASELINE.json (distilgpt2, Llama-3-8B, Zephyr-7B-beta = Mistral-7B, gemma-2-2b) plus tiny
+bee2bee/hf.py:23-32); these presets are the public architectures that are
+benchmarked (distilgpt2, Llama-3-8B, Zephyr-7B-beta = Mistral-7B, gemma-2-2b) plus tiny
 variants of each family for tests.  A config can also be read from a Hugging Face
 ``config.json`` (``ModelConfig.from_hf_dict``) so ``serve-hf --model <local dir>`` works.
 """
@@ -1156,7 +1156,7 @@ def piece_units(cfg: "ModelConfig", pieces: int, bounds: Optional[List[int]] = N
     pieces = max(1, min(pieces, cfg.n_layers))
     if pieces == 1 or not supports_half_layer_pieces(cfg):
         return [(UPL * r.start, UPL * r.stop) for r in balanced_split(cfg, pieces)]
-    # stage time model fitted to the measured decode step (profiles/decode_layer_breakdown.md, B200, 32 sequences):
+    # stage time model fitted to the measured decode step (B200, 32 sequences):
     # weight bytes at the measured 6.4 TB/s plus a fixed cost per kernel; the last piece adds the lm_head GEMM and the
     # sampler.  Llama-3-8B: attention block 34.1 us (measured 34.7), gate/up 40.7 (39.4), down 25.3 (24.9), head 201 (211).
     h, f = cfg.hidden_size, cfg.ffn_size

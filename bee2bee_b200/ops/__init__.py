@@ -136,7 +136,7 @@ PREFILL_SPLITK = os.environ.get("B2B_PREFILL_SPLITK", "1") == "1"
 
 def pick_prefill_tile(n_out: int, m_tok: int, k: int = 0):
     """(token tile, ring depth, cluster split-K) of a prefill GEMM (m_tok > 64) on gemm_tc.cu -- e4m3 operands and the bf16 calls
-    that ``use_wide`` leaves --, measured on B200 on the Llama-3-8B shapes (profiles/prefill_gemm.md).  0 = the tile's default depth / let ``pick_splitk`` decide.
+    that ``use_wide`` leaves --, measured on B200 on the Llama-3-8B shapes.  0 = the tile's default depth / let ``pick_splitk`` decide.
 
     * more tiles than SMs: TWO resident CTAs per SM with a shallow ring beat one CTA with a deep ring -- the epilogue of
       one tile (TMEM -> registers -> global) overlaps the main loop of the other (955 vs 787 TFLOP/s over the layer at
@@ -168,7 +168,7 @@ def pick_prefill_tile(n_out: int, m_tok: int, k: int = 0):
     return (128 if m_tok <= 512 else 256), 0, 0          # small chunks: not measured, the decode heuristic decides
 
 
-#: L2 weight prefetch: built, measured negative and REMOVED from the kernel (profiles/l2_prefetch.md; even
+#: L2 weight prefetch: built, measured negative and REMOVED from the kernel (even
 #: switched off its code and parameters cost ~20 us per decode step).  The value is accepted and ignored.
 L2_PREFETCH = 0
 

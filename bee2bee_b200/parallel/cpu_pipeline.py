@@ -1,5 +1,5 @@
 """Layer-piece pipeline over the *control-plane* mesh, for hosts without NVLink (CPU plumbing
-configuration of BASELINE.json: distilgpt2 split in two pieces over the loopback
+configuration: distilgpt2 split in two pieces over the loopback
 ``p2p_runtime``).  This is the generalisation of the reference's orphaned
 ``hf_part_load`` / ``hf_part_forward`` worker tasks (bee2bee/node.py:236-277)
 to decoder LMs with a KV cache:

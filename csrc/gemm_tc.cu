@@ -679,7 +679,7 @@ static int launch_bn_epi(const GemmParams& p, const CUtensorMap& tw, const CUten
 }
 
 // one compact kernel per (token tile, epilogue): a runtime `switch` in the 16x-unrolled epilogue
-// loop made the kernel instruction-fetch bound (5.4 us epilogue, see profiles/gemm_timeline.md)
+// loop made the kernel instruction-fetch bound (5.4 us epilogue)
 template <int BN>
 static int launch_bn(const GemmParams& p, const CUtensorMap& tw, const CUtensorMap& tx, cudaStream_t stream) {
 #define B2B_EPI_CASE(E)                                                                              \

@@ -8,7 +8,7 @@
 // Semantics follow the reference's generation defaults (bee2bee/hf.py:91-105):
 // repetition_penalty 1.15, top_p 0.95, do_sample iff temperature > 0, greedy otherwise.
 //
-// Performance notes (profiles/launches_decode_step.md): every pass over the 128k logits is
+// Performance notes: every pass over the 128k logits is
 // L2-latency bound, so logits are read 8 at a time per thread (2 x 128-bit loads in flight);
 // histogram mass is accumulated in 32.32 fixed point with native 32-bit shared-memory atomics
 // (float / 64-bit shared atomics are CAS loops).
@@ -96,7 +96,7 @@ __device__ __forceinline__ void hist_add(uint32_t* lo, uint32_t* hi, int bin, ui
 }
 
 // One CLUSTER of CS CTAs per sequence (grid = [B, 1, CS]); CTA r owns ids [r*W, (r+1)*W).  A single
-// SM is instruction-bound on a 128k vocabulary (about 28 us per pass, profiles/bench_history.md), so the
+// SM is instruction-bound on a 128k vocabulary (about 28 us per pass), so the
 // vocabulary is spread over CS SMs, each slice is read from L2 exactly once and then lives in shared
 // memory as exp(l - max); the per-level histograms are merged across the cluster through DSMEM.
 __global__ void __launch_bounds__(SAMP_THREADS, 1) sample_kernel(const SampleParams p, const int W) {

@@ -1,4 +1,4 @@
-"""BASELINE.json config 1 in one file: distilgpt2 split into two layer pieces hosted by two mesh
+"""distilgpt2 split into two layer pieces hosted by two mesh
 peers on this machine (CPU), hidden states hop over the loopback p2p runtime, generation through
 the FastAPI `/generate` route."""
 import os

@@ -88,7 +88,7 @@ def test_two_gpu_engine_waves_match_single_gpu():
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs >= 2 GPUs")
 @pytest.mark.parametrize("quant", ["mxfp8", "fp8"])
 def test_two_gpu_fp8_pipeline_matches_single_gpu(quant):
-    """BASELINE config 3 shape: block-scaled (mxfp8) / per-row fp8 pieces across the NVLink handoff, incl. a cut
+    """Block-scaled (mxfp8) / per-row fp8 pieces across the NVLink handoff, incl. a cut
     between a gate/up and a down GEMM, equal the single-GPU fp8 engine token for token."""
     kw = dict(B2B_QUANT=quant, B2B_STEPS="6", B2B_MX_FUSE="0")
     ref = _run(1, "tiny-llama", 2, 4, 0, **kw)

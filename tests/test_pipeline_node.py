@@ -1,4 +1,4 @@
-"""BASELINE.json config 1 -- distilgpt2 split into 2 layer pieces on CPU, hidden states hop over
+"""distilgpt2 split into 2 layer pieces on CPU, hidden states hop over
 the loopback p2p_runtime, /generate on a 16-token synthetic prompt -- plus the legacy
 coordinator/worker protocol (node.py) and the numpy MLP (intent of tests/test_model.py)."""
 import asyncio

@@ -1,4 +1,4 @@
-"""BASELINE config 1, measured: distilgpt2 split into 2 layer pieces hosted by two mesh peers on this machine (CPU),
+"""distilgpt2 split into 2 layer pieces hosted by two mesh peers on this machine (CPU),
 hidden states hop over the loopback WebSocket runtime as binary `hidden_forward` frames, generation through the FastAPI
 `POST /generate` route with a 16-token synthetic prompt.  Prints one JSON line with per-request latency, tokens/s and
 the per-hop payload (the reference ships the same hop as a JSON nested list of fp32, node.py:270-277)."""

@@ -1,4 +1,4 @@
-"""Concurrent multi-client load against the FastAPI sidecar (`POST /generate`), BASELINE config 5:
+"""Concurrent multi-client load against the FastAPI sidecar (`POST /generate`):
 N clients x R requests each, a mix of buffered and streamed generations; reports request latency percentiles,
 time to first streamed chunk, aggregate generated tokens/s (from the engine's own counters, `GET /metrics`) and
 the KV-cache page utilisation sampled while the load runs.

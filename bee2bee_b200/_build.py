@@ -22,7 +22,7 @@ BUILD = ROOT / "build" / "obj"
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 
-CU_SOURCES = ["gemm_tc.cu", "gemm_wide.cu", "elementwise.cu", "attention.cu", "attention_tc.cu", "attn_decode.cu", "sampler.cu", "hybrid.cu", "seqmix.cu", "postnorm.cu",
+CU_SOURCES = ["gemm_tc.cu", "gemm_wide.cu", "elementwise.cu", "attention.cu", "attention_tc.cu", "attn_decode.cu", "layer_chain.cu", "sampler.cu", "hybrid.cu", "seqmix.cu", "postnorm.cu",
               "mixed_attention.cu", "sandwich.cu", "diff_attention.cu",
               "lin_chunk.cu", "lin_span.cu"]
 # translation units whose arithmetic must be exact fp32 (no approximate division / exp / sqrt, no flush to zero)

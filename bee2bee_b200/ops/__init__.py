@@ -434,6 +434,13 @@ def attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, *, 
     return out
 
 
+def layer_chain(plan, x, positions, slots, q_start, q_len, kv_len, block_table):
+    """All layers of a decode step (one new token per sequence, up to 64) in one persistent kernel (csrc/layer_chain.cu); ``plan`` is the
+    piece's ``LayerChain``, which owns the weights' layout and the buffers.  The result is in the plan's ``xa``."""
+    plan.run(x, positions, slots, q_start, q_len, kv_len, block_table)
+    LAUNCHES[0] += 1
+
+
 def attention_fuses_quant(max_q: int, n_q: int, n_kv: int, head_dim: int, splits: int) -> bool:
     """True when ``attention`` will run the tcgen05 kernel without split-KV, i.e. can emit the e4m3 copy itself."""
     g = n_q // max(1, n_kv)

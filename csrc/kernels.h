@@ -45,6 +45,34 @@ unsigned attn_decode_gave_up();
 int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table, const int* q_start,
                        const int* q_len, const int* kv_len, int seqs, int max_pages, int n_tokens, int n_pages, int n_q, int n_kv,
                        int head_dim, int window, float softcap, void* q_out8, void* q_sf, int q_bn, cudaStream_t s);
+// all layers of a piece for one new token per sequence, up to 64 of them, in one persistent kernel (layer_chain.cu)
+struct ChainDims {
+  int hidden, ffn, n_q, n_kv, head_dim, pages;
+  int act_gelu, plus_one, post_norms;
+  float eps, rope_theta, q_scale, softcap;
+};
+struct ChainLayerPtrs {
+  const void *wqkv, *wo, *wgu, *w_down;
+  void *k_cache, *v_cache;
+  const void *post_attn, *post_ffn;      // or null
+  int window;
+};
+struct ChainCall {
+  const void* table;                     // layers x layer_chain_table_bytes(1), filled by layer_chain_fill
+  uint32_t* control;                     // layer_chain_control_words(layers), zero before the first launch; launches that share it are ordered
+  int layers, tokens, seqs, max_tokens, max_pages;
+  const void* x_in;                      // [tokens, hidden]; may be xa
+  void *xa, *xb, *q, *attn, *h, *norm;   // [max_tokens, ..] buffers; the result is in xa
+  const int *positions, *slots, *q_start, *q_len, *kv_len, *block_table;
+};
+bool layer_chain_supported(const ChainDims& d);
+size_t layer_chain_table_bytes(int layers);
+size_t layer_chain_control_words(int layers);
+int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w);
+int layer_chain_init(const ChainDims& d);
+int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s);
+int set_wait_policy_chain(uint32_t* abort_word, unsigned long long limit_ns);
+unsigned layer_chain_gave_up();          // launches whose bounded waits ran out so far, 0 unless there is a bug
 // spans of the hybrid graphs' softmax attention on the prefill kernel of attention_tc.cu (n_pages: pages of the cache)
 bool attention_tc_hybrid_supported(const float* q, const void* k_cache, const void* v_cache, const void* out, int ld_out, int H, int G, int D);
 int launch_attention_tc_hybrid(const float* q, const void* k_cache, const void* v_cache, void* out, int ld_out, const int* block_table,

@@ -1,0 +1,1237 @@
+// Decode steps: all layers of a piece in ONE persistent kernel whose weight stream goes on across the ends of operations.
+//
+// A decode step is a chain of small dependent operations per layer (QKV, attention, O, [norm], gate/up, down, [norm]), each of which streams its
+// weights or cache pages once.  As separate kernels each ends with its slowest block, starts with the latency of a launch and of its first loads, and
+// has only what fits beside the kernel before it on the way.  Here every SM runs one CTA for the whole step, and two producer warps walk the list
+// of weight tiles and cache pages of ALL operations: while an operation waits for the one before it, the next 200 KB per SM (4 us of the HBM
+// stream) land in the ring.
+//
+//   * operations are separated by a counter in global memory that every CTA adds to when its share of the results is stored; one warp per
+//     CTA polls it.  All CTAs are resident (cooperative launch).
+//   * weights are the 128 MMA rows, tokens the columns (16 / 32 / 64), as in gemm_tc.cu.  A cluster of four CTAs shares a run of rows and each takes a
+//     quarter of K (reading all of X in every CTA would double the traffic from L2 at 32 tokens); the partial sums travel to the CTA that finishes a
+//     quarter of the tokens with st.async, which counts its bytes on the receiver's mbarrier, and are added in the order of K.
+//   * attention as in attn_decode.cu (keys as MMA rows); its cache tiles pass through the same ring, so the pages that the new token does not touch
+//     are fetched while the QKV products run.  Few sequences: the CTAs of a cluster share the keys and merge through DSMEM.
+//   * the sums of squares for the next norm are left by the CTAs that write the rows, one number per CTA and token, added in a fixed order.
+//
+// Bound: the HBM stream and, between operations, the chain of last product, exchange, store, counter, poll and first activations (3 to 5 us, of
+// which the ring hides most).  Measured on B200, two Llama-3-8B layers, us (kernels one by one / here): one token behind 700 keys 190.7 / 177.3, 32
+// tokens behind 500 keys 218.9 / 201.0, 64 tokens behind 300 (Mistral-7B shapes) 255 / 224; two Gemma-2-2B layers: one token 124 / 105, 30 tokens 128 /
+// 115.  Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
+// All waits are bounded: one that runs out raises the abort word, every other wait then ends too, and the CTAs leave.
+#include "kernels.h"
+
+#include <cuda.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "activations.cuh"
+#include "common.cuh"
+#include "tmem.cuh"
+
+namespace b2b {
+
+int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, int elt_bytes);
+
+namespace {
+
+constexpr int LC_CL = 4;                           // CTAs of a cluster == parts of K
+constexpr int LC_THREADS = 256;
+constexpr int LC_PAGE = 64, LC_KEYS = 128, LC_HEADS = 16;
+constexpr int LC_BLOCK = 128 * 128;                // 128 rows x 64 bf16: a weight block, or 128 keys x 64 channels
+constexpr int LC_ENTRIES = 16;                     // entries of the ring in flight, at most
+constexpr uint32_t LC_SPINS = 1u << 23;            // polls of a counter (0.3 us or more each)
+constexpr int LC_SS = 64 * 64;
+constexpr float LC_LOG2E = 1.4426950408889634f;
+
+// operations of a layer; the norms are those behind O and down and exist in some models only
+enum LcOp : int { OP_QKV = 0, OP_ATT = 1, OP_O = 2, OP_NORM_A = 3, OP_GU = 4, OP_DOWN = 5, OP_NORM_F = 6, OP_COUNT = 7 };
+constexpr int LC_PRODUCTS = 4;
+__host__ __device__ constexpr int lc_weight(int op) { return op == OP_QKV ? 0 : (op == OP_O ? 1 : (op == OP_GU ? 2 : (op == OP_DOWN ? 3 : -1))); }
+
+// words of the control block in front of the operations' counters
+enum LcWord : int { LW_EXIT = 0, LW_ABORT = 1, LW_CTR = 32 };
+
+__device__ unsigned int g_chain_gave_up = 0;       // launches that ended early since the module was loaded
+
+// what a layer needs and no call changes
+struct alignas(128) LcLayer {
+  CUtensorMap w[4][5];                             // weights of the four products, boxes of 8, 16, .. 128 rows
+  CUtensorMap k, v;                                // cache pages: boxes of 64 keys x 64 channels
+  __nv_bfloat16* k_cache;
+  __nv_bfloat16* v_cache;
+  const __nv_bfloat16* post_attn;                  // weights of the norms behind O and down, or null
+  const __nv_bfloat16* post_ffn;
+  int window;
+};
+
+struct LcMaps {                                    // activations: boxes of 64 channels x the token tile (q: 16 heads)
+  CUtensorMap x_in, xa, xb, attn, h, q;
+};
+
+struct LcParams {
+  const LcLayer* layers;
+  int n_layers, T, seqs, hidden, ffn, n_q, n_kv, parts;
+  int act, plus_one, norms, x_rows;
+  float eps, rope_theta, q_scale, softcap;
+  const __nv_bfloat16* x_in;
+  __nv_bfloat16 *xa, *xb, *q, *attn, *h, *norm;
+  const int *positions, *slots, *q_start, *q_len, *kv_len, *block_table;
+  int max_pages;
+  uint32_t* ctl;
+  float* ss;                                       // [2][clusters][64 tokens] sums of squares
+};
+
+template <int BN>
+struct LcCfg {
+  static constexpr int kRing = BN == 64 ? 191 * 1024 : 208 * 1024;
+  static constexpr int kCols = BN / LC_CL;                         // tokens that a CTA of a cluster finishes
+  static constexpr int kZone = BN * 512 > 16384 ? BN * 512 : 16384;   // partial sums, or Q (8 KB: two of 128 channels or one of 256) and P
+  static constexpr int kSmem = 1024 + kRing + kZone + 512;
+  static constexpr uint32_t kS = 2 * BN, kO = 2 * BN + 2 * LC_HEADS;   // TMEM columns behind the two accumulators
+  static constexpr uint32_t kTmem = BN == 64 ? 256 : 128;
+};
+
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1,%2,%3,%4}, [%5];"
+               ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_release_gpu(uint32_t* p, uint32_t v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void lc_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }     // the epilogue warps
+__device__ __forceinline__ bool lc_vote(bool p) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred a, b;\n\t"
+      "setp.ne.u32 a, %1, 0;\n\t"
+      "barrier.cta.red.or.pred b, 1, 128, a;\n\t"
+      "selp.u32 %0, 1, 0, b;\n\t}\n"
+      : "=r"(r) : "r"(p ? 1u : 0u) : "memory");
+  return r != 0;
+}
+// wait on a barrier that the CTAs of the cluster arrive at
+__device__ __forceinline__ bool lc_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort) {
+  for (uint32_t spins = 0;; ++spins) {
+    if (try_wait_cluster(bar, parity)) return true;
+    if ((spins & 255u) == 255u && *abort != 0u) return false;
+    if (spins > MA_SPIN_LIMIT) {
+      *abort = 1u;
+      return false;
+    }
+  }
+}
+// wait until all CTAs have stored their results of an operation
+__device__ __noinline__ bool lc_wait_op(const uint32_t* ctr, uint32_t target, volatile uint32_t* abort, uint32_t* ctl) {
+  for (uint32_t spins = 0;; ++spins) {
+    if (ld_acquire_gpu(ctr) >= target) return true;
+    if ((spins & 63u) == 63u) {
+      if (*abort != 0u) return false;
+      if (*reinterpret_cast<volatile uint32_t*>(ctl + LW_ABORT) != 0u) { *abort = 1u; return false; }
+    }
+    if (spins > LC_SPINS) {
+      *abort = 1u;
+      return false;
+    }
+  }
+}
+
+// the same through the word that the CTA's polling thread keeps
+__device__ __forceinline__ bool lc_wait_due(const uint32_t* due_s, int n, volatile uint32_t* abort) {
+  for (uint32_t spins = 0;; ++spins) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(due_s)) : "memory");
+    if (static_cast<int>(v) >= n) return true;
+    if ((spins & 255u) == 255u && *abort != 0u) return false;
+    if (spins > (1u << 28)) {                          // (the polling thread gives up long before)
+      *abort = 1u;
+      return false;
+    }
+  }
+}
+
+template <int N>
+__device__ __forceinline__ void lc_ld(uint32_t taddr, float* v) {    // N columns of this thread's lane
+  if constexpr (N == 16) {
+    tmem_ld16(taddr, v);
+  } else {
+    uint32_t r[N];
+#pragma unroll
+    for (int i = 0; i < N; i += 32) ma_ld32(taddr + i, r + i);
+#pragma unroll
+    for (int i = 0; i < N; i += 32) ma_ld_fence(r + i);
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
+  }
+}
+template <int GP>
+__device__ __forceinline__ void lc_ld_heads(uint32_t taddr, float* v) {
+  uint32_t r[GP];
+  if constexpr (GP == 4)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+  else
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < GP; ++i) v[i] = __uint_as_float(r[i]);
+}
+template <int GP>
+__device__ __forceinline__ void lc_st_heads(uint32_t taddr, const float* v) {
+  if constexpr (GP == 4)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])),
+                 "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])) : "memory");
+  else
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(__float_as_uint(v[0])),
+                 "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
+                 "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])) : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// share of a product: units [u0, end) of the weights' rows, 64-channel blocks [kb0, kb0 + nkb) of K.  A unit is 8 rows (gate/up: 8 features).
+// Shares are cut at multiples of 32 rows (gate/up: 64 or 32 features) where that makes the largest share no more than 4 % larger: a tile then takes
+// one or two boxes per block of K.  With shares of single units gate/up needs up to 16, whose issue bound it at 2.3 TB/s.
+struct LcShare {
+  int u0, end, kb0, nkb;
+};
+__device__ LcShare lc_share(const LcParams& p, int op, int head_dim) {
+  LcShare s;
+  const int c = blockIdx.x / LC_CL, nc = gridDim.x / LC_CL, r = blockIdx.x % LC_CL;
+  const int rows = op == OP_QKV ? (p.n_q + 2 * p.n_kv) * head_dim : p.hidden;
+  const int nk = (op == OP_DOWN ? p.ffn : (op == OP_O ? p.n_q * head_dim : p.hidden)) / 64;
+  const int u = (op == OP_GU ? p.ffn : rows) / 8, most = (u + nc - 1) / nc;
+  int g = op == OP_GU ? 8 : 4;
+  while (g > 1 && (u % g != 0 || (u / g + nc - 1) / nc * g * 25 > most * 26)) g /= 2;
+  s.u0 = u / g * c / nc * g;
+  s.end = u / g * (c + 1) / nc * g;
+  s.kb0 = nk * r / LC_CL;
+  s.nkb = nk * (r + 1) / LC_CL - s.kb0;
+  return s;
+}
+// units of the tile that starts at u: up to 128 rows, gate/up tiles do not cross the 64-feature blocks of their rows
+__device__ __forceinline__ int lc_tile(int op, int u, int end) { return min(op == OP_GU ? 8 - (u & 7) : 16, end - u); }
+__device__ __forceinline__ int lc_rows(int op, int n) { return op == OP_GU ? n * 16 : n * 8; }
+
+// The ring holds entries of any size back to back (slots of a fixed size would be half empty in a tile of 64 rows): all roles walk the same list and
+// find the same places.
+template <int BYTES>
+struct LcRing {
+  uint32_t pos = 0, count = 0;
+  __device__ __forceinline__ uint32_t place(uint32_t bytes) {          // of the next entry
+    const uint32_t at = pos + bytes > BYTES ? 0u : pos;
+    pos = at + bytes;
+    return at;
+  }
+  __device__ __forceinline__ uint32_t entry() const { return count % LC_ENTRIES; }
+  __device__ __forceinline__ uint32_t parity() const { return count / LC_ENTRIES & 1u; }
+};
+// who fills the ring: also waits until there is room.  Both filling warps keep their own account (a word that one leaves for the other took a fence
+// per entry: 5 % of a decode step)
+template <int BYTES>
+struct LcFill : LcRing<BYTES> {
+  uint32_t tail = 0, used = 0;                     // the oldest entry in flight, bytes in flight
+  __device__ __forceinline__ bool room(uint32_t bytes, uint32_t& at, uint32_t* sizes, uint64_t* empty, volatile uint32_t* abort) {
+    const uint32_t before = this->pos;
+    at = this->place(bytes);
+    const uint32_t taken = at == before ? bytes : BYTES - before + bytes;
+#pragma unroll 1
+    while (used + taken > BYTES || this->count - tail >= LC_ENTRIES) {
+      if (!ma_wait(&empty[tail % LC_ENTRIES], tail / LC_ENTRIES & 1u, abort)) return false;
+      used -= sizes[tail % LC_ENTRIES];
+      ++tail;
+    }
+    used += taken;
+    sizes[this->entry()] = taken;
+    return true;
+  }
+};
+// weights of a tile per block of K: gate/up tiles of fewer than 64 features have their up rows at row 64 all the same
+__device__ __forceinline__ uint32_t lc_block_bytes(int op, int n) { return (op == OP_GU ? 8u + n : n) * 1024u; }
+
+// one (sequence, key/value head): this CTA's share of its key tiles
+struct LcItem {
+  int seq, kvh, kvlen, kv_lo, t0, nt;
+  bool active;
+};
+__device__ __forceinline__ LcItem lc_item(const LcParams& p, const int* kvlen_s, int window, int j, int part) {
+  LcItem it;
+  it.seq = j / p.n_kv;
+  it.kvh = j - it.seq * p.n_kv;
+  it.kvlen = kvlen_s[it.seq];                      // 0: the sequence takes no part
+  it.active = it.kvlen > 0;
+  it.kv_lo = window > 0 ? max(0, it.kvlen - window) : 0;
+  int lo = it.kv_lo / LC_KEYS, hi = it.active ? (it.kvlen + LC_KEYS - 1) / LC_KEYS : lo;
+  if (p.parts > 1) {
+    const int per = (hi - lo + p.parts - 1) / p.parts;
+    lo = min(hi, lo + part * per);
+    hi = min(hi, lo + per);
+  }
+  it.t0 = lo;
+  it.nt = hi - lo;
+  return it;
+}
+
+// D: channels of a head, GP: query heads of a key/value head rounded up to 4 or 8
+template <int BN, int D, int GP>
+__global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid_constant__ LcMaps maps, const LcParams p) {
+  using Cfg = LcCfg<BN>;
+  constexpr int CW = Cfg::kCols, DB = D / 64, MB = D / 128, NQ = 2 / MB;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* zone = smem + Cfg::kRing;          // partial sums of the cluster | up and gate halves | Q and P of the attention
+  uint64_t* full = reinterpret_cast<uint64_t*>(zone + Cfg::kZone);   // [LC_ENTRIES]
+  uint64_t* empty = full + LC_ENTRIES;             // [LC_ENTRIES]
+  uint64_t* acc_full = empty + LC_ENTRIES;                 // [2]
+  uint64_t* acc_empty = acc_full + 2;              // [2]
+  uint64_t* zone_full = acc_empty + 2;
+  uint64_t* zone_free = zone_full + 1;
+  uint64_t* q_full = zone_free + 1;                // [2]
+  uint64_t* q_empty = q_full + 2;                  // [2]
+  uint64_t* s_full = q_empty + 2;                  // [2]
+  uint64_t* p_ready = s_full + 2;                  // [2]
+  uint64_t* pv_done = p_ready + 2;                 // [2]
+  uint64_t* o_empty = pv_done + 2;
+  uint64_t* part_full = o_empty + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(part_full + 1);
+  volatile uint32_t* abort = tmem_slot + 1;
+  uint32_t* due_s = tmem_slot + 2;                 // operations whose results are complete, as the activation warp has seen it
+  __shared__ float rstd_s[CW];
+  __shared__ int pos_s[CW], slot_s[CW], kvlen_s[BN], q_start_s[BN];
+  __shared__ float red_s[4][GP];             // per warp: maxima
+  __shared__ float sq_s[4][CW > GP ? CW : GP];     // per warp: sums of squares, or of a row's weights
+  __shared__ float ml_s[2 * GP];             // this CTA's maxima and sums, read by the cluster
+  __shared__ LcShare share_s[LC_PRODUCTS];
+  __shared__ uint32_t entry_s[3][LC_ENTRIES];      // bytes of the ring's entries, with what was skipped in front of them
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_ctarank());
+  const uint32_t ctas = gridDim.x;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < LC_ENTRIES; ++i) {
+      mbar_init(&full[i], 3);                      // the two halves of the weights (or pages), the activations
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], 4);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_ready[i], 4);
+      mbar_init(&pv_done[i], 1);
+    }
+    mbar_init(zone_full, 1);
+    mbar_init(zone_free, 4 * LC_CL);
+    mbar_init(o_empty, 4);
+    mbar_init(part_full, static_cast<uint32_t>(p.parts));
+    *abort = 0u;
+    *due_s = 0u;
+    fence_barrier_init();
+  }
+  if (warp == 2)
+    for (int op = lane; op < OP_COUNT; op += 32)
+      if (lc_weight(op) >= 0) share_s[lc_weight(op)] = lc_share(p, op, D);
+  if (warp > 2)
+    for (int i = threadIdx.x - 96; i < p.seqs; i += LC_THREADS - 96) {
+      kvlen_s[i] = p.q_len[i] > 0 ? max(p.kv_len[i], 0) : 0;
+      q_start_s[i] = p.q_start[i];
+    }
+  if (warp == 1) tmem_alloc<Cfg::kTmem>(tmem_slot);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  cluster_arrive_release();
+  cluster_wait_acquire();
+  const uint32_t tmem = *tmem_slot;
+  const int G = p.n_q / p.n_kv;
+  const bool norms = p.norms != 0;
+  uint32_t* const ctr = p.ctl + LW_CTR;
+  const int item0 = blockIdx.x / p.parts, part = blockIdx.x % p.parts, item_step = gridDim.x / p.parts, items = p.seqs * p.n_kv;
+  const uint32_t x_bytes = static_cast<uint32_t>(p.x_rows) * 128u;     // activations of an entry per block of K
+  auto skip = [&](int op) { return !norms && (op == OP_NORM_A || op == OP_NORM_F); };
+  // (every role walks the operations in loops whose bodies appear once: a kernel of 250 KB of code spent microseconds per operation on
+  // fetching its instructions)
+
+  if (warp == 0 || warp == 7) {
+    // ------------------------------------------------------------------------- weights and cache pages, in the order of their use
+    // Two warps, each for one of the two blocks of an entry: the copies of one warp follow one another at 56 GB/s (16 KB boxes; 41 GB/s with 4 KB
+    // boxes), however many are asked for, and an SM that is late then cannot use what the others leave of the stream.
+    if (elect_one()) {
+      const int half = warp == 7;
+      uint32_t* sizes = entry_s[half];
+      const uint64_t pol = l2_policy_evict_first();
+      LcFill<Cfg::kRing> ring;
+      uint32_t place = 0;
+      bool ok = true;
+      int at = 0;                                    // operations so far, over the layers
+#pragma unroll 1
+      for (int l = 0; ok && l < p.n_layers; ++l) {
+        const LcLayer* L = p.layers + l;
+        const int window = L->window;
+        if (half && l + 1 < p.n_layers) {            // descriptors of the next layer
+#pragma unroll 1
+          for (int i = 0; i < 22; ++i) tma_prefetch_desc(&(L + 1)->w[0][0] + i);
+        }
+#pragma unroll 1
+        for (int op = 0; ok && op < OP_COUNT; ++op) {
+          if (skip(op)) continue;
+          ++at;
+          if (lc_weight(op) >= 0) {
+            const LcShare sh = share_s[lc_weight(op)];
+            const CUtensorMap* maps_w = L->w[lc_weight(op)];
+#pragma unroll 1
+            for (int u = sh.u0, n; ok && u < sh.end; u += n) {
+              n = lc_tile(op, u, sh.end);
+              // up to five boxes per block: rows of gate/up come in blocks of [64 gate | 64 up]: gate to rows 0.., up to rows 64.. of the tile
+              const bool halves = op == OP_GU && n < 8;
+              const int units = (op == OP_GU && !halves) ? 16 : n;
+              const int row0 = op == OP_GU ? (u >> 3) * 128 + (u & 7) * 8 : u * 8;
+              const uint32_t bytes = static_cast<uint32_t>(lc_rows(op, n)) * 128u, block = lc_block_bytes(op, n);
+#pragma unroll 1
+              for (int kb = 0; kb < sh.nkb; kb += 2) {
+                const int nb = min(2, sh.nkb - kb);
+                if (!(ok = ring.room((block + x_bytes) * nb, place, sizes, empty, abort))) break;
+                uint8_t* base = smem + place;
+                uint64_t* bar = &full[ring.entry()];
+                ++ring.count;
+                if (half >= nb) {
+                  mbar_arrive(bar);
+                  continue;
+                }
+                mbar_arrive_expect_tx(bar, bytes);
+                const int k = (sh.kb0 + kb + half) * 64;
+                uint8_t* dst = base + half * block;
+                if (units == 16) {
+                  tma_load_2d_hint(dst, maps_w + 4, bar, k, row0, pol);
+                  continue;
+                }
+                int row = row0;
+#pragma unroll 1
+                for (int i = 3; i >= 0; --i) {
+                  if (!(units >> i & 1)) continue;
+                  tma_load_2d_hint(dst, maps_w + i, bar, k, row, pol);
+                  if (halves) tma_load_2d_hint(dst + 64 * 128, maps_w + i, bar, k, row + 64, pol);
+                  dst += 1024 << i;
+                  row += 8 << i;
+                }
+              }
+            }
+          } else if (op == OP_ATT) {
+            bool appended = false;                   // the rows of the new tokens are in the cache
+            auto pages = [&](const LcItem& it, int n) {          // of a tile
+              const int page = 2 * (it.t0 + n), *bt = p.block_table + static_cast<size_t>(it.seq) * p.max_pages;
+              if (n >= it.nt) return make_int2(0, 0);
+              return make_int2(bt[page], bt[(page + 1) * LC_PAGE < it.kvlen ? page + 1 : page]);   // (past the end: any keys, they are masked)
+            };
+#pragma unroll 1
+            for (int j = item0; ok && j < items; j += item_step) {
+              const LcItem it = lc_item(p, kvlen_s, window, j, part);
+              int2 pg = pages(it, 0), pg1 = pages(it, 1);        // fetched ahead of their use
+              // K0, K1, V0, K2, V1, ..
+#pragma unroll 1
+              for (int i = 0; ok && i < 2 * it.nt; ++i) {
+                const bool values = i == 2 * it.nt - 1 || (i > 0 && (i & 1) == 0);
+                const int n = i == 0 ? 0 : (values ? (i - 1) >> 1 : (i + 1) >> 1);
+                const int2 where = values || i == 0 ? pg : pg1;
+                if ((2 * (it.t0 + n) + 2) * LC_PAGE >= it.kvlen && !appended) {                  // the tile with the new token's row
+                  if (!(ok = lc_wait_due(due_s, at - 1, abort))) break;
+                  fence_proxy_async_all();
+                  appended = true;
+                }
+#pragma unroll 1
+                for (int h = 0; h < MB; ++h) {       // 128 channels per slot
+                  if (!(ok = ring.room(2 * LC_BLOCK, place, sizes, empty, abort))) break;
+                  uint8_t* base = smem + place;
+                  uint64_t* bar = &full[ring.entry()];
+                  ++ring.count;
+                  mbar_arrive_expect_tx(bar, LC_BLOCK);
+                  if (half == 0) mbar_arrive(bar);   // (no activations)
+                  uint8_t* dst = base + half * LC_BLOCK;
+                  const CUtensorMap* m = values ? &L->v : &L->k;
+                  tma_load_2d(dst, m, bar, it.kvh * D + h * 128 + half * 64, where.x * LC_PAGE);
+                  tma_load_2d(dst + LC_PAGE * 128, m, bar, it.kvh * D + h * 128 + half * 64, where.y * LC_PAGE);
+                }
+                if (values) {
+                  pg = pg1;
+                  pg1 = pages(it, n + 2);
+                }
+              }
+            }
+          }
+        }
+      }
+    }
+  } else if (warp == 6) {
+    // --------------------------------------------------------------------------- activations, as soon as they are complete
+    if (elect_one()) {
+      const uint64_t pol = l2_policy_evict_last();
+      LcFill<Cfg::kRing> ring;
+      uint32_t nq = 0, place = 0;
+      bool ok = true;
+      int at = 0;
+#pragma unroll 1
+      for (int l = 0; ok && l < p.n_layers; ++l) {
+        const int window = p.layers[l].window;
+#pragma unroll 1
+        for (int op = 0; ok && op < OP_COUNT; ++op) {
+          if (skip(op)) continue;
+          if (at > 0) {                              // the operations so far are complete: this thread alone polls, the others of the CTA look at due_s
+            if (!(ok = lc_wait_op(ctr + at - 1, ctas, abort, p.ctl))) break;
+            asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(due_s)), "r"(at) : "memory");
+            fence_proxy_async_all();
+          }
+          ++at;
+          if (lc_weight(op) >= 0) {
+            const LcShare sh = share_s[lc_weight(op)];
+            const CUtensorMap* m = op == OP_QKV ? (l == 0 ? &maps.x_in : &maps.xa) : (op == OP_O ? &maps.attn : (op == OP_GU ? &maps.xb : &maps.h));
+#pragma unroll 1
+            for (int u = sh.u0, n; ok && u < sh.end; u += n) {
+              n = lc_tile(op, u, sh.end);
+              const uint32_t block = lc_block_bytes(op, n);
+#pragma unroll 1
+              for (int kb = 0; kb < sh.nkb; kb += 2) {
+                const int nb = min(2, sh.nkb - kb);
+                if (!(ok = ring.room((block + x_bytes) * nb, place, entry_s[2], empty, abort))) break;
+                uint8_t* base = smem + place + block * nb;
+                uint64_t* bar = &full[ring.entry()];
+                ++ring.count;
+                mbar_arrive_expect_tx(bar, x_bytes * nb);
+#pragma unroll 1
+                for (int b = 0; b < nb; ++b) tma_load_2d_hint(base + b * x_bytes, m, bar, (sh.kb0 + kb + b) * 64, 0, pol);
+              }
+            }
+          } else if (op == OP_ATT) {
+#pragma unroll 1
+            for (int j = item0; ok && j < items; j += item_step) {
+              const LcItem it = lc_item(p, kvlen_s, window, j, part);
+              if (it.nt <= 0) continue;
+              const uint32_t b = nq % NQ;
+              if (!(ok = ma_wait(&q_empty[b], ((nq / NQ) & 1u) ^ 1u, abort))) break;
+              ++nq;
+              mbar_arrive_expect_tx(&q_full[b], LC_HEADS * D * 2);
+#pragma unroll
+              for (int c = 0; c < DB; ++c)
+                tma_load_2d(zone + b * (LC_HEADS * D * 2) + c * (LC_HEADS * 128), &maps.q, &q_full[b], c * 64, q_start_s[it.seq] * p.n_q + it.kvh * G);
+#pragma unroll 1
+              for (int i = 0; ok && i < 2 * it.nt * MB; ++i, ++ring.count) ok = ring.room(2 * LC_BLOCK, place, entry_s[2], empty, abort);
+            }
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // -------------------------------------------------------------------------------------------------------- MMA issuer
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(128, BN);
+      constexpr uint32_t idesc_s = make_idesc_bf16(LC_KEYS, LC_HEADS);
+      constexpr uint32_t idesc_o = make_idesc_bf16(128, LC_HEADS) | (1u << 15);              // A (V) has its rows contiguous
+      const uint64_t desc0 = make_sw128_kmajor_desc(smem_u32(smem));         // + offset / 16 (a single thread issues: every instruction counts)
+      LcRing<Cfg::kRing> ring;
+      uint32_t na = 0, ns = 0, np = 0, nq = 0, no = 0;       // accumulators, score tiles, value tiles, items so far
+      bool ok = true;
+#pragma unroll 1
+      for (int l = 0; ok && l < p.n_layers; ++l) {
+        const int window = p.layers[l].window;
+#pragma unroll 1
+        for (int op = 0; ok && op < OP_COUNT; ++op) {
+          if (lc_weight(op) >= 0) {
+            const LcShare sh = share_s[lc_weight(op)];
+#pragma unroll 1
+            for (int u = sh.u0, n; ok && u < sh.end; u += n, ++na) {
+              n = lc_tile(op, u, sh.end);
+              const uint32_t block = lc_block_bytes(op, n);
+              if (!(ok = ma_wait(&acc_empty[na & 1u], ((na >> 1) & 1u) ^ 1u, abort))) break;
+              tc_fence_after();
+              const uint32_t acc = tmem + (na & 1u) * BN;
+              uint32_t more = 0u;
+#pragma unroll 1
+              for (int kb = 0; kb < sh.nkb; kb += 2) {
+                const uint32_t nb = min(2, sh.nkb - kb);
+                // (rows that the tile does not have are read from what lies behind it, and not used)
+                uint64_t a = desc0 + (ring.place((block + x_bytes) * nb) >> 4), x = a + (block * nb >> 4);
+                if (!(ok = ma_wait(&full[ring.entry()], ring.parity(), abort))) break;
+                tc_fence_after();
+                umma_bf16(acc, a, x, idesc, more);
+                umma_bf16(acc, a + 2, x + 2, idesc, 1u);
+                umma_bf16(acc, a + 4, x + 4, idesc, 1u);
+                umma_bf16(acc, a + 6, x + 6, idesc, 1u);
+                if (nb == 2) {
+                  a += block >> 4;
+                  x += x_bytes >> 4;
+                  umma_bf16(acc, a, x, idesc, 1u);
+                  umma_bf16(acc, a + 2, x + 2, idesc, 1u);
+                  umma_bf16(acc, a + 4, x + 4, idesc, 1u);
+                  umma_bf16(acc, a + 6, x + 6, idesc, 1u);
+                }
+                umma_commit(&empty[ring.entry()]);
+                ++ring.count;
+                more = 1u;
+              }
+              umma_commit(&acc_full[na & 1u]);
+            }
+          } else if (op == OP_ATT) {
+#pragma unroll 1
+            for (int j = item0; ok && j < items; j += item_step) {
+              const LcItem it = lc_item(p, kvlen_s, window, j, part);
+              if (it.nt <= 0) continue;
+              const uint32_t qb = nq % NQ;
+              if (!(ok = ma_wait(&q_full[qb], (nq / NQ) & 1u, abort))) break;
+              ++nq;
+              // S(0), S(1), PV(0), S(2), PV(1), ..: scores run while the softmax warps work on the tile before
+#pragma unroll 1
+              for (int i = 0; ok && i < 2 * it.nt; ++i) {
+                const bool values = i == 2 * it.nt - 1 || (i > 0 && (i & 1) == 0);
+                if (!values) {
+#pragma unroll 1
+                  for (int h = 0; h < MB; ++h) {
+                    const uint32_t base = smem_u32(smem) + ring.place(2 * LC_BLOCK);
+                    if (!(ok = ma_wait(&full[ring.entry()], ring.parity(), abort))) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int kk = 0; kk < 8; ++kk) {
+                      const uint64_t a = make_sw128_kmajor_desc(base + (kk / 4) * LC_BLOCK) + static_cast<uint64_t>((kk % 4) * 2);
+                      const uint64_t b = make_sw128_kmajor_desc(smem_u32(zone + qb * (LC_HEADS * D * 2) + (h * 2 + kk / 4) * (LC_HEADS * 128))) + static_cast<uint64_t>((kk % 4) * 2);
+                      umma_bf16(tmem + Cfg::kS + (ns & 1u) * LC_HEADS, a, b, idesc_s, (h > 0 || kk > 0) ? 1u : 0u);
+                    }
+                    umma_commit(&empty[ring.entry()]);
+                    ++ring.count;
+                  }
+                  umma_commit(&s_full[ns & 1u]);
+                  ++ns;
+                  if (i == max(0, 2 * it.nt - 3)) umma_commit(&q_empty[qb]);                 // the last scores: the queries have been read
+                } else {
+                  const bool first = i == (it.nt > 1 ? 2 : 1);
+                  if (first && !(ok = ma_wait(o_empty, (no & 1u) ^ 1u, abort))) break;
+                  if (!(ok = ma_wait(&p_ready[np & 1u], (np >> 1) & 1u, abort))) break;
+#pragma unroll 1
+                  for (int m = 0; m < MB; ++m) {
+                    const uint32_t base = smem_u32(smem) + ring.place(2 * LC_BLOCK);
+                    if (!(ok = ma_wait(&full[ring.entry()], ring.parity(), abort))) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int kk = 0; kk < LC_KEYS / 16; ++kk) {
+                      const uint64_t a = ma_value_desc(base + kk * (16 * 128));
+                      const uint64_t b = make_sw128_kmajor_desc(smem_u32(zone + 8192 + (np & 1u) * 4096 + (kk / 4) * (LC_HEADS * 128))) + static_cast<uint64_t>((kk % 4) * 2);
+                      umma_bf16(tmem + Cfg::kO + m * LC_HEADS, a, b, idesc_o, (!first || kk > 0) ? 1u : 0u);
+                    }
+                    umma_commit(&empty[ring.entry()]);
+                    ++ring.count;
+                  }
+                  umma_commit(&pv_done[np & 1u]);
+                  ++np;
+                }
+              }
+              ++no;
+            }
+          }
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------------------------------------ epilogues and softmax
+    // (a wait that gave up ends the others through the abort word; the loops go on, because every warp has to meet the others)
+    const int et = threadIdx.x - 64, q4 = warp & 3, row = q4 * 32 + lane;
+    const int col0 = rank * CW;                        // the tokens that this CTA finishes
+    const uint32_t lanes = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
+    const int q_dim = p.n_q * D, kv_dim = p.n_kv * D;
+    const float inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f, log_theta = p.rope_theta > 0.f ? log2f(p.rope_theta) : 0.f;
+    uint32_t na = 0, nx = 0, nt_all = 0, nparts = 0;   // accumulators, exchanges, key tiles, merges so far
+    int at = 0;                                        // operations so far, over the layers
+    bool ok = true;
+#pragma unroll 1
+    for (int l = 0; l < p.n_layers; ++l) {
+      const LcLayer* L = p.layers + l;
+      const __nv_bfloat16* x = l == 0 ? p.x_in : p.xa;
+      const int window = L->window;                    // (read here, ahead of their use)
+      __nv_bfloat16 *const k_cache = L->k_cache, *const v_cache = L->v_cache;
+#pragma unroll 1
+      for (int op = 0; op < OP_COUNT; ++op) {
+        if (skip(op)) continue;
+        if (lc_weight(op) >= 0) {
+          // ----------------------------------------------------------------------------------------------------- products
+          const LcShare sh = share_s[lc_weight(op)];
+          const bool work = sh.u0 < sh.end;
+          // O and down: + residual, unless a norm follows; then the sums of squares of the rows are left for the norm in the next product
+          const __nv_bfloat16* residual = norms ? nullptr : (op == OP_O ? x : p.xb);
+          __nv_bfloat16* out = norms ? p.norm : (op == OP_O ? p.xb : p.xa);
+          float sq[CW];
+#pragma unroll
+          for (int i = 0; i < CW; ++i) sq[i] = 0.f;
+          if (ok) ok = __all_sync(0xffffffffu, lc_wait_due(due_s, at, abort));
+          if (work && op == OP_QKV && et < CW) {
+            const int t = col0 + et;
+            pos_s[et] = (p.positions != nullptr && t < p.T) ? p.positions[t] : 0;
+            slot_s[et] = t < p.T ? p.slots[t] : -1;
+          }
+          if (work && op == OP_QKV && l == 0) {        // 1/rms of the rows: a warp per row
+            const int k8 = p.hidden / 8;
+#pragma unroll 1
+            for (int t = warp - 2; t < CW; t += 4) {
+              float ss = 0.f;
+              const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(min(col0 + t, p.T - 1)) * p.hidden);
+#pragma unroll 8
+              for (int i = lane; i < k8; i += 32) {
+                const uint4 v = src[i];
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float2 f = __bfloat1622float2(h[e]);
+                  ss += f.x * f.x + f.y * f.y;
+                }
+              }
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+              if (lane == 0) rstd_s[t] = rsqrtf(ss / static_cast<float>(p.hidden) + p.eps);
+            }
+          } else if (work && (op == OP_QKV || op == OP_GU)) {      // the same from the sums of squares left by those who wrote the rows
+            constexpr int TPT = 128 / CW;              // threads per token
+            const float* from = p.ss + (op == OP_GU ? LC_SS : 0) + col0 + et / TPT;
+            const int n = norms ? 1 : static_cast<int>(ctas) / LC_CL;
+            float a = 0.f;
+#pragma unroll 4
+            for (int i = et % TPT; i < n; i += TPT) a += __ldcg(from + i * 64);
+#pragma unroll
+            for (int o = TPT / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+            if (et % TPT == 0) rstd_s[et / TPT] = rsqrtf(a / static_cast<float>(p.hidden) + p.eps);
+          }
+          lc_sync();
+#pragma unroll 1
+          for (int u = sh.u0, n; u < sh.end; u += n) {
+            n = lc_tile(op, u, sh.end);
+            const int feat = u * 8 + row;
+            const bool live = op == OP_GU ? (row & 63) < n * 8 : row < n * 8;
+            const int sect = feat < q_dim ? 0 : (feat < q_dim + kv_dim ? 1 : 2);                  // (of QKV)
+            const int fs = feat - (sect == 0 ? 0 : (sect == 1 ? q_dim : q_dim + kv_dim));
+            const bool turn = sect < 2 && p.rope_theta > 0.f;
+            float c1[CW], c2[CW];                      // cosines and sines | residual
+            if (op == OP_QKV) {
+              const float freq = turn ? exp2f(-(2.f * ((fs % D) >> 1) / static_cast<float>(D)) * log_theta) : 0.f;
+#pragma unroll
+              for (int i = 0; i < CW; ++i) {
+                c1[i] = 1.f;
+                c2[i] = 0.f;
+                if (turn && col0 + i < p.T) sincosf(static_cast<float>(pos_s[i]) * freq, &c2[i], &c1[i]);
+              }
+            } else if (op != OP_GU) {
+#pragma unroll
+              for (int i = 0; i < CW; ++i)
+                c1[i] = (residual != nullptr && live && col0 + i < p.T) ? __bfloat162float(residual[static_cast<size_t>(col0 + i) * p.hidden + feat]) : 0.f;
+            }
+            if (ok) ok = __all_sync(0xffffffffu, ma_wait(&acc_full[na & 1u], (na >> 1) & 1u, abort));
+            tc_fence_after();
+            // partial sums of this CTA's quarter of K to the CTAs that finish the tokens; v = sums of this CTA's tokens, in the order of K
+            float v[CW];
+            {
+              float a[BN];
+              lc_ld<BN>(lanes + (na & 1u) * BN, a);
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&acc_empty[na & 1u]);
+              ++na;
+              if (nx > 0 && ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(zone_free, (nx - 1) & 1u, abort));
+              if (threadIdx.x == 64) mbar_arrive_expect_tx(zone_full, static_cast<uint32_t>(lc_rows(op, n) * LC_CL * CW * 4));
+              if (live && ok) {
+#pragma unroll
+                for (int d = 0; d < LC_CL; ++d) {
+                  const uint32_t to = mapa_smem(smem_u32(zone), d) + static_cast<uint32_t>((rank * (CW / 4) * 128 + row) * 16);
+                  const uint32_t bar = mapa_smem(smem_u32(zone_full), d);
+#pragma unroll
+                  for (int i = 0; i < CW / 4; ++i)
+                    st_async_v4(to + i * 2048, bar, a[d * CW + 4 * i], a[d * CW + 4 * i + 1], a[d * CW + 4 * i + 2], a[d * CW + 4 * i + 3]);
+                }
+              }
+              if (ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(zone_full, nx & 1u, abort));
+              ++nx;
+#pragma unroll
+              for (int i = 0; i < CW; ++i) v[i] = 0.f;
+#pragma unroll
+              for (int r = 0; r < LC_CL; ++r)
+#pragma unroll
+                for (int i = 0; i < CW / 4; ++i) {
+                  const float4 f = *reinterpret_cast<const float4*>(zone + ((r * (CW / 4) + i) * 128 + row) * 16);
+                  v[4 * i] += f.x; v[4 * i + 1] += f.y; v[4 * i + 2] += f.z; v[4 * i + 3] += f.w;
+                }
+            }
+            constexpr int HB = CW / 2;
+            const bool up = row >= 64;                 // gate/up: the up half finishes the second half of the tokens, the gate half the first
+            if (op == OP_GU) {
+              float* xch = reinterpret_cast<float*>(zone);         // [HB tokens][64] up values of the first half, then gate values of the second
+              lc_sync();                               // the sums have been read
+              float* to = xch + (up ? 0 : HB * 64) + (row & 63);
+#pragma unroll
+              for (int i = 0; i < HB; ++i) to[i * 64] = up ? v[i] : v[HB + i];
+              lc_sync();
+              const float* from = xch + (up ? HB * 64 : 0) + (row & 63);
+#pragma unroll
+              for (int i = 0; i < HB; ++i) c1[i] = from[i * 64];
+            }
+            __syncwarp();
+            if (lane < LC_CL) arrive_cluster(mapa_smem(smem_u32(zone_free), lane));               // the sums have been read
+            if (op == OP_GU) {
+              const int t0 = up ? HB : 0;
+#pragma unroll
+              for (int i = 0; i < HB; ++i) {
+                if (col0 + t0 + i >= p.T || !live || !ok) break;
+                const float rs = rstd_s[t0 + i], theirs = c1[i] * rs, mine = (up ? v[HB + i] : v[i]) * rs;
+                const float g = up ? theirs : mine, w = up ? mine : theirs;
+                p.h[static_cast<size_t>(col0 + t0 + i) * p.ffn + u * 8 + (row & 63)] = __float2bfloat16_rn((p.act ? gelu_tanh(g) : silu(g)) * w);
+              }
+            } else if (op == OP_QKV) {
+#pragma unroll
+              for (int i = 0; i < CW; ++i) {
+                const int tok = col0 + i;
+                if (tok >= p.T) break;                 // (the same for the warp)
+                const float a = v[i] * rstd_s[i];
+                // lanes (2j, 2j + 1) hold (x_j, x_{j + D / 2}) thanks to the row order of the weights
+                const float b = __shfl_xor_sync(0xffffffffu, a, 1);
+                const float o = turn ? ((lane & 1) ? (a * c1[i] + b * c2[i]) : (a * c1[i] - b * c2[i])) : a;
+                if (!live || !ok) continue;
+                if (sect == 0) {
+                  p.q[static_cast<size_t>(tok) * q_dim + fs] = __float2bfloat16_rn(o * p.q_scale);
+                } else if (slot_s[i] >= 0) {
+                  (sect == 1 ? k_cache : v_cache)[static_cast<size_t>(slot_s[i]) * kv_dim + fs] = __float2bfloat16_rn(o);
+                }
+              }
+            } else if (live && ok) {
+#pragma unroll
+              for (int i = 0; i < CW; ++i) {
+                if (col0 + i >= p.T) break;
+                const __nv_bfloat16 r = __float2bfloat16_rn(v[i] + c1[i]);
+                out[static_cast<size_t>(col0 + i) * p.hidden + feat] = r;
+                sq[i] += __bfloat162float(r) * __bfloat162float(r);
+              }
+            }
+          }
+          if (!norms && (op == OP_O || op == OP_DOWN)) {
+#pragma unroll
+            for (int i = 0; i < CW; ++i) {
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+              if (lane == 0) sq_s[q4][i] = sq[i];
+            }
+            lc_sync();
+            if (et < CW) p.ss[(op == OP_O ? LC_SS : 0) + blockIdx.x / LC_CL * 64 + col0 + et] = sq_s[0][et] + sq_s[1][et] + sq_s[2][et] + sq_s[3][et];
+          }
+        } else if (op == OP_ATT) {
+          // ---------------------------------------------------------------------------------------------------- attention
+#pragma unroll 1
+          for (int j = item0; j < items; j += item_step) {
+            const LcItem it = lc_item(p, kvlen_s, window, j, part);
+            if (!it.active) continue;                  // (the same for the CTAs that share its keys)
+            float m_ref[GP], lsum[GP];
+#pragma unroll
+            for (int g = 0; g < GP; ++g) {
+              m_ref[g] = -INFINITY;
+              lsum[g] = 0.f;
+            }
+#pragma unroll 1
+            for (int n = 0; n < it.nt; ++n, ++nt_all) {
+              const uint32_t b = nt_all & 1u;
+              const int key = (it.t0 + n) * LC_KEYS + row;
+              if (ok) ok = __all_sync(0xffffffffu, ma_wait(&s_full[b], (nt_all >> 1) & 1u, abort));
+              tc_fence_after();
+              float xs[GP] = {};
+              lc_ld_heads<GP>(lanes + Cfg::kS + b * LC_HEADS, xs);
+              const bool seen = key < it.kvlen && key >= it.kv_lo;
+              bool up = false;
+#pragma unroll
+              for (int g = 0; g < GP; ++g) {
+                if (p.softcap > 0.f) xs[g] = p.softcap * tanh_exp(xs[g] * inv_cap);
+                xs[g] = seen ? xs[g] * LC_LOG2E : -INFINITY;
+                up |= g < G && (xs[g] > m_ref[g] + 8.f || (m_ref[g] == -INFINITY && xs[g] > -INFINITY));
+              }
+              // P(n - 2) has been read; waited for in every tile so that no parity wait lags two phases behind
+              if (ok && nt_all > 1) ok = __all_sync(0xffffffffu, ma_wait(&pv_done[b], ((nt_all - 2) >> 1) & 1u, abort));
+              if (lc_vote(up)) {                       // new references: the maxima of this tile
+                float alpha[GP];
+#pragma unroll
+                for (int g = 0; g < GP; ++g) {
+                  float m = xs[g];
+#pragma unroll
+                  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                  if (lane == 0) red_s[q4][g] = m;
+                }
+                lc_sync();
+#pragma unroll
+                for (int g = 0; g < GP; ++g) {
+                  const float m = fmaxf(m_ref[g], fmaxf(fmaxf(red_s[0][g], red_s[1][g]), fmaxf(red_s[2][g], red_s[3][g])));
+                  alpha[g] = (m_ref[g] == -INFINITY || g >= G) ? 0.f : ex2(m_ref[g] - m);
+                  m_ref[g] = m;
+                  lsum[g] *= alpha[g];
+                }
+                lc_sync();                             // red_s may be written again
+                if (n > 0) {
+                  if (ok) ok = __all_sync(0xffffffffu, ma_wait(&pv_done[b ^ 1u], ((nt_all - 1) >> 1) & 1u, abort));
+                  tc_fence_after();
+#pragma unroll
+                  for (int m = 0; m < MB; ++m) {
+                    float y[GP];
+                    lc_ld_heads<GP>(lanes + Cfg::kO + m * LC_HEADS, y);
+#pragma unroll
+                    for (int g = 0; g < GP; ++g) y[g] *= alpha[g];
+                    lc_st_heads<GP>(lanes + Cfg::kO + m * LC_HEADS, y);
+                  }
+                }
+              }
+              uint8_t* pt = zone + 8192 + b * 4096 + (row >> 6) * (LC_HEADS * 128) + (row & 7) * 2;
+#pragma unroll
+              for (int g = 0; g < GP; ++g) {
+                if (g < G) {
+                  const float e = ex2(xs[g] - (m_ref[g] == -INFINITY ? 0.f : m_ref[g]));
+                  const __nv_bfloat16 w = __float2bfloat16_rn(e);
+                  lsum[g] += __bfloat162float(w);      // the sum of what the product sees: the rounding of a dominant weight cancels
+                  *reinterpret_cast<__nv_bfloat16*>(pt + g * 128 + ((((row & 63) >> 3) ^ (g & 7)) << 4)) = w;
+                }
+              }
+              fence_proxy_async_smem();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&p_ready[b]);
+            }
+#pragma unroll
+            for (int g = 0; g < GP; ++g)
+#pragma unroll
+              for (int sh = 16; sh > 0; sh >>= 1) lsum[g] += __shfl_xor_sync(0xffffffffu, lsum[g], sh);
+            if (lane == 0)
+#pragma unroll
+              for (int g = 0; g < GP; ++g) sq_s[q4][g] = lsum[g];
+            float o[MB][GP];
+            if (it.nt > 0) {
+              if (ok && it.nt > 1) ok = __all_sync(0xffffffffu, ma_wait(&pv_done[nt_all & 1u], ((nt_all - 2) >> 1) & 1u, abort));
+              if (ok) ok = __all_sync(0xffffffffu, ma_wait(&pv_done[(nt_all - 1) & 1u], ((nt_all - 1) >> 1) & 1u, abort));
+              tc_fence_after();
+#pragma unroll
+              for (int m = 0; m < MB; ++m) lc_ld_heads<GP>(lanes + Cfg::kO + m * LC_HEADS, o[m]);
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(o_empty);
+            } else {
+#pragma unroll
+              for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int g = 0; g < GP; ++g) o[m][g] = 0.f;
+            }
+            __nv_bfloat16* out = p.attn + static_cast<size_t>(q_start_s[it.seq]) * q_dim + it.kvh * G * D;
+            if (p.parts == 1) {
+              lc_sync();
+#pragma unroll
+              for (int g = 0; g < GP; ++g)
+                if (g < G && ok) {
+                  const float den = sq_s[0][g] + sq_s[1][g] + sq_s[2][g] + sq_s[3][g];
+#pragma unroll
+                  for (int m = 0; m < MB; ++m) out[g * D + m * 128 + row] = __float2bfloat16_rn(den == 0.f ? 0.f : o[m][g] / den);
+                }
+            } else {
+              float* part_s = reinterpret_cast<float*>(zone + 8192);       // [G][D], over the weights of tiles that have been used
+#pragma unroll
+              for (int g = 0; g < GP; ++g)
+                if (g < G) {
+#pragma unroll
+                  for (int m = 0; m < MB; ++m) part_s[g * D + m * 128 + row] = o[m][g];
+                  if (row == 0) ml_s[g] = m_ref[g];
+                }
+              lc_sync();
+              if (et < G) ml_s[GP + et] = sq_s[0][et] + sq_s[1][et] + sq_s[2][et] + sq_s[3][et];
+              lc_sync();
+              const int peer0 = rank - part;           // the CTAs of this item: consecutive ranks
+              if (et < p.parts) arrive_cluster(mapa_smem(smem_u32(part_full), peer0 + et));
+              if (ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(part_full, nparts & 1u, abort));
+              ++nparts;
+#pragma unroll 1
+              for (int e = part * 128 + row; e < G * D; e += p.parts * 128) {
+                const int g = e / D;
+                float mr[LC_CL], lr[LC_CL], nr[LC_CL], m = -INFINITY;      // (all loads in flight: each is a round trip to a neighbour)
+#pragma unroll
+                for (int r = 0; r < LC_CL; ++r) {
+                  const uint32_t from = static_cast<uint32_t>(peer0 + min(r, p.parts - 1));
+                  mr[r] = ld_cluster_f32(mapa_smem(smem_u32(&ml_s[g]), from));
+                  lr[r] = ld_cluster_f32(mapa_smem(smem_u32(&ml_s[GP + g]), from));
+                  nr[r] = ld_cluster_f32(mapa_smem(smem_u32(part_s + e), from));
+                }
+#pragma unroll
+                for (int r = 0; r < LC_CL; ++r)
+                  if (r < p.parts) m = fmaxf(m, mr[r]);
+                float num = 0.f, den = 0.f;
+#pragma unroll
+                for (int r = 0; r < LC_CL; ++r) {
+                  const float w = (r >= p.parts || mr[r] == -INFINITY) ? 0.f : ex2(mr[r] - m);
+                  if (r < p.parts) {
+                    den += w * lr[r];
+                    num += w * nr[r];
+                  }
+                }
+                if (ok) out[e] = __float2bfloat16_rn(den == 0.f ? 0.f : num / den);
+              }
+            }
+            lc_sync();                                 // the sums of the rows have been read
+          }
+        } else {
+          // ------------------------------------------------------------- out = residual + rmsnorm(x) w: a CTA per token
+          const __nv_bfloat16* w = op == OP_NORM_A ? L->post_attn : L->post_ffn;
+          const __nv_bfloat16* residual = op == OP_NORM_A ? x : p.xb;
+          __nv_bfloat16* out = op == OP_NORM_A ? p.xb : p.xa;
+          const int k8 = p.hidden / 8;
+#pragma unroll 1
+          for (int t = blockIdx.x; t < p.T; t += gridDim.x) {
+            const uint4* xr = reinterpret_cast<const uint4*>(p.norm + static_cast<size_t>(t) * p.hidden);
+            const uint4* rr = reinterpret_cast<const uint4*>(residual + static_cast<size_t>(t) * p.hidden);
+            uint4* orow = reinterpret_cast<uint4*>(out + static_cast<size_t>(t) * p.hidden);
+            constexpr int C = 4;                       // chunks of 8 channels per thread (hidden <= 4096)
+            uint4 xv[C], r[C], g[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {              // (the residual is older than the operation in front)
+              const int i = et + 128 * c;
+              xv[c] = r[c] = g[c] = make_uint4(0, 0, 0, 0);
+              if (i < k8) {
+                g[c] = reinterpret_cast<const uint4*>(w)[i];
+                r[c] = __ldcg(rr + i);
+              }
+            }
+            if (ok) ok = __all_sync(0xffffffffu, lc_wait_due(due_s, at, abort));
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+              if (et + 128 * c < k8) xv[c] = __ldcg(xr + et + 128 * c);
+            float ss = 0.f;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&xv[c]);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(h[j]);
+                ss += f.x * f.x + f.y * f.y;
+              }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lane == 0) red_s[q4][0] = ss;
+            lc_sync();
+            const float rs = rsqrtf((red_s[0][0] + red_s[1][0] + red_s[2][0] + red_s[3][0]) / p.hidden + p.eps);
+            float sq = 0.f;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              const int i = et + 128 * c;
+              if (i < k8 && ok) {
+                uint4 o;
+                const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&xv[c]);
+                const __nv_bfloat162* hr = reinterpret_cast<const __nv_bfloat162*>(&r[c]);
+                const __nv_bfloat162* hg = reinterpret_cast<const __nv_bfloat162*>(&g[c]);
+                __nv_bfloat162* ho = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float2 f = __bfloat1622float2(hx[j]), fr = __bfloat1622float2(hr[j]);
+                  float2 fg = __bfloat1622float2(hg[j]);
+                  if (p.plus_one) { fg.x += 1.f; fg.y += 1.f; }
+                  ho[j] = __floats2bfloat162_rn(f.x * rs * fg.x + fr.x, f.y * rs * fg.y + fr.y);
+                  const float2 f2 = __bfloat1622float2(ho[j]);
+                  sq += f2.x * f2.x + f2.y * f2.y;
+                }
+                orow[i] = o;
+              }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            if (lane == 0) sq_s[q4][0] = sq;
+            lc_sync();
+            if (et == 0) p.ss[(op == OP_NORM_A ? LC_SS : 0) + t] = sq_s[0][0] + sq_s[1][0] + sq_s[2][0] + sq_s[3][0];
+          }
+        }
+        // this CTA's results of the operation are stored
+        lc_sync();
+        if (threadIdx.x == 64) red_release_gpu(ctr + at, 1u);
+        ++at;
+      }
+    }
+  }
+
+  // ------------------------------------------------------------------------------------------------------------------ leaving
+  __syncwarp();
+  if (*abort != 0u) {                                  // copies in flight land before the shared memory is given back
+    if (lane == 0) *reinterpret_cast<volatile uint32_t*>(p.ctl + LW_ABORT) = 1u;
+    __nanosleep(200000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_arrive_release();                            // no CTA leaves while another writes to or reads from it
+  cluster_wait_acquire();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc<Cfg::kTmem>(tmem);
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(p.ctl + LW_EXIT, 1u) == ctas - 1) {  // the last CTA: ready for the next launch
+      __threadfence();
+      volatile uint32_t* c = p.ctl;
+      for (int i = 0; i < p.n_layers * OP_COUNT; ++i) c[LW_CTR + i] = 0u;
+      if (c[LW_ABORT] != 0u) {
+        c[LW_ABORT] = 0u;
+        if (g_abort_word != nullptr) *reinterpret_cast<volatile uint32_t*>(g_abort_word) = 1u;
+        atomicAdd(&g_chain_gave_up, 1u);
+      }
+      c[LW_EXIT] = 0u;
+      __threadfence();
+    }
+  }
+}
+
+// clusters of four that fit the device at once with this kernel, 0 if it cannot run
+template <int BN, int D, int GP>
+int chain_clusters() {
+  static int known[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 64 && known[dev] != 0) return known[dev] - 1;
+  int n = 0, coop = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  if (coop && cudaFuncSetAttribute(layer_chain_kernel<BN, D, GP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcCfg<BN>::kSmem) == cudaSuccess) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(LC_CL * 64);
+    cfg.blockDim = dim3(LC_THREADS);
+    cfg.dynamicSmemBytes = LcCfg<BN>::kSmem;
+    cudaLaunchAttribute a[1];
+    a[0].id = cudaLaunchAttributeClusterDimension;
+    a[0].val.clusterDim.x = LC_CL;
+    a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
+    cfg.attrs = a;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, layer_chain_kernel<BN, D, GP>, &cfg) != cudaSuccess) n = 0;
+  }
+  cudaGetLastError();
+  if (dev < 64) known[dev] = n + 1;
+  return n;
+}
+
+template <int BN, int D, int GP>
+int launch_chain_one(const LcMaps& maps, LcParams p, cudaStream_t s) {
+  const int clusters = std::min(chain_clusters<BN, D, GP>(), 64);
+  if (clusters <= 0) return -5;
+  const int ctas = clusters * LC_CL, items = p.seqs * p.n_kv;
+  p.parts = items * 4 <= ctas ? 4 : (items * 2 <= ctas ? 2 : 1);     // few sequences: CTAs of a cluster share the keys of one
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+  cfg.blockDim = dim3(LC_THREADS);
+  cfg.dynamicSmemBytes = LcCfg<BN>::kSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute a[2];
+  a[0].id = cudaLaunchAttributeClusterDimension;
+  a[0].val.clusterDim.x = LC_CL;
+  a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
+  a[1].id = cudaLaunchAttributeCooperative;                          // the CTAs wait on one another
+  a[1].val.cooperative = 1;
+  cfg.attrs = a;
+  cfg.numAttrs = 2;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, layer_chain_kernel<BN, D, GP>, maps, p));
+}
+
+#define B2B_CHAIN(FN, BN, ...) \
+  (d.head_dim == 128 ? (g <= 4 ? FN<BN, 128, 4>(__VA_ARGS__) : FN<BN, 128, 8>(__VA_ARGS__)) \
+                     : (g <= 4 ? FN<BN, 256, 4>(__VA_ARGS__) : FN<BN, 256, 8>(__VA_ARGS__)))
+
+}  // namespace
+
+size_t layer_chain_table_bytes(int layers) { return static_cast<size_t>(layers) * sizeof(LcLayer); }
+size_t layer_chain_control_words(int layers) { return (LW_CTR + static_cast<size_t>(layers) * 7 + 31) / 32 * 32 + 2 * LC_SS; }
+
+bool layer_chain_supported(const ChainDims& d) {
+  const int g = d.n_kv > 0 ? d.n_q / d.n_kv : 0;
+  return d.n_kv > 0 && d.n_q % d.n_kv == 0 && g <= 8 && (d.head_dim == 128 || d.head_dim == 256) && g * d.head_dim * 4 <= 8192 &&
+         d.hidden % 128 == 0 && d.hidden >= 256 && d.ffn % 64 == 0 && d.ffn >= 256 && d.n_q * d.head_dim >= 256 &&
+         (!d.post_norms || d.hidden <= 4096);
+}
+
+// tensor maps and pointers of one layer at `dst` (host memory)
+int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w) {
+  LcLayer L;
+  std::memset(&L, 0, sizeof(L));
+  const int q_dim = d.n_q * d.head_dim, kv_dim = d.n_kv * d.head_dim;
+  const void* ptr[4] = {w.wqkv, w.wo, w.wgu, w.w_down};
+  const uint64_t rows[4] = {static_cast<uint64_t>(q_dim + 2 * kv_dim), static_cast<uint64_t>(d.hidden), 2ull * d.ffn, static_cast<uint64_t>(d.hidden)};
+  const uint64_t cols[4] = {static_cast<uint64_t>(d.hidden), static_cast<uint64_t>(q_dim), static_cast<uint64_t>(d.hidden), static_cast<uint64_t>(d.ffn)};
+  for (int i = 0; i < 4; ++i)
+    for (int b = 0; b < 5; ++b)
+      if (const int r = make_tmap_shared(&L.w[i][b], ptr[i], rows[i], cols[i], cols[i], 8u << b, 2)) return r;
+  const uint64_t keys = static_cast<uint64_t>(d.pages) * LC_PAGE;
+  if (const int r = make_tmap_shared(&L.k, w.k_cache, keys, kv_dim, kv_dim, LC_PAGE, 2)) return r;
+  if (const int r = make_tmap_shared(&L.v, w.v_cache, keys, kv_dim, kv_dim, LC_PAGE, 2)) return r;
+  L.k_cache = static_cast<__nv_bfloat16*>(w.k_cache);
+  L.v_cache = static_cast<__nv_bfloat16*>(w.v_cache);
+  L.post_attn = static_cast<const __nv_bfloat16*>(w.post_attn);
+  L.post_ffn = static_cast<const __nv_bfloat16*>(w.post_ffn);
+  L.window = w.window;
+  std::memcpy(dst, &L, sizeof(L));
+  return 0;
+}
+
+int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
+  const int g = d.n_kv > 0 ? d.n_q / d.n_kv : 0;
+  if (!layer_chain_supported(d) || c.tokens < 1 || c.tokens > 64 || c.layers < 1) return -2;
+  const int bn = c.tokens <= 16 ? 16 : (c.tokens <= 32 ? 32 : 64), x_rows = c.tokens <= 8 ? 8 : bn, q_dim = d.n_q * d.head_dim;
+  LcMaps m;
+  auto act = [&](CUtensorMap* t, const void* ptr, uint64_t rows, int cols) { return make_tmap_shared(t, ptr, rows, cols, cols, x_rows, 2); };
+  int r;
+  if ((r = act(&m.x_in, c.x_in, c.tokens, d.hidden)) || (r = act(&m.xa, c.xa, c.max_tokens, d.hidden)) || (r = act(&m.xb, c.xb, c.max_tokens, d.hidden)) ||
+      (r = act(&m.attn, c.attn, c.max_tokens, q_dim)) || (r = act(&m.h, c.h, c.max_tokens, d.ffn)) ||
+      (r = make_tmap_shared(&m.q, c.q, static_cast<uint64_t>(c.max_tokens) * d.n_q, d.head_dim, d.head_dim, LC_HEADS, 2)))
+    return r;
+  LcParams p;
+  p.layers = static_cast<const LcLayer*>(c.table);
+  p.n_layers = c.layers; p.T = c.tokens; p.seqs = c.seqs;
+  p.hidden = d.hidden; p.ffn = d.ffn; p.n_q = d.n_q; p.n_kv = d.n_kv; p.parts = 1;
+  p.act = d.act_gelu; p.plus_one = d.plus_one; p.norms = d.post_norms; p.x_rows = x_rows;
+  p.eps = d.eps; p.rope_theta = d.rope_theta; p.q_scale = d.q_scale; p.softcap = d.softcap;
+  p.x_in = static_cast<const __nv_bfloat16*>(c.x_in);
+  p.xa = static_cast<__nv_bfloat16*>(c.xa); p.xb = static_cast<__nv_bfloat16*>(c.xb); p.q = static_cast<__nv_bfloat16*>(c.q);
+  p.attn = static_cast<__nv_bfloat16*>(c.attn); p.h = static_cast<__nv_bfloat16*>(c.h); p.norm = static_cast<__nv_bfloat16*>(c.norm);
+  p.positions = c.positions; p.slots = c.slots; p.q_start = c.q_start; p.q_len = c.q_len; p.kv_len = c.kv_len; p.block_table = c.block_table;
+  p.max_pages = c.max_pages;
+  p.ctl = c.control;
+  p.ss = reinterpret_cast<float*>(c.control + layer_chain_control_words(c.layers)) - 2 * LC_SS;
+  if (bn == 16) return B2B_CHAIN(launch_chain_one, 16, m, p, s);
+  if (bn == 32) return B2B_CHAIN(launch_chain_one, 32, m, p, s);
+  return B2B_CHAIN(launch_chain_one, 64, m, p, s);
+}
+
+// clusters that are resident at once (0: the kernel cannot run here); also sets the kernels' shared memory sizes, so that a first launch may
+// happen under graph capture
+int layer_chain_init(const ChainDims& d) {
+  const int g = d.n_kv > 0 ? d.n_q / d.n_kv : 0;
+  if (!layer_chain_supported(d)) return 0;
+  return std::min(B2B_CHAIN(chain_clusters, 16), std::min(B2B_CHAIN(chain_clusters, 32), B2B_CHAIN(chain_clusters, 64)));
+}
+
+int set_wait_policy_chain(uint32_t* abort_word, unsigned long long limit_ns) {
+  cudaError_t e = cudaMemcpyToSymbol(g_abort_word, &abort_word, sizeof(abort_word));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_wait_limit_ns, &limit_ns, sizeof(limit_ns));
+  return static_cast<int>(e);
+}
+
+unsigned layer_chain_gave_up() {
+  unsigned n = 0;
+  return cudaMemcpyFromSymbol(&n, g_chain_gave_up, sizeof(n)) == cudaSuccess ? n : ~0u;
+}
+
+}  // namespace b2b

@@ -1,0 +1,164 @@
+"""Decode steps in one persistent kernel (csrc/layer_chain.cu) against the kernels one by one, which the other tests hold against the oracle."""
+import dataclasses
+
+import pytest
+import torch
+
+from bee2bee_b200.models.config import resolve_config
+
+pytestmark = pytest.mark.gpu
+
+# Both sides keep every sum in fp32 and round the same intermediates to bf16 (queries, attention output, stream, MLP hidden); a sum in another order
+# flips some of those roundings by one unit.  Five roundings of at most 2^-9 each reach the result per layer, so two layers stay below 10 * 2^-9 in the
+# worst case and, because they are independent, near sqrt(10) * 2^-9 = 0.006; measured up to 0.004.
+REL = 2.0 ** -7
+
+
+def _tensors(cfg, layers, g):
+    H, F, Q, KV = cfg.hidden_size, cfg.ffn_size, cfg.q_dim, cfg.kv_dim
+    t = {}
+
+    def rnd(*shape, std):
+        return (torch.randn(*shape, generator=g, device="cuda") * std).to(torch.bfloat16)
+
+    for l in range(layers):
+        for n, r, c in (("wq", Q, H), ("wk", KV, H), ("wv", KV, H), ("wo", H, Q), ("w_gate", F, H), ("w_up", F, H), ("w_down", H, F)):
+            t[f"l{l}.{n}"] = rnd(r, c, std=c ** -0.5)
+        for n in ("ln1_w", "ln2_w") + (("post_attn_w", "post_ffn_w") if cfg.post_norms else ()):
+            t[f"l{l}.{n}"] = rnd(H, std=0.1) + (0.0 if cfg.gemma_norm else 1.0)
+    return t
+
+
+def _setup(cfg, layers, ctxs, seed=3, spare_pages=1):
+    from bee2bee_b200 import ops
+    from bee2bee_b200.models.native import BatchMeta, NativePiece
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    S = len(ctxs)
+    need = [(c + 64) // 64 for c in ctxs]                    # pages of ctx + 1 keys
+    order = (torch.randperm(sum(need), generator=g, device="cuda") + spare_pages).cpu().tolist()
+    table, at = [], 0
+    for n in need:
+        table.append(order[at:at + n] + [0] * (max(need) - n))
+        at += n
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    ops.native().init_kernels(0)
+    piece = NativePiece(cfg, range(layers), False, False, _tensors(cfg, layers, g), torch.device("cuda", 0), S, S, sum(need) + spare_pages)
+    meta = BatchMeta(ids=None, positions=i32(ctxs), slots=i32([table[s][c // 64] * 64 + c % 64 for s, c in enumerate(ctxs)]), q_start=i32(list(range(S))),
+                     q_len=i32([1] * S), kv_len=i32([c + 1 for c in ctxs]), block_table=i32(table), n_tokens=S, n_seqs=S, max_q=1)
+    caches = [torch.randn(c.shape, generator=g, device="cuda").to(torch.bfloat16) for c in list(piece.k_cache.values()) + list(piece.v_cache.values())]
+    x = torch.randn(S, cfg.hidden_size, generator=g, device="cuda").to(torch.bfloat16)
+    return piece, meta, caches, x
+
+
+def _run(piece, meta, caches, x, chain):
+    """one step: result and caches"""
+    cache = list(piece.k_cache.values()) + list(piece.v_cache.values())
+    for c, v in zip(cache, caches):
+        c.copy_(v)
+    plan = piece._chain
+    if not chain:
+        piece._chain = None
+    out = piece.forward(meta, x_in=x).clone()
+    if not chain:
+        piece._chain = plan
+    torch.cuda.synchronize()
+    return out, [c.clone() for c in cache]
+
+
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+def _compare(piece, meta, caches, x, rel=REL):
+    from bee2bee_b200 import ops
+
+    ref, ref_caches = _run(piece, meta, caches, x, False)
+    n0 = ops.LAUNCHES[0]
+    out, got = _run(piece, meta, caches, x, True)
+    assert ops.LAUNCHES[0] == n0 + 1                         # the persistent kernel ran
+    assert _rel(out, ref) < rel
+    assert all(_rel(a, b) < rel for a, b in zip(got, ref_caches))
+    again, _ = _run(piece, meta, caches, x, True)
+    assert torch.equal(again, out)                           # sums in a fixed order
+    assert ops.native().layer_chain_gave_up() == 0
+    return out
+
+
+@pytest.mark.parametrize("seqs", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("model", ["tiny-llama", "tiny-mistral", "tiny-gemma2"])
+def test_token_tiles(model, seqs):
+    """edges of the token tiles; few and many CTAs per (sequence, key/value head); windows that cut keys off; capped scores and norms behind O and down"""
+    _compare(*_setup(resolve_config(model), 2, [1 + (37 * i) % 290 for i in range(seqs)]))
+
+
+@pytest.mark.parametrize("hidden,heads,kv,dim,ffn", [(384, 4, 2, 128, 448), (2304, 8, 4, 256, 1216), (1024, 16, 2, 128, 8256), (4096, 32, 8, 128, 14336)])
+def test_shares_of_the_products(hidden, heads, kv, dim, ffn):
+    """odd numbers of blocks of K, CTAs without a share, tiles of fewer than 128 rows, gate/up shares that start inside a block of 64 features"""
+    cfg = dataclasses.replace(resolve_config("tiny-llama"), hidden_size=hidden, n_heads=heads, n_kv_heads=kv, head_dim=dim, ffn_size=ffn)
+    _compare(*_setup(cfg, 2, [5, 130, 64, 63, 127]))
+
+
+@pytest.mark.parametrize("model,ctxs", [("tiny-llama", [0]), ("tiny-llama", [127, 128, 129, 255, 256]), ("tiny-llama", [3000, 1, 700]), ("tiny-llama", [1500] * 20),
+                                        ("zephyr-7b-beta", [1200 - 13 * i for i in range(64)])])
+def test_key_tiles(model, ctxs):
+    """one key, the edges of a tile, long beside short sequences, and more tiles per CTA than the ring has entries"""
+    cfg = resolve_config(model)
+    _compare(*_setup(cfg, 1, ctxs))
+
+
+def test_sequences_that_take_no_part():
+    piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [50, 80, 0, 200])
+    meta.q_len[1] = 0                                        # as GpuRunner marks a free slot
+    meta.slots[1] = -1
+    ref, ref_caches = _run(piece, meta, caches, x, False)
+    piece.attn_buf.zero_()
+    out, got = _run(piece, meta, caches, x, True)
+    live = [0, 2, 3]
+    assert _rel(out[live], ref[live]) < REL
+    assert all(_rel(a, b) < REL for a, b in zip(got, ref_caches))
+
+
+def test_graph_replay_sees_new_inputs_and_lengths():
+    piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [60, 61, 62])
+    _run(piece, meta, caches, x, True)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            out = piece.forward(meta, x_in=x)
+    torch.cuda.current_stream().wait_stream(stream)
+    for step in range(3):
+        x.copy_(torch.randn(x.shape, device="cuda"))
+        meta.kv_len.fill_(20 + step)
+        meta.positions.fill_(19 + step)
+        meta.slots.copy_(meta.block_table[:, 0] * 64 + 19 + step)
+        ref, _ = _run(piece, meta, caches, x, False)
+        for c, v in zip(list(piece.k_cache.values()) + list(piece.v_cache.values()), caches):
+            c.copy_(v)
+        graph.replay()
+        assert _rel(out, ref) < REL
+
+
+def test_routes():
+    """what the persistent kernel does not take runs on the kernels one by one; replaced weights and caches are seen"""
+    from bee2bee_b200 import ops
+    from bee2bee_b200.models.native import Handoff
+
+    piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [30] * 65)
+    assert not piece._chain_takes(meta, x, Handoff())        # 65 tokens
+    piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [30, 40])
+    assert piece._chain_takes(meta, x, Handoff())
+    assert not piece._chain_takes(dataclasses.replace(meta, max_q=2), x, Handoff())
+    assert not piece._chain_takes(meta, x, Handoff(in_flag=1)) and not piece._chain_takes(meta, x, Handoff(out_x=1))
+    wide = torch.zeros(2, 2 * x.shape[1], device="cuda", dtype=torch.bfloat16)
+    wide[:, : x.shape[1]] = x
+    assert not piece._chain_takes(meta, wide[:, : x.shape[1]], Handoff())
+    to = torch.zeros_like(x)
+    n0 = ops.LAUNCHES[0]
+    piece.forward(meta, x_in=x, out_x=to)                    # a result that goes elsewhere
+    assert ops.LAUNCHES[0] > n0 + 1
+    old = _compare(piece, meta, caches, x)
+    piece.w["l1.w_down"] = piece.w["l1.w_down"] * 2
+    assert _rel(_compare(piece, meta, caches, x), old) > 0.1

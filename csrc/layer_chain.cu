@@ -3,8 +3,8 @@
 // A decode step is a chain of small dependent operations per layer (QKV, attention, O, [norm], gate/up, down, [norm]), each of which streams its
 // weights or cache pages once.  As separate kernels each ends with its slowest block, starts with the latency of a launch and of its first loads, and
 // has only what fits beside the kernel before it on the way.  Here every SM runs one CTA for the whole step, and two producer warps walk the list
-// of weight tiles and cache pages of ALL operations: while an operation waits for the one before it, the next 200 KB per SM (4 us of the HBM
-// stream) land in the ring.
+// of weight tiles and cache pages of ALL operations: while an operation waits for the one before it, the next 140 to 180 KB per SM (3 to 4 us of
+// the HBM stream) land in the ring.
 //
 //   * operations are separated by a counter in global memory that every CTA adds to when its share of the results is stored; one warp per
 //     CTA polls it.  All CTAs are resident (cooperative launch).
@@ -16,9 +16,9 @@
 //   * the sums of squares for the next norm are left by the CTAs that write the rows, one number per CTA and token, added in a fixed order.
 //
 // Bound: the HBM stream and, between operations, the chain of last product, exchange, store, counter, poll and first activations (3 to 5 us, of
-// which the ring hides most).  Measured on B200, two Llama-3-8B layers, us (kernels one by one / here): one token behind 700 keys 190.7 / 177.3, 32
-// tokens behind 500 keys 218.9 / 201.0, 64 tokens behind 300 (Mistral-7B shapes) 255 / 224; two Gemma-2-2B layers: one token 124 / 105, 30 tokens 128 /
-// 115.  Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
+// which the ring hides most).  Measured on B200, two Llama-3-8B layers, us (kernels one by one / here): one token behind 700 keys 188.5 / 171.5, 32
+// tokens behind 500 keys 217.0 / 193.7, 64 tokens behind 300 (Mistral-7B shapes) 257 / 219; two Gemma-2-2B layers: one token 124 / 106, 30 tokens 128 /
+// 116.  Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
 // All waits are bounded: one that runs out raises the abort word, every other wait then ends too, and the CTAs leave.
 #include "kernels.h"
 
@@ -34,6 +34,7 @@
 namespace b2b {
 
 int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, int elt_bytes);
+int make_blocks_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks);
 
 namespace {
 
@@ -41,6 +42,7 @@ constexpr int LC_CL = 4;                           // CTAs of a cluster == parts
 constexpr int LC_THREADS = 256;
 constexpr int LC_PAGE = 64, LC_KEYS = 128, LC_HEADS = 16;
 constexpr int LC_BLOCK = 128 * 128;                // 128 rows x 64 bf16: a weight block, or 128 keys x 64 channels
+constexpr int LC_XSLOTS = 6;                       // copies of activations in flight, at most
 constexpr int LC_ENTRIES = 16;                     // entries of the ring in flight, at most
 constexpr uint32_t LC_SPINS = 1u << 23;            // polls of a counter (0.3 us or more each)
 constexpr int LC_SS = 64 * 64;
@@ -67,7 +69,9 @@ struct alignas(128) LcLayer {
   int window;
 };
 
-struct LcMaps {                                    // activations: boxes of 64 channels x the token tile (q: 16 heads)
+// activations come in copies of two or four blocks of K of the whole token tile: with a copy per block their issue (0.45 us per entry of the ring) was
+// what a product that found its weights landed waited for (one token 177 -> 172 us, 32 tokens 201 -> 194)
+struct LcMaps {                                    // activations: boxes of kXBlocks 64-channel blocks x the token tile (q: 16 heads x 64 channels)
   CUtensorMap x_in, xa, xb, attn, h, q;
 };
 
@@ -86,10 +90,12 @@ struct LcParams {
 
 template <int BN>
 struct LcCfg {
-  static constexpr int kRing = BN == 64 ? 191 * 1024 : 208 * 1024;
+  static constexpr int kXBlocks = BN == 16 ? 4 : 2;                // 64-channel blocks per copy of activations
+  static constexpr int kX = (BN == 16 ? 24 : (BN == 32 ? 32 : 48)) * 1024;       // three copies, four at 32 tokens (six at 8 or fewer)
+  static constexpr int kRing = (BN == 64 ? 190 : 207) * 1024 - kX; // weights and cache pages
   static constexpr int kCols = BN / LC_CL;                         // tokens that a CTA of a cluster finishes
   static constexpr int kZone = BN * 512 > 16384 ? BN * 512 : 16384;   // partial sums, or Q (8 KB: two of 128 channels or one of 256) and P
-  static constexpr int kSmem = 1024 + kRing + kZone + 512;
+  static constexpr int kSmem = 1024 + kRing + kX + kZone + 640;
   static constexpr uint32_t kS = 2 * BN, kO = 2 * BN + 2 * LC_HEADS;   // TMEM columns behind the two accumulators
   static constexpr uint32_t kTmem = BN == 64 ? 256 : 128;
 };
@@ -133,6 +139,10 @@ __device__ __forceinline__ bool lc_vote(bool p) {
       "selp.u32 %0, 1, 0, b;\n\t}\n"
       : "=r"(r) : "r"(p ? 1u : 0u) : "memory");
   return r != 0;
+}
+__device__ __forceinline__ void tma_load_3d_hint(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2, uint64_t policy) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
+               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "l"(policy) : "memory");
 }
 // wait on a barrier that the CTAs of the cluster arrive at
 __device__ __forceinline__ bool lc_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort) {
@@ -249,7 +259,7 @@ struct LcRing {
   __device__ __forceinline__ uint32_t entry() const { return count % LC_ENTRIES; }
   __device__ __forceinline__ uint32_t parity() const { return count / LC_ENTRIES & 1u; }
 };
-// who fills the ring: also waits until there is room.  Both filling warps keep their own account (a word that one leaves for the other took a fence
+// who fills the ring: also waits until there is room.  The two filling warps keep an account each (a word that one leaves for the other took a fence
 // per entry: 5 % of a decode step)
 template <int BYTES>
 struct LcFill : LcRing<BYTES> {
@@ -299,13 +309,16 @@ __device__ __forceinline__ LcItem lc_item(const LcParams& p, const int* kvlen_s,
 template <int BN, int D, int GP>
 __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid_constant__ LcMaps maps, const LcParams p) {
   using Cfg = LcCfg<BN>;
-  constexpr int CW = Cfg::kCols, DB = D / 64, MB = D / 128, NQ = 2 / MB;
+  constexpr int XB = Cfg::kXBlocks, CW = Cfg::kCols, DB = D / 64, MB = D / 128, NQ = 2 / MB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* zone = smem + Cfg::kRing;          // partial sums of the cluster | up and gate halves | Q and P of the attention
+  uint8_t* x_s = smem + Cfg::kRing;                 // activations
+  uint8_t* zone = x_s + Cfg::kX;          // partial sums of the cluster | up and gate halves | Q and P of the attention
   uint64_t* full = reinterpret_cast<uint64_t*>(zone + Cfg::kZone);   // [LC_ENTRIES]
   uint64_t* empty = full + LC_ENTRIES;             // [LC_ENTRIES]
-  uint64_t* acc_full = empty + LC_ENTRIES;                 // [2]
+  uint64_t* x_full = empty + LC_ENTRIES;           // [LC_XSLOTS]
+  uint64_t* x_empty = x_full + LC_XSLOTS;          // [LC_XSLOTS]
+  uint64_t* acc_full = x_empty + LC_XSLOTS;                 // [2]
   uint64_t* acc_empty = acc_full + 2;              // [2]
   uint64_t* zone_full = acc_empty + 2;
   uint64_t* zone_free = zone_full + 1;
@@ -325,15 +338,19 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   __shared__ float sq_s[4][CW > GP ? CW : GP];     // per warp: sums of squares, or of a row's weights
   __shared__ float ml_s[2 * GP];             // this CTA's maxima and sums, read by the cluster
   __shared__ LcShare share_s[LC_PRODUCTS];
-  __shared__ uint32_t entry_s[3][LC_ENTRIES];      // bytes of the ring's entries, with what was skipped in front of them
+  __shared__ uint32_t entry_s[2][LC_ENTRIES];      // bytes of the ring's entries, with what was skipped in front of them
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank());
   const uint32_t ctas = gridDim.x;
   if (threadIdx.x == 0) {
     for (int i = 0; i < LC_ENTRIES; ++i) {
-      mbar_init(&full[i], 3);                      // the two halves of the weights (or pages), the activations
+      mbar_init(&full[i], 2);                      // the two halves
       mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < LC_XSLOTS; ++i) {
+      mbar_init(&x_full[i], 1);
+      mbar_init(&x_empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&q_full[i], 1);
@@ -371,7 +388,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   const bool norms = p.norms != 0;
   uint32_t* const ctr = p.ctl + LW_CTR;
   const int item0 = blockIdx.x / p.parts, part = blockIdx.x % p.parts, item_step = gridDim.x / p.parts, items = p.seqs * p.n_kv;
-  const uint32_t x_bytes = static_cast<uint32_t>(p.x_rows) * 128u;     // activations of an entry per block of K
+  const uint32_t x_bytes = static_cast<uint32_t>(p.x_rows) * 128u;     // activations per block of K
+  const uint32_t x_slots = Cfg::kX / (x_bytes * XB);
   auto skip = [&](int op) { return !norms && (op == OP_NORM_A || op == OP_NORM_F); };
   // (every role walks the operations in loops whose bodies appear once: a kernel of 250 KB of code spent microseconds per operation on
   // fetching its instructions)
@@ -414,7 +432,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
 #pragma unroll 1
               for (int kb = 0; kb < sh.nkb; kb += 2) {
                 const int nb = min(2, sh.nkb - kb);
-                if (!(ok = ring.room((block + x_bytes) * nb, place, sizes, empty, abort))) break;
+                if (!(ok = ring.room(block * nb, place, sizes, empty, abort))) break;
                 uint8_t* base = smem + place;
                 uint64_t* bar = &full[ring.entry()];
                 ++ring.count;
@@ -469,7 +487,6 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                   uint64_t* bar = &full[ring.entry()];
                   ++ring.count;
                   mbar_arrive_expect_tx(bar, LC_BLOCK);
-                  if (half == 0) mbar_arrive(bar);   // (no activations)
                   uint8_t* dst = base + half * LC_BLOCK;
                   const CUtensorMap* m = values ? &L->v : &L->k;
                   tma_load_2d(dst, m, bar, it.kvh * D + h * 128 + half * 64, where.x * LC_PAGE);
@@ -489,8 +506,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
     // --------------------------------------------------------------------------- activations, as soon as they are complete
     if (elect_one()) {
       const uint64_t pol = l2_policy_evict_last();
-      LcFill<Cfg::kRing> ring;
-      uint32_t nq = 0, place = 0;
+      uint32_t nq = 0, s = 0, ph = 0;
       bool ok = true;
       int at = 0;
 #pragma unroll 1
@@ -509,21 +525,14 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             const LcShare sh = share_s[lc_weight(op)];
             const CUtensorMap* m = op == OP_QKV ? (l == 0 ? &maps.x_in : &maps.xa) : (op == OP_O ? &maps.attn : (op == OP_GU ? &maps.xb : &maps.h));
 #pragma unroll 1
-            for (int u = sh.u0, n; ok && u < sh.end; u += n) {
-              n = lc_tile(op, u, sh.end);
-              const uint32_t block = lc_block_bytes(op, n);
+            for (int u = sh.u0; ok && u < sh.end; u += lc_tile(op, u, sh.end))
 #pragma unroll 1
-              for (int kb = 0; kb < sh.nkb; kb += 2) {
-                const int nb = min(2, sh.nkb - kb);
-                if (!(ok = ring.room((block + x_bytes) * nb, place, entry_s[2], empty, abort))) break;
-                uint8_t* base = smem + place + block * nb;
-                uint64_t* bar = &full[ring.entry()];
-                ++ring.count;
-                mbar_arrive_expect_tx(bar, x_bytes * nb);
-#pragma unroll 1
-                for (int b = 0; b < nb; ++b) tma_load_2d_hint(base + b * x_bytes, m, bar, (sh.kb0 + kb + b) * 64, 0, pol);
+              for (int kb = 0; kb < sh.nkb; kb += XB) {      // (whole copies, also where fewer blocks are left: they are not used)
+                if (!(ok = ma_wait(&x_empty[s], ph ^ 1u, abort))) break;
+                mbar_arrive_expect_tx(&x_full[s], x_bytes * XB);
+                tma_load_3d_hint(x_s + s * x_bytes * XB, m, &x_full[s], 0, 0, sh.kb0 + kb, pol);
+                if (++s == x_slots) { s = 0; ph ^= 1u; }
               }
-            }
           } else if (op == OP_ATT) {
 #pragma unroll 1
             for (int j = item0; ok && j < items; j += item_step) {
@@ -536,8 +545,6 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
 #pragma unroll
               for (int c = 0; c < DB; ++c)
                 tma_load_2d(zone + b * (LC_HEADS * D * 2) + c * (LC_HEADS * 128), &maps.q, &q_full[b], c * 64, q_start_s[it.seq] * p.n_q + it.kvh * G);
-#pragma unroll 1
-              for (int i = 0; ok && i < 2 * it.nt * MB; ++i, ++ring.count) ok = ring.room(2 * LC_BLOCK, place, entry_s[2], empty, abort);
             }
           }
         }
@@ -550,6 +557,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
       constexpr uint32_t idesc_s = make_idesc_bf16(LC_KEYS, LC_HEADS);
       constexpr uint32_t idesc_o = make_idesc_bf16(128, LC_HEADS) | (1u << 15);              // A (V) has its rows contiguous
       const uint64_t desc0 = make_sw128_kmajor_desc(smem_u32(smem));         // + offset / 16 (a single thread issues: every instruction counts)
+      const uint64_t desc_x = make_sw128_kmajor_desc(smem_u32(x_s));
+      const uint32_t x_chunk = x_bytes * XB >> 4;
+      uint32_t xs = 0, xph = 0;
       LcRing<Cfg::kRing> ring;
       uint32_t na = 0, ns = 0, np = 0, nq = 0, no = 0;       // accumulators, score tiles, value tiles, items so far
       bool ok = true;
@@ -569,27 +579,35 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               const uint32_t acc = tmem + (na & 1u) * BN;
               uint32_t more = 0u;
 #pragma unroll 1
-              for (int kb = 0; kb < sh.nkb; kb += 2) {
-                const uint32_t nb = min(2, sh.nkb - kb);
-                // (rows that the tile does not have are read from what lies behind it, and not used)
-                uint64_t a = desc0 + (ring.place((block + x_bytes) * nb) >> 4), x = a + (block * nb >> 4);
-                if (!(ok = ma_wait(&full[ring.entry()], ring.parity(), abort))) break;
-                tc_fence_after();
-                umma_bf16(acc, a, x, idesc, more);
-                umma_bf16(acc, a + 2, x + 2, idesc, 1u);
-                umma_bf16(acc, a + 4, x + 4, idesc, 1u);
-                umma_bf16(acc, a + 6, x + 6, idesc, 1u);
-                if (nb == 2) {
-                  a += block >> 4;
-                  x += x_bytes >> 4;
-                  umma_bf16(acc, a, x, idesc, 1u);
+              for (int kb = 0; kb < sh.nkb; kb += XB) {
+                if (!(ok = ma_wait(&x_full[xs], xph, abort))) break;
+                uint64_t x = desc_x + xs * x_chunk;
+#pragma unroll 1
+                for (int k2 = kb; k2 < min(kb + XB, sh.nkb); k2 += 2) {
+                  const uint32_t nb = min(2, sh.nkb - k2);
+                  // (rows that the tile does not have are read from what lies behind it, and not used)
+                  uint64_t a = desc0 + (ring.place(block * nb) >> 4);
+                  if (!(ok = ma_wait(&full[ring.entry()], ring.parity(), abort))) break;
+                  tc_fence_after();
+                  umma_bf16(acc, a, x, idesc, more);
                   umma_bf16(acc, a + 2, x + 2, idesc, 1u);
                   umma_bf16(acc, a + 4, x + 4, idesc, 1u);
                   umma_bf16(acc, a + 6, x + 6, idesc, 1u);
+                  if (nb == 2) {
+                    a += block >> 4;
+                    x += x_bytes >> 4;
+                    umma_bf16(acc, a, x, idesc, 1u);
+                    umma_bf16(acc, a + 2, x + 2, idesc, 1u);
+                    umma_bf16(acc, a + 4, x + 4, idesc, 1u);
+                    umma_bf16(acc, a + 6, x + 6, idesc, 1u);
+                    x += x_bytes >> 4;
+                  }
+                  umma_commit(&empty[ring.entry()]);
+                  ++ring.count;
+                  more = 1u;
                 }
-                umma_commit(&empty[ring.entry()]);
-                ++ring.count;
-                more = 1u;
+                umma_commit(&x_empty[xs]);
+                if (++xs == x_slots) { xs = 0; xph ^= 1u; }
               }
               umma_commit(&acc_full[na & 1u]);
             }
@@ -1191,7 +1209,7 @@ int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
   if (!layer_chain_supported(d) || c.tokens < 1 || c.tokens > 64 || c.layers < 1) return -2;
   const int bn = c.tokens <= 16 ? 16 : (c.tokens <= 32 ? 32 : 64), x_rows = c.tokens <= 8 ? 8 : bn, q_dim = d.n_q * d.head_dim;
   LcMaps m;
-  auto act = [&](CUtensorMap* t, const void* ptr, uint64_t rows, int cols) { return make_tmap_shared(t, ptr, rows, cols, cols, x_rows, 2); };
+  auto act = [&](CUtensorMap* t, const void* ptr, uint64_t rows, int cols) { return make_blocks_tmap(t, ptr, rows, cols, x_rows, bn == 16 ? LcCfg<16>::kXBlocks : LcCfg<32>::kXBlocks); };
   int r;
   if ((r = act(&m.x_in, c.x_in, c.tokens, d.hidden)) || (r = act(&m.xa, c.xa, c.max_tokens, d.hidden)) || (r = act(&m.xb, c.xb, c.max_tokens, d.hidden)) ||
       (r = act(&m.attn, c.attn, c.max_tokens, q_dim)) || (r = act(&m.h, c.h, c.max_tokens, d.ffn)) ||

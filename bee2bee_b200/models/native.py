@@ -1,7 +1,8 @@
 """One *piece* (contiguous layer range) resident on one B200, executed entirely by the
 hand-written sm_100a kernels in ``csrc/``.
 
-A decode step (one new token per sequence, up to 64) of whole bf16 layers is one persistent kernel (``csrc/layer_chain.cu``).
+A decode step (one new token per sequence, up to 64; GPT-2: prompts of up to 64 tokens too) of whole bf16 layers is one persistent
+kernel (``csrc/layer_chain.cu``).
 Prompts, quantised weights and pieces of a pipeline: per decoder layer (Llama / Mistral) exactly five launches, all on one stream:
 
     QKV GEMM  [fused: RMSNorm(x) via folded gamma + in-kernel 1/rms, RoPE, paged-KV append]
@@ -231,30 +232,39 @@ class NativePiece:
         self.attn_ws = torch.zeros(max_seqs * c.n_kv_heads * self.max_splits * rows * (c.head_dim + 2), device=dev,
                                    dtype=torch.float32)
         self._chain = self._chain_of = None
-        if units is None and self.layers and self.fused_norm and c.glu and not self.fp8 and self.device.type == "cuda":
+        self._chain_ln = not self.fused_norm and not c.glu and c.bias and not c.post_norms and c.rope_theta <= 0 and c.attn_softcap == 0
+        if units is None and self.layers and (self._chain_ln or (self.fused_norm and c.glu and not self.fp8)) and self.device.type == "cuda":
             with torch.cuda.device(dev):
-                if ops.native().layer_chain_supported(c.hidden_size, c.ffn_size, c.n_heads, c.n_kv_heads, c.head_dim, c.post_norms):
+                if ops.native().layer_chain_supported(c.hidden_size, c.ffn_size, c.n_heads, c.n_kv_heads, c.head_dim, c.post_norms, self._chain_ln):
                     self._plan_chain()
 
     # ------------------------------------------------------------------ helpers
     def _chain_tensors(self):
-        names = ("wqkv", "wo", "wgu", "w_down")
+        names = ("wqkv", "wo", "w_up" if self._chain_ln else "wgu", "w_down")
         post = ("post_attn_w", "post_ffn_w") if self.cfg.post_norms else ()
-        return [[self.w[f"l{l}.{n}"] for n in names] + [self.k_cache[l], self.v_cache[l]] + [self.w[f"l{l}.{n}"] for n in post]
+        if self._chain_ln:
+            post = ("bqkv", "bo", "b_up", "b_down", "ln2_w", "ln2_b")
+        rows = [[self.w[f"l{l}.{n}"] for n in names] + [self.k_cache[l], self.v_cache[l]] + [self.w[f"l{l}.{n}"] for n in post]
                 for l in self.layers]
+        if self._chain_ln:                     # the norm in front of the next layer
+            for row, l in zip(rows, self.layers[1:]):
+                row += [self.w[f"l{l}.ln1_w"], self.w[f"l{l}.ln1_b"]]
+        return rows
 
     def _plan_chain(self) -> None:
         """lays the layers out for the decode kernel (csrc/layer_chain.cu)"""
         c = self.cfg
         t = self._chain_tensors()
         self._chain = ops.native().LayerChain(t, [c.layer_window(l) for l in self.layers], self.xa, self.xb, self.q_buf, self.attn_buf, self.h_buf,
-                                              self.n_buf if c.post_norms else None, c.n_heads, c.n_kv_heads, c.head_dim,
-                                              int(c.act == "gelu_tanh"), c.gemma_norm, c.norm_eps, c.rope_theta, c.softmax_scale, c.attn_softcap)
+                                              self.n_buf if c.post_norms or self._chain_ln else None, c.n_heads, c.n_kv_heads, c.head_dim,
+                                              int(c.act == "gelu_tanh"), c.gemma_norm, c.norm_eps, c.rope_theta, c.softmax_scale, c.attn_softcap,
+                                              self._chain_ln)
         self._chain_of = [[x.data_ptr() for x in row] for row in t]
 
     def _chain_takes(self, m: BatchMeta, x: torch.Tensor, hand: Handoff) -> bool:
-        """a decode step (one new token per sequence, up to 64) of whole layers whose input and result stay on this GPU"""
-        if self._chain is None or m.max_q != 1 or not 1 <= m.n_tokens <= 64 or m.n_tokens != m.n_seqs:
+        """a decode step (one new token per sequence, up to 64) of whole layers whose input and result stay on this GPU; LayerNorm models:
+        prompts of up to 64 tokens too"""
+        if self._chain is None or not 1 <= m.n_tokens <= 64 or not (self._chain_ln or (m.max_q == 1 and m.n_tokens == m.n_seqs)):
             return False
         if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16:
             return False
@@ -348,6 +358,8 @@ class NativePiece:
             x = x_in[:T]
             wait_flag, wait_epoch = hand.in_flag, hand.in_epoch
         if out_x is None and self._chain_takes(m, x, hand):
+            if self._chain_ln:
+                ops.layernorm(x, self.w[f"l{self.layers[0]}.ln1_w"], self.w[f"l{self.layers[0]}.ln1_b"], self.n_buf[:T], eps)
             ops.layer_chain(self._chain, x, m.positions, m.slots, m.q_start, m.q_len, m.kv_len, m.block_table)
             return self._head(m, self.xa[:T], hand) if self.last else self.xa[:T]
         inline = self._use_inline_rstd(T)

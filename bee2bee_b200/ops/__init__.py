@@ -435,7 +435,7 @@ def attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, *, 
 
 
 def layer_chain(plan, x, positions, slots, q_start, q_len, kv_len, block_table):
-    """All layers of a decode step (one new token per sequence, up to 64) in one persistent kernel (csrc/layer_chain.cu); ``plan`` is the
+    """All layers of a decode step (one new token per sequence, up to 64; GPT-2: spans too) in one persistent kernel (csrc/layer_chain.cu); ``plan`` is the
     piece's ``LayerChain``, which owns the weights' layout and the buffers.  The result is in the plan's ``xa``."""
     plan.run(x, positions, slots, q_start, q_len, kv_len, block_table)
     LAUNCHES[0] += 1

@@ -267,11 +267,11 @@ void flag_signal(int64_t flag, int64_t epoch, int64_t bump_epoch, int64_t ack_fl
 
 // ------------------------------------------------------------- all layers of a decode step
 static b2b::ChainDims chain_dims(int64_t hidden, int64_t ffn, int64_t n_q, int64_t n_kv, int64_t head_dim, int64_t pages, int64_t act_gelu,
-                                 bool plus_one, bool post_norms, double eps, double rope_theta, double q_scale, double softcap) {
+                                 bool plus_one, bool post_norms, bool layer_norm, double eps, double rope_theta, double q_scale, double softcap) {
   b2b::ChainDims d;
   d.hidden = static_cast<int>(hidden); d.ffn = static_cast<int>(ffn); d.n_q = static_cast<int>(n_q); d.n_kv = static_cast<int>(n_kv);
   d.head_dim = static_cast<int>(head_dim); d.pages = static_cast<int>(pages);
-  d.act_gelu = static_cast<int>(act_gelu); d.plus_one = plus_one; d.post_norms = post_norms;
+  d.act_gelu = static_cast<int>(act_gelu); d.plus_one = plus_one; d.post_norms = post_norms; d.layer_norm = layer_norm;
   d.eps = static_cast<float>(eps); d.rope_theta = static_cast<float>(rope_theta); d.q_scale = static_cast<float>(q_scale);
   d.softcap = static_cast<float>(softcap);
   return d;
@@ -286,16 +286,17 @@ struct LayerChain {
   std::vector<Tensor> keep;
   Tensor xa, xb, q, attn, h, norm;
 
-  // per layer: wqkv, wo, wgu, w_down, k_cache, v_cache and, with post norms, their two weights
+  // per layer: wqkv, wo, wgu, w_down, k_cache, v_cache and, with post norms, their two weights; LayerNorm models: the biases of the four products (fp32),
+  // weight and bias of the norm in front of the MLP and, but for the last layer, of the next layer's first norm
   LayerChain(const std::vector<std::vector<Tensor>>& ls, const std::vector<int64_t>& windows, const Tensor& xa_, const Tensor& xb_,
              const Tensor& q_, const Tensor& attn_, const Tensor& h_, const OptT& norm_, int64_t n_q, int64_t n_kv, int64_t head_dim,
-             int64_t act_gelu, bool plus_one, double eps, double rope_theta, double q_scale, double softcap)
+             int64_t act_gelu, bool plus_one, double eps, double rope_theta, double q_scale, double softcap, bool layer_norm)
       : layers(static_cast<int>(ls.size())), max_tokens(static_cast<int>(xa_.size(0))), xa(xa_), xb(xb_), q(q_), attn(attn_), h(h_) {
     TORCH_CHECK(layers > 0 && windows.size() == ls.size(), "layer_chain: one window per layer");
-    const bool post = ls[0].size() == 8;
+    const bool post = !layer_norm && ls[0].size() == 8;
     const int64_t H = xa.size(1), F = h.size(1), Q = n_q * head_dim, KV = n_kv * head_dim;
-    if (post) {
-      TORCH_CHECK(norm_.has_value(), "layer_chain: post norms need a buffer");
+    if (post || layer_norm) {
+      TORCH_CHECK(norm_.has_value(), "layer_chain: norms need a buffer");
       norm = *norm_;
       check_bf16(norm, "norm");
       TORCH_CHECK(norm.size(0) >= max_tokens && norm.size(1) == H, "layer_chain: norm buffer size");
@@ -305,31 +306,46 @@ struct LayerChain {
       TORCH_CHECK(t->size(0) >= max_tokens, "layer_chain: buffers of max_tokens rows");
     }
     TORCH_CHECK(xb.size(1) == H && q.size(1) == Q && attn.size(1) == Q, "layer_chain: buffer widths");
-    d = chain_dims(H, F, n_q, n_kv, head_dim, ls[0].at(4).size(0), act_gelu, plus_one, post, eps, rope_theta, q_scale, softcap);
+    d = chain_dims(H, F, n_q, n_kv, head_dim, ls[0].at(4).size(0), act_gelu, plus_one, post, layer_norm, eps, rope_theta, q_scale, softcap);
     TORCH_CHECK(b2b::layer_chain_supported(d), "layer_chain: sizes not supported");
     const size_t one = b2b::layer_chain_table_bytes(1);
     Tensor host = at::empty({static_cast<int64_t>(one * layers)}, at::TensorOptions().dtype(at::kByte));
     for (int l = 0; l < layers; ++l) {
       const auto& t = ls[l];
-      TORCH_CHECK(t.size() == (post ? 8u : 6u), "layer_chain: tensors of layer ", l);
-      for (const Tensor& x : t) check_bf16(x, "layer_chain weight");
+      TORCH_CHECK(t.size() == (layer_norm ? (l + 1 < layers ? 14u : 12u) : (post ? 8u : 6u)), "layer_chain: tensors of layer ", l);
+      for (size_t i = 0; i < t.size(); ++i)
+        if (!layer_norm || i < 6 || i >= 10) check_bf16(t[i], "layer_chain weight");
       auto rows = [&](int i, int64_t r, int64_t c) {
         TORCH_CHECK(t[i].dim() == 2 && t[i].size(0) == r && t[i].size(1) == c && reinterpret_cast<uintptr_t>(t[i].data_ptr()) % 16 == 0,
                     "layer_chain: weight ", i, " of layer ", l);
       };
       rows(0, Q + 2 * KV, H);
       rows(1, H, Q);
-      rows(2, 2 * F, H);
+      rows(2, layer_norm ? F : 2 * F, H);
       rows(3, H, F);
       for (int i : {4, 5})
         TORCH_CHECK(t[i].size(0) == d.pages && t[i].numel() == static_cast<int64_t>(d.pages) * 64 * KV && reinterpret_cast<uintptr_t>(t[i].data_ptr()) % 16 == 0,
                     "layer_chain: cache of layer ", l);
       b2b::ChainLayerPtrs w{t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(), t[4].data_ptr(), t[5].data_ptr(), nullptr, nullptr,
-                            static_cast<int>(windows[l])};
+                            static_cast<int>(windows[l]), nullptr, nullptr, {nullptr, nullptr, nullptr, nullptr}};
       if (post) {
         TORCH_CHECK(t[6].numel() == H && t[7].numel() == H, "layer_chain: norm weights");
         w.post_attn = t[6].data_ptr();
         w.post_ffn = t[7].data_ptr();
+      }
+      if (layer_norm) {
+        const int64_t n[4] = {Q + 2 * KV, H, F, H};
+        for (int i = 0; i < 4; ++i) {
+          TORCH_CHECK(t[6 + i].is_cuda() && t[6 + i].scalar_type() == at::kFloat && t[6 + i].is_contiguous() && t[6 + i].numel() == n[i], "layer_chain: bias ", i);
+          w.bias[i] = static_cast<const float*>(t[6 + i].data_ptr());
+        }
+        for (size_t i = 10; i < t.size(); ++i) TORCH_CHECK(t[i].numel() == H && reinterpret_cast<uintptr_t>(t[i].data_ptr()) % 16 == 0, "layer_chain: norm weights");
+        w.post_attn = t[10].data_ptr();
+        w.post_attn_b = t[11].data_ptr();
+        if (t.size() == 14) {
+          w.post_ffn = t[12].data_ptr();
+          w.post_ffn_b = t[13].data_ptr();
+        }
       }
       check(b2b::layer_chain_fill(static_cast<uint8_t*>(host.data_ptr()) + one * l, d, w), "layer_chain_fill");
       keep.insert(keep.end(), t.begin(), t.end());
@@ -341,7 +357,8 @@ struct LayerChain {
     c10::cuda::getCurrentCUDAStream().synchronize();
   }
 
-  // one new token per sequence (rows of x_in in the order of the sequences); the result is in xa
+  // one new token per sequence (rows of x_in in the order of the sequences), LayerNorm models: spans too, the normed rows of x_in are in `norm`; the
+  // result is in xa
   void run(const Tensor& x_in, const OptT& positions, const Tensor& slots, const Tensor& q_start, const Tensor& q_len, const Tensor& kv_len,
            const Tensor& block_table) {
     check_bf16(x_in, "x_in");
@@ -350,7 +367,7 @@ struct LayerChain {
                 reinterpret_cast<uintptr_t>(x_in.data_ptr()) % 16 == 0, "layer_chain: 1 to 64 aligned rows of the hidden size");
     for (const Tensor* t : {&slots, &q_start, &q_len, &kv_len, &block_table})
       TORCH_CHECK(t->scalar_type() == at::kInt && t->is_contiguous() && t->device() == xa.device(), "layer_chain: int32 metadata");
-    TORCH_CHECK(S <= T && slots.numel() >= T && q_start.numel() >= S && kv_len.numel() >= S && block_table.dim() == 2 && block_table.size(0) >= S,
+    TORCH_CHECK((S <= T || d.layer_norm) && slots.numel() >= T && q_start.numel() >= S && kv_len.numel() >= S && block_table.dim() == 2 && block_table.size(0) >= S,
                 "layer_chain: metadata sizes");
     TORCH_CHECK(d.rope_theta <= 0.f || (positions.has_value() && positions->numel() >= T && positions->scalar_type() == at::kInt), "layer_chain: positions");
     c10::cuda::CUDAGuard guard(xa.device());
@@ -370,8 +387,8 @@ struct LayerChain {
 };
 
 // true if layer_chain.cu takes a piece of these sizes on the current device
-bool layer_chain_supported(int64_t hidden, int64_t ffn, int64_t n_q, int64_t n_kv, int64_t head_dim, bool post_norms) {
-  const b2b::ChainDims d = chain_dims(hidden, ffn, n_q, n_kv, head_dim, 1, 0, false, post_norms, 1e-5, 0.0, 1.0, 0.0);
+bool layer_chain_supported(int64_t hidden, int64_t ffn, int64_t n_q, int64_t n_kv, int64_t head_dim, bool post_norms, bool layer_norm) {
+  const b2b::ChainDims d = chain_dims(hidden, ffn, n_q, n_kv, head_dim, 1, 0, false, post_norms, layer_norm, 1e-5, 0.0, 1.0, 0.0);
   return b2b::layer_chain_supported(d) && b2b::layer_chain_init(d) > 0;
 }
 
@@ -1132,7 +1149,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   py::class_<LayerChain>(m, "LayerChain")
       .def(py::init<const std::vector<std::vector<Tensor>>&, const std::vector<int64_t>&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
-                    const Tensor&, const OptT&, int64_t, int64_t, int64_t, int64_t, bool, double, double, double, double>())
+                    const Tensor&, const OptT&, int64_t, int64_t, int64_t, int64_t, bool, double, double, double, double, bool>())
       .def("run", &LayerChain::run);
   m.def("layer_chain_supported", &layer_chain_supported);
   m.def("layer_chain_gave_up", &b2b::layer_chain_gave_up);

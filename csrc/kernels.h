@@ -45,24 +45,26 @@ unsigned attn_decode_gave_up();
 int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table, const int* q_start,
                        const int* q_len, const int* kv_len, int seqs, int max_pages, int n_tokens, int n_pages, int n_q, int n_kv,
                        int head_dim, int window, float softcap, void* q_out8, void* q_sf, int q_bn, cudaStream_t s);
-// all layers of a piece for one new token per sequence, up to 64 of them, in one persistent kernel (layer_chain.cu)
+// all layers of a piece for one new token per sequence (LayerNorm models: prompts too), up to 64 of them, in one persistent kernel (layer_chain.cu)
 struct ChainDims {
   int hidden, ffn, n_q, n_kv, head_dim, pages;
-  int act_gelu, plus_one, post_norms;
+  int act_gelu, plus_one, post_norms, layer_norm;
   float eps, rope_theta, q_scale, softcap;
 };
 struct ChainLayerPtrs {
   const void *wqkv, *wo, *wgu, *w_down;
   void *k_cache, *v_cache;
-  const void *post_attn, *post_ffn;      // or null
+  const void *post_attn, *post_ffn;      // weights of the norms behind O and down (LayerNorm models: in front of the MLP and of the next layer), or null
   int window;
+  const void *post_attn_b, *post_ffn_b;  // LayerNorm models
+  const float* bias[4];
 };
 struct ChainCall {
   const void* table;                     // layers x layer_chain_table_bytes(1), filled by layer_chain_fill
   uint32_t* control;                     // layer_chain_control_words(layers), zero before the first launch; launches that share it are ordered
   int layers, tokens, seqs, max_tokens, max_pages;
   const void* x_in;                      // [tokens, hidden]; may be xa
-  void *xa, *xb, *q, *attn, *h, *norm;   // [max_tokens, ..] buffers; the result is in xa
+  void *xa, *xb, *q, *attn, *h, *norm;   // [max_tokens, ..] buffers; the result is in xa (LayerNorm models: norm holds the normed rows of x_in)
   const int *positions, *slots, *q_start, *q_len, *kv_len, *block_table;
 };
 bool layer_chain_supported(const ChainDims& d);

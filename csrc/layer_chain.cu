@@ -13,12 +13,14 @@
 //     quarter of the tokens with st.async, which counts its bytes on the receiver's mbarrier, and are added in the order of K.
 //   * attention as in attn_decode.cu (keys as MMA rows); its cache tiles pass through the same ring, so the pages that the new token does not touch
 //     are fetched while the QKV products run.  Few sequences: the CTAs of a cluster share the keys and merge through DSMEM.
+//   * LayerNorm models with 64-wide heads (GPT-2): the norms are operations of a CTA per token, attention runs on CUDA cores (a warp or a CTA per
+//     token and head), so prompts of up to 64 tokens take the same path.
 //   * the sums of squares for the next norm are left by the CTAs that write the rows, one number per CTA and token, added in a fixed order.
 //
 // Bound: the HBM stream and, between operations, the chain of last product, exchange, store, counter, poll and first activations (3 to 5 us, of
 // which the ring hides most).  Measured on B200, two Llama-3-8B layers, us (kernels one by one / here): one token behind 700 keys 188.5 / 171.5, 32
 // tokens behind 500 keys 217.0 / 193.7, 64 tokens behind 300 (Mistral-7B shapes) 257 / 219; two Gemma-2-2B layers: one token 124 / 106, 30 tokens 128 /
-// 116.  Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
+// 116; all of distilgpt2, prompts of 19 / 60 tokens 267 / 209 and 333 / 254, gpt2, 64 tokens 649 / 507 (42 and 84 operations of 3 to 5 us).  Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
 // All waits are bounded: one that runs out raises the abort word, every other wait then ends too, and the CTAs leave.
 #include "kernels.h"
 
@@ -66,6 +68,9 @@ struct alignas(128) LcLayer {
   __nv_bfloat16* v_cache;
   const __nv_bfloat16* post_attn;                  // weights of the norms behind O and down, or null
   const __nv_bfloat16* post_ffn;
+  const __nv_bfloat16* post_attn_b;                // LayerNorm models: the norms in front of the MLP and of the next layer, and their biases
+  const __nv_bfloat16* post_ffn_b;
+  const float* bias[4];                            // of the products
   int window;
 };
 
@@ -77,7 +82,7 @@ struct LcMaps {                                    // activations: boxes of kXBl
 
 struct LcParams {
   const LcLayer* layers;
-  int n_layers, T, seqs, hidden, ffn, n_q, n_kv, parts;
+  int n_layers, T, seqs, hidden, ffn, n_q, n_kv, head_dim, parts;
   int act, plus_one, norms, x_rows;
   float eps, rope_theta, q_scale, softcap;
   const __nv_bfloat16* x_in;
@@ -228,13 +233,14 @@ __device__ __forceinline__ void lc_st_heads(uint32_t taddr, const float* v) {
 struct LcShare {
   int u0, end, kb0, nkb;
 };
+template <bool GLU>
 __device__ LcShare lc_share(const LcParams& p, int op, int head_dim) {
   LcShare s;
   const int c = blockIdx.x / LC_CL, nc = gridDim.x / LC_CL, r = blockIdx.x % LC_CL;
   const int rows = op == OP_QKV ? (p.n_q + 2 * p.n_kv) * head_dim : p.hidden;
   const int nk = (op == OP_DOWN ? p.ffn : (op == OP_O ? p.n_q * head_dim : p.hidden)) / 64;
   const int u = (op == OP_GU ? p.ffn : rows) / 8, most = (u + nc - 1) / nc;
-  int g = op == OP_GU ? 8 : 4;
+  int g = GLU && op == OP_GU ? 8 : 4;
   while (g > 1 && (u % g != 0 || (u / g + nc - 1) / nc * g * 25 > most * 26)) g /= 2;
   s.u0 = u / g * c / nc * g;
   s.end = u / g * (c + 1) / nc * g;
@@ -243,8 +249,10 @@ __device__ LcShare lc_share(const LcParams& p, int op, int head_dim) {
   return s;
 }
 // units of the tile that starts at u: up to 128 rows, gate/up tiles do not cross the 64-feature blocks of their rows
-__device__ __forceinline__ int lc_tile(int op, int u, int end) { return min(op == OP_GU ? 8 - (u & 7) : 16, end - u); }
-__device__ __forceinline__ int lc_rows(int op, int n) { return op == OP_GU ? n * 16 : n * 8; }
+template <bool GLU>
+__device__ __forceinline__ int lc_tile(int op, int u, int end) { return min(GLU && op == OP_GU ? 8 - (u & 7) : 16, end - u); }
+template <bool GLU>
+__device__ __forceinline__ int lc_rows(int op, int n) { return GLU && op == OP_GU ? n * 16 : n * 8; }
 
 // The ring holds entries of any size back to back (slots of a fixed size would be half empty in a tile of 64 rows): all roles walk the same list and
 // find the same places.
@@ -280,7 +288,8 @@ struct LcFill : LcRing<BYTES> {
   }
 };
 // weights of a tile per block of K: gate/up tiles of fewer than 64 features have their up rows at row 64 all the same
-__device__ __forceinline__ uint32_t lc_block_bytes(int op, int n) { return (op == OP_GU ? 8u + n : n) * 1024u; }
+template <bool GLU>
+__device__ __forceinline__ uint32_t lc_block_bytes(int op, int n) { return (GLU && op == OP_GU ? 8u + n : n) * 1024u; }
 
 // one (sequence, key/value head): this CTA's share of its key tiles
 struct LcItem {
@@ -305,10 +314,13 @@ __device__ __forceinline__ LcItem lc_item(const LcParams& p, const int* kvlen_s,
   return it;
 }
 
-// D: channels of a head, GP: query heads of a key/value head rounded up to 4 or 8
-template <int BN, int D, int GP>
+// D: channels of a head, GP: query heads of a key/value head rounded up to 4 or 8.  LN: LayerNorm models with biases, an MLP without a gate and 64-wide
+// heads (the norms are operations in front of the products; prompts too)
+template <int BN, int D, int GP, bool LN>
 __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid_constant__ LcMaps maps, const LcParams p) {
   using Cfg = LcCfg<BN>;
+  constexpr bool GLU = !LN;
+  const int hd = LN ? p.head_dim : D;               // channels of a head
   constexpr int XB = Cfg::kXBlocks, CW = Cfg::kCols, DB = D / 64, MB = D / 128, NQ = 2 / MB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -371,12 +383,26 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   }
   if (warp == 2)
     for (int op = lane; op < OP_COUNT; op += 32)
-      if (lc_weight(op) >= 0) share_s[lc_weight(op)] = lc_share(p, op, D);
-  if (warp > 2)
+      if (lc_weight(op) >= 0) share_s[lc_weight(op)] = lc_share<GLU>(p, op, hd);
+  if constexpr (LN) {                              // per token: its sequence (-1: none) and the keys that it sees
+    for (int t = threadIdx.x; t < p.T; t += LC_THREADS) {
+      int seq = -1, keys = 0;
+      for (int i = 0; i < p.seqs; ++i) {
+        const int o = t - p.q_start[i], n = p.q_len[i];
+        if (o >= 0 && o < n) {
+          seq = i;
+          keys = max(p.kv_len[i] - n + o + 1, 0);
+        }
+      }
+      q_start_s[t] = seq;
+      kvlen_s[t] = keys;
+    }
+  } else if (warp > 2) {
     for (int i = threadIdx.x - 96; i < p.seqs; i += LC_THREADS - 96) {
       kvlen_s[i] = p.q_len[i] > 0 ? max(p.kv_len[i], 0) : 0;
       q_start_s[i] = p.q_start[i];
     }
+  }
   if (warp == 1) tmem_alloc<Cfg::kTmem>(tmem_slot);
   tc_fence_before();
   __syncthreads();
@@ -390,7 +416,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   const int item0 = blockIdx.x / p.parts, part = blockIdx.x % p.parts, item_step = gridDim.x / p.parts, items = p.seqs * p.n_kv;
   const uint32_t x_bytes = static_cast<uint32_t>(p.x_rows) * 128u;     // activations per block of K
   const uint32_t x_slots = Cfg::kX / (x_bytes * XB);
-  auto skip = [&](int op) { return !norms && (op == OP_NORM_A || op == OP_NORM_F); };
+  auto skip = [&](int l, int op) {                 // (LayerNorm models: the norm in front of the next layer)
+    return LN ? (op == OP_NORM_F && l == p.n_layers - 1) : (!norms && (op == OP_NORM_A || op == OP_NORM_F));
+  };
   // (every role walks the operations in loops whose bodies appear once: a kernel of 250 KB of code spent microseconds per operation on
   // fetching its instructions)
 
@@ -416,19 +444,19 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
         }
 #pragma unroll 1
         for (int op = 0; ok && op < OP_COUNT; ++op) {
-          if (skip(op)) continue;
+          if (skip(l, op)) continue;
           ++at;
           if (lc_weight(op) >= 0) {
             const LcShare sh = share_s[lc_weight(op)];
             const CUtensorMap* maps_w = L->w[lc_weight(op)];
 #pragma unroll 1
             for (int u = sh.u0, n; ok && u < sh.end; u += n) {
-              n = lc_tile(op, u, sh.end);
+              n = lc_tile<GLU>(op, u, sh.end);
               // up to five boxes per block: rows of gate/up come in blocks of [64 gate | 64 up]: gate to rows 0.., up to rows 64.. of the tile
-              const bool halves = op == OP_GU && n < 8;
-              const int units = (op == OP_GU && !halves) ? 16 : n;
-              const int row0 = op == OP_GU ? (u >> 3) * 128 + (u & 7) * 8 : u * 8;
-              const uint32_t bytes = static_cast<uint32_t>(lc_rows(op, n)) * 128u, block = lc_block_bytes(op, n);
+              const bool halves = GLU && op == OP_GU && n < 8;
+              const int units = (GLU && op == OP_GU && !halves) ? 16 : n;
+              const int row0 = GLU && op == OP_GU ? (u >> 3) * 128 + (u & 7) * 8 : u * 8;
+              const uint32_t bytes = static_cast<uint32_t>(lc_rows<GLU>(op, n)) * 128u, block = lc_block_bytes<GLU>(op, n);
 #pragma unroll 1
               for (int kb = 0; kb < sh.nkb; kb += 2) {
                 const int nb = min(2, sh.nkb - kb);
@@ -458,7 +486,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                 }
               }
             }
-          } else if (op == OP_ATT) {
+          } else if (!LN && op == OP_ATT) {
             bool appended = false;                   // the rows of the new tokens are in the cache
             auto pages = [&](const LcItem& it, int n) {          // of a tile
               const int page = 2 * (it.t0 + n), *bt = p.block_table + static_cast<size_t>(it.seq) * p.max_pages;
@@ -514,7 +542,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
         const int window = p.layers[l].window;
 #pragma unroll 1
         for (int op = 0; ok && op < OP_COUNT; ++op) {
-          if (skip(op)) continue;
+          if (skip(l, op)) continue;
           if (at > 0) {                              // the operations so far are complete: this thread alone polls, the others of the CTA look at due_s
             if (!(ok = lc_wait_op(ctr + at - 1, ctas, abort, p.ctl))) break;
             asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(due_s)), "r"(at) : "memory");
@@ -525,7 +553,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             const LcShare sh = share_s[lc_weight(op)];
             const CUtensorMap* m = op == OP_QKV ? (l == 0 ? &maps.x_in : &maps.xa) : (op == OP_O ? &maps.attn : (op == OP_GU ? &maps.xb : &maps.h));
 #pragma unroll 1
-            for (int u = sh.u0; ok && u < sh.end; u += lc_tile(op, u, sh.end))
+            for (int u = sh.u0; ok && u < sh.end; u += lc_tile<GLU>(op, u, sh.end))
 #pragma unroll 1
               for (int kb = 0; kb < sh.nkb; kb += XB) {      // (whole copies, also where fewer blocks are left: they are not used)
                 if (!(ok = ma_wait(&x_empty[s], ph ^ 1u, abort))) break;
@@ -533,7 +561,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                 tma_load_3d_hint(x_s + s * x_bytes * XB, m, &x_full[s], 0, 0, sh.kb0 + kb, pol);
                 if (++s == x_slots) { s = 0; ph ^= 1u; }
               }
-          } else if (op == OP_ATT) {
+          } else if (!LN && op == OP_ATT) {
 #pragma unroll 1
             for (int j = item0; ok && j < items; j += item_step) {
               const LcItem it = lc_item(p, kvlen_s, window, j, part);
@@ -572,8 +600,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             const LcShare sh = share_s[lc_weight(op)];
 #pragma unroll 1
             for (int u = sh.u0, n; ok && u < sh.end; u += n, ++na) {
-              n = lc_tile(op, u, sh.end);
-              const uint32_t block = lc_block_bytes(op, n);
+              n = lc_tile<GLU>(op, u, sh.end);
+              const uint32_t block = lc_block_bytes<GLU>(op, n);
               if (!(ok = ma_wait(&acc_empty[na & 1u], ((na >> 1) & 1u) ^ 1u, abort))) break;
               tc_fence_after();
               const uint32_t acc = tmem + (na & 1u) * BN;
@@ -611,7 +639,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               }
               umma_commit(&acc_full[na & 1u]);
             }
-          } else if (op == OP_ATT) {
+          } else if (!LN && op == OP_ATT) {
 #pragma unroll 1
             for (int j = item0; ok && j < items; j += item_step) {
               const LcItem it = lc_item(p, kvlen_s, window, j, part);
@@ -675,7 +703,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
     const int et = threadIdx.x - 64, q4 = warp & 3, row = q4 * 32 + lane;
     const int col0 = rank * CW;                        // the tokens that this CTA finishes
     const uint32_t lanes = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
-    const int q_dim = p.n_q * D, kv_dim = p.n_kv * D;
+    const int q_dim = p.n_q * hd, kv_dim = p.n_kv * hd;
     const float inv_cap = p.softcap > 0.f ? 1.f / p.softcap : 0.f, log_theta = p.rope_theta > 0.f ? log2f(p.rope_theta) : 0.f;
     uint32_t na = 0, nx = 0, nt_all = 0, nparts = 0;   // accumulators, exchanges, key tiles, merges so far
     int at = 0;                                        // operations so far, over the layers
@@ -688,7 +716,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
       __nv_bfloat16 *const k_cache = L->k_cache, *const v_cache = L->v_cache;
 #pragma unroll 1
       for (int op = 0; op < OP_COUNT; ++op) {
-        if (skip(op)) continue;
+        if (skip(l, op)) continue;
         if (lc_weight(op) >= 0) {
           // ----------------------------------------------------------------------------------------------------- products
           const LcShare sh = share_s[lc_weight(op)];
@@ -696,6 +724,16 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           // O and down: + residual, unless a norm follows; then the sums of squares of the rows are left for the norm in the next product
           const __nv_bfloat16* residual = norms ? nullptr : (op == OP_O ? x : p.xb);
           __nv_bfloat16* out = norms ? p.norm : (op == OP_O ? p.xb : p.xa);
+          int ld = p.hidden;
+          const float* bias = nullptr;
+          if constexpr (LN) {
+            bias = L->bias[lc_weight(op)];
+            if (op == OP_GU) {
+              residual = nullptr;
+              out = p.h;
+              ld = p.ffn;
+            }
+          }
           float sq[CW];
 #pragma unroll
           for (int i = 0; i < CW; ++i) sq[i] = 0.f;
@@ -705,7 +743,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             pos_s[et] = (p.positions != nullptr && t < p.T) ? p.positions[t] : 0;
             slot_s[et] = t < p.T ? p.slots[t] : -1;
           }
-          if (work && op == OP_QKV && l == 0) {        // 1/rms of the rows: a warp per row
+          if (LN) {                                    // (the activations are normed)
+          } else if (work && op == OP_QKV && l == 0) { // 1/rms of the rows: a warp per row
             const int k8 = p.hidden / 8;
 #pragma unroll 1
             for (int t = warp - 2; t < CW; t += 4) {
@@ -739,12 +778,13 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           lc_sync();
 #pragma unroll 1
           for (int u = sh.u0, n; u < sh.end; u += n) {
-            n = lc_tile(op, u, sh.end);
+            n = lc_tile<GLU>(op, u, sh.end);
             const int feat = u * 8 + row;
-            const bool live = op == OP_GU ? (row & 63) < n * 8 : row < n * 8;
+            const bool live = GLU && op == OP_GU ? (row & 63) < n * 8 : row < n * 8;
+            const float bias_v = LN && live ? bias[feat] : 0.f;
             const int sect = feat < q_dim ? 0 : (feat < q_dim + kv_dim ? 1 : 2);                  // (of QKV)
             const int fs = feat - (sect == 0 ? 0 : (sect == 1 ? q_dim : q_dim + kv_dim));
-            const bool turn = sect < 2 && p.rope_theta > 0.f;
+            const bool turn = !LN && sect < 2 && p.rope_theta > 0.f;
             float c1[CW], c2[CW];                      // cosines and sines | residual
             if (op == OP_QKV) {
               const float freq = turn ? exp2f(-(2.f * ((fs % D) >> 1) / static_cast<float>(D)) * log_theta) : 0.f;
@@ -754,7 +794,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                 c2[i] = 0.f;
                 if (turn && col0 + i < p.T) sincosf(static_cast<float>(pos_s[i]) * freq, &c2[i], &c1[i]);
               }
-            } else if (op != OP_GU) {
+            } else if (LN || op != OP_GU) {
 #pragma unroll
               for (int i = 0; i < CW; ++i)
                 c1[i] = (residual != nullptr && live && col0 + i < p.T) ? __bfloat162float(residual[static_cast<size_t>(col0 + i) * p.hidden + feat]) : 0.f;
@@ -771,7 +811,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               if (lane == 0) mbar_arrive(&acc_empty[na & 1u]);
               ++na;
               if (nx > 0 && ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(zone_free, (nx - 1) & 1u, abort));
-              if (threadIdx.x == 64) mbar_arrive_expect_tx(zone_full, static_cast<uint32_t>(lc_rows(op, n) * LC_CL * CW * 4));
+              if (threadIdx.x == 64) mbar_arrive_expect_tx(zone_full, static_cast<uint32_t>(lc_rows<GLU>(op, n) * LC_CL * CW * 4));
               if (live && ok) {
 #pragma unroll
                 for (int d = 0; d < LC_CL; ++d) {
@@ -796,7 +836,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             }
             constexpr int HB = CW / 2;
             const bool up = row >= 64;                 // gate/up: the up half finishes the second half of the tokens, the gate half the first
-            if (op == OP_GU) {
+            if (GLU && op == OP_GU) {
               float* xch = reinterpret_cast<float*>(zone);         // [HB tokens][64] up values of the first half, then gate values of the second
               lc_sync();                               // the sums have been read
               float* to = xch + (up ? 0 : HB * 64) + (row & 63);
@@ -809,7 +849,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             }
             __syncwarp();
             if (lane < LC_CL) arrive_cluster(mapa_smem(smem_u32(zone_free), lane));               // the sums have been read
-            if (op == OP_GU) {
+            if (GLU && op == OP_GU) {
               const int t0 = up ? HB : 0;
 #pragma unroll
               for (int i = 0; i < HB; ++i) {
@@ -823,7 +863,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               for (int i = 0; i < CW; ++i) {
                 const int tok = col0 + i;
                 if (tok >= p.T) break;                 // (the same for the warp)
-                const float a = v[i] * rstd_s[i];
+                const float a = LN ? v[i] + bias_v : v[i] * rstd_s[i];
                 // lanes (2j, 2j + 1) hold (x_j, x_{j + D / 2}) thanks to the row order of the weights
                 const float b = __shfl_xor_sync(0xffffffffu, a, 1);
                 const float o = turn ? ((lane & 1) ? (a * c1[i] + b * c2[i]) : (a * c1[i] - b * c2[i])) : a;
@@ -838,13 +878,18 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
 #pragma unroll
               for (int i = 0; i < CW; ++i) {
                 if (col0 + i >= p.T) break;
-                const __nv_bfloat16 r = __float2bfloat16_rn(v[i] + c1[i]);
-                out[static_cast<size_t>(col0 + i) * p.hidden + feat] = r;
+                float a = v[i] + c1[i];
+                if constexpr (LN) {
+                  a += bias_v;
+                  if (op == OP_GU) a = gelu_tanh(a);
+                }
+                const __nv_bfloat16 r = __float2bfloat16_rn(a);
+                out[static_cast<size_t>(col0 + i) * ld + feat] = r;
                 sq[i] += __bfloat162float(r) * __bfloat162float(r);
               }
             }
           }
-          if (!norms && (op == OP_O || op == OP_DOWN)) {
+          if (!LN && !norms && (op == OP_O || op == OP_DOWN)) {
 #pragma unroll
             for (int i = 0; i < CW; ++i) {
 #pragma unroll
@@ -854,7 +899,105 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             lc_sync();
             if (et < CW) p.ss[(op == OP_O ? LC_SS : 0) + blockIdx.x / LC_CL * 64 + col0 + et] = sq_s[0][et] + sq_s[1][et] + sq_s[2][et] + sq_s[3][et];
           }
-        } else if (op == OP_ATT) {
+        } else if (LN && op == OP_ATT) {
+          // ---- attention of 64-wide heads, prompts and decode: a lane per key for the scores, two channels per lane for the values.  A (token, head)
+          // per warp while no token sees more than 128 keys, else per CTA, whose warps take every fourth run of 32 keys.  Bound by the latency
+          // of three dependent loads (page, key, value rows), so a run's rows are all fetched before the first is used.
+          float* q_s = reinterpret_cast<float*>(zone) + (warp - 2) * 64;           // per warp: the query
+          float *o_s = reinterpret_cast<float*>(zone) + 256, *m_s = o_s + 256, *l_s = m_s + 4;         // the warps' sums, maxima, sums of the weights
+          if (ok) ok = __all_sync(0xffffffffu, lc_wait_due(due_s, at, abort));
+          int most = 0;
+          for (int t = lane; t < p.T; t += 32) most = max(most, kvlen_s[t]);
+          for (int i = 16; i > 0; i >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, i));
+          const int w = warp - 2, parts = most > 128 ? 4 : 1, part = parts == 4 ? w : 0;
+#pragma unroll 1
+          for (int j = parts == 4 ? blockIdx.x : blockIdx.x * 4 + w; j < p.T * p.n_q; j += parts == 4 ? gridDim.x : gridDim.x * 4) {
+            const int t = j / p.n_q, head = j - t * p.n_q, seq = q_start_s[t], keys = kvlen_s[t];
+            if (seq < 0) continue;                     // (parts == 4: the same for the CTA)
+            const int kvh = head / (p.n_q / p.n_kv);
+            const int* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
+            const __nv_bfloat162 q2 = __ldcg(reinterpret_cast<const __nv_bfloat162*>(p.q + static_cast<size_t>(t) * q_dim + head * 64) + lane);
+            float m = -INFINITY, lsum = 0.f, o0 = 0.f, o1 = 0.f;
+            bool first = true;
+#pragma unroll 1
+            for (int k0 = part * 32; k0 < keys; k0 += parts * 32) {
+              const size_t row0 = (static_cast<size_t>(bt[k0 / LC_PAGE]) * LC_PAGE + k0 % LC_PAGE) * kv_dim + kvh * 64;      // (32 keys lie in one page)
+              const bool seen = k0 + lane < keys && (window <= 0 || k0 + lane >= keys - window);
+              const int n = min(32, keys - k0);
+              uint4 kv[8];
+              __nv_bfloat162 vv[32];
+              const uint4* src = reinterpret_cast<const uint4*>(k_cache + row0 + static_cast<size_t>(lane) * kv_dim);
+              const __nv_bfloat162* vsrc = reinterpret_cast<const __nv_bfloat162*>(v_cache + row0) + lane;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) kv[i] = seen ? __ldcg(src + i) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) vv[i] = i < n ? __ldcg(vsrc + static_cast<size_t>(i) * (kv_dim / 2)) : __floats2bfloat162_rn(0.f, 0.f);
+              if (first) {                             // (behind the rows' loads)
+                const float2 f = __bfloat1622float2(q2);
+                q_s[2 * lane] = f.x;
+                q_s[2 * lane + 1] = f.y;
+                __syncwarp();
+                first = false;
+              }
+              float s = 0.f;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&kv[i]);
+                const float4 qa = *reinterpret_cast<const float4*>(q_s + 8 * i), qb = *reinterpret_cast<const float4*>(q_s + 8 * i + 4);
+                const float2 f0 = __bfloat1622float2(h[0]), f1 = __bfloat1622float2(h[1]), f2 = __bfloat1622float2(h[2]), f3 = __bfloat1622float2(h[3]);
+                s += f0.x * qa.x + f0.y * qa.y + f1.x * qa.z + f1.y * qa.w + f2.x * qb.x + f2.y * qb.y + f3.x * qb.z + f3.y * qb.w;
+              }
+              s = seen ? s * LC_LOG2E : -INFINITY;
+              if (!__any_sync(0xffffffffu, !(s == -INFINITY))) continue;           // (no key of this run is seen; a NaN score goes on)
+              float top = s;
+#pragma unroll
+              for (int i = 16; i > 0; i >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, i));
+              top = fmaxf(top, m);
+              const float e = ex2(s - top), a = m == -INFINITY ? 0.f : ex2(m - top);
+              m = top;
+              lsum = lsum * a + e;
+              o0 *= a;
+              o1 *= a;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const float2 f = __bfloat1622float2(vv[i]);
+                const float pw = __shfl_sync(0xffffffffu, e, i);
+                if (i < n) {
+                  o0 += pw * f.x;
+                  o1 += pw * f.y;
+                }
+              }
+            }
+#pragma unroll
+            for (int i = 16; i > 0; i >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, i);
+            __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(p.attn + static_cast<size_t>(t) * q_dim + head * 64) + lane;
+            if (parts == 1) {
+              if (ok) *out = lsum == 0.f ? __floats2bfloat162_rn(0.f, 0.f) : __floats2bfloat162_rn(o0 / lsum, o1 / lsum);
+              __syncwarp();                            // the query has been read
+              continue;
+            }
+            o_s[w * 64 + 2 * lane] = o0;
+            o_s[w * 64 + 2 * lane + 1] = o1;
+            if (lane == 0) {
+              m_s[w] = m;
+              l_s[w] = lsum;
+            }
+            lc_sync();
+            if (w == 0 && ok) {
+              const float top = fmaxf(fmaxf(m_s[0], m_s[1]), fmaxf(m_s[2], m_s[3]));
+              float n0 = 0.f, n1 = 0.f, den = 0.f;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float a = m_s[i] == -INFINITY ? 0.f : ex2(m_s[i] - top);
+                n0 += a * o_s[i * 64 + 2 * lane];
+                n1 += a * o_s[i * 64 + 2 * lane + 1];
+                den += a * l_s[i];
+              }
+              *out = den == 0.f ? __floats2bfloat162_rn(0.f, 0.f) : __floats2bfloat162_rn(n0 / den, n1 / den);
+            }
+            lc_sync();                                 // the sums have been read
+          }
+        } else if (!LN && op == OP_ATT) {
           // ---------------------------------------------------------------------------------------------------- attention
 #pragma unroll 1
           for (int j = item0; j < items; j += item_step) {
@@ -1007,6 +1150,73 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             }
             lc_sync();                                 // the sums of the rows have been read
           }
+        } else if (LN) {
+          // ------------------------------------------------------------------------- out = LayerNorm(x): a CTA per token
+          const __nv_bfloat16* w = op == OP_NORM_A ? L->post_attn : L->post_ffn;
+          const __nv_bfloat16* wb = op == OP_NORM_A ? L->post_attn_b : L->post_ffn_b;
+          const __nv_bfloat16* src = op == OP_NORM_A ? p.xb : p.xa;
+          const int k8 = p.hidden / 8;
+#pragma unroll 1
+          for (int t = blockIdx.x; t < p.T; t += gridDim.x) {
+            constexpr int C = 4;                       // chunks of 8 channels per thread (hidden <= 4096)
+            uint4 xv[C], g[C], b[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              const int i = et + 128 * c;
+              xv[c] = g[c] = b[c] = make_uint4(0, 0, 0, 0);
+              if (i < k8) {
+                g[c] = reinterpret_cast<const uint4*>(w)[i];
+                b[c] = reinterpret_cast<const uint4*>(wb)[i];
+              }
+            }
+            if (ok) ok = __all_sync(0xffffffffu, lc_wait_due(due_s, at, abort));
+            float sum = 0.f, ss = 0.f;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              if (et + 128 * c < k8) xv[c] = __ldcg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * p.hidden) + et + 128 * c);
+              const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&xv[c]);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 f = __bfloat1622float2(h[j]);
+                sum += f.x + f.y;
+              }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (lane == 0) red_s[q4][0] = sum;
+            lc_sync();
+            const float mean = (red_s[0][0] + red_s[1][0] + red_s[2][0] + red_s[3][0]) / p.hidden;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&xv[c]);
+              if (et + 128 * c < k8)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float2 f = __bfloat1622float2(h[j]);
+                  ss += (f.x - mean) * (f.x - mean) + (f.y - mean) * (f.y - mean);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lane == 0) sq_s[q4][0] = ss;
+            lc_sync();
+            const float rs = rsqrtf((sq_s[0][0] + sq_s[1][0] + sq_s[2][0] + sq_s[3][0]) / p.hidden + p.eps);
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+              if (et + 128 * c < k8 && ok) {
+                uint4 o;
+                const __nv_bfloat162* hx = reinterpret_cast<const __nv_bfloat162*>(&xv[c]);
+                const __nv_bfloat162* hg = reinterpret_cast<const __nv_bfloat162*>(&g[c]);
+                const __nv_bfloat162* hb = reinterpret_cast<const __nv_bfloat162*>(&b[c]);
+                __nv_bfloat162* ho = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float2 f = __bfloat1622float2(hx[j]), fg = __bfloat1622float2(hg[j]), fb = __bfloat1622float2(hb[j]);
+                  ho[j] = __floats2bfloat162_rn((f.x - mean) * rs * fg.x + fb.x, (f.y - mean) * rs * fg.y + fb.y);
+                }
+                reinterpret_cast<uint4*>(p.norm + static_cast<size_t>(t) * p.hidden)[et + 128 * c] = o;
+              }
+          }
         } else {
           // ------------------------------------------------------------- out = residual + rmsnorm(x) w: a CTA per token
           const __nv_bfloat16* w = op == OP_NORM_A ? L->post_attn : L->post_ffn;
@@ -1117,7 +1327,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
 }
 
 // clusters of four that fit the device at once with this kernel, 0 if it cannot run
-template <int BN, int D, int GP>
+template <int BN, int D, int GP, bool LN>
 int chain_clusters() {
   static int known[64] = {};
   int dev = 0;
@@ -1125,7 +1335,7 @@ int chain_clusters() {
   if (dev < 64 && known[dev] != 0) return known[dev] - 1;
   int n = 0, coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  if (coop && cudaFuncSetAttribute(layer_chain_kernel<BN, D, GP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcCfg<BN>::kSmem) == cudaSuccess) {
+  if (coop && cudaFuncSetAttribute(layer_chain_kernel<BN, D, GP, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcCfg<BN>::kSmem) == cudaSuccess) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(LC_CL * 64);
     cfg.blockDim = dim3(LC_THREADS);
@@ -1136,16 +1346,16 @@ int chain_clusters() {
     a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
     cfg.attrs = a;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, layer_chain_kernel<BN, D, GP>, &cfg) != cudaSuccess) n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, layer_chain_kernel<BN, D, GP, LN>, &cfg) != cudaSuccess) n = 0;
   }
   cudaGetLastError();
   if (dev < 64) known[dev] = n + 1;
   return n;
 }
 
-template <int BN, int D, int GP>
+template <int BN, int D, int GP, bool LN>
 int launch_chain_one(const LcMaps& maps, LcParams p, cudaStream_t s) {
-  const int clusters = std::min(chain_clusters<BN, D, GP>(), 64);
+  const int clusters = std::min(chain_clusters<BN, D, GP, LN>(), 64);
   if (clusters <= 0) return -5;
   const int ctas = clusters * LC_CL, items = p.seqs * p.n_kv;
   p.parts = items * 4 <= ctas ? 4 : (items * 2 <= ctas ? 2 : 1);     // few sequences: CTAs of a cluster share the keys of one
@@ -1162,12 +1372,13 @@ int launch_chain_one(const LcMaps& maps, LcParams p, cudaStream_t s) {
   a[1].val.cooperative = 1;
   cfg.attrs = a;
   cfg.numAttrs = 2;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, layer_chain_kernel<BN, D, GP>, maps, p));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, layer_chain_kernel<BN, D, GP, LN>, maps, p));
 }
 
 #define B2B_CHAIN(FN, BN, ...) \
-  (d.head_dim == 128 ? (g <= 4 ? FN<BN, 128, 4>(__VA_ARGS__) : FN<BN, 128, 8>(__VA_ARGS__)) \
-                     : (g <= 4 ? FN<BN, 256, 4>(__VA_ARGS__) : FN<BN, 256, 8>(__VA_ARGS__)))
+  (d.layer_norm ? FN<BN, 128, 4, true>(__VA_ARGS__) : \
+   d.head_dim == 128 ? (g <= 4 ? FN<BN, 128, 4, false>(__VA_ARGS__) : FN<BN, 128, 8, false>(__VA_ARGS__)) \
+                     : (g <= 4 ? FN<BN, 256, 4, false>(__VA_ARGS__) : FN<BN, 256, 8, false>(__VA_ARGS__)))
 
 }  // namespace
 
@@ -1176,9 +1387,10 @@ size_t layer_chain_control_words(int layers) { return (LW_CTR + static_cast<size
 
 bool layer_chain_supported(const ChainDims& d) {
   const int g = d.n_kv > 0 ? d.n_q / d.n_kv : 0;
-  return d.n_kv > 0 && d.n_q % d.n_kv == 0 && g <= 8 && (d.head_dim == 128 || d.head_dim == 256) && g * d.head_dim * 4 <= 8192 &&
-         d.hidden % 128 == 0 && d.hidden >= 256 && d.ffn % 64 == 0 && d.ffn >= 256 && d.n_q * d.head_dim >= 256 &&
-         (!d.post_norms || d.hidden <= 4096);
+  if (d.n_kv <= 0 || d.n_q % d.n_kv != 0 || d.hidden % 128 != 0 || d.hidden < 256 || d.ffn % 64 != 0 || d.ffn < 256 || d.n_q * d.head_dim < 256)
+    return false;
+  if (d.layer_norm) return d.head_dim == 64 && (d.n_q * 64) % 128 == 0 && (d.n_kv * 64) % 128 == 0 && d.ffn % 128 == 0 && d.hidden <= 4096;
+  return g <= 8 && (d.head_dim == 128 || d.head_dim == 256) && g * d.head_dim * 4 <= 8192 && (!d.post_norms || d.hidden <= 4096);
 }
 
 // tensor maps and pointers of one layer at `dst` (host memory)
@@ -1187,7 +1399,7 @@ int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w) {
   std::memset(&L, 0, sizeof(L));
   const int q_dim = d.n_q * d.head_dim, kv_dim = d.n_kv * d.head_dim;
   const void* ptr[4] = {w.wqkv, w.wo, w.wgu, w.w_down};
-  const uint64_t rows[4] = {static_cast<uint64_t>(q_dim + 2 * kv_dim), static_cast<uint64_t>(d.hidden), 2ull * d.ffn, static_cast<uint64_t>(d.hidden)};
+  const uint64_t rows[4] = {static_cast<uint64_t>(q_dim + 2 * kv_dim), static_cast<uint64_t>(d.hidden), (d.layer_norm ? 1ull : 2ull) * d.ffn, static_cast<uint64_t>(d.hidden)};
   const uint64_t cols[4] = {static_cast<uint64_t>(d.hidden), static_cast<uint64_t>(q_dim), static_cast<uint64_t>(d.hidden), static_cast<uint64_t>(d.ffn)};
   for (int i = 0; i < 4; ++i)
     for (int b = 0; b < 5; ++b)
@@ -1199,6 +1411,9 @@ int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w) {
   L.v_cache = static_cast<__nv_bfloat16*>(w.v_cache);
   L.post_attn = static_cast<const __nv_bfloat16*>(w.post_attn);
   L.post_ffn = static_cast<const __nv_bfloat16*>(w.post_ffn);
+  L.post_attn_b = static_cast<const __nv_bfloat16*>(w.post_attn_b);
+  L.post_ffn_b = static_cast<const __nv_bfloat16*>(w.post_ffn_b);
+  for (int i = 0; i < 4; ++i) L.bias[i] = w.bias[i];
   L.window = w.window;
   std::memcpy(dst, &L, sizeof(L));
   return 0;
@@ -1206,19 +1421,22 @@ int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w) {
 
 int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
   const int g = d.n_kv > 0 ? d.n_q / d.n_kv : 0;
-  if (!layer_chain_supported(d) || c.tokens < 1 || c.tokens > 64 || c.layers < 1) return -2;
+  if (!layer_chain_supported(d) || c.tokens < 1 || c.tokens > 64 || c.layers < 1 || (!d.layer_norm && c.seqs > c.tokens)) return -2;
   const int bn = c.tokens <= 16 ? 16 : (c.tokens <= 32 ? 32 : 64), x_rows = c.tokens <= 8 ? 8 : bn, q_dim = d.n_q * d.head_dim;
   LcMaps m;
   auto act = [&](CUtensorMap* t, const void* ptr, uint64_t rows, int cols) { return make_blocks_tmap(t, ptr, rows, cols, x_rows, bn == 16 ? LcCfg<16>::kXBlocks : LcCfg<32>::kXBlocks); };
   int r;
-  if ((r = act(&m.x_in, c.x_in, c.tokens, d.hidden)) || (r = act(&m.xa, c.xa, c.max_tokens, d.hidden)) || (r = act(&m.xb, c.xb, c.max_tokens, d.hidden)) ||
+  // (LayerNorm models: the products read the normed rows)
+  const void *x_in = d.layer_norm ? c.norm : c.x_in, *xa = d.layer_norm ? c.norm : c.xa, *xb = d.layer_norm ? c.norm : c.xb;
+  if ((r = act(&m.x_in, x_in, d.layer_norm ? c.max_tokens : c.tokens, d.hidden)) || (r = act(&m.xa, xa, c.max_tokens, d.hidden)) ||
+      (r = act(&m.xb, xb, c.max_tokens, d.hidden)) ||
       (r = act(&m.attn, c.attn, c.max_tokens, q_dim)) || (r = act(&m.h, c.h, c.max_tokens, d.ffn)) ||
       (r = make_tmap_shared(&m.q, c.q, static_cast<uint64_t>(c.max_tokens) * d.n_q, d.head_dim, d.head_dim, LC_HEADS, 2)))
     return r;
   LcParams p;
   p.layers = static_cast<const LcLayer*>(c.table);
   p.n_layers = c.layers; p.T = c.tokens; p.seqs = c.seqs;
-  p.hidden = d.hidden; p.ffn = d.ffn; p.n_q = d.n_q; p.n_kv = d.n_kv; p.parts = 1;
+  p.hidden = d.hidden; p.ffn = d.ffn; p.n_q = d.n_q; p.n_kv = d.n_kv; p.head_dim = d.head_dim; p.parts = 1;
   p.act = d.act_gelu; p.plus_one = d.plus_one; p.norms = d.post_norms; p.x_rows = x_rows;
   p.eps = d.eps; p.rope_theta = d.rope_theta; p.q_scale = d.q_scale; p.softcap = d.softcap;
   p.x_in = static_cast<const __nv_bfloat16*>(c.x_in);

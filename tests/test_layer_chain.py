@@ -141,6 +141,59 @@ def test_graph_replay_sees_new_inputs_and_lengths():
         assert _rel(out, ref) < REL
 
 
+def _gpt2(hidden=256, heads=4, ffn=1024):
+    return dataclasses.replace(resolve_config("tiny-gpt2"), hidden_size=hidden, n_heads=heads, n_kv_heads=heads, head_dim=64, ffn_size=ffn)
+
+
+# spans (new tokens, cached tokens) of the sequences: edges of the token tiles; one key, the edges of a run of 32 and of a page; more than 128 keys (a CTA
+# per token and head) beside short ones; sequences without tokens and rows that belong to none (buckets)
+@pytest.mark.parametrize("spans,pad", [([(1, 0)], 0), ([(19, 0)], 0), ([(8, 0), (8, 57)], 0), ([(16, 31), (1, 64)], 0), ([(5, 0), (0, 0), (11, 3)], 5),
+                                       ([(33, 96)], 0), ([(31, 0), (2, 700)], 4), ([(64, 65)], 0), ([(1, 40 * i) for i in range(20)], 0)])
+@pytest.mark.parametrize("hidden,heads,ffn", [(256, 4, 1024), (768, 12, 3072), (384, 6, 512)])
+def test_layer_norm_models(spans, pad, hidden, heads, ffn):
+    """LayerNorm, biases, an MLP without a gate, 64-wide heads: prompts and decode steps; the norm in front of the first layer is a kernel of its own"""
+    from bee2bee_b200 import ops
+    from bee2bee_b200.models.native import BatchMeta, NativePiece
+
+    cfg, layers = _gpt2(hidden, heads, ffn), 3
+    g = torch.Generator(device="cuda").manual_seed(11)
+    rnd = lambda *shape, std=1.0: (torch.randn(*shape, generator=g, device="cuda") * std).to(torch.bfloat16)  # noqa: E731
+    t = {}
+    for l in range(layers):
+        for n, r, c in (("wq", hidden, hidden), ("wk", hidden, hidden), ("wv", hidden, hidden), ("wo", hidden, hidden), ("w_up", ffn, hidden), ("w_down", hidden, ffn)):
+            t[f"l{l}.{n}"] = rnd(r, c, std=c ** -0.5)
+        for n, m in (("bq", hidden), ("bk", hidden), ("bv", hidden), ("bo", hidden), ("b_up", ffn), ("b_down", hidden)):
+            t[f"l{l}.{n}"] = rnd(m, std=0.1)
+        for n in ("ln1", "ln2"):
+            t[f"l{l}.{n}_w"], t[f"l{l}.{n}_b"] = rnd(hidden, std=0.1) + 1.0, rnd(hidden, std=0.1)
+    need = [(n + c + 63) // 64 for n, c in spans]
+    order = (torch.randperm(sum(need), generator=g, device="cuda") + 1).cpu().tolist()
+    table, slots, at = [], [], 0
+    for (n, c), k in zip(spans, need):
+        table.append(order[at:at + k] + [0] * (max(need) - k))
+        slots += [table[-1][i // 64] * 64 + i % 64 for i in range(c, c + n)]
+        at += k
+    live = len(slots)
+    T = live + pad
+    starts = [sum(n for n, _ in spans[:i]) for i in range(len(spans))]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    ops.native().init_kernels(0)
+    piece = NativePiece(cfg, range(layers), False, False, t, torch.device("cuda", 0), T, len(spans), sum(need) + 1)
+    meta = BatchMeta(ids=None, positions=i32([0] * T), slots=i32(slots + [-1] * pad), q_start=i32(starts), q_len=i32([n for n, _ in spans]),
+                     kv_len=i32([n + c for n, c in spans]), block_table=i32(table), n_tokens=T, n_seqs=len(spans), max_q=max(n for n, _ in spans), bucket=pad > 0)
+    caches = [rnd(*c.shape) for c in list(piece.k_cache.values()) + list(piece.v_cache.values())]
+    x = rnd(T, hidden)
+    ref, ref_caches = _run(piece, meta, caches, x, False)
+    n0 = ops.LAUNCHES[0]
+    out, got = _run(piece, meta, caches, x, True)
+    assert ops.LAUNCHES[0] == n0 + 2
+    # (three layers: sqrt(15) roundings of 2^-9; the old kernels also round the weights of the attention)
+    assert _rel(out[:live], ref[:live]) < 2 * REL
+    assert all(_rel(a, b) < 2 * REL for a, b in zip(got, ref_caches))
+    assert torch.equal(_run(piece, meta, caches, x, True)[0][:live], out[:live])
+    assert ops.native().layer_chain_gave_up() == 0
+
+
 def test_routes():
     """what the persistent kernel does not take runs on the kernels one by one; replaced weights and caches are seen"""
     from bee2bee_b200 import ops

@@ -2,8 +2,8 @@
 hand-written sm_100a kernels in ``csrc/``.
 
 A decode step (one new token per sequence, up to 64; GPT-2: prompts of up to 64 tokens too) of whole bf16 layers is one persistent
-kernel (``csrc/layer_chain.cu``).
-Prompts, quantised weights and pieces of a pipeline: per decoder layer (Llama / Mistral) exactly five launches, all on one stream:
+kernel (``csrc/layer_chain.cu``); in block-scaled fp8 steps of up to 32 tokens are, behind the quantiser of the piece's input.
+Prompts, larger steps, weights with per-row scales and pieces of a pipeline: per decoder layer (Llama / Mistral) exactly five launches, all on one stream:
 
     QKV GEMM  [fused: RMSNorm(x) via folded gamma + in-kernel 1/rms, RoPE, paged-KV append]
     attention [paged KV, GQA]
@@ -233,9 +233,10 @@ class NativePiece:
                                    dtype=torch.float32)
         self._chain = self._chain_of = None
         self._chain_ln = not self.fused_norm and not c.glu and c.bias and not c.post_norms and c.rope_theta <= 0 and c.attn_softcap == 0
-        if units is None and self.layers and (self._chain_ln or (self.fused_norm and c.glu and not self.fp8)) and self.device.type == "cuda":
+        if units is None and self.layers and (self._chain_ln or (self.fused_norm and c.glu and self.fp8 == self.mx_fuse)) and self.device.type == "cuda":
             with torch.cuda.device(dev):
-                if ops.native().layer_chain_supported(c.hidden_size, c.ffn_size, c.n_heads, c.n_kv_heads, c.head_dim, c.post_norms, self._chain_ln):
+                if ops.native().layer_chain_supported(c.hidden_size, c.ffn_size, c.n_heads, c.n_kv_heads, c.head_dim, c.post_norms, self._chain_ln,
+                                                      self.mx_fuse):
                     self._plan_chain()
 
     # ------------------------------------------------------------------ helpers
@@ -245,7 +246,7 @@ class NativePiece:
         if self._chain_ln:
             post = ("bqkv", "bo", "b_up", "b_down", "ln2_w", "ln2_b")
         rows = [[self.w[f"l{l}.{n}"] for n in names] + [self.k_cache[l], self.v_cache[l]] + [self.w[f"l{l}.{n}"] for n in post]
-                for l in self.layers]
+                + ([self.wscale[f"l{l}.{n}"] for n in names] if self.mx_fuse else []) for l in self.layers]
         if self._chain_ln:                     # the norm in front of the next layer
             for row, l in zip(rows, self.layers[1:]):
                 row += [self.w[f"l{l}.ln1_w"], self.w[f"l{l}.ln1_b"]]
@@ -255,16 +256,20 @@ class NativePiece:
         """lays the layers out for the decode kernel (csrc/layer_chain.cu)"""
         c = self.cfg
         t = self._chain_tensors()
+        fp8 = []
+        if self.mx_fuse:
+            H, Q = c.hidden_size, c.q_dim
+            fp8 = [self._qbuf[H], self._qsf[H], self._fq_x, self._fq_sf_x, self._qbuf[Q], self._qsf[Q], self._fq_h, self._fq_sf_h]
         self._chain = ops.native().LayerChain(t, [c.layer_window(l) for l in self.layers], self.xa, self.xb, self.q_buf, self.attn_buf, self.h_buf,
                                               self.n_buf if c.post_norms or self._chain_ln else None, c.n_heads, c.n_kv_heads, c.head_dim,
                                               int(c.act == "gelu_tanh"), c.gemma_norm, c.norm_eps, c.rope_theta, c.softmax_scale, c.attn_softcap,
-                                              self._chain_ln)
+                                              self._chain_ln, fp8)
         self._chain_of = [[x.data_ptr() for x in row] for row in t]
 
     def _chain_takes(self, m: BatchMeta, x: torch.Tensor, hand: Handoff) -> bool:
-        """a decode step (one new token per sequence, up to 64) of whole layers whose input and result stay on this GPU; LayerNorm models:
+        """a decode step (one new token per sequence, up to 64; block-scaled fp8: 32) of whole layers whose input and result stay on this GPU; LayerNorm models:
         prompts of up to 64 tokens too"""
-        if self._chain is None or not 1 <= m.n_tokens <= 64 or not (self._chain_ln or (m.max_q == 1 and m.n_tokens == m.n_seqs)):
+        if self._chain is None or not 1 <= m.n_tokens <= self._chain.step_tokens or not (self._chain_ln or (m.max_q == 1 and m.n_tokens == m.n_seqs)):
             return False
         if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16:
             return False
@@ -358,6 +363,8 @@ class NativePiece:
             x = x_in[:T]
             wait_flag, wait_epoch = hand.in_flag, hand.in_epoch
         if out_x is None and self._chain_takes(m, x, hand):
+            if self.mx_fuse:
+                self._quant(x, with_rms=True)
             if self._chain_ln:
                 ops.layernorm(x, self.w[f"l{self.layers[0]}.ln1_w"], self.w[f"l{self.layers[0]}.ln1_b"], self.n_buf[:T], eps)
             ops.layer_chain(self._chain, x, m.positions, m.slots, m.q_start, m.q_len, m.kv_len, m.block_table)

@@ -267,11 +267,11 @@ void flag_signal(int64_t flag, int64_t epoch, int64_t bump_epoch, int64_t ack_fl
 
 // ------------------------------------------------------------- all layers of a decode step
 static b2b::ChainDims chain_dims(int64_t hidden, int64_t ffn, int64_t n_q, int64_t n_kv, int64_t head_dim, int64_t pages, int64_t act_gelu,
-                                 bool plus_one, bool post_norms, bool layer_norm, double eps, double rope_theta, double q_scale, double softcap) {
+                                 bool plus_one, bool post_norms, bool layer_norm, bool mx, double eps, double rope_theta, double q_scale, double softcap) {
   b2b::ChainDims d;
   d.hidden = static_cast<int>(hidden); d.ffn = static_cast<int>(ffn); d.n_q = static_cast<int>(n_q); d.n_kv = static_cast<int>(n_kv);
   d.head_dim = static_cast<int>(head_dim); d.pages = static_cast<int>(pages);
-  d.act_gelu = static_cast<int>(act_gelu); d.plus_one = plus_one; d.post_norms = post_norms; d.layer_norm = layer_norm;
+  d.act_gelu = static_cast<int>(act_gelu); d.plus_one = plus_one; d.post_norms = post_norms; d.layer_norm = layer_norm; d.mx = mx;
   d.eps = static_cast<float>(eps); d.rope_theta = static_cast<float>(rope_theta); d.q_scale = static_cast<float>(q_scale);
   d.softcap = static_cast<float>(softcap);
   return d;
@@ -285,15 +285,19 @@ struct LayerChain {
   Tensor table, control;
   std::vector<Tensor> keep;
   Tensor xa, xb, q, attn, h, norm;
+  std::vector<Tensor> fp8;                 // input, stream, attention output, MLP hidden in e4m3, each with its scale factors
 
   // per layer: wqkv, wo, wgu, w_down, k_cache, v_cache and, with post norms, their two weights; LayerNorm models: the biases of the four products (fp32),
-  // weight and bias of the norm in front of the MLP and, but for the last layer, of the next layer's first norm
+  // weight and bias of the norm in front of the MLP and, but for the last layer, of the next layer's first norm; block-scaled fp8: the scale factors of the
+  // four weights, and `fp8_`: buffers of [max_tokens, ..] values and their scale factors for input, stream, attention output and MLP hidden
   LayerChain(const std::vector<std::vector<Tensor>>& ls, const std::vector<int64_t>& windows, const Tensor& xa_, const Tensor& xb_,
              const Tensor& q_, const Tensor& attn_, const Tensor& h_, const OptT& norm_, int64_t n_q, int64_t n_kv, int64_t head_dim,
-             int64_t act_gelu, bool plus_one, double eps, double rope_theta, double q_scale, double softcap, bool layer_norm)
-      : layers(static_cast<int>(ls.size())), max_tokens(static_cast<int>(xa_.size(0))), xa(xa_), xb(xb_), q(q_), attn(attn_), h(h_) {
+             int64_t act_gelu, bool plus_one, double eps, double rope_theta, double q_scale, double softcap, bool layer_norm,
+             const std::vector<Tensor>& fp8_)
+      : layers(static_cast<int>(ls.size())), max_tokens(static_cast<int>(xa_.size(0))), xa(xa_), xb(xb_), q(q_), attn(attn_), h(h_), fp8(fp8_) {
+    const bool mx = !fp8.empty();
     TORCH_CHECK(layers > 0 && windows.size() == ls.size(), "layer_chain: one window per layer");
-    const bool post = !layer_norm && ls[0].size() == 8;
+    const bool post = !layer_norm && !mx && ls[0].size() == 8;
     const int64_t H = xa.size(1), F = h.size(1), Q = n_q * head_dim, KV = n_kv * head_dim;
     if (post || layer_norm) {
       TORCH_CHECK(norm_.has_value(), "layer_chain: norms need a buffer");
@@ -306,15 +310,28 @@ struct LayerChain {
       TORCH_CHECK(t->size(0) >= max_tokens, "layer_chain: buffers of max_tokens rows");
     }
     TORCH_CHECK(xb.size(1) == H && q.size(1) == Q && attn.size(1) == Q, "layer_chain: buffer widths");
-    d = chain_dims(H, F, n_q, n_kv, head_dim, ls[0].at(4).size(0), act_gelu, plus_one, post, layer_norm, eps, rope_theta, q_scale, softcap);
+    d = chain_dims(H, F, n_q, n_kv, head_dim, ls[0].at(4).size(0), act_gelu, plus_one, post, layer_norm, mx, eps, rope_theta, q_scale, softcap);
+    TORCH_CHECK(!mx || (fp8.size() == 8 && !layer_norm), "layer_chain: eight fp8 buffers");
+    if (mx) {
+      const int64_t width[4] = {H, H, Q, F};
+      for (int i = 0; i < 4; ++i) {
+        const Tensor &v = fp8[2 * i], &sf = fp8[2 * i + 1];
+        TORCH_CHECK(v.is_cuda() && v.scalar_type() == at::kFloat8_e4m3fn && v.is_contiguous() && v.size(0) >= max_tokens && v.size(1) == width[i] &&
+                    sf.scalar_type() == at::kByte && sf.is_contiguous() && sf.numel() >= width[i] / 128 * 512, "layer_chain: fp8 buffer ", i);
+      }
+    }
     TORCH_CHECK(b2b::layer_chain_supported(d), "layer_chain: sizes not supported");
     const size_t one = b2b::layer_chain_table_bytes(1);
     Tensor host = at::empty({static_cast<int64_t>(one * layers)}, at::TensorOptions().dtype(at::kByte));
     for (int l = 0; l < layers; ++l) {
       const auto& t = ls[l];
-      TORCH_CHECK(t.size() == (layer_norm ? (l + 1 < layers ? 14u : 12u) : (post ? 8u : 6u)), "layer_chain: tensors of layer ", l);
+      TORCH_CHECK(t.size() == (layer_norm ? (l + 1 < layers ? 14u : 12u) : (mx ? 10u : (post ? 8u : 6u))), "layer_chain: tensors of layer ", l);
       for (size_t i = 0; i < t.size(); ++i)
-        if (!layer_norm || i < 6 || i >= 10) check_bf16(t[i], "layer_chain weight");
+        if (mx && (i < 4 || i >= 6)) {
+          TORCH_CHECK(t[i].is_cuda() && t[i].is_contiguous() && t[i].scalar_type() == (i < 4 ? at::kFloat8_e4m3fn : at::kByte), "layer_chain: fp8 weight ", i);
+        } else if (!layer_norm || i < 6 || i >= 10) {
+          check_bf16(t[i], "layer_chain weight");
+        }
       auto rows = [&](int i, int64_t r, int64_t c) {
         TORCH_CHECK(t[i].dim() == 2 && t[i].size(0) == r && t[i].size(1) == c && reinterpret_cast<uintptr_t>(t[i].data_ptr()) % 16 == 0,
                     "layer_chain: weight ", i, " of layer ", l);
@@ -327,7 +344,12 @@ struct LayerChain {
         TORCH_CHECK(t[i].size(0) == d.pages && t[i].numel() == static_cast<int64_t>(d.pages) * 64 * KV && reinterpret_cast<uintptr_t>(t[i].data_ptr()) % 16 == 0,
                     "layer_chain: cache of layer ", l);
       b2b::ChainLayerPtrs w{t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), t[3].data_ptr(), t[4].data_ptr(), t[5].data_ptr(), nullptr, nullptr,
-                            static_cast<int>(windows[l]), nullptr, nullptr, {nullptr, nullptr, nullptr, nullptr}};
+                            static_cast<int>(windows[l]), nullptr, nullptr, {nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
+      if (mx)
+        for (int i = 0; i < 4; ++i) {
+          TORCH_CHECK(t[6 + i].numel() >= t[i].size(0) / 128 * (t[i].size(1) / 128) * 512, "layer_chain: scale factors ", i);
+          w.sf[i] = t[6 + i].data_ptr();
+        }
       if (post) {
         TORCH_CHECK(t[6].numel() == H && t[7].numel() == H, "layer_chain: norm weights");
         w.post_attn = t[6].data_ptr();
@@ -379,6 +401,9 @@ struct LayerChain {
     c.x_in = x_in.data_ptr();
     c.xa = xa.data_ptr(); c.xb = xb.data_ptr(); c.q = q.data_ptr(); c.attn = attn.data_ptr(); c.h = h.data_ptr();
     c.norm = norm.defined() ? norm.data_ptr() : nullptr;
+    void* f8[8] = {};
+    for (size_t i = 0; i < fp8.size(); ++i) f8[i] = fp8[i].data_ptr();
+    c.q8_in = f8[0]; c.sf_in = f8[1]; c.q8_x = f8[2]; c.sf_x = f8[3]; c.q8_attn = f8[4]; c.sf_attn = f8[5]; c.q8_h = f8[6]; c.sf_h = f8[7];
     auto ip = [](const Tensor& t) { return reinterpret_cast<const int*>(t.data_ptr()); };
     c.positions = positions.has_value() ? ip(*positions) : nullptr;
     c.slots = ip(slots); c.q_start = ip(q_start); c.q_len = ip(q_len); c.kv_len = ip(kv_len); c.block_table = ip(block_table);
@@ -387,8 +412,9 @@ struct LayerChain {
 };
 
 // true if layer_chain.cu takes a piece of these sizes on the current device
-bool layer_chain_supported(int64_t hidden, int64_t ffn, int64_t n_q, int64_t n_kv, int64_t head_dim, bool post_norms, bool layer_norm) {
-  const b2b::ChainDims d = chain_dims(hidden, ffn, n_q, n_kv, head_dim, 1, 0, false, post_norms, layer_norm, 1e-5, 0.0, 1.0, 0.0);
+bool layer_chain_supported(int64_t hidden, int64_t ffn, int64_t n_q, int64_t n_kv, int64_t head_dim, bool post_norms, bool layer_norm,
+                           bool mx) {
+  const b2b::ChainDims d = chain_dims(hidden, ffn, n_q, n_kv, head_dim, 1, 0, false, post_norms, layer_norm, mx, 1e-5, 0.0, 1.0, 0.0);
   return b2b::layer_chain_supported(d) && b2b::layer_chain_init(d) > 0;
 }
 
@@ -1149,7 +1175,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   py::class_<LayerChain>(m, "LayerChain")
       .def(py::init<const std::vector<std::vector<Tensor>>&, const std::vector<int64_t>&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
-                    const Tensor&, const OptT&, int64_t, int64_t, int64_t, int64_t, bool, double, double, double, double, bool>())
+                    const Tensor&, const OptT&, int64_t, int64_t, int64_t, int64_t, bool, double, double, double, double, bool, const std::vector<Tensor>&>())
+      .def_property_readonly("step_tokens", [](const LayerChain& c) { return b2b::layer_chain_tokens(c.d); })
       .def("run", &LayerChain::run);
   m.def("layer_chain_supported", &layer_chain_supported);
   m.def("layer_chain_gave_up", &b2b::layer_chain_gave_up);

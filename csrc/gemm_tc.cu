@@ -662,21 +662,22 @@ int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t co
   return make_tmap(m, ptr, rows, cols, ld, box_rows, elt_bytes);
 }
 
-// [rows, cols] bf16 as [cols / 64 blocks][rows][64], box = [box_blocks][box_rows][64], 128B swizzle: several blocks of K in one copy
-int make_blocks_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks) {
-  using Key = std::tuple<const void*, uint64_t, uint64_t, uint32_t, uint32_t>;
+// [rows, cols] as [blocks of 128 bytes][rows][128 bytes], box = [box_blocks][box_rows][128 bytes], 128B swizzle: several blocks of K in one copy
+int make_blocks_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks, int elt_bytes) {
+  using Key = std::tuple<const void*, uint64_t, uint64_t, uint32_t, uint32_t, int>;
   static std::map<Key, CUtensorMap> cache;
   static std::mutex mu;
   std::lock_guard<std::mutex> g(mu);
-  const Key key{ptr, rows, cols, box_rows, box_blocks};
+  const Key key{ptr, rows, cols, box_rows, box_blocks, elt_bytes};
   auto it = cache.find(key);
   if (it != cache.end()) { *m = it->second; return 0; }
   PFN_encodeTiled enc = get_encode();
   if (!enc) return -1;
-  cuuint64_t dims[3] = {64, rows, cols / 64}, strides[2] = {cols * 2, 128};
-  cuuint32_t box[3] = {64, box_rows, box_blocks}, estr[3] = {1, 1, 1};
-  const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const uint32_t per = ROW_BYTES / elt_bytes;
+  cuuint64_t dims[3] = {per, rows, cols / per}, strides[2] = {cols * elt_bytes, ROW_BYTES};
+  cuuint32_t box[3] = {per, box_rows, box_blocks}, estr[3] = {1, 1, 1};
+  const CUresult r = enc(m, elt_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return static_cast<int>(r);
   if (cache.size() > 65536) cache.clear();
   cache[key] = *m;

@@ -48,7 +48,7 @@ int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, 
 // all layers of a piece for one new token per sequence (LayerNorm models: prompts too), up to 64 of them, in one persistent kernel (layer_chain.cu)
 struct ChainDims {
   int hidden, ffn, n_q, n_kv, head_dim, pages;
-  int act_gelu, plus_one, post_norms, layer_norm;
+  int act_gelu, plus_one, post_norms, layer_norm, mx;
   float eps, rope_theta, q_scale, softcap;
 };
 struct ChainLayerPtrs {
@@ -58,6 +58,7 @@ struct ChainLayerPtrs {
   int window;
   const void *post_attn_b, *post_ffn_b;  // LayerNorm models
   const float* bias[4];
+  const void* sf[4];                     // block-scaled fp8 weights: their scale factors
 };
 struct ChainCall {
   const void* table;                     // layers x layer_chain_table_bytes(1), filled by layer_chain_fill
@@ -66,8 +67,12 @@ struct ChainCall {
   const void* x_in;                      // [tokens, hidden]; may be xa
   void *xa, *xb, *q, *attn, *h, *norm;   // [max_tokens, ..] buffers; the result is in xa (LayerNorm models: norm holds the normed rows of x_in)
   const int *positions, *slots, *q_start, *q_len, *kv_len, *block_table;
+  // block-scaled fp8: the input (quantised by the caller), the stream, the attention's output and the MLP hidden, [max_tokens, ..], and their scale factors
+  const void *q8_in, *sf_in;
+  void *q8_x, *sf_x, *q8_attn, *sf_attn, *q8_h, *sf_h;
 };
 bool layer_chain_supported(const ChainDims& d);
+int layer_chain_tokens(const ChainDims& d);                        // the most tokens of a step
 size_t layer_chain_table_bytes(int layers);
 size_t layer_chain_control_words(int layers);
 int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w);

@@ -15,16 +15,21 @@
 //     are fetched while the QKV products run.  Few sequences: the CTAs of a cluster share the keys and merge through DSMEM.
 //   * LayerNorm models with 64-wide heads (GPT-2): the norms are operations of a CTA per token, attention runs on CUDA cores (a warp or a CTA per
 //     token and head), so prompts of up to 64 tokens take the same path.
+//   * block-scaled fp8: weights, and the activations that the epilogues leave beside the bf16 ones, are e4m3 with a power of two per 32 channels; the scale
+//     factors travel behind the operands' blocks and go through TMEM (tcgen05.cp) to kind::mxf8f6f4.block_scale.
 //   * the sums of squares for the next norm are left by the CTAs that write the rows, one number per CTA and token, added in a fixed order.
 //
 // Bound: the HBM stream and, between operations, the chain of last product, exchange, store, counter, poll and first activations (3 to 5 us, of
 // which the ring hides most).  Measured on B200, two Llama-3-8B layers, us (kernels one by one / here): one token behind 700 keys 188.5 / 171.5, 32
 // tokens behind 500 keys 217.0 / 193.7, 64 tokens behind 300 (Mistral-7B shapes) 257 / 219; two Gemma-2-2B layers: one token 124 / 106, 30 tokens 128 /
-// 116; all of distilgpt2, prompts of 19 / 60 tokens 267 / 209 and 333 / 254, gpt2, 64 tokens 649 / 507 (42 and 84 operations of 3 to 5 us).  Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
+// 116; all of distilgpt2, prompts of 19 / 60 tokens 267 / 209 and 333 / 254, gpt2, 64 tokens 649 / 507 (42 and 84 operations of 3 to 5 us); block-scaled
+// fp8, two Llama-3-8B layers: one token 142 / 127, 8 tokens 143 / 129, 32 tokens 166 / 162 (a conversion behind each of three products).
+// Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
 // All waits are bounded: one that runs out raises the abort word, every other wait then ends too, and the CTAs leave.
 #include "kernels.h"
 
 #include <cuda.h>
+#include <cuda_fp8.h>
 
 #include <algorithm>
 #include <cstring>
@@ -36,7 +41,7 @@
 namespace b2b {
 
 int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, int elt_bytes);
-int make_blocks_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks);
+int make_blocks_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks, int elt_bytes);
 
 namespace {
 
@@ -71,6 +76,7 @@ struct alignas(128) LcLayer {
   const __nv_bfloat16* post_attn_b;                // LayerNorm models: the norms in front of the MLP and of the next layer, and their biases
   const __nv_bfloat16* post_ffn_b;
   const float* bias[4];                            // of the products
+  const uint8_t* sf[4];                            // block-scaled fp8: scale factors of the weights
   int window;
 };
 
@@ -91,9 +97,15 @@ struct LcParams {
   int max_pages;
   uint32_t* ctl;
   float* ss;                                       // [2][clusters][64 tokens] sums of squares
+  uint8_t *q8_x, *q8_attn, *q8_h;                  // block-scaled fp8: the stream, the attention's output and the MLP hidden as the products read them
+  uint8_t *sf_x, *sf_attn, *sf_h;                  // and their scale factors
+  const uint8_t* sf_in;                            // of the piece's input
 };
 
-template <int BN>
+// what the layers are made of: RMSNorm and a gated MLP in bf16; LayerNorm, biases and no gate; the first with operands in block-scaled fp8
+enum LcKind : int { KIND_RMS = 0, KIND_LN = 1, KIND_MX = 2 };
+
+template <int BN, int KIND>
 struct LcCfg {
   static constexpr int kXBlocks = BN == 16 ? 4 : 2;                // 64-channel blocks per copy of activations
   static constexpr int kX = (BN == 16 ? 24 : (BN == 32 ? 32 : 48)) * 1024;       // three copies, four at 32 tokens (six at 8 or fewer)
@@ -102,7 +114,7 @@ struct LcCfg {
   static constexpr int kZone = BN * 512 > 16384 ? BN * 512 : 16384;   // partial sums, or Q (8 KB: two of 128 channels or one of 256) and P
   static constexpr int kSmem = 1024 + kRing + kX + kZone + 640;
   static constexpr uint32_t kS = 2 * BN, kO = 2 * BN + 2 * LC_HEADS;   // TMEM columns behind the two accumulators
-  static constexpr uint32_t kTmem = BN == 64 ? 256 : 128;
+  static constexpr uint32_t kTmem = BN == 64 || KIND == KIND_MX ? 256 : 128;
 };
 
 __device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
@@ -227,30 +239,62 @@ __device__ __forceinline__ void lc_st_heads(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// block-scaled copy of a value per lane, 32 consecutive features of a token: e4m3 and the power of two that brings the largest (`most`) to at most 448, in
+// the layout of the product that reads it
+__device__ __forceinline__ void lc_store_mx(float r, float most, int tok, int feat, int ld, uint8_t* to, uint8_t* sf, int lane) {
+  const uint32_t b = __float_as_uint(most * (1.f / 448.f));
+  const int e = max(-126, min(127, static_cast<int>(b >> 23) - 127 + ((b & 0x7FFFFFu) ? 1 : 0)));
+  to[static_cast<size_t>(tok) * ld + feat] =
+      static_cast<uint8_t>(__nv_cvt_float_to_fp8(r * __uint_as_float(static_cast<uint32_t>(127 - e) << 23), __NV_SATFINITE, __NV_E4M3));
+  if (lane == 0) sf[static_cast<size_t>(feat >> 7) * 512 + (tok & 31) * 16 + (tok >> 5) * 4 + ((feat >> 5) & 3)] = static_cast<uint8_t>(e + 127);
+}
+// the same for tokens tok0 .. tok0 + N, `n` of them wanted, of the values as bf16 (like a separate quantiser): the N chains of shuffles run side by side
+template <int N>
+__device__ __forceinline__ void lc_put_mx(const float (&v)[N], int n, int tok0, int feat, int ld, uint8_t* to, uint8_t* sf, int lane) {
+  float r[N], most[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    r[i] = bf16_round(v[i]);
+    most[i] = fabsf(r[i]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < N; ++i) most[i] = fmaxf(most[i], __shfl_xor_sync(0xffffffffu, most[i], o));
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < n) {
+      lc_store_mx(r[i], most[i], tok0 + i, feat, ld, to, sf, lane);
+    }
+}
+
 // share of a product: units [u0, end) of the weights' rows, 64-channel blocks [kb0, kb0 + nkb) of K.  A unit is 8 rows (gate/up: 8 features).
 // Shares are cut at multiples of 32 rows (gate/up: 64 or 32 features) where that makes the largest share no more than 4 % larger: a tile then takes
 // one or two boxes per block of K.  With shares of single units gate/up needs up to 16, whose issue bound it at 2.3 TB/s.
 struct LcShare {
   int u0, end, kb0, nkb;
 };
-template <bool GLU>
+template <bool GLU, bool MX>
 __device__ LcShare lc_share(const LcParams& p, int op, int head_dim) {
   LcShare s;
   const int c = blockIdx.x / LC_CL, nc = gridDim.x / LC_CL, r = blockIdx.x % LC_CL;
   const int rows = op == OP_QKV ? (p.n_q + 2 * p.n_kv) * head_dim : p.hidden;
-  const int nk = (op == OP_DOWN ? p.ffn : (op == OP_O ? p.n_q * head_dim : p.hidden)) / 64;
+  const int nk = (op == OP_DOWN ? p.ffn : (op == OP_O ? p.n_q * head_dim : p.hidden)) / (MX ? 128 : 64);
   const int u = (op == OP_GU ? p.ffn : rows) / 8, most = (u + nc - 1) / nc;
-  int g = GLU && op == OP_GU ? 8 : 4;
-  while (g > 1 && (u % g != 0 || (u / g + nc - 1) / nc * g * 25 > most * 26)) g /= 2;
+  int g = GLU && op == OP_GU ? 8 : (MX ? 16 : 4);
+  while (g > (MX ? (GLU && op == OP_GU ? 8 : 4) : 1) && (u % g != 0 || (u / g + nc - 1) / nc * g * 25 > most * 26)) g /= 2;
   s.u0 = u / g * c / nc * g;
   s.end = u / g * (c + 1) / nc * g;
   s.kb0 = nk * r / LC_CL;
   s.nkb = nk * (r + 1) / LC_CL - s.kb0;
   return s;
 }
-// units of the tile that starts at u: up to 128 rows, gate/up tiles do not cross the 64-feature blocks of their rows
-template <bool GLU>
-__device__ __forceinline__ int lc_tile(int op, int u, int end) { return min(GLU && op == OP_GU ? 8 - (u & 7) : 16, end - u); }
+// units of the tile that starts at u: up to 128 rows, gate/up tiles do not cross the 64-feature blocks of their rows.  Scale factors come in runs of 128
+// rows, a column of TMEM for 32 of them: block-scaled tiles do not cross the runs, and have their rows where the run has them (lc_first)
+template <bool GLU, bool MX>
+__device__ __forceinline__ int lc_tile(int op, int u, int end) { return min(GLU && op == OP_GU ? 8 - (u & 7) : (MX ? 16 - (u & 15) : 16), end - u); }
+template <bool GLU, bool MX>
+__device__ __forceinline__ int lc_first(int op, int u) { return MX && !(GLU && op == OP_GU) ? u & 15 : 0; }
 template <bool GLU>
 __device__ __forceinline__ int lc_rows(int op, int n) { return GLU && op == OP_GU ? n * 16 : n * 8; }
 
@@ -314,11 +358,12 @@ __device__ __forceinline__ LcItem lc_item(const LcParams& p, const int* kvlen_s,
   return it;
 }
 
-// D: channels of a head, GP: query heads of a key/value head rounded up to 4 or 8.  LN: LayerNorm models with biases, an MLP without a gate and 64-wide
-// heads (the norms are operations in front of the products; prompts too)
-template <int BN, int D, int GP, bool LN>
+// D: channels of a head, GP: query heads of a key/value head rounded up to 4 or 8.  KIND_LN: 64-wide heads, the norms are operations in
+// front of the products; prompts too
+template <int BN, int D, int GP, int KIND>
 __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid_constant__ LcMaps maps, const LcParams p) {
-  using Cfg = LcCfg<BN>;
+  using Cfg = LcCfg<BN, KIND>;
+  constexpr bool LN = KIND == KIND_LN, MX = KIND == KIND_MX;
   constexpr bool GLU = !LN;
   const int hd = LN ? p.head_dim : D;               // channels of a head
   constexpr int XB = Cfg::kXBlocks, CW = Cfg::kCols, DB = D / 64, MB = D / 128, NQ = 2 / MB;
@@ -383,7 +428,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   }
   if (warp == 2)
     for (int op = lane; op < OP_COUNT; op += 32)
-      if (lc_weight(op) >= 0) share_s[lc_weight(op)] = lc_share<GLU>(p, op, hd);
+      if (lc_weight(op) >= 0) share_s[lc_weight(op)] = lc_share<GLU, MX>(p, op, hd);
   if constexpr (LN) {                              // per token: its sequence (-1: none) and the keys that it sees
     for (int t = threadIdx.x; t < p.T; t += LC_THREADS) {
       int seq = -1, keys = 0;
@@ -415,7 +460,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   uint32_t* const ctr = p.ctl + LW_CTR;
   const int item0 = blockIdx.x / p.parts, part = blockIdx.x % p.parts, item_step = gridDim.x / p.parts, items = p.seqs * p.n_kv;
   const uint32_t x_bytes = static_cast<uint32_t>(p.x_rows) * 128u;     // activations per block of K
-  const uint32_t x_slots = Cfg::kX / (x_bytes * XB);
+  const uint32_t x_slot = x_bytes * XB + (MX ? XB * 512u : 0u), x_slots = min(static_cast<uint32_t>(LC_XSLOTS), Cfg::kX / x_slot);
   auto skip = [&](int l, int op) {                 // (LayerNorm models: the norm in front of the next layer)
     return LN ? (op == OP_NORM_F && l == p.n_layers - 1) : (!norms && (op == OP_NORM_A || op == OP_NORM_F));
   };
@@ -449,18 +494,19 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           if (lc_weight(op) >= 0) {
             const LcShare sh = share_s[lc_weight(op)];
             const CUtensorMap* maps_w = L->w[lc_weight(op)];
+            const int k_blocks = (op == OP_DOWN ? p.ffn : (op == OP_O ? p.n_q * hd : p.hidden)) / 128;           // (MX)
 #pragma unroll 1
             for (int u = sh.u0, n; ok && u < sh.end; u += n) {
-              n = lc_tile<GLU>(op, u, sh.end);
+              n = lc_tile<GLU, MX>(op, u, sh.end);
               // up to five boxes per block: rows of gate/up come in blocks of [64 gate | 64 up]: gate to rows 0.., up to rows 64.. of the tile
               const bool halves = GLU && op == OP_GU && n < 8;
-              const int units = (GLU && op == OP_GU && !halves) ? 16 : n;
+              const int units = (GLU && op == OP_GU && !halves) ? 16 : n, first = lc_first<GLU, MX>(op, u);
               const int row0 = GLU && op == OP_GU ? (u >> 3) * 128 + (u & 7) * 8 : u * 8;
-              const uint32_t bytes = static_cast<uint32_t>(lc_rows<GLU>(op, n)) * 128u, block = lc_block_bytes<GLU>(op, n);
+              const uint32_t bytes = static_cast<uint32_t>(lc_rows<GLU>(op, n)) * 128u, block = lc_block_bytes<GLU>(op, first + n);
 #pragma unroll 1
               for (int kb = 0; kb < sh.nkb; kb += 2) {
                 const int nb = min(2, sh.nkb - kb);
-                if (!(ok = ring.room(block * nb, place, sizes, empty, abort))) break;
+                if (!(ok = ring.room(block * nb + (MX ? 1024u : 0u), place, sizes, empty, abort))) break;
                 uint8_t* base = smem + place;
                 uint64_t* bar = &full[ring.entry()];
                 ++ring.count;
@@ -468,9 +514,12 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                   mbar_arrive(bar);
                   continue;
                 }
-                mbar_arrive_expect_tx(bar, bytes);
-                const int k = (sh.kb0 + kb + half) * 64;
-                uint8_t* dst = base + half * block;
+                mbar_arrive_expect_tx(bar, bytes + (MX && half == 0 ? nb * 512u : 0u));
+                const int k = (sh.kb0 + kb + half) * (MX ? 128 : 64);
+                if constexpr (MX)
+                  if (half == 0)                     // scale factors of both blocks, behind them
+                    bulk_load(base + nb * block, L->sf[lc_weight(op)] + (static_cast<size_t>(row0 >> 7) * k_blocks + sh.kb0 + kb) * 512, nb * 512u, bar);
+                uint8_t* dst = base + half * block + first * 1024;
                 if (units == 16) {
                   tma_load_2d_hint(dst, maps_w + 4, bar, k, row0, pol);
                   continue;
@@ -553,12 +602,16 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             const LcShare sh = share_s[lc_weight(op)];
             const CUtensorMap* m = op == OP_QKV ? (l == 0 ? &maps.x_in : &maps.xa) : (op == OP_O ? &maps.attn : (op == OP_GU ? &maps.xb : &maps.h));
 #pragma unroll 1
-            for (int u = sh.u0; ok && u < sh.end; u += lc_tile<GLU>(op, u, sh.end))
+            for (int u = sh.u0; ok && u < sh.end; u += lc_tile<GLU, MX>(op, u, sh.end))
 #pragma unroll 1
               for (int kb = 0; kb < sh.nkb; kb += XB) {      // (whole copies, also where fewer blocks are left: they are not used)
                 if (!(ok = ma_wait(&x_empty[s], ph ^ 1u, abort))) break;
-                mbar_arrive_expect_tx(&x_full[s], x_bytes * XB);
-                tma_load_3d_hint(x_s + s * x_bytes * XB, m, &x_full[s], 0, 0, sh.kb0 + kb, pol);
+                const uint32_t sf_bytes = MX ? min(XB, sh.nkb - kb) * 512u : 0u;
+                mbar_arrive_expect_tx(&x_full[s], x_bytes * XB + sf_bytes);
+                tma_load_3d_hint(x_s + s * x_slot, m, &x_full[s], 0, 0, sh.kb0 + kb, pol);
+                if constexpr (MX)
+                  bulk_load(x_s + s * x_slot + x_bytes * XB, (op == OP_QKV ? (l == 0 ? p.sf_in : p.sf_x) : op == OP_O ? p.sf_attn : op == OP_GU ? p.sf_x : p.sf_h) +
+                            static_cast<size_t>(sh.kb0 + kb) * 512, sf_bytes, &x_full[s]);
                 if (++s == x_slots) { s = 0; ph ^= 1u; }
               }
           } else if (!LN && op == OP_ATT) {
@@ -581,12 +634,13 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   } else if (warp == 1) {
     // -------------------------------------------------------------------------------------------------------- MMA issuer
     if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(128, BN);
+      constexpr uint32_t idesc = MX ? make_idesc_mxf8(128, BN) : make_idesc_bf16(128, BN);
       constexpr uint32_t idesc_s = make_idesc_bf16(LC_KEYS, LC_HEADS);
       constexpr uint32_t idesc_o = make_idesc_bf16(128, LC_HEADS) | (1u << 15);              // A (V) has its rows contiguous
       const uint64_t desc0 = make_sw128_kmajor_desc(smem_u32(smem));         // + offset / 16 (a single thread issues: every instruction counts)
       const uint64_t desc_x = make_sw128_kmajor_desc(smem_u32(x_s));
-      const uint32_t x_chunk = x_bytes * XB >> 4;
+      const uint32_t x_chunk = x_slot >> 4;
+      uint32_t nblk = 0;                             // blocks of K so far (their scale factors alternate between two sets of columns)
       uint32_t xs = 0, xph = 0;
       LcRing<Cfg::kRing> ring;
       uint32_t na = 0, ns = 0, np = 0, nq = 0, no = 0;       // accumulators, score tiles, value tiles, items so far
@@ -600,8 +654,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             const LcShare sh = share_s[lc_weight(op)];
 #pragma unroll 1
             for (int u = sh.u0, n; ok && u < sh.end; u += n, ++na) {
-              n = lc_tile<GLU>(op, u, sh.end);
-              const uint32_t block = lc_block_bytes<GLU>(op, n);
+              n = lc_tile<GLU, MX>(op, u, sh.end);
+              const uint32_t block = lc_block_bytes<GLU>(op, lc_first<GLU, MX>(op, u) + n);
               if (!(ok = ma_wait(&acc_empty[na & 1u], ((na >> 1) & 1u) ^ 1u, abort))) break;
               tc_fence_after();
               const uint32_t acc = tmem + (na & 1u) * BN;
@@ -614,21 +668,39 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                 for (int k2 = kb; k2 < min(kb + XB, sh.nkb); k2 += 2) {
                   const uint32_t nb = min(2, sh.nkb - k2);
                   // (rows that the tile does not have are read from what lies behind it, and not used)
-                  uint64_t a = desc0 + (ring.place(block * nb) >> 4);
+                  const uint32_t at_w = ring.place(block * nb + (MX ? 1024u : 0u));
+                  uint64_t a = desc0 + (at_w >> 4);
                   if (!(ok = ma_wait(&full[ring.entry()], ring.parity(), abort))) break;
                   tc_fence_after();
-                  umma_bf16(acc, a, x, idesc, more);
-                  umma_bf16(acc, a + 2, x + 2, idesc, 1u);
-                  umma_bf16(acc, a + 4, x + 4, idesc, 1u);
-                  umma_bf16(acc, a + 6, x + 6, idesc, 1u);
-                  if (nb == 2) {
-                    a += block >> 4;
-                    x += x_bytes >> 4;
-                    umma_bf16(acc, a, x, idesc, 1u);
+                  if constexpr (MX) {
+                    // (scale factors: two sets of 16 columns behind the attention's)
+                    const uint32_t sfa = smem_u32(smem) + at_w + nb * block, sfb = smem_u32(x_s) + xs * x_slot + x_bytes * XB + (k2 - kb) * 512;
+#pragma unroll 1
+                    for (uint32_t b = 0; b < nb; ++b, ++nblk) {
+                      const uint32_t ta = tmem + Cfg::kO + 2 * LC_HEADS + (nblk & 1u) * 16, tb = ta + 4;
+                      tmem_cp_32x128b_warpx4(ta, make_sf_desc(sfa + b * 512));
+                      tmem_cp_32x128b_warpx4(tb, make_sf_desc(sfb + b * 512));
+#pragma unroll
+                      for (int k = 0; k < 4; ++k)
+                        umma_mxf8(acc, a + 2 * k, x + 2 * k, idesc | (static_cast<uint32_t>(k) << 4) | (static_cast<uint32_t>(k) << 29),
+                                  (more != 0u || b > 0 || k > 0) ? 1u : 0u, ta, tb);
+                      a += block >> 4;
+                      x += x_bytes >> 4;
+                    }
+                  } else {
+                    umma_bf16(acc, a, x, idesc, more);
                     umma_bf16(acc, a + 2, x + 2, idesc, 1u);
                     umma_bf16(acc, a + 4, x + 4, idesc, 1u);
                     umma_bf16(acc, a + 6, x + 6, idesc, 1u);
-                    x += x_bytes >> 4;
+                    if (nb == 2) {
+                      a += block >> 4;
+                      x += x_bytes >> 4;
+                      umma_bf16(acc, a, x, idesc, 1u);
+                      umma_bf16(acc, a + 2, x + 2, idesc, 1u);
+                      umma_bf16(acc, a + 4, x + 4, idesc, 1u);
+                      umma_bf16(acc, a + 6, x + 6, idesc, 1u);
+                      x += x_bytes >> 4;
+                    }
                   }
                   umma_commit(&empty[ring.entry()]);
                   ++ring.count;
@@ -778,9 +850,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           lc_sync();
 #pragma unroll 1
           for (int u = sh.u0, n; u < sh.end; u += n) {
-            n = lc_tile<GLU>(op, u, sh.end);
-            const int feat = u * 8 + row;
-            const bool live = GLU && op == OP_GU ? (row & 63) < n * 8 : row < n * 8;
+            n = lc_tile<GLU, MX>(op, u, sh.end);
+            const int own = row - lc_first<GLU, MX>(op, u) * 8, feat = u * 8 + own;
+            const bool live = GLU && op == OP_GU ? (row & 63) < n * 8 : (own >= 0 && own < n * 8);
             const float bias_v = LN && live ? bias[feat] : 0.f;
             const int sect = feat < q_dim ? 0 : (feat < q_dim + kv_dim ? 1 : 2);                  // (of QKV)
             const int fs = feat - (sect == 0 ? 0 : (sect == 1 ? q_dim : q_dim + kv_dim));
@@ -851,12 +923,19 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             if (lane < LC_CL) arrive_cluster(mapa_smem(smem_u32(zone_free), lane));               // the sums have been read
             if (GLU && op == OP_GU) {
               const int t0 = up ? HB : 0;
+              float h[HB];
 #pragma unroll
               for (int i = 0; i < HB; ++i) {
-                if (col0 + t0 + i >= p.T || !live || !ok) break;
                 const float rs = rstd_s[t0 + i], theirs = c1[i] * rs, mine = (up ? v[HB + i] : v[i]) * rs;
                 const float g = up ? theirs : mine, w = up ? mine : theirs;
-                p.h[static_cast<size_t>(col0 + t0 + i) * p.ffn + u * 8 + (row & 63)] = __float2bfloat16_rn((p.act ? gelu_tanh(g) : silu(g)) * w);
+                h[i] = (p.act ? gelu_tanh(g) : silu(g)) * w;
+              }
+              if constexpr (MX) {                      // (whole blocks of 64 features: every lane has one)
+                lc_put_mx<HB>(h, ok ? p.T - col0 - t0 : 0, col0 + t0, u * 8 + (row & 63), p.ffn, p.q8_h, p.sf_h, lane);
+              } else if (live && ok) {
+#pragma unroll
+                for (int i = 0; i < HB; ++i)
+                  if (col0 + t0 + i < p.T) p.h[static_cast<size_t>(col0 + t0 + i) * p.ffn + u * 8 + (row & 63)] = __float2bfloat16_rn(h[i]);
               }
             } else if (op == OP_QKV) {
 #pragma unroll
@@ -874,19 +953,24 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                   (sect == 1 ? k_cache : v_cache)[static_cast<size_t>(slot_s[i]) * kv_dim + fs] = __float2bfloat16_rn(o);
                 }
               }
-            } else if (live && ok) {
+            } else {
 #pragma unroll
               for (int i = 0; i < CW; ++i) {
-                if (col0 + i >= p.T) break;
-                float a = v[i] + c1[i];
+                v[i] += c1[i];
                 if constexpr (LN) {
-                  a += bias_v;
-                  if (op == OP_GU) a = gelu_tanh(a);
+                  v[i] += bias_v;
+                  if (op == OP_GU) v[i] = gelu_tanh(v[i]);
                 }
-                const __nv_bfloat16 r = __float2bfloat16_rn(a);
-                out[static_cast<size_t>(col0 + i) * ld + feat] = r;
-                sq[i] += __bfloat162float(r) * __bfloat162float(r);
               }
+              if (live && ok)
+#pragma unroll
+                for (int i = 0; i < CW; ++i)
+                  if (col0 + i < p.T) {
+                    const __nv_bfloat16 r = __float2bfloat16_rn(v[i]);
+                    out[static_cast<size_t>(col0 + i) * ld + feat] = r;
+                    sq[i] += __bfloat162float(r) * __bfloat162float(r);
+                  }
+              if constexpr (MX) lc_put_mx<CW>(v, live && ok ? p.T - col0 : 0, col0, feat, p.hidden, p.q8_x, p.sf_x, lane);
             }
           }
           if (!LN && !norms && (op == OP_O || op == OP_DOWN)) {
@@ -1099,13 +1183,35 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
             __nv_bfloat16* out = p.attn + static_cast<size_t>(q_start_s[it.seq]) * q_dim + it.kvh * G * D;
             if (p.parts == 1) {
               lc_sync();
+              float den[GP];
 #pragma unroll
-              for (int g = 0; g < GP; ++g)
-                if (g < G && ok) {
-                  const float den = sq_s[0][g] + sq_s[1][g] + sq_s[2][g] + sq_s[3][g];
+              for (int g = 0; g < GP; ++g) den[g] = g < G ? sq_s[0][g] + sq_s[1][g] + sq_s[2][g] + sq_s[3][g] : 0.f;
 #pragma unroll
-                  for (int m = 0; m < MB; ++m) out[g * D + m * 128 + row] = __float2bfloat16_rn(den == 0.f ? 0.f : o[m][g] / den);
+              for (int m = 0; m < MB; ++m) {
+#pragma unroll
+                for (int g = 0; g < GP; ++g) o[m][g] = den[g] == 0.f ? 0.f : o[m][g] / den[g];
+                if constexpr (MX) {                    // (G heads side by side: "rows" of D features)
+                  float r[GP], most[GP];
+#pragma unroll
+                  for (int g = 0; g < GP; ++g) {
+                    r[g] = bf16_round(o[m][g]);
+                    most[g] = fabsf(r[g]);
+                  }
+#pragma unroll
+                  for (int sh = 16; sh > 0; sh >>= 1)
+#pragma unroll
+                    for (int g = 0; g < GP; ++g) most[g] = fmaxf(most[g], __shfl_xor_sync(0xffffffffu, most[g], sh));
+#pragma unroll
+                  for (int g = 0; g < GP; ++g)
+                    if (g < G && ok) {
+                      lc_store_mx(r[g], most[g], q_start_s[it.seq], it.kvh * G * D + g * D + m * 128 + row, q_dim, p.q8_attn, p.sf_attn, lane);
+                    }
+                } else {
+#pragma unroll
+                  for (int g = 0; g < GP; ++g)
+                    if (g < G && ok) out[g * D + m * 128 + row] = __float2bfloat16_rn(o[m][g]);
                 }
+              }
             } else {
               float* part_s = reinterpret_cast<float*>(zone + 8192);       // [G][D], over the weights of tiles that have been used
 #pragma unroll
@@ -1145,7 +1251,13 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                     num += w * nr[r];
                   }
                 }
-                if (ok) out[e] = __float2bfloat16_rn(den == 0.f ? 0.f : num / den);
+                const float v = den == 0.f ? 0.f : num / den;
+                if (!ok) continue;
+                if constexpr (MX) {
+                  const float one[1] = {v};
+                  lc_put_mx<1>(one, 1, q_start_s[it.seq], it.kvh * G * D + e, q_dim, p.q8_attn, p.sf_attn, lane);
+                }
+                else out[e] = __float2bfloat16_rn(v);
               }
             }
             lc_sync();                                 // the sums of the rows have been read
@@ -1327,7 +1439,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
 }
 
 // clusters of four that fit the device at once with this kernel, 0 if it cannot run
-template <int BN, int D, int GP, bool LN>
+template <int BN, int D, int GP, int KIND>
 int chain_clusters() {
   static int known[64] = {};
   int dev = 0;
@@ -1335,34 +1447,34 @@ int chain_clusters() {
   if (dev < 64 && known[dev] != 0) return known[dev] - 1;
   int n = 0, coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  if (coop && cudaFuncSetAttribute(layer_chain_kernel<BN, D, GP, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcCfg<BN>::kSmem) == cudaSuccess) {
+  if (coop && cudaFuncSetAttribute(layer_chain_kernel<BN, D, GP, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, LcCfg<BN, KIND>::kSmem) == cudaSuccess) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(LC_CL * 64);
     cfg.blockDim = dim3(LC_THREADS);
-    cfg.dynamicSmemBytes = LcCfg<BN>::kSmem;
+    cfg.dynamicSmemBytes = LcCfg<BN, KIND>::kSmem;
     cudaLaunchAttribute a[1];
     a[0].id = cudaLaunchAttributeClusterDimension;
     a[0].val.clusterDim.x = LC_CL;
     a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
     cfg.attrs = a;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, layer_chain_kernel<BN, D, GP, LN>, &cfg) != cudaSuccess) n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, layer_chain_kernel<BN, D, GP, KIND>, &cfg) != cudaSuccess) n = 0;
   }
   cudaGetLastError();
   if (dev < 64) known[dev] = n + 1;
   return n;
 }
 
-template <int BN, int D, int GP, bool LN>
+template <int BN, int D, int GP, int KIND>
 int launch_chain_one(const LcMaps& maps, LcParams p, cudaStream_t s) {
-  const int clusters = std::min(chain_clusters<BN, D, GP, LN>(), 64);
+  const int clusters = std::min(chain_clusters<BN, D, GP, KIND>(), 64);
   if (clusters <= 0) return -5;
   const int ctas = clusters * LC_CL, items = p.seqs * p.n_kv;
   p.parts = items * 4 <= ctas ? 4 : (items * 2 <= ctas ? 2 : 1);     // few sequences: CTAs of a cluster share the keys of one
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas));
   cfg.blockDim = dim3(LC_THREADS);
-  cfg.dynamicSmemBytes = LcCfg<BN>::kSmem;
+  cfg.dynamicSmemBytes = LcCfg<BN, KIND>::kSmem;
   cfg.stream = s;
   cudaLaunchAttribute a[2];
   a[0].id = cudaLaunchAttributeClusterDimension;
@@ -1372,13 +1484,15 @@ int launch_chain_one(const LcMaps& maps, LcParams p, cudaStream_t s) {
   a[1].val.cooperative = 1;
   cfg.attrs = a;
   cfg.numAttrs = 2;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, layer_chain_kernel<BN, D, GP, LN>, maps, p));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, layer_chain_kernel<BN, D, GP, KIND>, maps, p));
 }
 
-#define B2B_CHAIN(FN, BN, ...) \
-  (d.layer_norm ? FN<BN, 128, 4, true>(__VA_ARGS__) : \
-   d.head_dim == 128 ? (g <= 4 ? FN<BN, 128, 4, false>(__VA_ARGS__) : FN<BN, 128, 8, false>(__VA_ARGS__)) \
-                     : (g <= 4 ? FN<BN, 256, 4, false>(__VA_ARGS__) : FN<BN, 256, 8, false>(__VA_ARGS__)))
+#define B2B_CHAIN64(FN, ...) B2B_CHAIN_OF(FN, 64, KIND_RMS, __VA_ARGS__)
+#define B2B_CHAIN_OF(FN, BN, KIND, ...) \
+  (d.layer_norm ? FN<BN, 128, 4, KIND_LN>(__VA_ARGS__) : \
+   d.head_dim == 128 ? (g <= 4 ? FN<BN, 128, 4, KIND>(__VA_ARGS__) : FN<BN, 128, 8, KIND>(__VA_ARGS__)) \
+                     : (g <= 4 ? FN<BN, 256, 4, KIND>(__VA_ARGS__) : FN<BN, 256, 8, KIND>(__VA_ARGS__)))
+#define B2B_CHAIN(FN, BN, ...) (d.mx ? B2B_CHAIN_OF(FN, BN, KIND_MX, __VA_ARGS__) : B2B_CHAIN_OF(FN, BN, KIND_RMS, __VA_ARGS__))
 
 }  // namespace
 
@@ -1390,6 +1504,7 @@ bool layer_chain_supported(const ChainDims& d) {
   if (d.n_kv <= 0 || d.n_q % d.n_kv != 0 || d.hidden % 128 != 0 || d.hidden < 256 || d.ffn % 64 != 0 || d.ffn < 256 || d.n_q * d.head_dim < 256)
     return false;
   if (d.layer_norm) return d.head_dim == 64 && (d.n_q * 64) % 128 == 0 && (d.n_kv * 64) % 128 == 0 && d.ffn % 128 == 0 && d.hidden <= 4096;
+  if (d.mx && (d.post_norms || d.ffn % 128 != 0 || d.hidden < 512 || d.ffn < 512 || d.n_q * d.head_dim < 512)) return false;
   return g <= 8 && (d.head_dim == 128 || d.head_dim == 256) && g * d.head_dim * 4 <= 8192 && (!d.post_norms || d.hidden <= 4096);
 }
 
@@ -1403,7 +1518,7 @@ int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w) {
   const uint64_t cols[4] = {static_cast<uint64_t>(d.hidden), static_cast<uint64_t>(q_dim), static_cast<uint64_t>(d.hidden), static_cast<uint64_t>(d.ffn)};
   for (int i = 0; i < 4; ++i)
     for (int b = 0; b < 5; ++b)
-      if (const int r = make_tmap_shared(&L.w[i][b], ptr[i], rows[i], cols[i], cols[i], 8u << b, 2)) return r;
+      if (const int r = make_tmap_shared(&L.w[i][b], ptr[i], rows[i], cols[i], cols[i], 8u << b, d.mx ? 1 : 2)) return r;
   const uint64_t keys = static_cast<uint64_t>(d.pages) * LC_PAGE;
   if (const int r = make_tmap_shared(&L.k, w.k_cache, keys, kv_dim, kv_dim, LC_PAGE, 2)) return r;
   if (const int r = make_tmap_shared(&L.v, w.v_cache, keys, kv_dim, kv_dim, LC_PAGE, 2)) return r;
@@ -1413,7 +1528,10 @@ int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w) {
   L.post_ffn = static_cast<const __nv_bfloat16*>(w.post_ffn);
   L.post_attn_b = static_cast<const __nv_bfloat16*>(w.post_attn_b);
   L.post_ffn_b = static_cast<const __nv_bfloat16*>(w.post_ffn_b);
-  for (int i = 0; i < 4; ++i) L.bias[i] = w.bias[i];
+  for (int i = 0; i < 4; ++i) {
+    L.bias[i] = w.bias[i];
+    L.sf[i] = static_cast<const uint8_t*>(w.sf[i]);
+  }
   L.window = w.window;
   std::memcpy(dst, &L, sizeof(L));
   return 0;
@@ -1421,16 +1539,24 @@ int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w) {
 
 int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
   const int g = d.n_kv > 0 ? d.n_q / d.n_kv : 0;
-  if (!layer_chain_supported(d) || c.tokens < 1 || c.tokens > 64 || c.layers < 1 || (!d.layer_norm && c.seqs > c.tokens)) return -2;
+  if (!layer_chain_supported(d) || c.tokens < 1 || c.tokens > layer_chain_tokens(d) || c.layers < 1 || (!d.layer_norm && c.seqs > c.tokens)) return -2;
   const int bn = c.tokens <= 16 ? 16 : (c.tokens <= 32 ? 32 : 64), x_rows = c.tokens <= 8 ? 8 : bn, q_dim = d.n_q * d.head_dim;
   LcMaps m;
-  auto act = [&](CUtensorMap* t, const void* ptr, uint64_t rows, int cols) { return make_blocks_tmap(t, ptr, rows, cols, x_rows, bn == 16 ? LcCfg<16>::kXBlocks : LcCfg<32>::kXBlocks); };
+  auto act = [&](CUtensorMap* t, const void* ptr, uint64_t rows, int cols) {
+    return make_blocks_tmap(t, ptr, rows, cols, x_rows, bn == 16 ? LcCfg<16, KIND_RMS>::kXBlocks : LcCfg<32, KIND_RMS>::kXBlocks, d.mx ? 1 : 2);
+  };
   int r;
-  // (LayerNorm models: the products read the normed rows)
-  const void *x_in = d.layer_norm ? c.norm : c.x_in, *xa = d.layer_norm ? c.norm : c.xa, *xb = d.layer_norm ? c.norm : c.xb;
-  if ((r = act(&m.x_in, x_in, d.layer_norm ? c.max_tokens : c.tokens, d.hidden)) || (r = act(&m.xa, xa, c.max_tokens, d.hidden)) ||
-      (r = act(&m.xb, xb, c.max_tokens, d.hidden)) ||
-      (r = act(&m.attn, c.attn, c.max_tokens, q_dim)) || (r = act(&m.h, c.h, c.max_tokens, d.ffn)) ||
+  // what the products read: LayerNorm models the normed rows, fp8 ones the copies in fp8
+  const void *x_in = c.x_in, *xa = c.xa, *xb = c.xb, *attn = c.attn, *h = c.h;
+  if (d.layer_norm) x_in = xa = xb = c.norm;
+  if (d.mx) {
+    x_in = c.q8_in;
+    xa = xb = c.q8_x;
+    attn = c.q8_attn;
+    h = c.q8_h;
+  }
+  if ((r = act(&m.x_in, x_in, x_in == c.x_in ? c.tokens : c.max_tokens, d.hidden)) || (r = act(&m.xa, xa, c.max_tokens, d.hidden)) ||
+      (r = act(&m.xb, xb, c.max_tokens, d.hidden)) || (r = act(&m.attn, attn, c.max_tokens, q_dim)) || (r = act(&m.h, h, c.max_tokens, d.ffn)) ||
       (r = make_tmap_shared(&m.q, c.q, static_cast<uint64_t>(c.max_tokens) * d.n_q, d.head_dim, d.head_dim, LC_HEADS, 2)))
     return r;
   LcParams p;
@@ -1444,19 +1570,27 @@ int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
   p.attn = static_cast<__nv_bfloat16*>(c.attn); p.h = static_cast<__nv_bfloat16*>(c.h); p.norm = static_cast<__nv_bfloat16*>(c.norm);
   p.positions = c.positions; p.slots = c.slots; p.q_start = c.q_start; p.q_len = c.q_len; p.kv_len = c.kv_len; p.block_table = c.block_table;
   p.max_pages = c.max_pages;
+  p.q8_x = static_cast<uint8_t*>(c.q8_x); p.q8_attn = static_cast<uint8_t*>(c.q8_attn); p.q8_h = static_cast<uint8_t*>(c.q8_h);
+  p.sf_x = static_cast<uint8_t*>(c.sf_x); p.sf_attn = static_cast<uint8_t*>(c.sf_attn); p.sf_h = static_cast<uint8_t*>(c.sf_h);
+  p.sf_in = static_cast<const uint8_t*>(c.sf_in);
   p.ctl = c.control;
   p.ss = reinterpret_cast<float*>(c.control + layer_chain_control_words(c.layers)) - 2 * LC_SS;
   if (bn == 16) return B2B_CHAIN(launch_chain_one, 16, m, p, s);
   if (bn == 32) return B2B_CHAIN(launch_chain_one, 32, m, p, s);
-  return B2B_CHAIN(launch_chain_one, 64, m, p, s);
+  return B2B_CHAIN64(launch_chain_one, m, p, s);
 }
+
+// Block-scaled fp8 steps of 33 tokens and more stay with the kernels one by one: half the bytes of bf16, and the conversions of 64 tokens' results, put
+// them behind (two layers of Zephyr-7B, 40 tokens: 193.5 us one by one, 195.0 here; 64 tokens: 194.0 and 196.0).
+int layer_chain_tokens(const ChainDims& d) { return d.mx ? 32 : 64; }
 
 // clusters that are resident at once (0: the kernel cannot run here); also sets the kernels' shared memory sizes, so that a first launch may
 // happen under graph capture
 int layer_chain_init(const ChainDims& d) {
   const int g = d.n_kv > 0 ? d.n_q / d.n_kv : 0;
   if (!layer_chain_supported(d)) return 0;
-  return std::min(B2B_CHAIN(chain_clusters, 16), std::min(B2B_CHAIN(chain_clusters, 32), B2B_CHAIN(chain_clusters, 64)));
+  const int n = std::min(B2B_CHAIN(chain_clusters, 16), B2B_CHAIN(chain_clusters, 32));
+  return d.mx ? n : std::min(n, B2B_CHAIN64(chain_clusters));
 }
 
 int set_wait_policy_chain(uint32_t* abort_word, unsigned long long limit_ns) {

@@ -57,3 +57,30 @@ def test_spans(H, G, D, news, ctxs, window, keep, cap, sink):
             assert float((out[at:at + n].double() - ref).norm() / ref.norm()) < BOUND
         at += n
     assert float(wide[:, H * D:].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("cap", [3.0, 9.0, 30.0, 1000.0])
+def test_cap_of_small_and_large_scores(D, cap):
+    """scores below half the cap (a polynomial) and rows far above it (exponentials), in warps of their own and beside one another; an infinite score; what
+    lies behind the last key is not a number and stays out"""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n, H = 150, 2
+    k, v = (torch.randn(4, 64, 1, D, generator=g, device="cuda").bfloat16() for _ in "kv")
+    k[3, n - 128:] = float("nan")
+    v[3, n - 128:] = 0.0
+    q = torch.randn(n, H * D, generator=g, device="cuda")
+    q[40:43] *= 30.0                                         # (beside small rows)
+    q[64:96] *= 30.0                                         # (a warp's rows)
+    q[20, :D] = 0.0
+    q[20, 0] = 1e38                                          # (infinite as a product with a key: plus or minus the cap)
+    out = torch.zeros(n, H * D, device="cuda", dtype=torch.bfloat16)
+    scale = D ** -0.5
+    ops.softmax_attention(q, k, v, out, i32([[1, 2, 3]]), i32([0]), i32([n]), i32([n]), 1, n, H, 1, D, D, 0, scale, softcap=cap)
+    kk, vv = (c.view(-1, D)[64:64 + n].double() for c in (k, v))
+    sc = cap * torch.tanh(torch.einsum("qhd,kd->hqk", (q * scale).bfloat16().double().view(n, H, D), kk) / cap)
+    ref = torch.einsum("hqk,kd->qhd", sc.masked_fill(~torch.ones(n, n, device="cuda", dtype=torch.bool).tril(), float("-inf")).softmax(-1), vv).reshape(n, H * D)
+    # (the queries are rounded on both sides.  A score in fp32 is off by sqrt(D) 2^-24 of its largest products, up to 150 here, less than 2^-12 of a weight;
+    # the weights' roundings to bf16 and the result's are 2^-9 each)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.5 * 2.0 ** -9
+    assert bool(torch.isfinite(out).all())

@@ -8,10 +8,13 @@
 // Semantics follow the reference's generation defaults (bee2bee/hf.py:91-105):
 // repetition_penalty 1.15, top_p 0.95, do_sample iff temperature > 0, greedy otherwise.
 //
-// Performance notes: every pass over the 128k logits is
-// L2-latency bound, so logits are read 8 at a time per thread (2 x 128-bit loads in flight);
-// histogram mass is accumulated in 32.32 fixed point with native 32-bit shared-memory atomics
-// (float / 64-bit shared atomics are CAS loops).
+// Performance notes: the pass over the 128k logits is L2-latency bound, so logits are read 16 at a time
+// per thread (4 x 128-bit loads in flight); histogram mass is accumulated in 32.32 fixed point with native
+// 32-bit shared-memory atomics (float / 64-bit shared atomics are CAS loops).  Bound: the latency of four
+// cluster barriers and the steps between them (12 us at any size; it was 20 while every CTA read the
+// histograms of all), then the atomics of a flat distribution.  Measured on B200, top_p 0.95, us before /
+// now: 32 rows of 128256, flat 28.0 / 22.2, peaked (50 likely ids) 35.6 / 20.1, all ids kept 50 / 36; one
+// row 24.0 / 16.7; 8 rows of 32000 21.7 / 13.2.
 #include "kernels.h"
 
 #include "common.cuh"
@@ -20,7 +23,7 @@
 namespace b2b {
 
 constexpr int SAMP_THREADS = 1024;
-constexpr int NBINS = 4096;
+constexpr int P1 = 4;                // quads of logits per thread in flight
 
 __device__ __forceinline__ uint32_t hash_u32(uint32_t x) {
   x ^= x >> 16; x *= 0x7feb352dU; x ^= x >> 15; x *= 0x846ca68bU; x ^= x >> 16;
@@ -65,8 +68,7 @@ constexpr int MAX_SLICE = 36864;     // ids per CTA kept in shared memory (144 K
 struct __align__(16) SampShared {
   uint32_t h1_lo[SBINS], h1_hi[SBINS];      // level-1 histogram, 32.32 fixed point split in two native-atomic words
   uint32_t h2_lo[SBINS], h2_hi[SBINS];      // level-2 histogram (inside the boundary bin)
-  unsigned long long merged[SBINS];         // cluster-wide sum of the level being scanned
-  unsigned long long wsum[32];
+  unsigned long long chunk[2][MAX_CS][32];  // per level and CTA: sums of 64 bins (written by every peer)
   unsigned long long red_u[32];
   unsigned long long cz[MAX_CS];            // per-CTA partition-function partials (written by every peer)
   float cmax[MAX_CS];
@@ -98,7 +100,7 @@ __device__ __forceinline__ void hist_add(uint32_t* lo, uint32_t* hi, int bin, ui
 // One CLUSTER of CS CTAs per sequence (grid = [B, 1, CS]); CTA r owns ids [r*W, (r+1)*W).  A single
 // SM is instruction-bound on a 128k vocabulary (about 28 us per pass), so the
 // vocabulary is spread over CS SMs, each slice is read from L2 exactly once and then lives in shared
-// memory as exp(l - max); the per-level histograms are merged across the cluster through DSMEM.
+// memory as exp(l - max); the per-level histograms are searched across the cluster through DSMEM.
 __global__ void __launch_bounds__(SAMP_THREADS, 1) sample_kernel(const SampleParams p, const int W) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   SampShared& S = *reinterpret_cast<SampShared*>(smem_raw);
@@ -171,33 +173,29 @@ __global__ void __launch_bounds__(SAMP_THREADS, 1) sample_kernel(const SamplePar
       ebuf[i - lo] = l;
       if (l > mx) { mx = l; amx = i; }
     };
-    for (int q = tid; q < n4; q += 2 * SAMP_THREADS) {
-      const int q2 = q + SAMP_THREADS;
-      const bool has2 = q2 < n4;
-      const int i0 = lo + 4 * q, i1 = lo + 4 * q2;
-      float a[4], c[4] = {0.f, 0.f, 0.f, 0.f};
-      if (vec_ok) {
-        const float4 va = *reinterpret_cast<const float4*>(logits + i0);
-        a[0] = va.x; a[1] = va.y; a[2] = va.z; a[3] = va.w;
-        if (has2) {
-          const float4 vc = *reinterpret_cast<const float4*>(logits + i1);
-          c[0] = vc.x; c[1] = vc.y; c[2] = vc.z; c[3] = vc.w;
-        }
-      } else {
+    for (int q0 = tid; q0 < n4; q0 += P1 * SAMP_THREADS) {
+      float a[P1][4];
+      uint32_t sw[P1];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) a[k] = logits[i0 + k];
-        if (has2) {
+      for (int j = 0; j < P1; ++j) {
+        const int q = q0 + j * SAMP_THREADS, i0 = lo + 4 * q;
+        sw[j] = 0u;
+        if (q >= n4) continue;
+        if (vec_ok) {
+          const float4 v = *reinterpret_cast<const float4*>(logits + i0);
+          a[j][0] = v.x; a[j][1] = v.y; a[j][2] = v.z; a[j][3] = v.w;
+        } else {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) c[k] = logits[i1 + k];
+          for (int k = 0; k < 4; ++k) a[j][k] = logits[i0 + k];
         }
+        if (seen_r) sw[j] = seen_r[i0 >> 5];
       }
-      const uint32_t sa = seen_r ? seen_r[i0 >> 5] : 0u;
-      const uint32_t sc = (seen_r && has2) ? seen_r[i1 >> 5] : 0u;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) take(i0 + k, a[k], sa);
-      if (has2) {
+      for (int j = 0; j < P1; ++j) {
+        const int q = q0 + j * SAMP_THREADS, i0 = lo + 4 * q;
+        if (q >= n4) break;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) take(i1 + k, c[k], sc);
+        for (int k = 0; k < 4; ++k) take(i0 + k, a[j][k], sw[j]);
       }
     }
     for (int i = lo + 4 * n4 + tid; i < hi; i += SAMP_THREADS) take(i, logits[i], seen_r ? seen_r[i >> 5] : 0u);
@@ -235,28 +233,28 @@ __global__ void __launch_bounds__(SAMP_THREADS, 1) sample_kernel(const SamplePar
     return;
   }
 
-  // ---- phase 2: e = exp(l - max) in place; level-1 histogram (top 11 key bits) and partition function
+  // ---- phase 2: e = exp(l - max) in place, partition function, level-1 histogram (top 11 key bits).  A value below (1 - top_p) Z / V is never the boundary:
+  // all of those together weigh less than what is cut off.  Z is at least one, the largest value, so what is below (1 - top_p) / V stays out of the
+  // histogram: a fifth of flat logits, and nearly all of peaked ones, whose small values would all meet in a few bins.
+  const uint32_t least = max(1u, static_cast<uint32_t>(fminf(0.99f * (1.f - top_p) * 4294967296.0f / static_cast<float>(V), 4294967040.0f)));
   unsigned long long zsum = 0ull;
   {
+    auto add = [&](float e) {
+      const uint32_t f = fx32(e);
+      zsum += f;
+      if (f >= least) hist_add(S.h1_lo, S.h1_hi, dkey(e) >> 17, f);
+    };
     float4* e4 = reinterpret_cast<float4*>(ebuf);
     for (int q = tid; q < n4; q += SAMP_THREADS) {
       float4 v = e4[q];
       v.x = __expf(v.x - mx); v.y = __expf(v.y - mx); v.z = __expf(v.z - mx); v.w = __expf(v.w - mx);
       e4[q] = v;
-      const float ev[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t f = fx32(ev[k]);
-        zsum += f;
-        hist_add(S.h1_lo, S.h1_hi, dkey(ev[k]) >> 17, f);
-      }
+      add(v.x); add(v.y); add(v.z); add(v.w);
     }
     for (int j = 4 * n4 + tid; j < n; j += SAMP_THREADS) {
       const float e = __expf(ebuf[j] - mx);
       ebuf[j] = e;
-      const uint32_t f = fx32(e);
-      zsum += f;
-      hist_add(S.h1_lo, S.h1_hi, dkey(e) >> 17, f);
+      add(e);
     }
   }
 #pragma unroll
@@ -269,68 +267,72 @@ __global__ void __launch_bounds__(SAMP_THREADS, 1) sample_kernel(const SamplePar
     for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
     if (lane < CS) st_dsmem_u64(mapa_smem(smem_u32(&S.cz[r]), lane), z);
   }
-  cluster_sync_all();
-
-  // cluster-wide histogram -> S.merged (every CTA computes the same sum), then a top-down search for the
-  // highest bin whose suffix mass (plus `carry`) reaches `need`.  Results: s_i[0] = bin, s_u[0] = mass above it.
-  auto merge_and_find = [&](uint32_t* hlo, uint32_t* hhi, unsigned long long carry, unsigned long long need) {
-    {
-      const int bin = 2 * tid;        // SBINS == 2 * SAMP_THREADS
-      unsigned long long m0 = 0ull, m1 = 0ull;
-      const uint32_t alo = smem_u32(&hlo[bin]), ahi = smem_u32(&hhi[bin]);
-      for (int c = 0; c < CS; ++c) {
-        const uint2 l2 = ld_dsmem_v2u32(mapa_smem(alo, c));
-        const uint2 h2 = ld_dsmem_v2u32(mapa_smem(ahi, c));
-        m0 += (static_cast<unsigned long long>(h2.x) << 32) | l2.x;
-        m1 += (static_cast<unsigned long long>(h2.y) << 32) | l2.y;
-      }
-      S.merged[bin] = m0; S.merged[bin + 1] = m1;
-      unsigned long long ws = m0 + m1;      // warp w covers bins [64w, 64w + 64)
+  // Highest bin whose suffix mass over the cluster (plus `carry`) reaches `need`: the CTAs leave sums of 64 bins with every peer, one warp finds the 64 bins
+  // there and reads only those from the peers.  (Every CTA reading all bins of all was 128 KB at 8 CTAs, twice: 5 us of it each.)  s_i[0] = bin, s_u[0] =
+  // mass above it.
+  auto leave_sums = [&](int level, const uint32_t* hlo, const uint32_t* hhi) {                // (behind a barrier)
+    const uint2 l2 = *reinterpret_cast<const uint2*>(&hlo[2 * tid]), h2 = *reinterpret_cast<const uint2*>(&hhi[2 * tid]);          // SBINS == 2 * SAMP_THREADS
+    unsigned long long ws = (static_cast<unsigned long long>(h2.x) << 32) + l2.x + (static_cast<unsigned long long>(h2.y) << 32) + l2.y;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
-      if (lane == 0) S.wsum[warp] = ws;
-    }
-    __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+    if (lane < CS) st_dsmem_u64(mapa_smem(smem_u32(&S.chunk[level][r][warp]), lane), ws);
+    cluster_sync_all();
+  };
+  auto find = [&](int level, const uint32_t* hlo, const uint32_t* hhi, unsigned long long carry, unsigned long long need) {
     if (warp == 0) {
-      // lane l looks at warp-chunk 31 - l (highest bins first)
-      const unsigned long long v = S.wsum[31 - lane];
-      unsigned long long pre = v;
+      auto scan = [&](unsigned long long v) {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const unsigned long long t = __shfl_up_sync(0xffffffffu, pre, o); if (lane >= o) pre += t; }
+        for (int o = 1; o < 32; o <<= 1) { const unsigned long long t = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += t; }
+        return v;
+      };
+      unsigned long long v = 0ull;         // lane l looks at sum 31 - l (highest bins first)
+      for (int c = 0; c < CS; ++c) v += S.chunk[level][c][31 - lane];
+      const unsigned long long pre = scan(v);
       const unsigned ball = __ballot_sync(0xffffffffu, carry + pre >= need);
-      int found = -1;
+      int found = 0;
       unsigned long long above = carry;
       if (ball) {
         const int l0 = __ffs(ball) - 1;
-        unsigned long long run = carry + __shfl_sync(0xffffffffu, pre, l0) - __shfl_sync(0xffffffffu, v, l0);
-        const int cbase = (31 - l0) * 64;
-        for (int base = cbase + 32; base >= cbase && found < 0; base -= 32) {
-          const unsigned long long bv = S.merged[base + (31 - lane)];
-          unsigned long long bp = bv;
+        const unsigned long long run = carry + __shfl_sync(0xffffffffu, pre - v, l0);
+        const int bin = (31 - l0) * 64 + 62 - 2 * lane;                // this lane's two bins
+        const uint32_t alo = smem_u32(&hlo[bin]), ahi = smem_u32(&hhi[bin]);
+        unsigned long long m0 = 0ull, m1 = 0ull;
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) { const unsigned long long t = __shfl_up_sync(0xffffffffu, bp, o); if (lane >= o) bp += t; }
-          const unsigned hit = __ballot_sync(0xffffffffu, run + bp >= need);
-          if (hit) {
-            const int l1 = __ffs(hit) - 1;
-            found = base + (31 - l1);
-            above = run + __shfl_sync(0xffffffffu, bp, l1) - __shfl_sync(0xffffffffu, bv, l1);
-          } else {
-            run += __shfl_sync(0xffffffffu, bp, 31);
-          }
+        for (int c0 = 0; c0 < MAX_CS; c0 += 4) {                       // (four peers at a time: one by one each would wait for the one before)
+          uint2 l2[4], h2[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c0 + c < CS) {
+              l2[c] = ld_dsmem_v2u32(mapa_smem(alo, c0 + c));
+              h2[c] = ld_dsmem_v2u32(mapa_smem(ahi, c0 + c));
+            }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (c0 + c < CS) {
+              m0 += (static_cast<unsigned long long>(h2[c].x) << 32) | l2[c].x;
+              m1 += (static_cast<unsigned long long>(h2[c].y) << 32) | l2[c].y;
+            }
         }
+        const unsigned long long upto = run + scan(m0 + m1), from = upto - m0 - m1;
+        const unsigned hit = __ballot_sync(0xffffffffu, upto >= need);
+        const int l1 = hit ? __ffs(hit) - 1 : 31;
+        const bool upper = from + m1 >= need;
+        found = __shfl_sync(0xffffffffu, upper ? bin + 1 : bin, l1);
+        above = __shfl_sync(0xffffffffu, upper ? from : from + m1, l1);
       }
-      if (lane == 0) { S.s_i[0] = found < 0 ? 0 : found; S.s_u[0] = found < 0 ? carry : above; }
+      if (lane == 0) { S.s_i[0] = found; S.s_u[0] = above; }
     }
     __syncthreads();
   };
+  leave_sums(0, S.h1_lo, S.h1_hi);
 
   unsigned long long Z = 0ull;
   for (int c = 0; c < CS; ++c) Z += S.cz[c];
   const unsigned long long need = static_cast<unsigned long long>(static_cast<double>(top_p) * static_cast<double>(Z));
-  merge_and_find(S.h1_lo, S.h1_hi, 0ull, need);
+  find(0, S.h1_lo, S.h1_hi, 0ull, need);
   const int B1 = S.s_i[0];
   const unsigned long long above1 = S.s_u[0];       // mass strictly above the boundary bin
-  __syncthreads();                                   // s_i / merged are reused by the second level
+  __syncthreads();                                   // s_i / s_u are reused by the second level
 
   // ---- phase 3: level-2 histogram inside the boundary bin (next 11 key bits)
   {
@@ -350,8 +352,8 @@ __global__ void __launch_bounds__(SAMP_THREADS, 1) sample_kernel(const SamplePar
     }
   }
   __syncthreads();
-  cluster_sync_all();
-  merge_and_find(S.h2_lo, S.h2_hi, above1, need);
+  leave_sums(1, S.h2_lo, S.h2_hi);
+  find(1, S.h2_lo, S.h2_hi, above1, need);
   const uint32_t thr = (static_cast<uint32_t>(B1) << 17) | (static_cast<uint32_t>(S.s_i[0]) << 6);
 
   // ---- phase 4: multinomial draw over the kept set {dkey(e) >= thr}, in id order.
@@ -413,7 +415,38 @@ __global__ void __launch_bounds__(SAMP_THREADS, 1) sample_kernel(const SamplePar
   if (warp != wsel) return;
   float run = my_excl + __shfl_sync(0xffffffffu, wpre - wt, wsel);
   int pick = -1, last_kept = -1;
-  for (int base = c0; base < c1 && pick < 0; base += 32) {
+  // Groups of 32 ids in front of the target are passed over: a lane adds up a group (in the order of the scan below, so the same bits), 32 groups side by
+  // side, and the running sum goes through them one by one.  A scan per group would be 32 times 200 cycles.  Sums within rounding of the target are scanned.
+  int first = c0;
+  while (first + 32 * 32 <= ((c1 - c0) & ~1023) + c0) {
+    const float4* g4 = reinterpret_cast<const float4*>(ebuf + first + 32 * lane);
+    float part[8];
+    int kept_at = -1;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float4 v = g4[k];
+      const bool x = dkey(v.x) >= thr, y = dkey(v.y) >= thr, z = dkey(v.z) >= thr, w = dkey(v.w) >= thr;
+      part[k] = ((x ? v.x : 0.f) + (y ? v.y : 0.f)) + ((z ? v.z : 0.f) + (w ? v.w : 0.f));
+      if ((x && v.x > 0.f) || (y && v.y > 0.f) || (z && v.z > 0.f) || (w && v.w > 0.f))
+        kept_at = first + 32 * lane + 4 * k + (w && v.w > 0.f ? 3 : (z && v.z > 0.f ? 2 : (y && v.y > 0.f ? 1 : 0)));
+    }
+    const float tot = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+    int stop = 32;
+    float at = run;
+#pragma unroll
+    for (int gi = 0; gi < 32; ++gi) {
+      const float t = __shfl_sync(0xffffffffu, tot, gi);
+      if (stop == 32) {
+        if (at + t * 1.00001f >= target * 0.99999f) stop = gi;
+        else at += t;
+      }
+    }
+    run = at;
+    for (int gi = 0; gi < stop; ++gi) last_kept = max(last_kept, __shfl_sync(0xffffffffu, kept_at, gi));
+    first += 32 * stop;
+    if (stop < 32) break;
+  }
+  for (int base = first; base < c1 && pick < 0; base += 32) {
     const int j = base + lane;
     float v = 0.f;
     if (j < c1) { const float e = ebuf[j]; if (dkey(e) >= thr) v = e; }

@@ -233,7 +233,7 @@ class NativePiece:
                                    dtype=torch.float32)
         self._chain = self._chain_of = None
         self._chain_ln = not self.fused_norm and not c.glu and c.bias and not c.post_norms and c.rope_theta <= 0 and c.attn_softcap == 0
-        if units is None and self.layers and (self._chain_ln or (self.fused_norm and c.glu and self.fp8 == self.mx_fuse)) and self.device.type == "cuda":
+        if self.head_mode == 0 and self.tail_mode == 2 and self.layers and (self._chain_ln or (self.fused_norm and c.glu and self.fp8 == self.mx_fuse)) and self.device.type == "cuda":
             with torch.cuda.device(dev):
                 if ops.native().layer_chain_supported(c.hidden_size, c.ffn_size, c.n_heads, c.n_kv_heads, c.head_dim, c.post_norms, self._chain_ln,
                                                       self.mx_fuse):

@@ -282,6 +282,7 @@ static b2b::ChainDims chain_dims(int64_t hidden, int64_t ffn, int64_t n_q, int64
 struct LayerChain {
   b2b::ChainDims d;
   int layers, max_tokens;
+  uint32_t polls = 0;                      // of a counter before a launch gives up, 0: seconds of them
   Tensor table, control;
   std::vector<Tensor> keep;
   Tensor xa, xb, q, attn, h, norm;
@@ -398,6 +399,7 @@ struct LayerChain {
     c.control = reinterpret_cast<uint32_t*>(control.data_ptr());
     c.layers = layers; c.tokens = static_cast<int>(T); c.seqs = static_cast<int>(S); c.max_tokens = max_tokens;
     c.max_pages = static_cast<int>(block_table.size(1));
+    c.polls = polls;
     c.x_in = x_in.data_ptr();
     c.xa = xa.data_ptr(); c.xb = xb.data_ptr(); c.q = q.data_ptr(); c.attn = attn.data_ptr(); c.h = h.data_ptr();
     c.norm = norm.defined() ? norm.data_ptr() : nullptr;
@@ -1177,6 +1179,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def(py::init<const std::vector<std::vector<Tensor>>&, const std::vector<int64_t>&, const Tensor&, const Tensor&, const Tensor&, const Tensor&,
                     const Tensor&, const OptT&, int64_t, int64_t, int64_t, int64_t, bool, double, double, double, double, bool, const std::vector<Tensor>&>())
       .def_property_readonly("step_tokens", [](const LayerChain& c) { return b2b::layer_chain_tokens(c.d); })
+      .def_readwrite("polls", &LayerChain::polls)
+      .def_readonly("control", &LayerChain::control)
       .def("run", &LayerChain::run);
   m.def("layer_chain_supported", &layer_chain_supported);
   m.def("layer_chain_gave_up", &b2b::layer_chain_gave_up);

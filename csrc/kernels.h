@@ -64,6 +64,7 @@ struct ChainCall {
   const void* table;                     // layers x layer_chain_table_bytes(1), filled by layer_chain_fill
   uint32_t* control;                     // layer_chain_control_words(layers), zero before the first launch; launches that share it are ordered
   int layers, tokens, seqs, max_tokens, max_pages;
+  uint32_t polls;                        // of a counter before the launch gives up, 0: the default (seconds)
   const void* x_in;                      // [tokens, hidden]; may be xa
   void *xa, *xb, *q, *attn, *h, *norm;   // [max_tokens, ..] buffers; the result is in xa (LayerNorm models: norm holds the normed rows of x_in)
   const int *positions, *slots, *q_start, *q_len, *kv_len, *block_table;

@@ -51,7 +51,7 @@ constexpr int LC_PAGE = 64, LC_KEYS = 128, LC_HEADS = 16;
 constexpr int LC_BLOCK = 128 * 128;                // 128 rows x 64 bf16: a weight block, or 128 keys x 64 channels
 constexpr int LC_XSLOTS = 6;                       // copies of activations in flight, at most
 constexpr int LC_ENTRIES = 16;                     // entries of the ring in flight, at most
-constexpr uint32_t LC_SPINS = 1u << 23;            // polls of a counter (0.3 us or more each)
+constexpr uint32_t LC_SPINS = 1u << 23;            // polls of a counter (0.3 us or more each) unless the plan asks for fewer
 constexpr int LC_SS = 64 * 64;
 constexpr float LC_LOG2E = 1.4426950408889634f;
 
@@ -61,7 +61,7 @@ constexpr int LC_PRODUCTS = 4;
 __host__ __device__ constexpr int lc_weight(int op) { return op == OP_QKV ? 0 : (op == OP_O ? 1 : (op == OP_GU ? 2 : (op == OP_DOWN ? 3 : -1))); }
 
 // words of the control block in front of the operations' counters
-enum LcWord : int { LW_EXIT = 0, LW_ABORT = 1, LW_CTR = 32 };
+enum LcWord : int { LW_EXIT = 0, LW_ABORT = 1, LW_GAVE_UP = 2, LW_CTR = 32 };   // LW_GAVE_UP: launches that ended early, never reset
 
 __device__ unsigned int g_chain_gave_up = 0;       // launches that ended early since the module was loaded
 
@@ -95,6 +95,7 @@ struct LcParams {
   __nv_bfloat16 *xa, *xb, *q, *attn, *h, *norm;
   const int *positions, *slots, *q_start, *q_len, *kv_len, *block_table;
   int max_pages;
+  uint32_t polls;                                  // of a counter, then the launch gives up
   uint32_t* ctl;
   float* ss;                                       // [2][clusters][64 tokens] sums of squares
   uint8_t *q8_x, *q8_attn, *q8_h;                  // block-scaled fp8: the stream, the attention's output and the MLP hidden as the products read them
@@ -161,11 +162,14 @@ __device__ __forceinline__ void tma_load_3d_hint(void* dst, const CUtensorMap* m
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
                ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "l"(policy) : "memory");
 }
-// wait on a barrier that the CTAs of the cluster arrive at
-__device__ __forceinline__ bool lc_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort) {
+// wait on a barrier that the CTAs of the cluster arrive at; one that gave up arrives no more, but raises the launch's abort word
+__device__ __forceinline__ bool lc_wait_cluster(uint64_t* bar, uint32_t parity, volatile uint32_t* abort, uint32_t* ctl) {
   for (uint32_t spins = 0;; ++spins) {
     if (try_wait_cluster(bar, parity)) return true;
-    if ((spins & 255u) == 255u && *abort != 0u) return false;
+    if ((spins & 255u) == 255u) {
+      if (*abort != 0u) return false;
+      if (*reinterpret_cast<volatile uint32_t*>(ctl + LW_ABORT) != 0u) { *abort = 1u; return false; }
+    }
     if (spins > MA_SPIN_LIMIT) {
       *abort = 1u;
       return false;
@@ -173,21 +177,26 @@ __device__ __forceinline__ bool lc_wait_cluster(uint64_t* bar, uint32_t parity, 
   }
 }
 // wait until all CTAs have stored their results of an operation
-__device__ __noinline__ bool lc_wait_op(const uint32_t* ctr, uint32_t target, volatile uint32_t* abort, uint32_t* ctl) {
+__device__ __noinline__ bool lc_wait_op(const uint32_t* ctr, uint32_t target, uint32_t polls, volatile uint32_t* abort, uint32_t* ctl) {
   for (uint32_t spins = 0;; ++spins) {
     if (ld_acquire_gpu(ctr) >= target) return true;
     if ((spins & 63u) == 63u) {
       if (*abort != 0u) return false;
       if (*reinterpret_cast<volatile uint32_t*>(ctl + LW_ABORT) != 0u) { *abort = 1u; return false; }
     }
-    if (spins > LC_SPINS) {
+    if (spins >= polls) {
       *abort = 1u;
       return false;
     }
   }
 }
+// wait for copies or products in flight, also after a wait that ran out; nothing depends on the result but when this CTA's memory is given back
+__device__ __noinline__ void lc_drain(uint64_t* bar, uint32_t parity) {
+  for (uint32_t spins = 0; spins < (1u << 16) && !mbar_try_wait(bar, parity); ++spins) {
+  }
+}
 
-// the same through the word that the CTA's polling thread keeps
+// wait for an operation through the word that the CTA's polling thread keeps
 __device__ __forceinline__ bool lc_wait_due(const uint32_t* due_s, int n, volatile uint32_t* abort) {
   for (uint32_t spins = 0;; ++spins) {
     uint32_t v;
@@ -386,7 +395,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   uint64_t* pv_done = p_ready + 2;                 // [2]
   uint64_t* o_empty = pv_done + 2;
   uint64_t* part_full = o_empty + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(part_full + 1);
+  uint64_t* mma_done = part_full + 1;              // all products that were asked for
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
   volatile uint32_t* abort = tmem_slot + 1;
   uint32_t* due_s = tmem_slot + 2;                 // operations whose results are complete, as the activation warp has seen it
   __shared__ float rstd_s[CW];
@@ -396,6 +406,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   __shared__ float ml_s[2 * GP];             // this CTA's maxima and sums, read by the cluster
   __shared__ LcShare share_s[LC_PRODUCTS];
   __shared__ uint32_t entry_s[2][LC_ENTRIES];      // bytes of the ring's entries, with what was skipped in front of them
+  __shared__ uint32_t issued_s[4];                 // copies asked for: ring entries of the two filling warps, activations, queries
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank());
@@ -422,6 +433,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
     mbar_init(zone_free, 4 * LC_CL);
     mbar_init(o_empty, 4);
     mbar_init(part_full, static_cast<uint32_t>(p.parts));
+    mbar_init(mma_done, 1);
     *abort = 0u;
     *due_s = 0u;
     fence_barrier_init();
@@ -578,12 +590,13 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           }
         }
       }
+      issued_s[half] = ring.count;
     }
   } else if (warp == 6) {
     // --------------------------------------------------------------------------- activations, as soon as they are complete
     if (elect_one()) {
       const uint64_t pol = l2_policy_evict_last();
-      uint32_t nq = 0, s = 0, ph = 0;
+      uint32_t nq = 0, nx = 0, s = 0, ph = 0;
       bool ok = true;
       int at = 0;
 #pragma unroll 1
@@ -593,7 +606,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
         for (int op = 0; ok && op < OP_COUNT; ++op) {
           if (skip(l, op)) continue;
           if (at > 0) {                              // the operations so far are complete: this thread alone polls, the others of the CTA look at due_s
-            if (!(ok = lc_wait_op(ctr + at - 1, ctas, abort, p.ctl))) break;
+            if (!(ok = lc_wait_op(ctr + at - 1, ctas, p.polls, abort, p.ctl))) break;
             asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(due_s)), "r"(at) : "memory");
             fence_proxy_async_all();
           }
@@ -612,6 +625,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                 if constexpr (MX)
                   bulk_load(x_s + s * x_slot + x_bytes * XB, (op == OP_QKV ? (l == 0 ? p.sf_in : p.sf_x) : op == OP_O ? p.sf_attn : op == OP_GU ? p.sf_x : p.sf_h) +
                             static_cast<size_t>(sh.kb0 + kb) * 512, sf_bytes, &x_full[s]);
+                ++nx;
                 if (++s == x_slots) { s = 0; ph ^= 1u; }
               }
           } else if (!LN && op == OP_ATT) {
@@ -630,6 +644,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           }
         }
       }
+      issued_s[2] = nx;
+      issued_s[3] = nq;
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------------------------------------------------- MMA issuer
@@ -768,10 +784,12 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           }
         }
       }
+      umma_commit(mma_done);
     }
   } else {
     // ------------------------------------------------------------------------------------------------ epilogues and softmax
-    // (a wait that gave up ends the others through the abort word; the loops go on, because every warp has to meet the others)
+    // (a wait that gave up ends the others through the abort word; the loops go on, because every warp has to meet the others, but nothing is sent to
+    // the cluster any more: its barriers count the bytes and arrivals of every exchange)
     const int et = threadIdx.x - 64, q4 = warp & 3, row = q4 * 32 + lane;
     const int col0 = rank * CW;                        // the tokens that this CTA finishes
     const uint32_t lanes = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
@@ -882,8 +900,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               __syncwarp();
               if (lane == 0) mbar_arrive(&acc_empty[na & 1u]);
               ++na;
-              if (nx > 0 && ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(zone_free, (nx - 1) & 1u, abort));
-              if (threadIdx.x == 64) mbar_arrive_expect_tx(zone_full, static_cast<uint32_t>(lc_rows<GLU>(op, n) * LC_CL * CW * 4));
+              if (nx > 0 && ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(zone_free, (nx - 1) & 1u, abort, p.ctl));
+              if (threadIdx.x == 64 && ok) mbar_arrive_expect_tx(zone_full, static_cast<uint32_t>(lc_rows<GLU>(op, n) * LC_CL * CW * 4));
               if (live && ok) {
 #pragma unroll
                 for (int d = 0; d < LC_CL; ++d) {
@@ -894,7 +912,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                     st_async_v4(to + i * 2048, bar, a[d * CW + 4 * i], a[d * CW + 4 * i + 1], a[d * CW + 4 * i + 2], a[d * CW + 4 * i + 3]);
                 }
               }
-              if (ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(zone_full, nx & 1u, abort));
+              if (ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(zone_full, nx & 1u, abort, p.ctl));
               ++nx;
 #pragma unroll
               for (int i = 0; i < CW; ++i) v[i] = 0.f;
@@ -920,7 +938,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               for (int i = 0; i < HB; ++i) c1[i] = from[i * 64];
             }
             __syncwarp();
-            if (lane < LC_CL) arrive_cluster(mapa_smem(smem_u32(zone_free), lane));               // the sums have been read
+            if (lane < LC_CL && ok) arrive_cluster(mapa_smem(smem_u32(zone_free), lane));         // the sums have been read
             if (GLU && op == OP_GU) {
               const int t0 = up ? HB : 0;
               float h[HB];
@@ -1226,7 +1244,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               lc_sync();
               const int peer0 = rank - part;           // the CTAs of this item: consecutive ranks
               if (et < p.parts) arrive_cluster(mapa_smem(smem_u32(part_full), peer0 + et));
-              if (ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(part_full, nparts & 1u, abort));
+              if (ok) ok = __all_sync(0xffffffffu, lc_wait_cluster(part_full, nparts & 1u, abort, p.ctl));
               ++nparts;
 #pragma unroll 1
               for (int e = part * 128 + row; e < G * D; e += p.parts * 128) {
@@ -1409,14 +1427,28 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
 
   // ------------------------------------------------------------------------------------------------------------------ leaving
   __syncwarp();
-  if (*abort != 0u) {                                  // copies in flight land before the shared memory is given back
-    if (lane == 0) *reinterpret_cast<volatile uint32_t*>(p.ctl + LW_ABORT) = 1u;
-    __nanosleep(200000);
-  }
+  if (*abort != 0u && lane == 0) *reinterpret_cast<volatile uint32_t*>(p.ctl + LW_ABORT) = 1u;
   tc_fence_before();
-  __syncthreads();
+  __syncthreads();                                     // (no role waits behind this: the abort word is the same for all)
+  const bool gave_up = *abort != 0u;
+  if (threadIdx.x == 0) {
+    lc_drain(mma_done, 0u);
+    if (gave_up) {                                     // what was asked for and nobody waited for: it lands before the shared memory is given back
+      const uint32_t n0 = issued_s[0], n1 = issued_s[1], n = max(n0, n1), slots = x_slots;
+      for (uint32_t i = min(n0, n1); i < n; ++i) mbar_arrive(&full[i % LC_ENTRIES]);         // for the half that was not asked for
+      for (uint32_t i = n - min(n, static_cast<uint32_t>(LC_ENTRIES)); i < n; ++i) lc_drain(&full[i % LC_ENTRIES], i / LC_ENTRIES & 1u);
+      for (uint32_t i = issued_s[2] - min(issued_s[2], slots); i < issued_s[2]; ++i) lc_drain(&x_full[i % slots], i / slots & 1u);
+      for (uint32_t i = issued_s[3] - min(issued_s[3], static_cast<uint32_t>(NQ)); i < issued_s[3]; ++i) lc_drain(&q_full[i % NQ], i / NQ & 1u);
+    }
+  }
   cluster_arrive_release();                            // no CTA leaves while another writes to or reads from it
   cluster_wait_acquire();
+  if (gave_up && threadIdx.x == 0) {                   // sums that a neighbour sent and nobody waited for: they are on their way for a microsecond
+    const unsigned long long t0 = globaltimer_ns();
+    for (int i = 0; i < (1 << 20) && globaltimer_ns() - t0 < 100000ull; ++i) {
+    }
+  }
+  __syncthreads();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc<Cfg::kTmem>(tmem);
@@ -1429,6 +1461,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
       for (int i = 0; i < p.n_layers * OP_COUNT; ++i) c[LW_CTR + i] = 0u;
       if (c[LW_ABORT] != 0u) {
         c[LW_ABORT] = 0u;
+        c[LW_GAVE_UP] = c[LW_GAVE_UP] + 1u;
         if (g_abort_word != nullptr) *reinterpret_cast<volatile uint32_t*>(g_abort_word) = 1u;
         atomicAdd(&g_chain_gave_up, 1u);
       }
@@ -1570,6 +1603,7 @@ int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
   p.attn = static_cast<__nv_bfloat16*>(c.attn); p.h = static_cast<__nv_bfloat16*>(c.h); p.norm = static_cast<__nv_bfloat16*>(c.norm);
   p.positions = c.positions; p.slots = c.slots; p.q_start = c.q_start; p.q_len = c.q_len; p.kv_len = c.kv_len; p.block_table = c.block_table;
   p.max_pages = c.max_pages;
+  p.polls = c.polls > 0 ? c.polls : LC_SPINS;
   p.q8_x = static_cast<uint8_t*>(c.q8_x); p.q8_attn = static_cast<uint8_t*>(c.q8_attn); p.q8_h = static_cast<uint8_t*>(c.q8_h);
   p.sf_x = static_cast<uint8_t*>(c.sf_x); p.sf_attn = static_cast<uint8_t*>(c.sf_attn); p.sf_h = static_cast<uint8_t*>(c.sf_h);
   p.sf_in = static_cast<const uint8_t*>(c.sf_in);

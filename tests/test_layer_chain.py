@@ -66,6 +66,11 @@ def _run(piece, meta, caches, x, chain):
     return out, [c.clone() for c in cache]
 
 
+def _gave_up(piece):
+    """launches of the piece's plan that ended early"""
+    return int(piece._chain.control[2])
+
+
 def _rel(a, b):
     return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
 
@@ -81,7 +86,7 @@ def _compare(piece, meta, caches, x, rel=REL, launches=1):
     assert all(_rel(a, b) < rel for a, b in zip(got, ref_caches))
     again, _ = _run(piece, meta, caches, x, True)
     assert torch.equal(again, out)                           # sums in a fixed order
-    assert ops.native().layer_chain_gave_up() == 0
+    assert _gave_up(piece) == 0
     return out
 
 
@@ -191,7 +196,7 @@ def test_layer_norm_models(spans, pad, hidden, heads, ffn):
     assert _rel(out[:live], ref[:live]) < 2 * REL
     assert all(_rel(a, b) < 2 * REL for a, b in zip(got, ref_caches))
     assert torch.equal(_run(piece, meta, caches, x, True)[0][:live], out[:live])
-    assert ops.native().layer_chain_gave_up() == 0
+    assert _gave_up(piece) == 0
 
 
 # Both sides round the same values to e4m3 with the same rule.  A bf16 rounding that falls the other way moves its e4m3 value by one unit (2^-3 of it at
@@ -203,6 +208,37 @@ def test_block_scaled_fp8(seqs, hidden, heads, kv, dim, ffn):
     """edges of the token tiles; shares that start inside a run of 128 rows; the quantiser of the piece's input is a kernel of its own"""
     cfg = dataclasses.replace(resolve_config("tiny-llama"), hidden_size=hidden, n_heads=heads, n_kv_heads=kv, head_dim=dim, ffn_size=ffn)
     _compare(*_setup(cfg, 2, [1 + (37 * i) % 290 for i in range(seqs)], quant="mxfp8"), rel=2.0 ** -4, launches=2)
+
+
+@pytest.mark.parametrize("seqs,quant", [(1, "bf16"), (8, "bf16"), (40, "bf16"), (5, "mxfp8"), (30, "mxfp8")])
+def test_a_wait_that_runs_out(seqs, quant):
+    """the launch ends, says so and leaves its counters ready for the next one, while weights, cache pages and activations were on their way"""
+    from bee2bee_b200 import ops
+
+    cfg = dataclasses.replace(resolve_config("tiny-llama"), hidden_size=2048, n_heads=16, n_kv_heads=4, head_dim=128, ffn_size=5632)
+    piece, meta, caches, x = _setup(cfg, 3, [300] * seqs, quant=quant)
+    C = ops.native()
+    ref, _ = _run(piece, meta, caches, x, True)
+    n0 = C.layer_chain_gave_up()
+    word = C.peer_alloc(256)
+    told = C.tensor_from_ptr(word, [64], "i32", 0)
+    told.zero_()
+    torch.cuda.synchronize()
+    C.set_wait_policy(word, 1000.0)
+    try:
+        piece._chain.polls = 1                               # (a product takes several microseconds, a poll less than one)
+        for i in range(3):
+            _run(piece, meta, caches, x, True)
+            assert C.layer_chain_gave_up() == n0 + i + 1 and _gave_up(piece) == i + 1 and int(told[0]) == 1
+            words = piece._chain.control[:32 + 7 * 3].clone()
+            words[2] = 0
+            assert not bool(words.any())
+    finally:
+        C.set_wait_policy(0, 0.0)
+        C.peer_free(word)
+    piece._chain.polls = 0
+    out, _ = _run(piece, meta, caches, x, True)
+    assert torch.equal(out, ref) and _gave_up(piece) == 3
 
 
 def test_routes():

@@ -232,6 +232,7 @@ class NativePiece:
         self.attn_ws = torch.zeros(max_seqs * c.n_kv_heads * self.max_splits * rows * (c.head_dim + 2), device=dev,
                                    dtype=torch.float32)
         self._chain = self._chain_of = None
+        self._chain_recorded, self._chain_kept = False, []       # the plan is in a graph; plans that were and have been replaced
         self._chain_ln = not self.fused_norm and not c.glu and c.bias and not c.post_norms and c.rope_theta <= 0 and c.attn_softcap == 0
         if self.head_mode == 0 and self.tail_mode == 2 and self.layers and (self._chain_ln or (self.fused_norm and c.glu and self.fp8 == self.mx_fuse)) and self.device.type == "cuda":
             with torch.cuda.device(dev):
@@ -256,6 +257,9 @@ class NativePiece:
         """lays the layers out for the decode kernel (csrc/layer_chain.cu)"""
         c = self.cfg
         t = self._chain_tensors()
+        if self._chain_recorded:               # graphs go on reading its table and counters
+            self._chain_kept.append(self._chain)
+            self._chain_recorded = False
         fp8 = []
         if self.mx_fuse:
             H, Q = c.hidden_size, c.q_dim
@@ -273,10 +277,12 @@ class NativePiece:
             return False
         if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16:
             return False
+        recording = torch.cuda.is_current_stream_capturing()
         if self._chain_of != [[t.data_ptr() for t in row] for row in self._chain_tensors()]:       # weights or caches were replaced
-            if torch.cuda.is_current_stream_capturing():
+            if recording:
                 return False
             self._plan_chain()
+        self._chain_recorded |= recording
         return True
 
     def has_attn(self, l: int) -> bool:

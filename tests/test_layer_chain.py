@@ -1,12 +1,13 @@
 """Decode steps in one persistent kernel (csrc/layer_chain.cu) against the kernels one by one, which the other tests hold against the oracle."""
 import dataclasses
+import weakref
 
 import pytest
 import torch
 
 from bee2bee_b200.models.config import resolve_config
 
-pytestmark = pytest.mark.gpu
+gpu = pytest.mark.gpu
 
 # Both sides keep every sum in fp32 and round the same intermediates to bf16 (queries, attention output, stream, MLP hidden); a sum in another order
 # flips some of those roundings by one unit.  Five roundings of at most 2^-9 each reach the result per layer, so two layers stay below 10 * 2^-9 in the
@@ -90,6 +91,60 @@ def _compare(piece, meta, caches, x, rel=REL, launches=1):
     return out
 
 
+class _Plan:
+    """stands in for the native plan where there is no GPU"""
+    step_tokens = 64
+
+    def __init__(self, *args):
+        self.args = args
+
+
+def _cpu_piece(monkeypatch, layers=2):
+    """a piece of a small Llama on the CPU, planned as on a GPU"""
+    import types
+
+    from bee2bee_b200 import ops
+    from bee2bee_b200.models.native import NativePiece
+
+    cfg = resolve_config("tiny-llama")
+    H, F, Q, KV = cfg.hidden_size, cfg.ffn_size, cfg.q_dim, cfg.kv_dim
+    t = {f"l{l}.{n}": torch.randn(r, c) for l in range(layers)
+         for n, r, c in (("wq", Q, H), ("wk", KV, H), ("wv", KV, H), ("wo", H, Q), ("w_gate", F, H), ("w_up", F, H), ("w_down", H, F))}
+    t.update({f"l{l}.{n}": torch.ones(H) for l in range(layers) for n in ("ln1_w", "ln2_w")})
+    piece = NativePiece(cfg, range(layers), False, False, t, torch.device("cpu"), 4, 4, 8)
+    monkeypatch.setattr(ops, "native", lambda: types.SimpleNamespace(LayerChain=_Plan))
+    piece._plan_chain()
+    return piece
+
+
+def _step(n=1):
+    from bee2bee_b200.models.native import BatchMeta
+
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32)  # noqa: E731
+    return BatchMeta(ids=None, positions=i32([3] * n), slots=i32([67] * n), q_start=i32(list(range(n))), q_len=i32([1] * n), kv_len=i32([4] * n),
+                     block_table=i32([[1, 0]] * n), n_tokens=n, n_seqs=n, max_q=1)
+
+
+def test_plans_of_graphs_are_kept(monkeypatch):
+    from bee2bee_b200.models.native import Handoff
+
+    piece = _cpu_piece(monkeypatch)
+    x = torch.zeros(1, piece.cfg.hidden_size, dtype=torch.bfloat16)
+    recording = [True]
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: recording[0])
+    assert piece._chain_takes(_step(), x, Handoff())
+    first = weakref.ref(piece._chain)
+    recording[0] = False
+    piece.w["l0.wo"] = piece.w["l0.wo"].clone()
+    assert piece._chain_takes(_step(), x, Handoff()) and piece._chain is not first()
+    assert first() is not None                               # a graph reads it
+    second = weakref.ref(piece._chain)
+    piece.w["l0.wo"] = piece.w["l0.wo"].clone()
+    assert piece._chain_takes(_step(), x, Handoff())
+    assert second() is None                                  # no graph does
+
+
+@gpu
 @pytest.mark.parametrize("seqs", [1, 8, 9, 16, 17, 32, 33, 64])
 @pytest.mark.parametrize("model", ["tiny-llama", "tiny-mistral", "tiny-gemma2"])
 def test_token_tiles(model, seqs):
@@ -97,6 +152,7 @@ def test_token_tiles(model, seqs):
     _compare(*_setup(resolve_config(model), 2, [1 + (37 * i) % 290 for i in range(seqs)]))
 
 
+@gpu
 @pytest.mark.parametrize("hidden,heads,kv,dim,ffn", [(384, 4, 2, 128, 448), (2304, 8, 4, 256, 1216), (1024, 16, 2, 128, 8256), (4096, 32, 8, 128, 14336)])
 def test_shares_of_the_products(hidden, heads, kv, dim, ffn):
     """odd numbers of blocks of K, CTAs without a share, tiles of fewer than 128 rows, gate/up shares that start inside a block of 64 features"""
@@ -104,6 +160,7 @@ def test_shares_of_the_products(hidden, heads, kv, dim, ffn):
     _compare(*_setup(cfg, 2, [5, 130, 64, 63, 127]))
 
 
+@gpu
 @pytest.mark.parametrize("model,ctxs", [("tiny-llama", [0]), ("tiny-llama", [127, 128, 129, 255, 256]), ("tiny-llama", [3000, 1, 700]), ("tiny-llama", [1500] * 20),
                                         ("zephyr-7b-beta", [1200 - 13 * i for i in range(64)])])
 def test_key_tiles(model, ctxs):
@@ -112,6 +169,7 @@ def test_key_tiles(model, ctxs):
     _compare(*_setup(cfg, 1, ctxs))
 
 
+@gpu
 def test_sequences_that_take_no_part():
     piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [50, 80, 0, 200])
     meta.q_len[1] = 0                                        # as GpuRunner marks a free slot
@@ -124,6 +182,7 @@ def test_sequences_that_take_no_part():
     assert all(_rel(a, b) < REL for a, b in zip(got, ref_caches))
 
 
+@gpu
 def test_graph_replay_sees_new_inputs_and_lengths():
     piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [60, 61, 62])
     _run(piece, meta, caches, x, True)
@@ -146,12 +205,36 @@ def test_graph_replay_sees_new_inputs_and_lengths():
         assert _rel(out, ref) < REL
 
 
+@gpu
+def test_a_graph_outlives_its_plan():
+    """a graph that was recorded before a weight was replaced goes on reading what it was recorded with"""
+    piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [60, 61, 62])
+    ref, _ = _run(piece, meta, caches, x, True)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            out = piece.forward(meta, x_in=x)
+    torch.cuda.current_stream().wait_stream(stream)
+    old = piece.w["l1.w_down"]                               # (the graph's own inputs stay the caller's to keep)
+    piece.w["l1.w_down"] = old * 2
+    assert _rel(_run(piece, meta, caches, x, True)[0], ref) > 0.1
+    fill = [torch.full((n,), 255, device="cuda", dtype=torch.uint8) for n in [512 * k for k in range(1, 65)] for _ in range(8)]
+    for c, v in zip(list(piece.k_cache.values()) + list(piece.v_cache.values()), caches):
+        c.copy_(v)
+    graph.replay()
+    assert torch.equal(out, ref)
+    del fill
+
+
 def _gpt2(hidden=256, heads=4, ffn=1024):
     return dataclasses.replace(resolve_config("tiny-gpt2"), hidden_size=hidden, n_heads=heads, n_kv_heads=heads, head_dim=64, ffn_size=ffn)
 
 
 # spans (new tokens, cached tokens) of the sequences: edges of the token tiles; one key, the edges of a run of 32 and of a page; more than 128 keys (a CTA
 # per token and head) beside short ones; sequences without tokens and rows that belong to none (buckets)
+@gpu
 @pytest.mark.parametrize("spans,pad", [([(1, 0)], 0), ([(19, 0)], 0), ([(8, 0), (8, 57)], 0), ([(16, 31), (1, 64)], 0), ([(5, 0), (0, 0), (11, 3)], 5),
                                        ([(33, 96)], 0), ([(31, 0), (2, 700)], 4), ([(64, 65)], 0), ([(1, 40 * i) for i in range(20)], 0)])
 @pytest.mark.parametrize("hidden,heads,ffn", [(256, 4, 1024), (768, 12, 3072), (384, 6, 512)])
@@ -202,6 +285,7 @@ def test_layer_norm_models(spans, pad, hidden, heads, ffn):
 # Both sides round the same values to e4m3 with the same rule.  A bf16 rounding that falls the other way moves its e4m3 value by one unit (2^-3 of it at
 # most), or, where it is the largest of its 32, their common power of two, which moves all of them by less than a unit: less than 2^-4 of the result
 # even if half of all values moved.  Measured up to 0.027.
+@gpu
 @pytest.mark.parametrize("seqs", [1, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("hidden,heads,kv,dim,ffn", [(512, 4, 2, 128, 1024), (640, 8, 1, 128, 1152), (1024, 4, 2, 256, 4224), (4096, 32, 8, 128, 14336)])
 def test_block_scaled_fp8(seqs, hidden, heads, kv, dim, ffn):
@@ -210,6 +294,7 @@ def test_block_scaled_fp8(seqs, hidden, heads, kv, dim, ffn):
     _compare(*_setup(cfg, 2, [1 + (37 * i) % 290 for i in range(seqs)], quant="mxfp8"), rel=2.0 ** -4, launches=2)
 
 
+@gpu
 @pytest.mark.parametrize("seqs,quant", [(1, "bf16"), (8, "bf16"), (40, "bf16"), (5, "mxfp8"), (30, "mxfp8")])
 def test_a_wait_that_runs_out(seqs, quant):
     """the launch ends, says so and leaves its counters ready for the next one, while weights, cache pages and activations were on their way"""
@@ -241,6 +326,7 @@ def test_a_wait_that_runs_out(seqs, quant):
     assert torch.equal(out, ref) and _gave_up(piece) == 3
 
 
+@gpu
 def test_routes():
     """what the persistent kernel does not take runs on the kernels one by one; replaced weights and caches are seen"""
     from bee2bee_b200 import ops

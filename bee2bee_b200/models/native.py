@@ -268,7 +268,12 @@ class NativePiece:
                                               self.n_buf if c.post_norms or self._chain_ln else None, c.n_heads, c.n_kv_heads, c.head_dim,
                                               int(c.act == "gelu_tanh"), c.gemma_norm, c.norm_eps, c.rope_theta, c.softmax_scale, c.attn_softcap,
                                               self._chain_ln, fp8)
-        self._chain_of = [[x.data_ptr() for x in row] for row in t]
+        self._chain_of = self._chain_key(t)
+
+    @staticmethod
+    def _chain_key(tensors):
+        """all that a plan takes from its weights and caches; it does not hold them"""
+        return [[(x.data_ptr(), x.shape, x.stride(), x.dtype) for x in row] for row in tensors]
 
     def _chain_takes(self, m: BatchMeta, x: torch.Tensor, hand: Handoff) -> bool:
         """a decode step (one new token per sequence, up to 64; block-scaled fp8: 32) of whole layers whose input and result stay on this GPU; LayerNorm models:
@@ -278,7 +283,7 @@ class NativePiece:
         if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16:
             return False
         recording = torch.cuda.is_current_stream_capturing()
-        if self._chain_of != [[t.data_ptr() for t in row] for row in self._chain_tensors()]:       # weights or caches were replaced
+        if self._chain_of != self._chain_key(self._chain_tensors()):       # weights or caches were replaced
             if recording:
                 return False
             self._plan_chain()

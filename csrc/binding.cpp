@@ -277,14 +277,14 @@ static b2b::ChainDims chain_dims(int64_t hidden, int64_t ffn, int64_t n_q, int64
   return d;
 }
 
-// A piece's weights, caches and buffers laid out for layer_chain.cu.  Holds the tensors it points to; launches that use one plan are ordered by
-// their stream, like the buffers they share.
+// A piece's weights, caches and buffers laid out for layer_chain.cu.  Holds the buffers; weights and caches stay the piece's, which makes a new plan before
+// the first launch after it has replaced one (a plan that held them kept what was replaced).  Launches that use one plan are ordered by their stream, like
+// the buffers they share.
 struct LayerChain {
   b2b::ChainDims d;
   int layers, max_tokens;
   uint32_t polls = 0;                      // of a counter before a launch gives up, 0: seconds of them
   Tensor table, control;
-  std::vector<Tensor> keep;
   Tensor xa, xb, q, attn, h, norm;
   std::vector<Tensor> fp8;                 // input, stream, attention output, MLP hidden in e4m3, each with its scale factors
 
@@ -371,7 +371,6 @@ struct LayerChain {
         }
       }
       check(b2b::layer_chain_fill(static_cast<uint8_t*>(host.data_ptr()) + one * l, d, w), "layer_chain_fill");
-      keep.insert(keep.end(), t.begin(), t.end());
     }
     c10::cuda::CUDAGuard guard(xa.device());
     table = host.to(xa.device());

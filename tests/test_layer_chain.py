@@ -113,6 +113,7 @@ def _cpu_piece(monkeypatch, layers=2):
     t.update({f"l{l}.{n}": torch.ones(H) for l in range(layers) for n in ("ln1_w", "ln2_w")})
     piece = NativePiece(cfg, range(layers), False, False, t, torch.device("cpu"), 4, 4, 8)
     monkeypatch.setattr(ops, "native", lambda: types.SimpleNamespace(LayerChain=_Plan))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     piece._plan_chain()
     return piece
 
@@ -142,6 +143,20 @@ def test_plans_of_graphs_are_kept(monkeypatch):
     piece.w["l0.wo"] = piece.w["l0.wo"].clone()
     assert piece._chain_takes(_step(), x, Handoff())
     assert second() is None                                  # no graph does
+
+
+def test_plans_follow_shapes_and_types(monkeypatch):
+    """what replaces a weight may lie where the old one lay"""
+    from bee2bee_b200.models.native import Handoff
+
+    piece = _cpu_piece(monkeypatch)
+    x = torch.zeros(1, piece.cfg.hidden_size, dtype=torch.bfloat16)
+    w = piece.w["l0.wo"]
+    for new in (w.view(-1, 64), w.view(torch.float16), w.t()):
+        old = piece._chain
+        assert piece._chain_takes(_step(), x, Handoff()) and piece._chain is old
+        piece.w["l0.wo"] = new
+        assert piece._chain_takes(_step(), x, Handoff()) and piece._chain is not old
 
 
 @gpu
@@ -226,6 +241,20 @@ def test_a_graph_outlives_its_plan():
     graph.replay()
     assert torch.equal(out, ref)
     del fill
+
+
+@gpu
+def test_replaced_weights_are_let_go():
+    """a plan holds no weight or cache that its piece has replaced, also while no decode step follows"""
+    piece, meta, caches, x = _setup(dataclasses.replace(resolve_config("tiny-llama"), hidden_size=2048, ffn_size=8192), 2, [60, 61])
+    _run(piece, meta, caches, x, True)
+    new = [piece.w["l1.w_down"].clone(), piece.k_cache[0].clone()]
+    held = torch.cuda.memory_allocated()
+    gone = piece.w["l1.w_down"].nbytes + piece.k_cache[0].nbytes
+    piece.w["l1.w_down"], piece.k_cache[0] = new
+    del new
+    assert torch.cuda.memory_allocated() <= held - gone
+    _compare(piece, meta, caches, x)
 
 
 def _gpt2(hidden=256, heads=4, ffn=1024):

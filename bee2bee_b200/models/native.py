@@ -90,6 +90,35 @@ class BatchMeta:
     bucket: bool = False                      # the sizes are a bucket's: fewer sequences and tokens may be live (q_len says which)
 
 
+# What the persistent decode kernel and the kernels one by one take for attention, us per 128 keys of a 128-wide key/value head (64 KB; wider heads in
+# proportion): one CTA of either (the persistent one has two issuing warps; attn_decode.cu one, and two CTAs per SM at 128 channels) and the whole chip's
+# stream.  Measured on B200 over 1 to 64 sequences of Llama-3-8B and Gemma-2-2B behind 100 to 16000 keys.
+CHAIN_TILE_US, DECODE_TILE_US, STREAM_TILE_US = 0.87, {128: 1.17, 256: 1.4}, 0.0101
+
+
+def chain_attention_us(seqs: int, n_kv: int, head_dim: int, keys: int, window: int, ctas: int) -> float:
+    """what attention of one layer costs more (less: negative) in the persistent decode kernel than in a kernel of its own.
+
+    A (sequence, key/value head) is an item.  The persistent kernel has one CTA per SM on ``ctas`` SMs and shares an item among at most 4 of them; items that
+    do not fill its last round leave most CTAs waiting for the few that walk one more (17 to 24 Llama-3-8B sequences behind 8000 keys: 20 to 37 us per layer
+    lost).  The other kernel shares an item among up to 8 CTAs and starts new ones as the first end."""
+    if window > 0:
+        keys = min(keys, window + 127)
+    items, unit, tiles = seqs * n_kv, head_dim / 128, (keys + 127) // 128
+
+    def rounds(slots: int, parts: int, tile: float) -> float:
+        full, rest = divmod(items, max(1, slots // parts))
+        per = (tiles + parts - 1) // parts
+        last = per * max(tile, rest * parts * STREAM_TILE_US * unit) if rest else 0.0
+        return full * per * max(tile, slots * STREAM_TILE_US * unit) + last
+
+    parts = 4 if items * 4 <= ctas else (2 if items * 2 <= ctas else 1)
+    slots, own = (296 if head_dim == 128 else 148), 1
+    while own < 8 and items * own * 2 <= slots and own * 2 <= tiles:
+        own *= 2
+    return rounds(ctas, parts, CHAIN_TILE_US * unit) - rounds(slots, own, DECODE_TILE_US[head_dim])
+
+
 class NativePiece:
     def __init__(self, cfg: ModelConfig, layers: Iterable[int], first: bool, last: bool, tensors: Tensors,
                  device: torch.device, max_tokens: int, max_seqs: int, num_pages: int, quant: str = "bf16",
@@ -275,12 +304,28 @@ class NativePiece:
         """all that a plan takes from its weights and caches; it does not hold them"""
         return [[(x.data_ptr(), x.shape, x.stride(), x.dtype) for x in row] for row in tensors]
 
+    def _chain_pays(self, m: BatchMeta) -> bool:
+        """the persistent kernel is the faster one for as many keys as the tokens of ``m`` may see.  Per layer it gains (products and launches) 9.5 us on Llama and
+        Mistral shapes, 5 behind post norms, 11.5 from 33 tokens on; block-scaled fp8 5 up to 16 tokens and nothing beyond (measured as above, the smaller
+        ones of each)."""
+        c = self.cfg
+        keys = m.block_table.shape[1] * ops.PAGE
+        if self._chain_ln:
+            return True
+        if self.mx_fuse:
+            gain = 5.0 if m.n_tokens <= 16 else 0.25
+        else:
+            gain = 11.5 if m.n_tokens > 32 else (5.0 if c.post_norms else 9.5)
+        windows = [c.layer_window(l) for l in self.layers]
+        lost = sum(windows.count(w) * chain_attention_us(m.n_seqs, c.n_kv_heads, c.head_dim, keys, w, self._chain.ctas) for w in set(windows))
+        return lost <= gain * len(windows)
+
     def _chain_takes(self, m: BatchMeta, x: torch.Tensor, hand: Handoff) -> bool:
         """a decode step (one new token per sequence, up to 64; block-scaled fp8: 32) of whole layers whose input and result stay on this GPU; LayerNorm models:
-        prompts of up to 64 tokens too"""
+        prompts of up to 64 tokens too; all while the keys are not too many (``_chain_pays``)"""
         if self._chain is None or not 1 <= m.n_tokens <= self._chain.step_tokens or not (self._chain_ln or (m.max_q == 1 and m.n_tokens == m.n_seqs)):
             return False
-        if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16:
+        if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16 or not self._chain_pays(m):
             return False
         recording = torch.cuda.is_current_stream_capturing()
         if self._chain_of != self._chain_key(self._chain_tensors()):       # weights or caches were replaced

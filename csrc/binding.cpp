@@ -282,7 +282,7 @@ static b2b::ChainDims chain_dims(int64_t hidden, int64_t ffn, int64_t n_q, int64
 // the buffers they share.
 struct LayerChain {
   b2b::ChainDims d;
-  int layers, max_tokens;
+  int layers, max_tokens, ctas;            // ctas: of a launch
   uint32_t polls = 0;                      // of a counter before a launch gives up, 0: seconds of them
   Tensor table, control;
   Tensor xa, xb, q, attn, h, norm;
@@ -375,7 +375,8 @@ struct LayerChain {
     c10::cuda::CUDAGuard guard(xa.device());
     table = host.to(xa.device());
     control = at::zeros({static_cast<int64_t>(b2b::layer_chain_control_words(layers))}, xa.options().dtype(at::kInt));
-    TORCH_CHECK(b2b::layer_chain_init(d) > 0, "layer_chain: the device cannot hold its CTAs at once");
+    ctas = 4 * std::min(b2b::layer_chain_init(d), 64);
+    TORCH_CHECK(ctas > 0, "layer_chain: the device cannot hold its CTAs at once");
     c10::cuda::getCurrentCUDAStream().synchronize();
   }
 
@@ -1180,6 +1181,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_property_readonly("step_tokens", [](const LayerChain& c) { return b2b::layer_chain_tokens(c.d); })
       .def_readwrite("polls", &LayerChain::polls)
       .def_readonly("control", &LayerChain::control)
+      .def_readonly("ctas", &LayerChain::ctas)
       .def("run", &LayerChain::run);
   m.def("layer_chain_supported", &layer_chain_supported);
   m.def("layer_chain_gave_up", &b2b::layer_chain_gave_up);

@@ -58,11 +58,13 @@ def _run(piece, meta, caches, x, chain):
     for c, v in zip(cache, caches):
         c.copy_(v)
     plan = piece._chain
+    piece._chain_pays = lambda m: True                       # (the kernel is held against the others also where it is the slower one)
     if not chain:
         piece._chain = None
     out = piece.forward(meta, x_in=x).clone()
     if not chain:
         piece._chain = plan
+    del piece._chain_pays
     torch.cuda.synchronize()
     return out, [c.clone() for c in cache]
 
@@ -93,7 +95,7 @@ def _compare(piece, meta, caches, x, rel=REL, launches=1):
 
 class _Plan:
     """stands in for the native plan where there is no GPU"""
-    step_tokens = 64
+    step_tokens, ctas = 64, 132
 
     def __init__(self, *args):
         self.args = args
@@ -124,6 +126,44 @@ def _step(n=1):
     i32 = lambda v: torch.tensor(v, dtype=torch.int32)  # noqa: E731
     return BatchMeta(ids=None, positions=i32([3] * n), slots=i32([67] * n), q_start=i32(list(range(n))), q_len=i32([1] * n), kv_len=i32([4] * n),
                      block_table=i32([[1, 0]] * n), n_tokens=n, n_seqs=n, max_q=1)
+
+
+# measured on B200, two layers, us: kernels one by one / the persistent kernel
+@pytest.mark.parametrize("seqs,keys,takes", [(1, 500, True),          # 191 / 173
+                                             (1, 8000, True),         # 207 / 197
+                                             (8, 8000, True),         # 271 / 251
+                                             (17, 500, True),         # 207 / 190
+                                             (17, 4000, False),       # 282 / 304
+                                             (20, 8000, False),       # 397 / 434
+                                             (32, 8000, True),        # 502 / 482
+                                             (34, 8000, False),       # 540 / 602
+                                             (40, 8000, True),        # 655 / 607
+                                             (50, 8000, False),       # 703 / 751
+                                             (64, 8000, True)])       # 817 / 787
+def test_route_follows_the_keys(monkeypatch, seqs, keys, takes):
+    """attention of the persistent kernel leaves most CTAs waiting where the (sequence, head) pairs do not fill its last round: behind many keys that costs more
+    than the kernel gains.  The block table says how many there may be"""
+    from bee2bee_b200.models.native import Handoff
+
+    piece = _cpu_piece(monkeypatch)
+    piece.cfg = dataclasses.replace(piece.cfg, n_heads=32, n_kv_heads=8, head_dim=128)       # (Llama-3-8B's)
+    meta = dataclasses.replace(_step(seqs), block_table=torch.zeros(seqs, (keys + 64) // 64, dtype=torch.int32))
+    assert piece._chain_takes(meta, torch.zeros(seqs, 256, dtype=torch.bfloat16), Handoff()) == takes
+
+
+# Gemma-2-2B (4 heads of 256 channels, a window of 4096 in every other layer) and block-scaled fp8
+@pytest.mark.parametrize("seqs,kv,dim,windows,keys,gain,pays", [(1, 4, 256, (4096, 0), 500, 5.0, True),        # 125 / 110
+                                                                (2, 4, 256, (4096, 0), 4000, 5.0, False),      # 126 / 129
+                                                                (8, 4, 256, (4096, 0), 8000, 5.0, True),       # 180 / 167
+                                                                (34, 4, 256, (4096, 0), 4000, 11.5, False),    # 305 / 364
+                                                                (40, 4, 256, (4096, 0), 8000, 11.5, True),     # 502 / 494
+                                                                (17, 8, 128, (0,), 500, 0.25, False),          # 156 / 160
+                                                                (32, 8, 128, (0,), 500, 0.25, True),           # 169 / 166
+                                                                (10, 8, 128, (0,), 16000, 5.0, False)])        # 343 / 351
+def test_what_attention_costs(seqs, kv, dim, windows, keys, gain, pays):
+    from bee2bee_b200.models.native import chain_attention_us
+
+    assert (sum(chain_attention_us(seqs, kv, dim, keys, w, 132) for w in windows) / len(windows) <= gain) == pays
 
 
 def test_plans_of_graphs_are_kept(monkeypatch):

@@ -309,10 +309,12 @@ class GpuRunner:
         mq = min(_pow2_at_least(max_q, 16), tb)
         return tb, sb, mq
 
-    def _pf_state(self, key: tuple) -> dict:
+    def _pf_state(self, key: tuple, keys: int = 0) -> dict:
         """state of a chunk bucket: ``(tokens, sequences, max_q, parity)`` for generation chunks (one logits row per
-        sequence, sampled), ``(..., rows, True)`` for scoring chunks (``rows`` logits rows, nothing sampled)"""
-        st = self._pf.get(key)
+        sequence, sampled), ``(..., rows, True)`` for scoring chunks (``rows`` logits rows, nothing sampled).
+        ``keys`` > 0: chunks whose tokens see no more keys than that, where the piece has another kernel for them"""
+        entry = (key, keys) if keys else key
+        st = self._pf.get(entry)
         if st is not None:
             return st
         tb, sb, mq, parity = key[:4]
@@ -340,7 +342,7 @@ class GpuRunner:
                 h_in = self.C.tensor_from_ptr(hand.in_h, [tb, self.cfg.ffn_size], "bf16", dev.index)
         meta = BatchMeta(ids=v["ids"], positions=v["pos"], slots=v["slots"], q_start=v["q_start"], q_len=v["q_len"],
                          kv_len=v["kv_len"], block_table=v["bt"], n_tokens=tb, n_seqs=sb, max_q=mq,
-                         last_idx=v["last_idx"], seq_slot=v["seq_slot"], n_out=ob, bucket=True)
+                         last_idx=v["last_idx"], seq_slot=v["seq_slot"], n_out=ob, max_keys=keys, bucket=True)
         st["meta"] = meta       # captured kernels address these views by raw pointer: keep them alive
 
         def body():
@@ -377,7 +379,7 @@ class GpuRunner:
                     body()
                 st["launches"] = ops.LAUNCHES[0] - n0        # kernels recorded into this chunk graph
                 st["graph"] = g
-        self._pf[key] = st
+        self._pf[entry] = st
         return st
 
     def _run_chunk(self, chunk: List[Tuple[SeqInit, int, int]], want_rows: Optional[Sequence[int]] = None) -> None:
@@ -389,7 +391,8 @@ class GpuRunner:
         parity = (self.pf_chunks & 1) if self.world > 1 else 0
         score = want_rows is not None
         ob = min(_pow2_at_least(max(1, len(want_rows))), self.max_logit_rows) if score else sb
-        st = self._pf_state((tb, sb, mq, parity, ob, True) if score else (tb, sb, mq, parity))
+        few = 0 if self.cfg.hybrid else self.piece.span_keys(tb)
+        st = self._pf_state((tb, sb, mq, parity, ob, True) if score else (tb, sb, mq, parity), few if max(c1 for _, _, c1 in chunk) <= few else 0)
         turn = st["turn"]
         st["turn"] = (turn + 1) % len(st["hosts"])
         if st["events"][turn] is not None:

@@ -87,6 +87,7 @@ class BatchMeta:
     splits: int = 1
     seq_slot: Optional[torch.Tensor] = None   # [S] int32 batch slot of each sequence (per-sequence recurrent state)
     n_out: int = 0                            # rows of logits wanted (0 = one per sequence)
+    max_keys: int = 0                         # no token sees more keys than this (0 = as many as the block table holds)
     bucket: bool = False                      # the sizes are a bucket's: fewer sequences and tokens may be live (q_len says which)
 
 
@@ -117,6 +118,15 @@ def chain_attention_us(seqs: int, n_kv: int, head_dim: int, keys: int, window: i
     while own < 8 and items * own * 2 <= slots and own * 2 <= tiles:
         own *= 2
     return rounds(ctas, parts, CHAIN_TILE_US * unit) - rounds(slots, own, DECODE_TILE_US[head_dim])
+
+
+def chain_key_limit(tokens: int, heads: int, ctas: int) -> int:
+    """LayerNorm models: the most keys that a token may see for the persistent kernel to be the faster one.  Its attention reads all keys of a (token, head) for
+    that one alone, on a warp up to 128 keys and on a CTA beyond; the kernel of its own reads them once for 16 tokens.  gpt2, us per layer gained, by
+    rounds of (token, head) over the CTAs: one round 3 to 9 at 900 keys; two 4 at 256 to 300, -4 to -23 at 500 to 900; three and four 3 to 7 at 128, 2 to
+    -1 at 170; more 4 at 115, 1 to -1 at 124."""
+    rounds = -(-tokens * heads // ctas)
+    return 1024 if rounds <= 1 else (256 if rounds == 2 else (128 if rounds <= 4 else 112))
 
 
 class NativePiece:
@@ -304,14 +314,20 @@ class NativePiece:
         """all that a plan takes from its weights and caches; it does not hold them"""
         return [[(x.data_ptr(), x.shape, x.stride(), x.dtype) for x in row] for row in tensors]
 
+    def span_keys(self, tokens: int) -> int:
+        """spans of so many new tokens run in the persistent kernel while none of them sees more keys than this (0: spans never do)"""
+        if self._chain is None or not self._chain_ln or tokens > self._chain.step_tokens:
+            return 0
+        return chain_key_limit(tokens, self.cfg.n_heads, self._chain.ctas)
+
     def _chain_pays(self, m: BatchMeta) -> bool:
         """the persistent kernel is the faster one for as many keys as the tokens of ``m`` may see.  Per layer it gains (products and launches) 9.5 us on Llama and
         Mistral shapes, 5 behind post norms, 11.5 from 33 tokens on; block-scaled fp8 5 up to 16 tokens and nothing beyond (measured as above, the smaller
         ones of each)."""
         c = self.cfg
-        keys = m.block_table.shape[1] * ops.PAGE
-        if self._chain_ln:
-            return True
+        keys = m.max_keys or m.block_table.shape[1] * ops.PAGE
+        if self._chain_ln:                     # (their positions come from a table)
+            return min(keys, c.max_position) <= self.span_keys(m.n_tokens)
         if self.mx_fuse:
             gain = 5.0 if m.n_tokens <= 16 else 0.25
         else:

@@ -135,7 +135,8 @@ class GpuPieceHost:
                              slots=slots, q_start=torch.zeros(1, device=dev, dtype=i32),
                              q_len=torch.tensor([T], device=dev, dtype=i32),
                              kv_len=torch.tensor([pos0 + T], device=dev, dtype=i32), block_table=pages[None, :].contiguous(),
-                             n_tokens=T, n_seqs=1, max_q=T, last_idx=torch.tensor([T - 1], device=dev, dtype=torch.int64))
+                             n_tokens=T, n_seqs=1, max_q=T, last_idx=torch.tensor([T - 1], device=dev, dtype=torch.int64),
+                             max_keys=pos0 + T)
             out = self.piece.forward(meta, x_in=hidden)
             s["len"] = pos0 + T
             self.launches += 5 * len(self.layers) + 2

@@ -101,18 +101,19 @@ class _Plan:
         self.args = args
 
 
-def _cpu_piece(monkeypatch, layers=2):
-    """a piece of a small Llama on the CPU, planned as on a GPU"""
+def _cpu_piece(monkeypatch, cfg=None, layers=2):
+    """a piece (of a small Llama) on the CPU, planned as on a GPU"""
     import types
 
     from bee2bee_b200 import ops
     from bee2bee_b200.models.native import NativePiece
 
-    cfg = resolve_config("tiny-llama")
+    cfg = cfg or resolve_config("tiny-llama")
     H, F, Q, KV = cfg.hidden_size, cfg.ffn_size, cfg.q_dim, cfg.kv_dim
     t = {f"l{l}.{n}": torch.randn(r, c) for l in range(layers)
          for n, r, c in (("wq", Q, H), ("wk", KV, H), ("wv", KV, H), ("wo", H, Q), ("w_gate", F, H), ("w_up", F, H), ("w_down", H, F))}
-    t.update({f"l{l}.{n}": torch.ones(H) for l in range(layers) for n in ("ln1_w", "ln2_w")})
+    t.update({f"l{l}.{n}": torch.ones(H) for l in range(layers) for n in ("ln1_w", "ln2_w", "ln1_b", "ln2_b")})
+    t.update({f"l{l}.{n}": torch.ones(w) for l in range(layers) for n, w in (("bq", Q), ("bk", KV), ("bv", KV), ("bo", H), ("b_up", F), ("b_down", H))})
     piece = NativePiece(cfg, range(layers), False, False, t, torch.device("cpu"), 4, 4, 8)
     monkeypatch.setattr(ops, "native", lambda: types.SimpleNamespace(LayerChain=_Plan))
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
@@ -149,6 +150,32 @@ def test_route_follows_the_keys(monkeypatch, seqs, keys, takes):
     piece.cfg = dataclasses.replace(piece.cfg, n_heads=32, n_kv_heads=8, head_dim=128)       # (Llama-3-8B's)
     meta = dataclasses.replace(_step(seqs), block_table=torch.zeros(seqs, (keys + 64) // 64, dtype=torch.int32))
     assert piece._chain_takes(meta, torch.zeros(seqs, 256, dtype=torch.bfloat16), Handoff()) == takes
+
+
+# measured on B200, all of gpt2, us: kernels one by one / the persistent kernel
+@pytest.mark.parametrize("tokens,keys,takes", [(1, 900, True),        # 555 / 487
+                                               (8, 1024, True),       # 561 / 504
+                                               (12, 256, True),       # 520 / 434
+                                               (16, 900, False),      # 612 / 696
+                                               (24, 124, True),       # 474 / 437
+                                               (32, 300, False),      # 523 / 576
+                                               (64, 64, True),        # 617 / 472
+                                               (64, 184, False),      # 648 / 698
+                                               (64, 964, False),      # 756 / 1566
+                                               (65, 65, False)])
+def test_route_of_layer_norm_models_follows_the_keys(monkeypatch, tokens, keys, takes):
+    """the persistent kernel reads all keys of a (token, head) for that one alone; a call that knows how many there are says so"""
+    from bee2bee_b200.models.native import BatchMeta, Handoff
+
+    piece = _cpu_piece(monkeypatch, _gpt2(768, 12, 768), layers=1)
+    x = torch.zeros(tokens, 768, dtype=torch.bfloat16)
+    i32 = lambda *shape: torch.zeros(shape, dtype=torch.int32)  # noqa: E731
+    meta = BatchMeta(ids=None, positions=i32(tokens), slots=i32(tokens), q_start=i32(1), q_len=i32(1), kv_len=i32(1), block_table=i32(1, (keys + 63) // 64),
+                     n_tokens=tokens, n_seqs=1, max_q=tokens, max_keys=keys)
+    assert piece._chain_takes(meta, x, Handoff()) == takes
+    # without that the block table's width is taken, at most the model's positions
+    assert piece._chain_takes(dataclasses.replace(meta, max_keys=0, block_table=i32(1, 64)), x, Handoff()) == (tokens * 12 <= 132)
+    assert piece._chain_takes(dataclasses.replace(meta, max_keys=0, block_table=i32(1, 1)), x, Handoff()) == (tokens <= 64)
 
 
 # Gemma-2-2B (4 heads of 256 channels, a window of 4096 in every other layer) and block-scaled fp8

@@ -1,5 +1,7 @@
 """Whole-piece numerics on the GPU: NativePiece (hand-written kernels, paged KV, fused
 epilogues, CUDA graphs) against the plain-PyTorch fp32 oracle, for every model family."""
+import dataclasses
+
 import pytest
 import torch
 
@@ -119,6 +121,33 @@ def test_piece_fp8_close_to_oracle(name, quant):
                 cos = torch.nn.functional.cosine_similarity(got[b].float(), ref.float(), dim=0).item()
                 assert cos > 0.98, cos
     runner.close()
+
+
+def test_prefill_buckets_know_whether_keys_are_few():
+    """GPT-2: chunks of up to 64 tokens have a graph for few keys (the persistent kernel) and one for many; both give what the kernels one by one give."""
+    cfg = dataclasses.replace(resolve_config("tiny-gpt2"), hidden_size=256, n_heads=4, n_kv_heads=4, head_dim=64, ffn_size=1024)
+    outs = []
+    for chain in (True, False):
+        r = GpuRunner(cfg, "", 0, 1, torch.device("cuda:0"), max_batch=4, groups=1, max_seq_len=512, max_prefill_tokens=64, seed=0)
+        if not chain:
+            r.piece._chain = None
+            r._pf.clear()
+        logits = []
+        for slot, L in enumerate((40, 64, 300)):                   # 300 tokens: five chunks, the later ones behind up to 256 keys
+            s = SeqInit(slot=slot, prompt=[(3 * i + slot) % cfg.vocab_size for i in range(L)], pages=list(range(1 + 8 * slot, 9 + 8 * slot)),
+                        temperature=0.0, top_p=1.0, repetition_penalty=1.0, seed=slot)
+            r.prefill([s])
+            r.sync()
+            logits.append(r.piece.logits[0, :cfg.vocab_size].clone())
+        outs.append(torch.stack(logits))
+        few = r.piece.span_keys(64)
+        assert few == (256 if chain else 0)
+        if chain:                                                  # (44 tokens of the last chunk, behind 256 keys: many)
+            assert set(r._pf) == {((64, 1, 64, 0), 256), (64, 1, 64, 0)}
+            assert r._pf[(64, 1, 64, 0)]["launches"] > r._pf[((64, 1, 64, 0), 256)]["launches"]
+        r.close()
+    # (roundings of bf16 through two layers and the head; the kernels one by one also round the attention's weights)
+    assert _rel_err(outs[0], outs[1]) < 0.02
 
 
 def test_graph_prefill_matches_eager_prefill():

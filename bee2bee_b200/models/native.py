@@ -348,6 +348,8 @@ class NativePiece:
             if recording:
                 return False
             self._plan_chain()
+        if self._chain is None or self._chain.refused:
+            return False
         self._chain_recorded |= recording
         return True
 
@@ -439,8 +441,9 @@ class NativePiece:
                 self._quant(x, with_rms=True)
             if self._chain_ln:
                 ops.layernorm(x, self.w[f"l{self.layers[0]}.ln1_w"], self.w[f"l{self.layers[0]}.ln1_b"], self.n_buf[:T], eps)
-            ops.layer_chain(self._chain, x, m.positions, m.slots, m.q_start, m.q_len, m.kv_len, m.block_table)
-            return self._head(m, self.xa[:T], hand) if self.last else self.xa[:T]
+            if ops.layer_chain(self._chain, x, m.positions, m.slots, m.q_start, m.q_len, m.kv_len, m.block_table):
+                return self._head(m, self.xa[:T], hand) if self.last else self.xa[:T]
+            # (refused: x is as it was)
         inline = self._use_inline_rstd(T)
         n_layers = len(self.layers)
         fuse = self.mx_fuse

@@ -436,9 +436,12 @@ def attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, *, 
 
 def layer_chain(plan, x, positions, slots, q_start, q_len, kv_len, block_table):
     """All layers of a decode step (one new token per sequence, up to 64; GPT-2: spans too) in one persistent kernel (csrc/layer_chain.cu); ``plan`` is the
-    piece's ``LayerChain``, which owns the weights' layout and the buffers.  The result is in the plan's ``xa``."""
-    plan.run(x, positions, slots, q_start, q_len, kv_len, block_table)
+    piece's ``LayerChain``, which owns the weights' layout and the buffers.  The result is in the plan's ``xa``.  False: the device refused the launch and
+    nothing ran (``plan.refused`` from then on)."""
+    if not plan.run(x, positions, slots, q_start, q_len, kv_len, block_table):
+        return False
     LAUNCHES[0] += 1
+    return True
 
 
 def attention_fuses_quant(max_q: int, n_q: int, n_kv: int, head_dim: int, splits: int) -> bool:

@@ -284,6 +284,7 @@ struct LayerChain {
   b2b::ChainDims d;
   int layers, max_tokens, ctas;            // ctas: of a launch
   uint32_t polls = 0;                      // of a counter before a launch gives up, 0: seconds of them
+  bool refused = false;
   Tensor table, control;
   Tensor xa, xb, q, attn, h, norm;
   std::vector<Tensor> fp8;                 // input, stream, attention output, MLP hidden in e4m3, each with its scale factors
@@ -381,8 +382,9 @@ struct LayerChain {
   }
 
   // one new token per sequence (rows of x_in in the order of the sequences), LayerNorm models: spans too, the normed rows of x_in are in `norm`; the
-  // result is in xa
-  void run(const Tensor& x_in, const OptT& positions, const Tensor& slots, const Tensor& q_start, const Tensor& q_len, const Tensor& kv_len,
+  // result is in xa.  False, here and from then on: the device refused the launch (fewer SMs than the plan counts on, no cooperative launches, ..) and nothing
+  // ran
+  bool run(const Tensor& x_in, const OptT& positions, const Tensor& slots, const Tensor& q_start, const Tensor& q_len, const Tensor& kv_len,
            const Tensor& block_table) {
     check_bf16(x_in, "x_in");
     const int64_t T = x_in.size(0), S = q_len.numel();
@@ -409,7 +411,12 @@ struct LayerChain {
     auto ip = [](const Tensor& t) { return reinterpret_cast<const int*>(t.data_ptr()); };
     c.positions = positions.has_value() ? ip(*positions) : nullptr;
     c.slots = ip(slots); c.q_start = ip(q_start); c.q_len = ip(q_len); c.kv_len = ip(kv_len); c.block_table = ip(block_table);
-    check(b2b::launch_layer_chain(d, c, cur_stream()), "layer_chain");
+    const int err = b2b::launch_layer_chain(d, c, cur_stream());
+    if (err == 0) return true;
+    cudaGetLastError();
+    check(static_cast<int>(cudaGetLastError()), "layer_chain");        // (an error that stays is not this launch's)
+    refused = true;
+    return false;
   }
 };
 
@@ -1182,6 +1189,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("polls", &LayerChain::polls)
       .def_readonly("control", &LayerChain::control)
       .def_readonly("ctas", &LayerChain::ctas)
+      .def_readonly("refused", &LayerChain::refused)
       .def("run", &LayerChain::run);
   m.def("layer_chain_supported", &layer_chain_supported);
   m.def("layer_chain_gave_up", &b2b::layer_chain_gave_up);

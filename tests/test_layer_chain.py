@@ -95,7 +95,7 @@ def _compare(piece, meta, caches, x, rel=REL, launches=1):
 
 class _Plan:
     """stands in for the native plan where there is no GPU"""
-    step_tokens, ctas = 64, 132
+    step_tokens, ctas, refused = 64, 132, False
 
     def __init__(self, *args):
         self.args = args
@@ -420,6 +420,36 @@ def test_a_wait_that_runs_out(seqs, quant):
     piece._chain.polls = 0
     out, _ = _run(piece, meta, caches, x, True)
     assert torch.equal(out, ref) and _gave_up(piece) == 3
+
+
+class _Refused:
+    """a plan whose launches the device refuses"""
+    refused, asked = False, 0
+
+    def __init__(self, plan):
+        self.plan = plan
+
+    def __getattr__(self, name):
+        return getattr(self.plan, name)
+
+    def run(self, *args):
+        self.asked += 1
+        self.refused = True
+        return False
+
+
+@gpu
+@pytest.mark.parametrize("quant", ["bf16", "mxfp8"])
+def test_a_launch_that_is_refused(quant):
+    """the kernels one by one take the step and the ones after it"""
+    cfg = dataclasses.replace(resolve_config("tiny-llama"), hidden_size=512, n_heads=4, n_kv_heads=2, head_dim=128, ffn_size=1024)
+    piece, meta, caches, x = _setup(cfg, 2, [30, 40, 200], quant=quant)
+    ref, ref_caches = _run(piece, meta, caches, x, False)
+    piece._chain = plan = _Refused(piece._chain)
+    for _ in range(2):
+        out, got = _run(piece, meta, caches, x, True)
+        assert torch.equal(out, ref) and all(torch.equal(a, b) for a, b in zip(got, ref_caches))
+    assert plan.asked == 1
 
 
 @gpu

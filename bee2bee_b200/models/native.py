@@ -303,11 +303,14 @@ class NativePiece:
         if self.mx_fuse:
             H, Q = c.hidden_size, c.q_dim
             fp8 = [self._qbuf[H], self._qsf[H], self._fq_x, self._fq_sf_x, self._qbuf[Q], self._qsf[Q], self._fq_h, self._fq_sf_h]
-        self._chain = ops.native().LayerChain(t, [c.layer_window(l) for l in self.layers], self.xa, self.xb, self.q_buf, self.attn_buf, self.h_buf,
-                                              self.n_buf if c.post_norms or self._chain_ln else None, c.n_heads, c.n_kv_heads, c.head_dim,
-                                              int(c.act == "gelu_tanh"), c.gemma_norm, c.norm_eps, c.rope_theta, c.softmax_scale, c.attn_softcap,
-                                              self._chain_ln, fp8)
         self._chain_of = self._chain_key(t)
+        try:
+            self._chain = ops.native().LayerChain(t, [c.layer_window(l) for l in self.layers], self.xa, self.xb, self.q_buf, self.attn_buf, self.h_buf,
+                                                  self.n_buf if c.post_norms or self._chain_ln else None, c.n_heads, c.n_kv_heads, c.head_dim,
+                                                  int(c.act == "gelu_tanh"), c.gemma_norm, c.norm_eps, c.rope_theta, c.softmax_scale, c.attn_softcap,
+                                                  self._chain_ln, fp8)
+        except RuntimeError:                   # weights or caches that only the kernels one by one take, or refuse themselves
+            self._chain = None
 
     @staticmethod
     def _chain_key(tensors):
@@ -338,17 +341,17 @@ class NativePiece:
 
     def _chain_takes(self, m: BatchMeta, x: torch.Tensor, hand: Handoff) -> bool:
         """a decode step (one new token per sequence, up to 64; block-scaled fp8: 32) of whole layers whose input and result stay on this GPU; LayerNorm models:
-        prompts of up to 64 tokens too; all while the keys are not too many (``_chain_pays``)"""
-        if self._chain is None or not 1 <= m.n_tokens <= self._chain.step_tokens or not (self._chain_ln or (m.max_q == 1 and m.n_tokens == m.n_seqs)):
+        prompts of up to 64 tokens too; all while the keys are not too many (``_chain_pays``) and attention on tensor cores is not switched off"""
+        if self._chain_of is None or not 1 <= m.n_tokens <= 64 or not (self._chain_ln or (m.max_q == 1 and m.n_tokens == m.n_seqs == m.q_len.numel())):
             return False
-        if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16 or not self._chain_pays(m):
+        if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16 or ops.get_attn_tc_min_q() <= 0:
             return False
         recording = torch.cuda.is_current_stream_capturing()
         if self._chain_of != self._chain_key(self._chain_tensors()):       # weights or caches were replaced
             if recording:
                 return False
             self._plan_chain()
-        if self._chain is None or self._chain.refused:
+        if self._chain is None or self._chain.refused or m.n_tokens > self._chain.step_tokens or not self._chain_pays(m):
             return False
         self._chain_recorded |= recording
         return True

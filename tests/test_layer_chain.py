@@ -115,7 +115,7 @@ def _cpu_piece(monkeypatch, cfg=None, layers=2):
     t.update({f"l{l}.{n}": torch.ones(H) for l in range(layers) for n in ("ln1_w", "ln2_w", "ln1_b", "ln2_b")})
     t.update({f"l{l}.{n}": torch.ones(w) for l in range(layers) for n, w in (("bq", Q), ("bk", KV), ("bv", KV), ("bo", H), ("b_up", F), ("b_down", H))})
     piece = NativePiece(cfg, range(layers), False, False, t, torch.device("cpu"), 4, 4, 8)
-    monkeypatch.setattr(ops, "native", lambda: types.SimpleNamespace(LayerChain=_Plan))
+    monkeypatch.setattr(ops, "native", lambda: types.SimpleNamespace(LayerChain=_Plan, get_attn_tc_min_q=lambda: 2))
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     piece._plan_chain()
     return piece
@@ -210,6 +210,34 @@ def test_plans_of_graphs_are_kept(monkeypatch):
     piece.w["l0.wo"] = piece.w["l0.wo"].clone()
     assert piece._chain_takes(_step(), x, Handoff())
     assert second() is None                                  # no graph does
+
+
+def test_what_a_plan_refuses(monkeypatch):
+    """weights and metadata that the persistent kernel does not take are no error: the kernels one by one have them"""
+    from bee2bee_b200 import ops
+    from bee2bee_b200.models.native import Handoff
+
+    piece = _cpu_piece(monkeypatch)
+    x = torch.zeros(2, piece.cfg.hidden_size, dtype=torch.bfloat16)
+    meta = _step(2)
+    # room for more sequences than take part
+    assert not piece._chain_takes(dataclasses.replace(meta, q_len=torch.tensor([1, 1, 0], dtype=torch.int32)), x, Handoff())
+    assert piece._chain_takes(meta, x, Handoff())
+    with monkeypatch.context() as mp:                        # attention on CUDA cores
+        mp.setattr(ops, "get_attn_tc_min_q", lambda: 0)
+        assert not piece._chain_takes(meta, x, Handoff())
+
+    def refuse(self, *args):
+        raise RuntimeError("sizes")
+
+    old = piece.w["l0.wo"]
+    with monkeypatch.context() as mp:
+        mp.setattr(_Plan, "__init__", refuse)
+        piece.w["l0.wo"] = old[:, :-8]
+        for _ in range(2):
+            assert not piece._chain_takes(meta, x, Handoff())
+    piece.w["l0.wo"] = old
+    assert piece._chain_takes(meta, x, Handoff())
 
 
 def test_plans_follow_shapes_and_types(monkeypatch):

@@ -57,13 +57,8 @@ def _run(piece, meta, caches, x, chain):
     cache = list(piece.k_cache.values()) + list(piece.v_cache.values())
     for c, v in zip(cache, caches):
         c.copy_(v)
-    plan = piece._chain
-    piece._chain_pays = lambda m: True                       # (the kernel is held against the others also where it is the slower one)
-    if not chain:
-        piece._chain = None
+    piece._chain_pays = lambda m: chain                      # (the kernel is held against the others also where it is the slower one)
     out = piece.forward(meta, x_in=x).clone()
-    if not chain:
-        piece._chain = plan
     del piece._chain_pays
     torch.cuda.synchronize()
     return out, [c.clone() for c in cache]

@@ -317,6 +317,10 @@ class NativePiece:
         """all that a plan takes from its weights and caches; it does not hold them"""
         return [[(x.data_ptr(), x.shape, x.stride(), x.dtype) for x in row] for row in tensors]
 
+    def gave_up(self) -> Optional[torch.Tensor]:
+        """[1] int32 on the device: launches of the persistent kernel that a wait ended early, whose results are not to be used (None: there are none)"""
+        return None if self._chain is None else self._chain.control[2:3]
+
     def span_keys(self, tokens: int) -> int:
         """spans of so many new tokens run in the persistent kernel while none of them sees more keys than this (0: spans never do)"""
         if self._chain is None or not self._chain_ln or tokens > self._chain.step_tokens:

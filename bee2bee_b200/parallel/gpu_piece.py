@@ -71,6 +71,7 @@ class GpuPieceHost:
         self.max_sessions = max_sessions
         self.x_in = torch.zeros((max_tokens, cfg.hidden_size), device=self.device, dtype=torch.bfloat16)
         self.stream = torch.cuda.Stream(device=self.device)
+        self._gave_up = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.launches = 0
 
     # ------------------------------------------------------------------ sessions (KV residency)
@@ -138,19 +139,33 @@ class GpuPieceHost:
                              n_tokens=T, n_seqs=1, max_q=T, last_idx=torch.tensor([T - 1], device=dev, dtype=torch.int64),
                              max_keys=pos0 + T)
             out = self.piece.forward(meta, x_in=hidden)
-            s["len"] = pos0 + T
             self.launches += 5 * len(self.layers) + 2
             if self.last:
                 logits = out[:1, :c.vocab_size].float()
-                self.stream.synchronize()
+                self._finish(s, pos0 + T)
                 return {"logits": logits}
             if keep_on_device:
                 ptr = self.C.peer_alloc(T * c.hidden_size * 2)
                 self.C.memcpy_peer(ptr, dev.index, out.data_ptr(), dev.index, T * c.hidden_size * 2)
-                self.stream.synchronize()
+                try:
+                    self._finish(s, pos0 + T)
+                except RuntimeError:
+                    self.C.peer_free(ptr)
+                    raise
                 ent = register_buffer(ptr, dev.index, [T, c.hidden_size])
                 return {"hidden_ref": {"ref": ent["ref"], "device": dev.index, "shape": [T, c.hidden_size],
                                        "ipc": bytes(self.C.ipc_export(ptr)).hex()}}
             res = out[:T].clone()
-        self.stream.synchronize()
+            self._finish(s, pos0 + T)
         return {"hidden": res}
+
+    def _finish(self, session: dict, length: int) -> None:
+        """waits for the hop; one that a kernel's wait ended early is an error, and the session stays as it was"""
+        gave_up = self.piece.gave_up()
+        if gave_up is not None:
+            self._gave_up.copy_(gave_up, non_blocking=True)
+        self.stream.synchronize()
+        if gave_up is not None and int(self._gave_up):
+            gave_up.zero_()
+            raise RuntimeError("the decode kernel gave up waiting for its own results; the hop was discarded")
+        session["len"] = length

@@ -501,3 +501,26 @@ def test_routes():
     old = _compare(piece, meta, caches, x)
     piece.w["l1.w_down"] = piece.w["l1.w_down"] * 2
     assert _rel(_compare(piece, meta, caches, x), old) > 0.1
+
+
+def _host(seed=0):
+    from bee2bee_b200.parallel.gpu_piece import GpuPieceHost
+
+    return GpuPieceHost("tiny-llama", 0, 99, device="cuda:0", max_tokens=64, max_sessions=2, max_seq_len=256, seed=seed)
+
+
+@gpu
+def test_piece_host_reports_a_launch_that_gave_up():
+    """a hop whose kernel gave up is an error and leaves its session as it was"""
+    host, ref = _host(), _host()
+    for h in (host, ref):
+        h.forward("a", ids=list(range(3, 40)))
+    want = [ref.forward("a", ids=[t])["logits"].clone() for t in (7, 9)]
+    assert torch.equal(host.forward("a", ids=[7])["logits"], want[0])
+    host.piece._chain.polls = 1
+    for _ in range(2):
+        with pytest.raises(RuntimeError, match="gave up"):
+            host.forward("a", ids=[9])
+    host.piece._chain.polls = 0
+    assert host.sessions["a"]["len"] == ref.sessions["a"]["len"] - 1
+    assert torch.equal(host.forward("a", ids=[9])["logits"], want[1])

@@ -163,6 +163,7 @@ class GpuRunner:
         self._pf: Dict[tuple, dict] = {}           # prefill state (staging + graph) per bucket
         self.stream = torch.cuda.Stream(device=dev)
         self.kernel_launches = 0
+        self._decode_launches = 0
         self.h2d_bytes = 0
         self.d2h_bytes = 0
         self.decode_splits = 1
@@ -198,9 +199,10 @@ class GpuRunner:
         return t[g * self.gb:(g + 1) * self.gb]
 
     def launches_per_decode_step(self) -> int:
-        """Native kernel launches one rank issues per group decode step: counted while the decode graph was recorded
-        (``ops.LAUNCHES``); before the first capture, an estimate from the layer structure."""
-        if getattr(self, "_decode_launches", 0):
+        """Native kernel launches one rank issues per group decode step: counted while the step was warmed up or its graph recorded
+        (``ops.LAUNCHES``); before that (pieces of a pipeline, whose layers are kernels one by one), an estimate from the layer
+        structure."""
+        if self._decode_launches:
             return self._decode_launches
         c, n = self.cfg, len(self.layers)
         if c.norm == "ln":
@@ -430,12 +432,13 @@ class GpuRunner:
         ev = torch.cuda.Event()
         ev.record(self.stream)
         st["events"][turn] = ev
+        n0 = ops.LAUNCHES[0]
         if st["graph"] is not None:
             st["graph"].replay()
         else:
             st["body"]()
         self.pf_chunks += 1
-        self.kernel_launches += st.get("launches") or (self.launches_per_decode_step() + 1)
+        self.kernel_launches += st.get("launches") or (ops.LAUNCHES[0] - n0)
 
     # ------------------------------------------------------------------ scoring (given tokens, no sampling)
     def score_step(self, spans: Sequence[Tuple[SeqInit, int]], want: Sequence[Sequence[int]]) -> torch.Tensor:
@@ -555,9 +558,11 @@ class GpuRunner:
         saved = self.q_len.clone()
         self.q_len.zero_()
         pos, kvl = self.positions.clone(), self.kv_len.clone()
+        n0 = ops.LAUNCHES[0]
         with torch.cuda.stream(self.stream):
             for g in range(self.groups):
                 self._decode_group(g)
+        self._decode_launches = (ops.LAUNCHES[0] - n0) // self.groups
         self.stream.synchronize()
         self.q_len.copy_(saved)
         self.positions.copy_(pos)

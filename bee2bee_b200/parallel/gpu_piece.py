@@ -138,8 +138,9 @@ class GpuPieceHost:
                              kv_len=torch.tensor([pos0 + T], device=dev, dtype=i32), block_table=pages[None, :].contiguous(),
                              n_tokens=T, n_seqs=1, max_q=T, last_idx=torch.tensor([T - 1], device=dev, dtype=torch.int64),
                              max_keys=pos0 + T)
+            before = ops.LAUNCHES[0]
             out = self.piece.forward(meta, x_in=hidden)
-            self.launches += 5 * len(self.layers) + 2
+            self.launches += ops.LAUNCHES[0] - before
             if self.last:
                 logits = out[:1, :c.vocab_size].float()
                 self._finish(s, pos0 + T)

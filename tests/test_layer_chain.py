@@ -524,3 +524,19 @@ def test_piece_host_reports_a_launch_that_gave_up():
     host.piece._chain.polls = 0
     assert host.sessions["a"]["len"] == ref.sessions["a"]["len"] - 1
     assert torch.equal(host.forward("a", ids=[9])["logits"], want[1])
+
+
+@gpu
+def test_launch_counts():
+    """what is reported is what was launched: a decode step of whole layers is the persistent kernel, embedding and head"""
+    from bee2bee_b200.engine.runner import GpuRunner
+
+    host = _host()
+    host.forward("a", ids=list(range(3, 40)))
+    n0 = host.launches
+    host.forward("a", ids=[7])
+    assert host.launches - n0 == 3
+    for graphs in (False, True):
+        r = GpuRunner(resolve_config("tiny-llama"), "", 0, 1, torch.device("cuda:0"), max_batch=4, max_seq_len=256, use_graphs=graphs)
+        assert r.launches_per_decode_step() == 5             # (and the positions' advance and the sampler)
+        r.close()

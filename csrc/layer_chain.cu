@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
   uint32_t* due_s = tmem_slot + 2;                 // operations whose results are complete, as the activation warp has seen it
   __shared__ float rstd_s[CW];
   __shared__ int pos_s[CW], slot_s[CW], kvlen_s[BN], q_start_s[BN];
+  __shared__ int fresh_s[2][LN ? 1 : BN];    // per filling warp: the first key of a sequence that this step writes, -1: not looked for
   __shared__ float red_s[4][GP];             // per warp: maxima
   __shared__ float sq_s[4][CW > GP ? CW : GP];     // per warp: sums of squares, or of a row's weights
   __shared__ float ml_s[2 * GP];             // this CTA's maxima and sums, read by the cluster
@@ -456,6 +457,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
     }
   } else if (warp > 2) {
     for (int i = threadIdx.x - 96; i < p.seqs; i += LC_THREADS - 96) {
+      fresh_s[0][i] = fresh_s[1][i] = -1;
       kvlen_s[i] = p.q_len[i] > 0 ? max(p.kv_len[i], 0) : 0;
       q_start_s[i] = p.q_start[i];
     }
@@ -564,10 +566,28 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                 const bool values = i == 2 * it.nt - 1 || (i > 0 && (i & 1) == 0);
                 const int n = i == 0 ? 0 : (values ? (i - 1) >> 1 : (i + 1) >> 1);
                 const int2 where = values || i == 0 ? pg : pg1;
-                if ((2 * (it.t0 + n) + 2) * LC_PAGE >= it.kvlen && !appended) {                  // the tile with the new token's row
-                  if (!(ok = lc_wait_due(due_s, at - 1, abort))) break;
-                  fence_proxy_async_all();
-                  appended = true;
+                // tiles with rows of this step: the new token's, and, where tokens of one text come as sequences that share its pages, of the ones in front of
+                // it (looked for once; taking the last T keys of every sequence for written delayed pages by 0.6 us per layer at 32 sequences)
+                const int end = (2 * (it.t0 + n) + 2) * LC_PAGE;
+                if (end > it.kvlen - p.T && !appended) {
+                  int first = it.kvlen - 1;
+                  if (end <= first && (first = fresh_s[half][it.seq]) < 0) {
+                    first = it.kvlen - 1;
+                    const int* bt = p.block_table + static_cast<size_t>(it.seq) * p.max_pages + first / LC_PAGE;
+                    const int page0 = first / LC_PAGE * LC_PAGE, page = bt[0], before = bt[-1];            // (a tile lies in front of this one)
+#pragma unroll 8
+                    for (int t = 0; t < p.T; ++t) {
+                      const int slot = p.slots[t];
+                      if (slot >= 0 && slot / LC_PAGE == page) first = min(first, page0 + slot % LC_PAGE);
+                      if (slot >= 0 && slot / LC_PAGE == before) first = min(first, page0 - LC_PAGE + slot % LC_PAGE);
+                    }
+                    fresh_s[half][it.seq] = first;
+                  }
+                  if (end > first) {
+                    if (!(ok = lc_wait_due(due_s, at - 1, abort))) break;
+                    fence_proxy_async_all();
+                    appended = true;
+                  }
                 }
 #pragma unroll 1
                 for (int h = 0; h < MB; ++h) {       // 128 channels per slot

@@ -370,6 +370,20 @@ def test_sequences_that_take_no_part():
 
 
 @gpu
+@pytest.mark.parametrize("first", [120, 126, 127, 250])
+@pytest.mark.parametrize("rows", [2, 5, 20])
+def test_tokens_of_one_text_as_sequences(first, rows):
+    """consecutive tokens of a text as sequences that share its pages: each sees the keys and values that the ones in front of it leave in the same step"""
+    piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, list(range(first, first + rows)))
+    table = meta.block_table[-1].tolist()
+    meta.block_table[:] = meta.block_table[-1]
+    meta.slots.copy_(torch.tensor([table[p // 64] * 64 + p % 64 for p in range(first, first + rows)], dtype=torch.int32))
+    for c in caches:                                         # what lies there before the step would be seen
+        c.view(-1, c.shape[2] * c.shape[3])[meta.slots.long()] = 50.0
+    _compare(piece, meta, caches, x)
+
+
+@gpu
 def test_graph_replay_sees_new_inputs_and_lengths():
     piece, meta, caches, x = _setup(resolve_config("tiny-llama"), 2, [60, 61, 62])
     _run(piece, meta, caches, x, True)

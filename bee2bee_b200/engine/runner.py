@@ -393,7 +393,7 @@ class GpuRunner:
         parity = (self.pf_chunks & 1) if self.world > 1 else 0
         score = want_rows is not None
         ob = min(_pow2_at_least(max(1, len(want_rows))), self.max_logit_rows) if score else sb
-        few = 0 if self.cfg.hybrid else self.piece.span_keys(tb)
+        few = 0 if self.cfg.hybrid or self.world > 1 else self.piece.span_keys(tb)
         st = self._pf_state((tb, sb, mq, parity, ob, True) if score else (tb, sb, mq, parity), few if max(c1 for _, _, c1 in chunk) <= few else 0)
         turn = st["turn"]
         st["turn"] = (turn + 1) % len(st["hosts"])

@@ -2,7 +2,8 @@
 hand-written sm_100a kernels in ``csrc/``.
 
 A decode step (one new token per sequence, up to 64; GPT-2: prompts of up to 64 tokens too) of whole bf16 layers is one persistent
-kernel (``csrc/layer_chain.cu``); in block-scaled fp8 steps of up to 32 tokens are, behind the quantiser of the piece's input.
+kernel (``csrc/layer_chain.cu``); in block-scaled fp8 steps of up to 32 tokens are, behind the quantiser of the piece's input.  All where
+the keys are not so many that attention is slower there (``NativePiece._chain_pays``).
 Prompts, larger steps, weights with per-row scales and pieces of a pipeline: per decoder layer (Llama / Mistral) exactly five launches, all on one stream:
 
     QKV GEMM  [fused: RMSNorm(x) via folded gamma + in-kernel 1/rms, RoPE, paged-KV append]
@@ -87,8 +88,8 @@ class BatchMeta:
     splits: int = 1
     seq_slot: Optional[torch.Tensor] = None   # [S] int32 batch slot of each sequence (per-sequence recurrent state)
     n_out: int = 0                            # rows of logits wanted (0 = one per sequence)
-    max_keys: int = 0                         # no token sees more keys than this (0 = as many as the block table holds)
     bucket: bool = False                      # the sizes are a bucket's: fewer sequences and tokens may be live (q_len says which)
+    max_keys: int = 0                         # no token sees more keys than this (0 = as many as the block table holds)
 
 
 # What the persistent decode kernel and the kernels one by one take for attention, us per 128 keys of a 128-wide key/value head (64 KB; wider heads in

@@ -399,8 +399,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         return row_valid && kvpos <= qpos && kvpos < kvlen && (p.window <= 0 || kvpos > qpos - p.window || (Q32 && kvpos < p.keep_first));
       };
       // Q32: exponential and reciprocal of the cap and the exponential of the weight are 3 of the hardware's 16 per cycle for each score, 1.6 us per 64 keys of two
-      // CTAs; while all scores of the warp are at most half the cap it is a polynomial: 2048 tokens, 16 / 4 heads of 128, window 1024, 53 -> 43 us (37 without a
-      // cap).  (The bf16 models' hardware tanh is one instruction: 8 / 4 heads of 256 took 78 us with either.)
+      // CTAs; while all scores of the warp are at most half the cap it is a polynomial: 2048 tokens, 16 / 4 heads of 128, window 1024, 53 -> 43 us one at a time
+      // (37 without a cap), 64 -> 52 under sustained load.  (The bf16 models' hardware tanh is one instruction: 8 / 4 heads of 256 took 78 us with either.)
       bool small = false;
       if constexpr (SOFTCAP && Q32) {
         float am[4] = {0.f, 0.f, 0.f, 0.f};

@@ -2,9 +2,10 @@
 //
 // A decode step is a chain of small dependent operations per layer (QKV, attention, O, [norm], gate/up, down, [norm]), each of which streams its
 // weights or cache pages once.  As separate kernels each ends with its slowest block, starts with the latency of a launch and of its first loads, and
-// has only what fits beside the kernel before it on the way.  Here every SM runs one CTA for the whole step, and two producer warps walk the list
-// of weight tiles and cache pages of ALL operations: while an operation waits for the one before it, the next 140 to 180 KB per SM (3 to 4 us of
-// the HBM stream) land in the ring.
+// has only what fits beside the kernel before it on the way.  Here 132 SMs run one CTA each for the whole step (33 clusters of four fit the device; 16 SMs
+// have none), and two producer warps walk the list of weight tiles and cache pages of ALL operations: while an operation waits for the one before it, the
+// next 140 to 180 KB per SM (3 to 4 us of the HBM stream) land in the ring.  132 CTAs ask for 11 to 14 TB/s with two issuing warps each, so the stream
+// misses no SM; attention of few sequences, which fewer CTAs share, does (the rule in models/native.py leaves such steps to attn_decode.cu).
 //
 //   * operations are separated by a counter in global memory that every CTA adds to when its share of the results is stored; one warp per
 //     CTA polls it.  All CTAs are resident (cooperative launch).
@@ -20,10 +21,10 @@
 //   * the sums of squares for the next norm are left by the CTAs that write the rows, one number per CTA and token, added in a fixed order.
 //
 // Bound: the HBM stream and, between operations, the chain of last product, exchange, store, counter, poll and first activations (3 to 5 us, of
-// which the ring hides most).  Measured on B200, two Llama-3-8B layers, us (kernels one by one / here): one token behind 700 keys 188.5 / 171.5, 32
-// tokens behind 500 keys 217.0 / 193.7, 64 tokens behind 300 (Mistral-7B shapes) 257 / 219; two Gemma-2-2B layers: one token 124 / 106, 30 tokens 128 /
-// 116; all of distilgpt2, prompts of 19 / 60 tokens 267 / 209 and 333 / 254, gpt2, 64 tokens 649 / 507 (42 and 84 operations of 3 to 5 us); block-scaled
-// fp8, two Llama-3-8B layers: one token 142 / 127, 8 tokens 143 / 129, 32 tokens 166 / 162 (a conversion behind each of three products).
+// which the ring hides most).  Measured on B200, replayed back to back, two Llama-3-8B layers behind 500 keys, us (kernels one by one / here): one token 191 /
+// 173, 32 tokens 221 / 200, 64 tokens 280 / 243; two Gemma-2-2B layers: one token 125 / 110, 32 tokens 146 / 134; the layers of distilgpt2, 19 tokens 231 /
+// 182, of gpt2, 64 tokens 617 / 472 (42 and 84 operations of 3 to 5 us); block-scaled fp8, two Llama-3-8B layers: one token 142 / 126, 8 tokens 143 / 131,
+// 32 tokens 169 / 166 (a conversion behind each of three products).
 // Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
 // All waits are bounded: one that runs out raises the abort word, every other wait then ends too, and the CTAs leave.
 #include "kernels.h"

@@ -1551,7 +1551,7 @@ int launch_softmax_attention(const float* q, const void* k_cache, const void* v_
   const bool wide_v = V > 32 * SMX_VR;      // values of 257 .. 512 channels: 16 channels per lane
   if (ldv <= 0) ldv = Gv * V;               // values in a cache of their own; otherwise a view into wider rows
   // longer spans of plain 64- and 128-wide heads: the tcgen05 kernel of the dense models (one span of
-  // 2048 tokens, 16 / 4 heads of 128, window 1024, capped: 43 us against 167 on mma.sync below; 40 tokens: 9 against 10)
+  // 2048 tokens, 16 / 4 heads of 128, window 1024, capped: 52 us under sustained load against 167 on mma.sync below; 40 tokens: 9 against 10)
   if (!f32 && plain && D == V && ldv == G * V && max_q >= SMX_TC_MIN_Q && n_pages > 0 && attention_tc_hybrid_supported(q, k_cache, v_cache, out, ld_out, H, G, D))
     return launch_attention_tc_hybrid(q, k_cache, v_cache, out, ld_out, block_table, max_pages, n_pages, q_start, q_len, kv_len, n_seqs, max_q,
                                       H, G, D, window, scale, softcap, keep_first, sink, s);

@@ -281,21 +281,26 @@ class NativePiece:
                     self._plan_chain()
 
     # ------------------------------------------------------------------ helpers
-    def _chain_tensors(self):
+    def _chain_slots(self):
+        """where the plan's tensors are, per layer: (dict, key)"""
         names = ("wqkv", "wo", "w_up" if self._chain_ln else "wgu", "w_down")
         post = ("post_attn_w", "post_ffn_w") if self.cfg.post_norms else ()
         if self._chain_ln:
             post = ("bqkv", "bo", "b_up", "b_down", "ln2_w", "ln2_b")
-        rows = [[self.w[f"l{l}.{n}"] for n in names] + [self.k_cache[l], self.v_cache[l]] + [self.w[f"l{l}.{n}"] for n in post]
-                + ([self.wscale[f"l{l}.{n}"] for n in names] if self.mx_fuse else []) for l in self.layers]
+        rows = [[(self.w, f"l{l}.{n}") for n in names] + [(self.k_cache, l), (self.v_cache, l)] + [(self.w, f"l{l}.{n}") for n in post]
+                + ([(self.wscale, f"l{l}.{n}") for n in names] if self.mx_fuse else []) for l in self.layers]
         if self._chain_ln:                     # the norm in front of the next layer
             for row, l in zip(rows, self.layers[1:]):
-                row += [self.w[f"l{l}.ln1_w"], self.w[f"l{l}.ln1_b"]]
+                row += [(self.w, f"l{l}.ln1_w"), (self.w, f"l{l}.ln1_b")]
         return rows
+
+    def _chain_tensors(self):
+        return [[d[k] for d, k in row] for row in self._chain_at]
 
     def _plan_chain(self) -> None:
         """lays the layers out for the decode kernel (csrc/layer_chain.cu)"""
         c = self.cfg
+        self._chain_at = self._chain_slots()
         t = self._chain_tensors()
         if self._chain_recorded:               # graphs go on reading its table and counters
             self._chain_kept.append(self._chain)
@@ -304,7 +309,7 @@ class NativePiece:
         if self.mx_fuse:
             H, Q = c.hidden_size, c.q_dim
             fp8 = [self._qbuf[H], self._qsf[H], self._fq_x, self._fq_sf_x, self._qbuf[Q], self._qsf[Q], self._fq_h, self._fq_sf_h]
-        self._chain_of = self._chain_key(t)
+        self._chain_of = ops.native().tensor_stamp(t)          # all that a plan takes from its weights and caches; it does not hold them
         try:
             self._chain = ops.native().LayerChain(t, [c.layer_window(l) for l in self.layers], self.xa, self.xb, self.q_buf, self.attn_buf, self.h_buf,
                                                   self.n_buf if c.post_norms or self._chain_ln else None, c.n_heads, c.n_kv_heads, c.head_dim,
@@ -312,11 +317,6 @@ class NativePiece:
                                                   self._chain_ln, fp8)
         except RuntimeError:                   # weights or caches that only the kernels one by one take, or refuse themselves
             self._chain = None
-
-    @staticmethod
-    def _chain_key(tensors):
-        """all that a plan takes from its weights and caches; it does not hold them"""
-        return [[(x.data_ptr(), x.shape, x.stride(), x.dtype) for x in row] for row in tensors]
 
     def gave_up(self) -> Optional[torch.Tensor]:
         """[1] int32 on the device: launches of the persistent kernel that a wait ended early, whose results are not to be used (None: there are none)"""
@@ -352,7 +352,7 @@ class NativePiece:
         if hand.in_flag or hand.out_x or hand.out_h or not x.is_contiguous() or x.data_ptr() % 16 or ops.get_attn_tc_min_q() <= 0:
             return False
         recording = torch.cuda.is_current_stream_capturing()
-        if self._chain_of != self._chain_key(self._chain_tensors()):       # weights or caches were replaced
+        if self._chain_of != ops.native().tensor_stamp(self._chain_tensors()):       # weights or caches were replaced
             if recording:
                 return False
             self._plan_chain()

@@ -194,7 +194,14 @@ def _cpu_piece(monkeypatch, cfg=None, layers=2):
     t.update({f"l{l}.{n}": torch.ones(H) for l in range(layers) for n in ("ln1_w", "ln2_w", "ln1_b", "ln2_b")})
     t.update({f"l{l}.{n}": torch.ones(w) for l in range(layers) for n, w in (("bq", Q), ("bk", KV), ("bv", KV), ("bo", H), ("b_up", F), ("b_down", H))})
     piece = NativePiece(cfg, range(layers), False, False, t, torch.device("cpu"), 4, 4, 8)
-    monkeypatch.setattr(ops, "native", lambda: types.SimpleNamespace(LayerChain=_Plan, get_attn_tc_min_q=lambda: 2))
+    def stamp(rows):                                         # (the native one where the extension is built)
+        return [[(x.data_ptr(), x.shape, x.stride(), x.dtype) for x in row] for row in rows]
+
+    try:
+        stamp = ops.native().tensor_stamp
+    except RuntimeError:
+        pass
+    monkeypatch.setattr(ops, "native", lambda: types.SimpleNamespace(LayerChain=_Plan, get_attn_tc_min_q=lambda: 2, tensor_stamp=stamp))
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     piece._plan_chain()
     return piece

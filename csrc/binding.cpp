@@ -153,7 +153,7 @@ void set_wait_policy(int64_t abort_word, double limit_ms) {
   check(b2b::set_wait_policy_gemm(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(gemm)");
   check(b2b::set_wait_policy_wide(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(wide)");
   check(b2b::set_wait_policy_decode(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(decode)");
-  check(b2b::set_wait_policy_chain(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(chain)");
+  check(b2b::set_wait_policy_chain(as_ptr<uint32_t>(abort_word)), "set_wait_policy(chain)");
   check(b2b::set_wait_policy_elementwise(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(elementwise)");
   check(b2b::set_wait_policy_mixed(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(mixed)");
   check(b2b::set_wait_policy_diff(as_ptr<uint32_t>(abort_word), ns), "set_wait_policy(diff)");

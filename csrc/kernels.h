@@ -79,7 +79,7 @@ size_t layer_chain_control_words(int layers);
 int layer_chain_fill(void* dst, const ChainDims& d, const ChainLayerPtrs& w);
 int layer_chain_init(const ChainDims& d);
 int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s);
-int set_wait_policy_chain(uint32_t* abort_word, unsigned long long limit_ns);
+int set_wait_policy_chain(uint32_t* abort_word);
 unsigned layer_chain_gave_up();          // launches whose bounded waits ran out so far, 0 unless there is a bug
 // spans of the hybrid graphs' softmax attention on the prefill kernel of attention_tc.cu (n_pages: pages of the cache)
 bool attention_tc_hybrid_supported(const float* q, const void* k_cache, const void* v_cache, const void* out, int ld_out, int H, int G, int D);

@@ -1648,11 +1648,8 @@ int layer_chain_init(const ChainDims& d) {
   return d.mx ? n : std::min(n, B2B_CHAIN64(chain_clusters));
 }
 
-int set_wait_policy_chain(uint32_t* abort_word, unsigned long long limit_ns) {
-  cudaError_t e = cudaMemcpyToSymbol(g_abort_word, &abort_word, sizeof(abort_word));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_wait_limit_ns, &limit_ns, sizeof(limit_ns));
-  return static_cast<int>(e);
-}
+// (its own waits are counted in polls: the process's limit in time is for flags of other GPUs)
+int set_wait_policy_chain(uint32_t* abort_word) { return static_cast<int>(cudaMemcpyToSymbol(g_abort_word, &abort_word, sizeof(abort_word))); }
 
 unsigned layer_chain_gave_up() {
   unsigned n = 0;

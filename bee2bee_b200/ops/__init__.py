@@ -135,8 +135,8 @@ PREFILL_SPLITK = os.environ.get("B2B_PREFILL_SPLITK", "1") == "1"
 
 
 def pick_prefill_tile(n_out: int, m_tok: int, k: int = 0):
-    """(token tile, ring depth, cluster split-K) of a prefill GEMM (m_tok > 64) on gemm_tc.cu -- e4m3 operands and the bf16 calls
-    that ``use_wide`` leaves --, measured on B200 on the Llama-3-8B shapes.  0 = the tile's default depth / let ``pick_splitk`` decide.
+    """(token tile, ring depth, cluster split-K) of a prefill GEMM (m_tok > 64) on gemm_tc.cu -- e4m3 operands with a scale per row and the bf16
+    calls that ``use_wide`` leaves --, measured on B200 on the Llama-3-8B shapes.  0 = the tile's default depth / let ``pick_splitk`` decide.
 
     * more tiles than SMs: TWO resident CTAs per SM with a shallow ring beat one CTA with a deep ring -- the epilogue of
       one tile (TMEM -> registers -> global) overlaps the main loop of the other (955 vs 787 TFLOP/s over the layer at
@@ -179,13 +179,15 @@ GEMM_STAGES = int(os.environ.get("B2B_GEMM_STAGES", "0"))
 #: tuning hook: {"buf": int64 cuda tensor, "off": 0, "log": []} makes every GEMM record a per-CTA timeline
 TIMELINE = None
 
-def use_wide(n_out: int, m_tok: int) -> bool:
+def use_wide(n_out: int, m_tok: int, mx: bool = False) -> bool:
     """bf16 products of many tokens run on the CTA-pair kernel (csrc/gemm_wide.cu, which picks its own tiles) where it takes the
     call.  Measured on the Llama-3-8B and Gemma-2-2B layer shapes: from 129 tokens on it is the faster one for all of them (160
     tokens: 17 against 40 us for 6144 x 4096, 55 against 84 for 28672 x 4096); at 65 .. 128 tokens, where both read the weights
     once, it is while gemm_tc.cu has no more than one tile per SM (128 tokens: 17 against 33 us for 6144 x 4096, 30 against 63 for
-    4096 x 14336, 23 against 27 for 18432 x 2304, but 54 against 51 for 28672 x 4096)."""
-    return m_tok > 128 or (m_tok > 64 and n_out <= 128 * NUM_SMS)
+    4096 x 14336, 23 against 27 for 18432 x 2304, but 54 against 51 for 28672 x 4096).  Block-scaled fp8 (``mx``): for all of them from 65
+    tokens on (gate/up 28672 x 4096, gemm_tc.cu / CTA pairs: 96 tokens 79 / 47 us, 256 170 / 48, 1000 463 / 100, 4096 1718 / 335; 4096 x 14336:
+    59 / 31, 59 / 31, 120 / 58, 414 / 178; with cold caches and the latency of a launch)."""
+    return m_tok > 128 or (m_tok > 64 and (mx or n_out <= 128 * NUM_SMS))
 
 
 #: (n_out, k) -> split-K override (tuning / sweeps)
@@ -240,7 +242,7 @@ def gemm(w: torch.Tensor, x: torch.Tensor, out: Optional[torch.Tensor] = None, *
     m_tok, k = x.shape
     n_out = w.shape[0]
     # (calls that name a tile, split or ring depth get the kernel those belong to)
-    wide = int(bn <= 0 and splitk <= 0 and stages < 0 and use_wide(n_out, m_tok)) if wide_tile <= 0 else wide_tile
+    wide = int(bn <= 0 and splitk <= 0 and stages < 0 and use_wide(n_out, m_tok, sfa is not None)) if wide_tile <= 0 else wide_tile
     if bn <= 0:
         if sfa is not None:
             bn = pick_bn_mx(m_tok)

@@ -92,6 +92,7 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
   p.q_sf = as_ptr<uint8_t>(q_sf);
   p.ld_q = static_cast<int>(ld_q);
   p.q_bn = static_cast<int16_t>(q_bn > 0 ? q_bn : 32);
+  p.sf_bn = static_cast<int16_t>(p.sfb != nullptr ? bn : 0);
   p.sumsq_out = as_ptr<float>(sumsq_out);
   p.zero_buf = as_ptr<float>(zero_buf);
   p.sumsq = as_ptr<const float>(sumsq);

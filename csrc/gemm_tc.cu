@@ -662,6 +662,27 @@ int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t co
   return make_tmap(m, ptr, rows, cols, ld, box_rows, elt_bytes);
 }
 
+// runs of 512 bytes (scale factors of 128 rows and 128 K), a run per copy, not swizzled
+int make_sf_tmap(CUtensorMap* m, const void* ptr, uint64_t chunks) {
+  using Key = std::tuple<const void*, uint64_t>;
+  static std::map<Key, CUtensorMap> cache;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> g(mu);
+  const Key key{ptr, chunks};
+  auto it = cache.find(key);
+  if (it != cache.end()) { *m = it->second; return 0; }
+  PFN_encodeTiled enc = get_encode();
+  if (!enc) return -1;
+  cuuint64_t dims[2] = {128, chunks}, strides[1] = {512};
+  cuuint32_t box[2] = {128, 1}, estr[2] = {1, 1};
+  const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return static_cast<int>(r);
+  if (cache.size() > 65536) cache.clear();
+  cache[key] = *m;
+  return 0;
+}
+
 // [rows, cols] as [blocks of 128 bytes][rows][128 bytes], box = [box_blocks][box_rows][128 bytes], 128B swizzle: several blocks of K in one copy
 int make_blocks_tmap(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks, int elt_bytes) {
   using Key = std::tuple<const void*, uint64_t, uint64_t, uint32_t, uint32_t, int>;

@@ -57,6 +57,7 @@ struct GemmParams {
   uint8_t* q_sf;                  // scale-factor chunks of the consumer GEMM's activation operand
   int ld_q;                       // row stride of q_out8 in elements (= consumer K)
   int16_t q_bn;                   // consumer token tile (chunk layout), >= 32
+  int16_t sf_bn;                  // token tile that `sfb` is laid out for
   float* sumsq_out;               // [m_tok] += sum over this CTA's features of out^2, or null
   float* zero_buf;                // [m_tok] accumulator to clear (read by an earlier GEMM, re-filled by a later one), or null
   const float* sumsq;             // consumer side: per-token sum of squares of X -> rstd = rsqrt(sumsq / k + eps)
@@ -95,7 +96,7 @@ struct GemmParams {
 // Host launcher (gemm_tc.cu). Returns cudaError_t as int.
 int gemm_tc_max_splitk(int bn, int epi, int stages);
 int launch_gemm_tc(const GemmParams& p, const void* w, const void* x, int bn, cudaStream_t stream);
-// many tokens (gemm_wide.cu): bf16 operands, 16-byte aligned rows; bn: feature tile 128 / 192 / 256, split: last round cut along K (0 / 1);
+// many tokens (gemm_wide.cu): bf16 or block-scaled fp8 operands, 16-byte aligned rows; bn: feature tile 128 / 192 / 256, split: last round cut along K (0 / 1);
 // any other value: chosen by size.  -4: no such tile for this call
 bool gemm_wide_supported(const GemmParams& p);
 int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, int split, cudaStream_t stream);

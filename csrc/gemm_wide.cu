@@ -1,6 +1,6 @@
 // Prefill GEMM: many tokens, pairs of CTAs, persistent tiles.
 //
-//   out[t, n] = epilogue( sum_k X[t, k] * W[n, k] )        (the epilogues of gemm_tc.cu, bf16 operands, fp32 accumulators)
+//   out[t, n] = epilogue( sum_k X[t, k] * W[n, k] )        (the epilogues of gemm_tc.cu, bf16 or block-scaled fp8 operands, fp32 accumulators)
 //
 // gemm_tc.cu makes the weights the 128 MMA rows and the tokens the columns, which is what few tokens want.  With hundreds of tokens
 // it is bound by shared memory (a CTA reads 128 + 256 operand rows per 128 x 256 tile) and by its epilogue (a lane owns one feature,
@@ -26,8 +26,22 @@
 //   4096 tokens: QKV 218 (945) -> 131 (1573), O 157 (875) -> 96 (1436), gate/up 1041 (924) -> 595 (1616), down 404 (1191) -> 342 (1405)
 //    512 tokens: QKV 39 (656) -> 22 (1193),   O 27 (633) -> 18 (978),   gate/up 139 (866) -> 91 (1326),   down 59 (1019) -> 50 (1198)
 //    160 tokens: QKV 40 -> 17, O 33 -> 14, gate/up 84 -> 55, down 60 -> 30 (the weights alone: 8, 5, 36, 18)
+//
+// Block-scaled fp8 (MX): the same tiles with 128 K per stage; the scale factors come through the ring in runs of 512 bytes and are copied to tensor
+// memory in front of their products.  The epilogue's lane has whole blocks of 32 features of its token, so the e4m3 copy that the next product reads
+// needs no exchange between lanes.  256-wide tiles leave no columns for scale factors beside two accumulators, so these overlap by 32 columns, which
+// the epilogue takes first (128-wide tiles have none of that, but twice the rounds: gate/up of 4096 tokens 384 us against 335).  gemm_tc.cu reads
+// 128 + 256 operand rows per 128 x 256 tile and has no second accumulator.  Llama-3-8B layer shapes, us, with cold caches and the latency of a launch,
+// gemm_tc.cu -> here:
+//   4096 tokens: QKV 349 -> 91, O 282 -> 74, gate/up 1718 -> 335 (2.9 PFLOP/s), down 414 -> 178
+//    512 tokens: QKV  78 -> 27, O  53 -> 23, gate/up  290 -> 66, down 88 -> 41
+//    128 tokens: QKV  41 -> 21, O  25 -> 21, gate/up   90 -> 48, down 62 -> 31
 // Roles (192 threads): warp 0 = TMA producer (both CTAs), warp 1 = TMEM owner, MMA issuer in the pair's even CTA, warps 2..5 = epilogue.
 #include "gemm_tc.cuh"
+
+#include <cuda_fp8.h>
+
+#include <type_traits>
 
 #include "activations.cuh"
 #include "common.cuh"
@@ -38,11 +52,12 @@
 namespace b2b {
 
 int make_tmap_shared(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, int elt_bytes);
+int make_sf_tmap(CUtensorMap* m, const void* ptr, uint64_t chunks);
 
 namespace {
 
 constexpr int WM = 128;                    // token rows per CTA (256 per pair)
-constexpr int WK = 64;                     // K elements per stage (one 128-byte swizzled row)
+constexpr int WK = 64;                     // K elements per stage (one 128-byte swizzled row; block-scaled fp8: 128)
 constexpr int WA_BYTES = WM * 128;
 constexpr int WIDE_THREADS = 192;
 constexpr int WIDE_PAIRS = 74;             // of the 148 SMs
@@ -51,15 +66,23 @@ constexpr int EPI_BYTES = 4 * 32 * EPI_PITCH;
 
 __device__ unsigned int g_wide_gave_up = 0;        // CTAs whose waits ran out since the module was loaded
 
-template <int BN>
+template <int BN, bool MX>
 struct WideCfg {
   static constexpr int kBBytes = BN / 2 * 128;                           // this CTA's half of the weight rows
   static constexpr int kStageBytes = WA_BYTES + kBBytes;
+  static constexpr int kSfBytes = MX ? 512 + BN / 128 * 512 : 0;         // scale factors: this CTA's token rows, all weight rows of the pair
   static constexpr int kStages = BN == 256 ? 6 : (BN == 192 ? 7 : 8);
   static constexpr int kLandPitch = BN / 2 + 4;                          // floats per row of the split-K landing zone
-  static constexpr int kSmem = 1024 + kStages * kStageBytes + EPI_BYTES + 512;
-  static constexpr uint32_t kTmemCols = BN == 128 ? 256 : 512;
+  static constexpr int kSmem = 1024 + kStages * (kStageBytes + kSfBytes) + EPI_BYTES + 512;
+  static constexpr uint32_t kTmemCols = (MX || BN != 128) ? 512 : 256;
+  // Accumulators: two of BN columns.  Behind two of 256 no columns are left for scale factors, so those of block-scaled tiles share 32: the
+  // epilogue takes the shared columns into registers before anything else, and only then may the next tile begin.
+  static constexpr bool kShared = MX && BN == 256;
+  static constexpr uint32_t kAccStride = kShared ? 224 : BN;
+  static constexpr uint32_t kSfCol = kAccStride + BN;                    // two sets of 16 columns
+  static_assert(!MX || kSfCol + 32 <= kTmemCols, "scale factors lie behind the accumulators");
   static_assert(WM * kLandPitch * 4 <= kStages * kStageBytes, "the landing zone reuses the ring");
+  static_assert(kSmem <= 232448, "shared memory of an SM");
 };
 
 template <uint32_t kCols>
@@ -78,6 +101,19 @@ __device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t adesc, uint
       "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// block-scaled e4m3: scale factors of both operands in tensor memory, each CTA's own token rows and all weight rows of the pair
+__device__ __forceinline__ void umma2_mxf8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
+      : "memory");
+}
+// scale factors of 128 rows, shared memory -> tensor memory, in both CTAs of the pair
+__device__ __forceinline__ void tmem_cp2_32x128b_warpx4(uint32_t taddr, uint64_t sdesc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
 // arrives on the barrier at this offset in the CTAs of `mask` once the MMAs issued so far have retired
 __device__ __forceinline__ void umma2_commit(uint64_t* bar, uint16_t mask) {
@@ -154,16 +190,23 @@ struct Plan {
   }
 };
 
-template <int BN, int EPI>
+struct NoMaps {};
+struct SfMaps {                            // scale factors as rows of 512 bytes
+  CUtensorMap w, x;
+};
+
+template <int BN, int EPI, bool MX>
 __global__ void __launch_bounds__(WIDE_THREADS, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const GemmParams p,
-                 const int allow_split) {
-  using Cfg = WideCfg<BN>;
+                 const int allow_split, const __grid_constant__ std::conditional_t<MX, SfMaps, NoMaps> sf_maps) {
+  using Cfg = WideCfg<BN, MX>;
   constexpr int STAGES = Cfg::kStages;
+  constexpr int KE = MX ? 128 : WK;                // K elements per stage
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stage_out = smem + STAGES * Cfg::kStageBytes;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(stage_out + EPI_BYTES);
+  uint8_t* sf_s = stage_out + EPI_BYTES;           // [STAGES][kSfBytes]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sf_s + STAGES * Cfg::kSfBytes);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* acc_full = empty_bar + STAGES;         // [2]
   uint64_t* acc_empty = acc_full + 2;              // [2], of the pair's even CTA
@@ -180,7 +223,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   Plan plan;
   plan.tok_tiles = (p.m_tok + 2 * WM - 1) / (2 * WM);
   plan.tiles = plan.tok_tiles * ((p.n_out + BN - 1) / BN);
-  plan.nkb = p.k / WK;
+  plan.nkb = p.k / KE;
   plan.pairs = static_cast<int>(gridDim.x >> 1);
   plan.full = plan.tiles / plan.pairs * plan.pairs;
   plan.rest = plan.tiles - plan.full;
@@ -189,6 +232,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
+    if constexpr (MX) {
+      tma_prefetch_desc(&sf_maps.w);
+      tma_prefetch_desc(&sf_maps.x);
+    }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
@@ -225,10 +272,21 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         uint8_t* st = smem + s * Cfg::kStageBytes;
         const uint32_t bar = mapa_smem(smem_u32(&full_bar[s]), lead);
         if (w) {
-          if (!odd) mbar_arrive_expect_tx(&full_bar[s], 2 * Cfg::kStageBytes);
-          tma_load2(st + WA_BYTES, &tmap_w, bar, kb * WK, n0 + (odd ? BN / 2 : 0));
+          if (!odd) mbar_arrive_expect_tx(&full_bar[s], 2 * (Cfg::kStageBytes + Cfg::kSfBytes));
+          tma_load2(st + WA_BYTES, &tmap_w, bar, kb * KE, n0 + (odd ? BN / 2 : 0));
+          if constexpr (MX) {
+#pragma unroll
+            for (int j = 0; j < BN / 128; ++j)     // (rows behind the last are not there: zeros, for features that are not stored)
+              tma_load2(sf_s + s * Cfg::kSfBytes + 512 + j * 512, &sf_maps.w, bar, 0, (n0 / 128 + j) * plan.nkb + kb);
+          }
         }
-        if (x) tma_load2(st, &tmap_x, bar, kb * WK, m0 + (odd ? WM : 0));
+        if (x) {
+          tma_load2(st, &tmap_x, bar, kb * KE, m0 + (odd ? WM : 0));
+          if constexpr (MX) {                      // runs of 128 tokens, or (sf_bn 256) of 256 whose halves lie side by side
+            const int half = odd ? 1 : 0, run = p.sf_bn > 128 ? (m0 / 256 * plan.nkb + kb) * 2 + half : (m0 / 128 + half) * plan.nkb + kb;
+            tma_load2(sf_s + s * Cfg::kSfBytes, &sf_maps.x, bar, 0, run);
+          }
+        }
       };
       for (int i = 0; ok && plan.get(i, pair, it); ++i) {
         const int m0 = it.t % plan.tok_tiles * (2 * WM), n0 = it.t / plan.tok_tiles * BN;
@@ -243,7 +301,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           for (int j = 0; j < pre; ++j, ++n) fill(kb + j, n0, m0, false, true);
           kb += pre;
         }
-        if (i == 2) wait_downstream(p);            // (two accumulators: from here on the ring waits for the epilogue, too)
+        if (i == (Cfg::kShared ? 1 : 2)) wait_downstream(p);      // (two accumulators: from here on the ring waits for the epilogue, too)
         for (; kb < it.kb1; ++kb, ++n) {
           if (!(ok = ma_wait(&empty_bar[n % STAGES], (n / STAGES & 1u) ^ 1u, abort))) break;
           fill(kb, n0, m0, true, true);
@@ -253,7 +311,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   } else if (warp == 1) {
     // -------------------------------------------------------------------------------------------------- MMA issuer
     if (!odd && elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(2 * WM, BN);
+      constexpr uint32_t idesc = MX ? make_idesc_mxf8(2 * WM, BN) : make_idesc_bf16(2 * WM, BN);
       const uint16_t both = static_cast<uint16_t>(3u << lead);
       uint32_t n = 0;
       for (int i = 0; ok && plan.get(i, pair, it); ++i) {
@@ -262,8 +320,12 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           pdl_wait();                              // (no result is needed; the waits below may count once the producer's input is there)
           wait_upstream(p);
         }
-        if (i == 2) wait_downstream(p);
-        if (!(ok = ma_wait(&acc_empty[b], (i >> 1 & 1) ^ 1u, abort))) break;
+        if (i == (Cfg::kShared ? 1 : 2)) wait_downstream(p);
+        if constexpr (Cfg::kShared) {              // the tile before has left the shared columns, the one before that all of them
+          if (i > 0 && !(ok = ma_wait(&acc_empty[b ^ 1u], (i - 1) >> 1 & 1, abort))) break;
+        } else {
+          if (!(ok = ma_wait(&acc_empty[b], (i >> 1 & 1) ^ 1u, abort))) break;
+        }
         tc_fence_after();
         for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
           const uint32_t s = n % STAGES;
@@ -271,8 +333,20 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           tc_fence_after();
           const uint64_t a = make_sw128_kmajor_desc(smem_u32(smem + s * Cfg::kStageBytes));
           const uint64_t w = make_sw128_kmajor_desc(smem_u32(smem + s * Cfg::kStageBytes + WA_BYTES));
+          if constexpr (MX) {
+            // two sets of columns alternate: copies and products run in the order of their issue
+            const uint32_t ta = tmem + Cfg::kSfCol + (n & 1u) * 16, sf = smem_u32(sf_s + s * Cfg::kSfBytes);
+            tmem_cp2_32x128b_warpx4(ta, make_sf_desc(sf));
 #pragma unroll
-          for (int k = 0; k < WK / 16; ++k) umma2_bf16(tmem + b * BN, a + 2 * k, w + 2 * k, idesc, (kb > it.kb0 || k > 0) ? 1u : 0u);
+            for (int j = 0; j < BN / 128; ++j) tmem_cp2_32x128b_warpx4(ta + 4 + 4 * j, make_sf_desc(sf + 512 + 512 * j));
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              umma2_mxf8(tmem + b * Cfg::kAccStride, a + 2 * k, w + 2 * k, idesc | (static_cast<uint32_t>(k) << 4) | (static_cast<uint32_t>(k) << 29),
+                         (kb > it.kb0 || k > 0) ? 1u : 0u, ta, ta + 4);
+          } else {
+#pragma unroll
+            for (int k = 0; k < WK / 16; ++k) umma2_bf16(tmem + b * BN, a + 2 * k, w + 2 * k, idesc, (kb > it.kb0 || k > 0) ? 1u : 0u);
+          }
           umma2_commit(&empty_bar[s], both);
         }
         if (ok) umma2_commit(&acc_full[b], both);
@@ -290,6 +364,12 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     pdl_wait();
     wait_upstream(p);
     wait_downstream(p);
+    if constexpr (MX) {                            // sums of squares that an earlier product has read and a later one adds to
+      if (p.zero_buf != nullptr && blockIdx.x == 0)
+        for (int t = threadIdx.x - 64; t < p.m_tok; t += 128) p.zero_buf[t] = 0.f;
+    }
+    uint32_t hold[Cfg::kShared ? 32 : 1];          // the accumulator columns that two tiles share
+    int hold_c = -1;                               // the first of them in the tile that is worked on
 
     // the residual values of a 64-column block in the coalesced view, in flight while the accumulators are awaited or worked on
     uint4 res[EPI == EPI_RESIDUAL ? 8 : 1];
@@ -309,7 +389,9 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const int tok = m0 + row;
       const bool live = tok < p.m_tok;
       if (m0 + q * 32 >= p.m_tok) return;          // no token of this warp (warp-uniform)
-      const float rs = (p.rstd != nullptr && live) ? p.rstd[tok] : 1.f;
+      float rs = (p.rstd != nullptr && live) ? p.rstd[tok] : 1.f, ssq = 0.f;
+      if constexpr (MX)
+        if (p.sumsq != nullptr && live) rs *= rsqrtf(p.sumsq[tok] / static_cast<float>(p.k) + p.eps);
       int slot = -1;
       float pos = 0.f;
       if constexpr (EPI == EPI_QKV_ROPE) {
@@ -320,6 +402,11 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         uint32_t r[32];
         ma_ld32(acc + c, r);
         ma_ld_fence(r);
+        if constexpr (Cfg::kShared) {              // (the next tile may be writing there)
+          if (c == hold_c)
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = hold[j];
+        }
         if (land != nullptr) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
@@ -361,6 +448,58 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         __syncwarp();
       };
+      // Block-scaled copy of 64 finished features (this lane's staged bf16 row) for the product that reads them: e4m3, a power of two per 32 of them in
+      // the layout of that product's operand, and the row's sum of squares.  A lane has whole blocks of its token: no exchange.
+      auto emit_q = [&](int feat) {
+        uint32_t e8[16];
+        uint32_t exps = 0u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float r[32], most = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint4 w = *reinterpret_cast<const uint4*>(srow + h * 64 + j * 16);
+            const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&w);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 f = __bfloat1622float2(x[e]);
+              r[8 * j + 2 * e] = f.x;
+              r[8 * j + 2 * e + 1] = f.y;
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            most = fmaxf(most, fabsf(r[j]));
+            ssq += r[j] * r[j];
+          }
+          const uint32_t b = __float_as_uint(most * (1.f / 448.f));
+          const int ex = max(-126, min(127, static_cast<int>(b >> 23) - 127 + ((b & 0x7FFFFFu) ? 1 : 0)));
+          const float inv = __uint_as_float(static_cast<uint32_t>(127 - ex) << 23);
+          exps |= static_cast<uint32_t>(ex + 127) << (8 * h);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j] * inv, r[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j + 2] * inv, r[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+            e8[8 * h + j] = lo | (hi << 16);
+          }
+        }
+        if (live) {
+          const int n = tok % p.q_bn, rr = n & 127, run = p.q_bn > 128 ? 1024 : 512;
+          *reinterpret_cast<uint16_t*>(p.q_sf + (static_cast<size_t>(tok / p.q_bn) * (p.ld_q >> 7) + (feat >> 7)) * run + (n >> 7) * 512 + (rr & 31) * 16 +
+                                       (rr >> 5) * 4 + ((feat >> 5) & 3)) = static_cast<uint16_t>(exps);
+        }
+        __syncwarp();                              // the bf16 rows have been stored
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(srow + j * 16) = make_uint4(e8[4 * j], e8[4 * j + 1], e8[4 * j + 2], e8[4 * j + 3]);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {              // 64 bytes of a row, 8 rows at a time
+          const int r = (lane >> 2) + 8 * i, t = m0 + q * 32 + r;
+          const uint4 w = *reinterpret_cast<const uint4*>(sbuf + r * EPI_PITCH + (lane & 3) * 16);
+          if (t < p.m_tok) *reinterpret_cast<uint4*>(p.q_out8 + static_cast<size_t>(t) * p.ld_q + feat + (lane & 3) * 16) = w;
+        }
+        __syncwarp();
+      };
 
       if constexpr (EPI == EPI_GLU) {              // 64 gate columns, then 64 up columns -> 64 outputs
         for (int c = c0; c < c1 && n0 + c < p.n_out; c += 128) {
@@ -373,7 +512,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             for (int j = 0; j < 32; ++j) g[j] = (p.act_gelu ? gelu_tanh(g[j]) : silu(g[j])) * u[j];
             put(half, g);
           }
-          flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>((n0 + c) / 2) * 2, static_cast<size_t>(p.ld_out) * 2);
+          if (!MX || p.out != nullptr)
+            flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>((n0 + c) / 2) * 2, static_cast<size_t>(p.ld_out) * 2);
+          if constexpr (MX)
+            if (p.q_out8 != nullptr) emit_q((n0 + c) / 2);
         }
       } else if (EPI == EPI_PLAIN && p.out_fp32) {
         for (int c = c0; c < c1 && n0 + c < p.n_out; c += 32) {
@@ -459,7 +601,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(n) * 2, static_cast<size_t>(p.ld_out) * 2);
             if (EPI == EPI_RESIDUAL && p.out2 != nullptr)
               flush(reinterpret_cast<uint8_t*>(p.out2) + static_cast<size_t>(n) * 2, static_cast<size_t>(p.ld_out) * 2);
+            if constexpr (MX && EPI == EPI_RESIDUAL)
+              if (p.q_out8 != nullptr) emit_q(n);
           }
+        }
+      }
+      if constexpr (MX) {
+        if (p.sumsq_out != nullptr && live) {
+          if (p.signal_flag != nullptr) atomicAdd_system(&p.sumsq_out[tok], ssq);          // the tail of a piece: they are the peer's
+          else atomicAdd(&p.sumsq_out[tok], ssq);
         }
       }
     };
@@ -477,14 +627,25 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         tail = true;
         break;
       }
-      finish(lanes + b * BN, m0, n0, 0, BN, nullptr);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) arrive_cluster(mapa_smem(smem_u32(&acc_empty[b]), lead));
+      if constexpr (Cfg::kShared) {
+        hold_c = b ? 0 : static_cast<int>(Cfg::kAccStride);
+        ma_ld32(lanes + Cfg::kAccStride, hold);
+        ma_ld_fence(hold);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_cluster(mapa_smem(smem_u32(&acc_empty[b]), lead));
+        finish(lanes + b * Cfg::kAccStride, m0, n0, 0, BN, nullptr);
+        hold_c = -1;
+      } else {
+        finish(lanes + b * BN, m0, n0, 0, BN, nullptr);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_cluster(mapa_smem(smem_u32(&acc_empty[b]), lead));
+      }
     }
     if (plan.split) {
       // ------------------------------------- exchange of a split tile: pair 0 finishes columns [0, BN/2), pair 1 the others
-      const uint32_t acc = lanes + (i & 1) * BN;
+      const uint32_t acc = lanes + (i & 1) * Cfg::kAccStride;
       const int mine = (crank >> 1) ? BN / 2 : 0, theirs = BN / 2 - mine;
       cluster_arrive_release();                    // every MMA of the cluster has retired: the rings are free
       cluster_wait_acquire();
@@ -539,30 +700,34 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 }
 
 // One launch: `pairs` pairs of CTAs in clusters of 2, or (split) of 4.
-template <int BN, int EPI>
-int launch_wide_one(const GemmParams& p, const CUtensorMap& tw, const CUtensorMap& tx, int pairs, bool split, cudaStream_t stream) {
+template <int BN, int EPI, bool MX>
+int launch_wide_one(const GemmParams& p, const CUtensorMap& tw, const CUtensorMap& tx, const SfMaps& sf, int pairs, bool split, cudaStream_t stream) {
   static bool set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !set[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_wide_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<BN>::kSmem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_wide_kernel<BN, EPI, MX>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<BN, MX>::kSmem);
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev < 64) set[dev] = true;
   }
-  return static_cast<int>(launch_kernel_cx(gemm_wide_kernel<BN, EPI>, dim3(2 * pairs), dim3(WIDE_THREADS), WideCfg<BN>::kSmem, stream,
-                                           split ? 4u : 2u, tw, tx, p, split ? 1 : 0));
+  std::conditional_t<MX, SfMaps, NoMaps> maps;
+  if constexpr (MX) maps = sf;
+  return static_cast<int>(launch_kernel_cx(gemm_wide_kernel<BN, EPI, MX>, dim3(2 * pairs), dim3(WIDE_THREADS), WideCfg<BN, MX>::kSmem, stream,
+                                           split ? 4u : 2u, tw, tx, p, split ? 1 : 0, maps));
 }
 
-template <int BN>
-int launch_wide_bn(const GemmParams& p, const CUtensorMap& tw, const CUtensorMap& tx, int pairs, bool split, cudaStream_t stream) {
+template <int BN, bool MX>
+int launch_wide_bn(const GemmParams& p, const CUtensorMap& tw, const CUtensorMap& tx, const SfMaps& sf, int pairs, bool split, cudaStream_t stream) {
   switch (p.epi) {
-    case EPI_PLAIN: return launch_wide_one<BN, EPI_PLAIN>(p, tw, tx, pairs, split, stream);
-    case EPI_RESIDUAL: return launch_wide_one<BN, EPI_RESIDUAL>(p, tw, tx, pairs, split, stream);
+    case EPI_PLAIN: return launch_wide_one<BN, EPI_PLAIN, MX>(p, tw, tx, sf, pairs, split, stream);
+    case EPI_RESIDUAL: return launch_wide_one<BN, EPI_RESIDUAL, MX>(p, tw, tx, sf, pairs, split, stream);
     case EPI_GLU:
-      if constexpr (BN % 128 == 0) return launch_wide_one<BN, EPI_GLU>(p, tw, tx, pairs, split, stream);
+      if constexpr (BN % 128 == 0) return launch_wide_one<BN, EPI_GLU, MX>(p, tw, tx, sf, pairs, split, stream);
       return -4;
-    case EPI_QKV_ROPE: return launch_wide_one<BN, EPI_QKV_ROPE>(p, tw, tx, pairs, split, stream);
-    case EPI_GELU: return launch_wide_one<BN, EPI_GELU>(p, tw, tx, pairs, split, stream);
+    case EPI_QKV_ROPE: return launch_wide_one<BN, EPI_QKV_ROPE, MX>(p, tw, tx, sf, pairs, split, stream);
+    case EPI_GELU:
+      if constexpr (!MX) return launch_wide_one<BN, EPI_GELU, MX>(p, tw, tx, sf, pairs, split, stream);
+      return -4;
     default: return -4;
   }
 }
@@ -577,7 +742,7 @@ int wide_clusters4() {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(148);
   cfg.blockDim = dim3(WIDE_THREADS);
-  cfg.dynamicSmemBytes = WideCfg<256>::kSmem;
+  cfg.dynamicSmemBytes = WideCfg<256, false>::kSmem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 4;
@@ -585,8 +750,8 @@ int wide_clusters4() {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaFuncSetAttribute(gemm_wide_kernel<256, EPI_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<256>::kSmem) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, gemm_wide_kernel<256, EPI_PLAIN>, &cfg) != cudaSuccess || n < 1) {
+  if (cudaFuncSetAttribute(gemm_wide_kernel<256, EPI_PLAIN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg<256, false>::kSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_wide_kernel<256, EPI_PLAIN, false>, &cfg) != cudaSuccess || n < 1) {
     cudaGetLastError();
     n = 1;
   }
@@ -622,8 +787,17 @@ WideChoice wide_choice(const GemmParams& p, int bn, bool split) {
 
 bool gemm_wide_supported(const GemmParams& p) {
   const int elt = (p.epi == EPI_PLAIN && p.out_fp32) ? 4 : 2;
-  if (p.fp8 || p.norm_src || p.dbg || p.q_out8 || p.sumsq || p.sumsq_out || p.zero_buf) return false;
-  if (p.n_out % 128 != 0 || p.k % WK != 0 || p.k < 2 * WK || p.m_tok <= 0) return false;
+  const bool mx = p.fp8 && p.sfa != nullptr;
+  if (p.norm_src || p.dbg || (p.fp8 && !mx)) return false;
+  if (!mx && (p.q_out8 || p.sumsq || p.sumsq_out || p.zero_buf)) return false;
+  const int ke = mx ? 128 : WK;
+  if (p.n_out % 128 != 0 || p.k % ke != 0 || p.k < 2 * ke || p.m_tok <= 0) return false;
+  if (mx) {
+    if (p.epi == EPI_GELU || p.w_scale || p.sfb == nullptr || p.sf_bn < 128) return false;
+    if ((reinterpret_cast<uintptr_t>(p.sfa) | reinterpret_cast<uintptr_t>(p.sfb)) & 15) return false;
+    if (p.q_out8 && (((reinterpret_cast<uintptr_t>(p.q_out8) | static_cast<uintptr_t>(p.ld_q)) & 15) || (reinterpret_cast<uintptr_t>(p.q_sf) & 1))) return false;
+    if (p.q_out8 && p.q_bn < 128) return false;
+  }
   if (p.epi == EPI_GELU && p.act_gelu == 4) return false;
   if (p.bias && (reinterpret_cast<uintptr_t>(p.bias) & 15)) return false;
   if (p.epi == EPI_QKV_ROPE) {
@@ -637,11 +811,12 @@ bool gemm_wide_supported(const GemmParams& p) {
 
 int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, int split, cudaStream_t stream) {
   if (!gemm_wide_supported(p)) return -2;
-  const bool can_split = p.k / WK >= 8;
+  const bool mx = p.fp8;
+  const bool can_split = p.k / (mx ? 128 : WK) >= 8;
   WideChoice best{0, 0, false, 1e30};
   for (int b = 256; b >= 128; b -= 64) {
     if (bn >= 128 && bn <= 256 && b != bn) continue;
-    if (b == 192 && p.epi == EPI_GLU) continue;                                  // (gate/up pairs are 128 columns wide)
+    if (b == 192 && (p.epi == EPI_GLU || mx)) continue;                          // (gate/up pairs, and runs of scale factors, are 128 columns wide)
     for (int s = 0; s < 2; ++s) {
       if ((split == 0 || split == 1) && s != split) continue;
       if (s && (!can_split || b == 192 || (b == 128 && p.epi == EPI_GLU))) continue;     // halves are whole 64-column blocks
@@ -651,12 +826,20 @@ int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, 
   }
   if (best.bn == 0) return -4;
   CUtensorMap tw, tx;
-  int r = make_tmap_shared(&tw, w, p.n_out, p.k, p.k, best.bn / 2, 2);
+  SfMaps sf;
+  int r = make_tmap_shared(&tw, w, p.n_out, p.k, p.k, best.bn / 2, mx ? 1 : 2);
   if (r) return r;
-  if ((r = make_tmap_shared(&tx, x, p.m_tok, p.k, p.k, WM, 2))) return r;
-  if (best.bn == 192) return launch_wide_bn<192>(p, tw, tx, best.pairs, false, stream);
-  return best.bn == 128 ? launch_wide_bn<128>(p, tw, tx, best.pairs, best.split, stream)
-                        : launch_wide_bn<256>(p, tw, tx, best.pairs, best.split, stream);
+  if ((r = make_tmap_shared(&tx, x, p.m_tok, p.k, p.k, WM, mx ? 1 : 2))) return r;
+  if (mx) {
+    const uint64_t nkb = p.k / 128;
+    if ((r = make_sf_tmap(&sf.w, p.sfa, p.n_out / 128 * nkb))) return r;
+    if ((r = make_sf_tmap(&sf.x, p.sfb, (p.m_tok + p.sf_bn - 1) / p.sf_bn * (p.sf_bn / 128) * nkb))) return r;
+    return best.bn == 128 ? launch_wide_bn<128, true>(p, tw, tx, sf, best.pairs, best.split, stream)
+                          : launch_wide_bn<256, true>(p, tw, tx, sf, best.pairs, best.split, stream);
+  }
+  if (best.bn == 192) return launch_wide_bn<192, false>(p, tw, tx, sf, best.pairs, false, stream);
+  return best.bn == 128 ? launch_wide_bn<128, false>(p, tw, tx, sf, best.pairs, best.split, stream)
+                        : launch_wide_bn<256, false>(p, tw, tx, sf, best.pairs, best.split, stream);
 }
 
 int set_wait_policy_wide(uint32_t* abort_word, unsigned long long limit_ns) {

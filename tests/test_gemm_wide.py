@@ -195,3 +195,54 @@ def test_neighbour_that_never_comes(abort_word):
     assert int(abort[0]) == 1
     assert word.tolist() == [0, 0, 1, 0, 0, 0, 0, 0]
     abort.zero_()
+
+
+# Block-scaled fp8: the runs of scale factors of tokens come in tiles of 128 (m <= 512: 129 and 300 leave half a pair without one) or 256 (513), those of
+# weights per 128 features: 640 and 896 leave the second run of the last 256-wide tile out.  k 256: two stages; 1152: 9, no multiple of a ring, halves of 4 and 5 blocks;
+# 18944 features (74 and 148 tiles of 256): accumulators that overlap, as the rule picks them.
+def spread(rows, k, seed):
+    """rows whose blocks of 32 lie powers of two apart: a scale factor from another place is a large error"""
+    g = torch.Generator(device="cuda").manual_seed(seed + rows + k)
+    e = torch.randint(-3, 4, (rows, k // 32), generator=g, device="cuda").double().repeat_interleave(32, 1)
+    return (torch.randn(rows, k, generator=g, device="cuda").double() * torch.exp2(e)).to(torch.bfloat16)
+
+
+MX_TILES = [(0, -1), (128, 0), (128, 1), (256, 0), (256, 1)]
+
+
+@pytest.mark.parametrize("tile,split", MX_TILES)
+@pytest.mark.parametrize("m,n,k", [(65, 128, 1152), (129, 896, 256), (300, 640, 1152), (513, 1280, 1024), (700, 18944, 256)])
+def test_block_scaled(tile, split, m, n, k):
+    if split == 1 and k < 1024:
+        pytest.skip("fewer than 8 stages are not cut")
+    kw = dict(wide_tile=tile, wide_split=split) if tile else {}
+    wq, sfa = ops.quantize_weight_mxfp8(spread(n, k, 1))
+    bn = ops.pick_bn_mx(m)
+    ss = torch.zeros(m, device="cuda")
+    xq, sfb = ops.quant_mxfp8_rows(spread(m, k, 2), bn, sumsq_out=ss)
+    w = ops.mx_dequant(wq, ops.mx_unchunk(sfa, n, k)).double()
+    ref = ops.mx_dequant(xq, ops.mx_unchunk(sfb, m, k, bn)).double() @ w.t()
+    sf = dict(sfa=sfa, sfb=sfb, **kw)
+    near(ops.gemm(wq, xq, out_fp32=True, **sf), ref, 1e-5)
+
+    def quantised(call, width):
+        """a call that leaves a quantised copy of its bf16 result: the one that quantising the result gives, its sums of squares, and words cleared"""
+        q8 = torch.zeros(m, width, device="cuda", dtype=torch.float8_e4m3fn)
+        q_sf = torch.full(((m + bn - 1) // bn * (width // 128) * (bn // 128) * 512,), 127, device="cuda", dtype=torch.uint8)
+        sums, clear = torch.zeros(m, device="cuda"), torch.ones(m, device="cuda")
+        out = call(fq_out=q8, fq_sf=q_sf, fq_bn=bn, sumsq_out=sums, zero_buf=clear)
+        want, want_sf = ops.quant_mxfp8_rows(out, bn)
+        assert torch.equal(q8.view(torch.uint8), want.view(torch.uint8))
+        assert torch.equal(ops.mx_unchunk(q_sf, m, width, bn), ops.mx_unchunk(want_sf, m, width, bn))
+        near(sums, out.double().pow(2).sum(1), 1e-5)
+        assert not clear.any()
+        return out
+
+    res = bf(m, n)
+    rs = (ss.double() / k + 1e-5).rsqrt()[:, None]
+    near(quantised(lambda **q: ops.gemm(wq, xq, epi=ops.EPI_RESIDUAL, residual=res, sumsq=ss, eps=1e-5, **q, **sf), n), ref * rs + res.double())
+    if n % 256 == 0 and (tile != 128 or split <= 0):                       # (a gate / up pair is 128 columns wide)
+        gu = (ref * rs).view(m, n // 128, 2, 64)
+        near(quantised(lambda **q: ops.gemm(wq, xq, epi=ops.EPI_GLU, sumsq=ss, eps=1e-5, out=torch.empty(m, n // 2, device="cuda", dtype=torch.bfloat16),
+                                            **q, **sf), n // 2), (torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]).flatten(1))
+    assert ops.native().gemm_wide_gave_up() == 0

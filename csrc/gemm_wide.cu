@@ -12,8 +12,8 @@
 //   * one pair per two SMs walks the tiles (persistent); the accumulator is double-buffered in tensor memory, so
 //     the epilogue of a tile runs under the main loop of the next one;
 //   * a lane owns one token and 32 adjacent features per TMEM read: rotary pairs, gate/up pairs and residual rows are in its own
-//     registers or 16-byte accesses away, and the finished 32 x 128-byte block goes through shared memory so that a warp
-//     stores whole 128-byte rows;
+//     registers or 16-byte accesses away, and the finished 32 x 64-byte block goes through shared memory so that a warp
+//     stores pieces of 64 bytes;
 //   * tiles left over after the last full round may be split (clusters of four CTAs then): the two pairs of a cluster take half of K each
 //     and exchange half of the columns through distributed shared memory, which halves the time of that round;
 //   * the piece handoff of gemm_tc.cu is here too (wait for the upstream flag, stores into the peer, release flag), so that pieces on
@@ -36,7 +36,7 @@
 //   4096 tokens: QKV 349 -> 91, O 282 -> 74, gate/up 1718 -> 335 (2.9 PFLOP/s), down 414 -> 178
 //    512 tokens: QKV  78 -> 27, O  53 -> 23, gate/up  290 -> 66, down 88 -> 41
 //    128 tokens: QKV  41 -> 21, O  25 -> 21, gate/up   90 -> 48, down 62 -> 31
-// Roles (192 threads): warp 0 = TMA producer (both CTAs), warp 1 = TMEM owner, MMA issuer in the pair's even CTA, warps 2..5 = epilogue.
+// Roles (320 threads): warp 0 = TMA producer (both CTAs), warp 1 = TMEM owner, MMA issuer in the pair's even CTA, warps 2..9 = epilogue.
 #include "gemm_tc.cuh"
 
 #include <cuda_fp8.h>
@@ -59,10 +59,11 @@ namespace {
 constexpr int WM = 128;                    // token rows per CTA (256 per pair)
 constexpr int WK = 64;                     // K elements per stage (one 128-byte swizzled row; block-scaled fp8: 128)
 constexpr int WA_BYTES = WM * 128;
-constexpr int WIDE_THREADS = 192;
+constexpr int EPI_WARPS = 8;               // two per 32 token rows, each with 32 of every 64 features
+constexpr int WIDE_THREADS = 64 + 32 * EPI_WARPS;
 constexpr int WIDE_PAIRS = 74;             // of the 148 SMs
-constexpr int EPI_PITCH = 144;             // bytes per staged row of 128: 16-byte accesses of 8 lanes fall into distinct banks
-constexpr int EPI_BYTES = 4 * 32 * EPI_PITCH;
+constexpr int EPI_PITCH = 80;              // bytes per staged row of 64: 16-byte accesses of 8 lanes fall into distinct banks
+constexpr int EPI_BYTES = EPI_WARPS * 32 * EPI_PITCH;
 
 __device__ unsigned int g_wide_gave_up = 0;        // CTAs whose waits ran out since the module was loaded
 
@@ -242,7 +243,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 8);                 // the epilogue warps of both CTAs
+      mbar_init(&acc_empty[b], 2 * EPI_WARPS);     // the epilogue warps of both CTAs
     }
     *abort = 0u;
     fence_barrier_init();
@@ -263,48 +264,46 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
   bool ok = true;
   Item it;
+  auto fill = [&](uint32_t n, int kb, int n0, int m0, bool w, bool x) {       // stage n of this CTA
+    const uint32_t s = n % STAGES;
+    uint8_t* st = smem + s * Cfg::kStageBytes;
+    const uint32_t bar = mapa_smem(smem_u32(&full_bar[s]), lead);
+    if (w) {
+      if (!odd) mbar_arrive_expect_tx(&full_bar[s], 2 * (Cfg::kStageBytes + Cfg::kSfBytes));
+      tma_load2(st + WA_BYTES, &tmap_w, bar, kb * KE, n0 + (odd ? BN / 2 : 0));
+      if constexpr (MX) {
+#pragma unroll
+        for (int j = 0; j < BN / 128; ++j)     // (rows behind the last are not there: zeros, for features that are not stored)
+          tma_load2(sf_s + s * Cfg::kSfBytes + 512 + j * 512, &sf_maps.w, bar, 0, (n0 / 128 + j) * plan.nkb + kb);
+      }
+    }
+    if (x) {
+      tma_load2(st, &tmap_x, bar, kb * KE, m0 + (odd ? WM : 0));
+      if constexpr (MX) {                      // runs of 128 tokens, or (sf_bn 256) of 256 whose halves lie side by side
+        const int half = odd ? 1 : 0, run = p.sf_bn > 128 ? (m0 / 256 * plan.nkb + kb) * 2 + half : (m0 / 128 + half) * plan.nkb + kb;
+        tma_load2(sf_s + s * Cfg::kSfBytes, &sf_maps.x, bar, 0, run);
+      }
+    }
+  };
   if (warp == 0) {
     // ------------------------------------------------------------------------------------------------ TMA producer
     if (elect_one()) {
       uint32_t n = 0;                              // stages filled so far
-      auto fill = [&](int kb, int n0, int m0, bool w, bool x) {
-        const uint32_t s = n % STAGES;
-        uint8_t* st = smem + s * Cfg::kStageBytes;
-        const uint32_t bar = mapa_smem(smem_u32(&full_bar[s]), lead);
-        if (w) {
-          if (!odd) mbar_arrive_expect_tx(&full_bar[s], 2 * (Cfg::kStageBytes + Cfg::kSfBytes));
-          tma_load2(st + WA_BYTES, &tmap_w, bar, kb * KE, n0 + (odd ? BN / 2 : 0));
-          if constexpr (MX) {
-#pragma unroll
-            for (int j = 0; j < BN / 128; ++j)     // (rows behind the last are not there: zeros, for features that are not stored)
-              tma_load2(sf_s + s * Cfg::kSfBytes + 512 + j * 512, &sf_maps.w, bar, 0, (n0 / 128 + j) * plan.nkb + kb);
-          }
-        }
-        if (x) {
-          tma_load2(st, &tmap_x, bar, kb * KE, m0 + (odd ? WM : 0));
-          if constexpr (MX) {                      // runs of 128 tokens, or (sf_bn 256) of 256 whose halves lie side by side
-            const int half = odd ? 1 : 0, run = p.sf_bn > 128 ? (m0 / 256 * plan.nkb + kb) * 2 + half : (m0 / 128 + half) * plan.nkb + kb;
-            tma_load2(sf_s + s * Cfg::kSfBytes, &sf_maps.x, bar, 0, run);
-          }
-        }
-      };
       for (int i = 0; ok && plan.get(i, pair, it); ++i) {
         const int m0 = it.t % plan.tok_tiles * (2 * WM), n0 = it.t / plan.tok_tiles * BN;
         int kb = it.kb0;
         if (i == 0) {                              // the weights depend on no earlier kernel: fill the ring with them first
           const int pre = min(STAGES, it.kb1 - it.kb0);
-          for (int j = 0; j < pre; ++j, ++n) fill(kb + j, n0, m0, true, false);
-          pdl_wait();
+          for (; n < static_cast<uint32_t>(pre); ++n) fill(n, kb + n, n0, m0, true, false);
+          pdl_wait();                              // (the tokens' part of these stages: an epilogue warp)
           wait_upstream(p);                        // head of a piece: X is written by the upstream GPU
           if (p.wait_flag != nullptr) fence_proxy_async_all();      // peer-written (generic proxy) data -> TMA (async proxy) reads
-          n = 0;
-          for (int j = 0; j < pre; ++j, ++n) fill(kb + j, n0, m0, false, true);
           kb += pre;
         }
         if (i == (Cfg::kShared ? 1 : 2)) wait_downstream(p);      // (two accumulators: from here on the ring waits for the epilogue, too)
         for (; kb < it.kb1; ++kb, ++n) {
           if (!(ok = ma_wait(&empty_bar[n % STAGES], (n / STAGES & 1u) ^ 1u, abort))) break;
-          fill(kb, n0, m0, true, true);
+          fill(n, kb, n0, m0, true, true);
         }
       }
     }
@@ -354,31 +353,40 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
   } else {
     // ---------------------------------------------------------------------------------------------------- epilogue
-    const int q = warp & 3;
+    // Two warps per 32 rows (with one, each scheduler had a single chain of reads, activations and stores): the last tile's epilogue is in nobody's shadow, and
+    // with a short K all of them take longer than a main loop.  From the last product to the last store, four warps -> eight, us: 512 tokens QKV 3.1 -> 2.8,
+    // O 3.8 -> 2.8, gate/up 9.5 -> 6.7, down 3.6 -> 3.1; up with GELU 768 x 3072, 240 tokens (three activations in one loop before) 9.0 -> 4.3.
+    const int q = warp & 3, hw = (warp - 2) >> 2;
     const int row = q * 32 + lane;                 // TMEM lane == token row of this CTA
     const uint32_t lanes = tmem + (static_cast<uint32_t>(q * 32) << 16);
     uint8_t* sbuf = stage_out + (warp - 2) * 32 * EPI_PITCH;
     uint8_t* srow = sbuf + lane * EPI_PITCH;       // this lane's staged row
-    const int sr = lane >> 3, sc = (lane & 7) * 16;        // coalesced view: rows sr + 4 i, byte column sc
+    const int sr = lane >> 2, sc = (lane & 3) * 16;        // coalesced view: rows sr + 8 i, byte column sc
     const int q_dim = p.n_q_heads * p.head_dim, kv_dim = p.n_kv_heads * p.head_dim;
     pdl_wait();
     wait_upstream(p);
+    if (warp == 2 && plan.get(0, pair, it) && elect_one()) {       // X of the first stages: the producer may still be issuing their weights
+      if (p.wait_flag != nullptr) fence_proxy_async_all();
+      for (int j = 0; j < min(STAGES, it.kb1 - it.kb0); ++j)
+        fill(j, it.kb0 + j, it.t / plan.tok_tiles * BN, it.t % plan.tok_tiles * (2 * WM), false, true);
+    }
+    __syncwarp();
     wait_downstream(p);
     if constexpr (MX) {                            // sums of squares that an earlier product has read and a later one adds to
       if (p.zero_buf != nullptr && blockIdx.x == 0)
-        for (int t = threadIdx.x - 64; t < p.m_tok; t += 128) p.zero_buf[t] = 0.f;
+        for (int t = threadIdx.x - 64; t < p.m_tok; t += 32 * EPI_WARPS) p.zero_buf[t] = 0.f;
     }
     uint32_t hold[Cfg::kShared ? 32 : 1];          // the accumulator columns that two tiles share
     int hold_c = -1;                               // the first of them in the tile that is worked on
 
-    // the residual values of a 64-column block in the coalesced view, in flight while the accumulators are awaited or worked on
-    uint4 res[EPI == EPI_RESIDUAL ? 8 : 1];
+    // the residual values of this warp's 32 columns in the coalesced view, in flight while the accumulators are awaited or worked on
+    uint4 res[EPI == EPI_RESIDUAL ? 4 : 1];
     auto fetch_res = [&](int m0, int n) {
       if constexpr (EPI == EPI_RESIDUAL) {
         const uint8_t* src = reinterpret_cast<const uint8_t*>(p.residual + n) + sc;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int t = m0 + q * 32 + sr + 4 * i;
+        for (int i = 0; i < 4; ++i) {
+          const int t = m0 + q * 32 + sr + 8 * i;
           res[i] = make_uint4(0u, 0u, 0u, 0u);
           if (t < p.m_tok && n < p.n_out) res[i] = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(t) * p.ld_res * 2);
         }
@@ -431,156 +439,158 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           }
         }
       };
-      auto put = [&](int half, const float* v) {   // 32 values as bf16 into this lane's staged row
+      auto put = [&](const float* v) {             // 32 values as bf16 into this lane's staged row
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          *reinterpret_cast<uint4*>(srow + half * 64 + j * 16) = make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
-                                                                            pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
+          *reinterpret_cast<uint4*>(srow + j * 16) = make_uint4(pack2(v[8 * j], v[8 * j + 1]), pack2(v[8 * j + 2], v[8 * j + 3]),
+                                                                pack2(v[8 * j + 4], v[8 * j + 5]), pack2(v[8 * j + 6], v[8 * j + 7]));
       };
-      // staged rows -> memory: `base` = address of token m0's row at this block's first column, `ld` in bytes
+      // staged rows -> memory: `base` = address of token m0's row at this warp's first column, `ld` in bytes
       auto flush = [&](uint8_t* base, size_t ld) {
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int r = sr + 4 * i, t = q * 32 + r;
+        for (int i = 0; i < 4; ++i) {
+          const int r = sr + 8 * i, t = q * 32 + r;
           const uint4 w = *reinterpret_cast<const uint4*>(sbuf + r * EPI_PITCH + sc);
           if (m0 + t < p.m_tok) *reinterpret_cast<uint4*>(base + static_cast<size_t>(m0 + t) * ld + sc) = w;
         }
         __syncwarp();
       };
-      // Block-scaled copy of 64 finished features (this lane's staged bf16 row) for the product that reads them: e4m3, a power of two per 32 of them in
-      // the layout of that product's operand, and the row's sum of squares.  A lane has whole blocks of its token: no exchange.
+
+      // Block-scaled copy of 32 finished features (this lane's staged bf16 row) for the product that reads them: e4m3, a power of two in the layout of
+      // that product's operand, and the row's sum of squares.  A lane has the whole block of its token: no exchange.
       auto emit_q = [&](int feat) {
-        uint32_t e8[16];
-        uint32_t exps = 0u;
+        uint32_t e8[8];
+        float r[32], most = 0.f;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float r[32], most = 0.f;
+        for (int j = 0; j < 4; ++j) {
+          const uint4 w = *reinterpret_cast<const uint4*>(srow + j * 16);
+          const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&w);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint4 w = *reinterpret_cast<const uint4*>(srow + h * 64 + j * 16);
-            const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&w);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 f = __bfloat1622float2(x[e]);
-              r[8 * j + 2 * e] = f.x;
-              r[8 * j + 2 * e + 1] = f.y;
-            }
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(x[e]);
+            r[8 * j + 2 * e] = f.x;
+            r[8 * j + 2 * e + 1] = f.y;
           }
+        }
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            most = fmaxf(most, fabsf(r[j]));
-            ssq += r[j] * r[j];
-          }
-          const uint32_t b = __float_as_uint(most * (1.f / 448.f));
-          const int ex = max(-126, min(127, static_cast<int>(b >> 23) - 127 + ((b & 0x7FFFFFu) ? 1 : 0)));
-          const float inv = __uint_as_float(static_cast<uint32_t>(127 - ex) << 23);
-          exps |= static_cast<uint32_t>(ex + 127) << (8 * h);
+        for (int j = 0; j < 32; ++j) {
+          most = fmaxf(most, fabsf(r[j]));
+          ssq += r[j] * r[j];
+        }
+        const uint32_t b = __float_as_uint(most * (1.f / 448.f));
+        const int ex = max(-126, min(127, static_cast<int>(b >> 23) - 127 + ((b & 0x7FFFFFu) ? 1 : 0)));
+        const float inv = __uint_as_float(static_cast<uint32_t>(127 - ex) << 23);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j] * inv, r[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j + 2] * inv, r[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-            e8[8 * h + j] = lo | (hi << 16);
-          }
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j] * inv, r[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+          const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j + 2] * inv, r[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+          e8[j] = lo | (hi << 16);
         }
         if (live) {
           const int n = tok % p.q_bn, rr = n & 127, run = p.q_bn > 128 ? 1024 : 512;
-          *reinterpret_cast<uint16_t*>(p.q_sf + (static_cast<size_t>(tok / p.q_bn) * (p.ld_q >> 7) + (feat >> 7)) * run + (n >> 7) * 512 + (rr & 31) * 16 +
-                                       (rr >> 5) * 4 + ((feat >> 5) & 3)) = static_cast<uint16_t>(exps);
+          p.q_sf[(static_cast<size_t>(tok / p.q_bn) * (p.ld_q >> 7) + (feat >> 7)) * run + (n >> 7) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 +
+                 ((feat >> 5) & 3)] = static_cast<uint8_t>(ex + 127);
         }
         __syncwarp();                              // the bf16 rows have been stored
-#pragma unroll
-        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(srow + j * 16) = make_uint4(e8[4 * j], e8[4 * j + 1], e8[4 * j + 2], e8[4 * j + 3]);
+        *reinterpret_cast<uint4*>(srow) = make_uint4(e8[0], e8[1], e8[2], e8[3]);
+        *reinterpret_cast<uint4*>(srow + 16) = make_uint4(e8[4], e8[5], e8[6], e8[7]);
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {              // 64 bytes of a row, 8 rows at a time
-          const int r = (lane >> 2) + 8 * i, t = m0 + q * 32 + r;
-          const uint4 w = *reinterpret_cast<const uint4*>(sbuf + r * EPI_PITCH + (lane & 3) * 16);
-          if (t < p.m_tok) *reinterpret_cast<uint4*>(p.q_out8 + static_cast<size_t>(t) * p.ld_q + feat + (lane & 3) * 16) = w;
+        for (int i = 0; i < 2; ++i) {              // 32 bytes of a row, 16 rows at a time
+          const int r = (lane >> 1) + 16 * i, t = m0 + q * 32 + r;
+          const uint4 w = *reinterpret_cast<const uint4*>(sbuf + r * EPI_PITCH + (lane & 1) * 16);
+          if (t < p.m_tok) *reinterpret_cast<uint4*>(p.q_out8 + static_cast<size_t>(t) * p.ld_q + feat + (lane & 1) * 16) = w;
         }
         __syncwarp();
       };
 
       if constexpr (EPI == EPI_GLU) {              // 64 gate columns, then 64 up columns -> 64 outputs
-        for (int c = c0; c < c1 && n0 + c < p.n_out; c += 128) {
 #pragma unroll 1
-          for (int half = 0; half < 2; ++half) {
-            float g[32], u[32];
-            load(c + half * 32, g);
-            load(c + 64 + half * 32, u);
+        for (int c = c0 + hw * 32; c < c1 && n0 + c < p.n_out; c += 128) {
+          float g[32], u[32];
+          load(c, g);
+          load(c + 64, u);
+          if (p.act_gelu) {                        // (the branch outside: code that is not taken is not fetched either)
 #pragma unroll
-            for (int j = 0; j < 32; ++j) g[j] = (p.act_gelu ? gelu_tanh(g[j]) : silu(g[j])) * u[j];
-            put(half, g);
+            for (int j = 0; j < 32; ++j) g[j] = gelu_tanh(g[j]) * u[j];
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) g[j] = silu(g[j]) * u[j];
           }
-          if (!MX || p.out != nullptr)
-            flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>((n0 + c) / 2) * 2, static_cast<size_t>(p.ld_out) * 2);
+          put(g);
+          const int f = (n0 + c - hw * 32) / 2 + hw * 32;
+          if (!MX || p.out != nullptr) flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(f) * 2, static_cast<size_t>(p.ld_out) * 2);
           if constexpr (MX)
-            if (p.q_out8 != nullptr) emit_q((n0 + c) / 2);
+            if (p.q_out8 != nullptr) emit_q(f);
         }
       } else if (EPI == EPI_PLAIN && p.out_fp32) {
-        for (int c = c0; c < c1 && n0 + c < p.n_out; c += 32) {
+#pragma unroll 1
+        for (int c = c0 + hw * 32; c < c1 && n0 + c < p.n_out; c += 64) {
           float v[32];
           load(c, v);
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4*>(srow + j * 16) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-          flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(n0 + c) * 4, static_cast<size_t>(p.ld_out) * 4);
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              *reinterpret_cast<float4*>(srow + j * 16) = make_float4(v[16 * h + 4 * j], v[16 * h + 4 * j + 1], v[16 * h + 4 * j + 2], v[16 * h + 4 * j + 3]);
+            flush(reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(n0 + c + 16 * h) * 4, static_cast<size_t>(p.ld_out) * 4);
+          }
         }
       } else {
-        for (int c = c0; c < c1 && n0 + c < p.n_out; c += 64) {
+#pragma unroll 1
+        for (int c = c0 + hw * 32; c < c1 && n0 + c < p.n_out; c += 64) {
           const int n = n0 + c;
           if constexpr (EPI == EPI_RESIDUAL) {     // the residual rows of this block, whole rows at a time
 #pragma unroll
-            for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(sbuf + (sr + 4 * i) * EPI_PITCH + sc) = res[i];
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(sbuf + (sr + 8 * i) * EPI_PITCH + sc) = res[i];
             if (c + 64 < c1) fetch_res(m0, n + 64);
             __syncwarp();
           }
-#pragma unroll 1
-          for (int half = 0; half < 2; ++half) {
-            float v[32];
-            load(c + half * 32, v);
-            if constexpr (EPI == EPI_RESIDUAL) {
+          float v[32];
+          load(c, v);
+          if constexpr (EPI == EPI_RESIDUAL) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint4 w = *reinterpret_cast<const uint4*>(srow + half * 64 + j * 16);
-                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w);
+            for (int j = 0; j < 4; ++j) {
+              const uint4 w = *reinterpret_cast<const uint4*>(srow + j * 16);
+              const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&w);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float2 f = __bfloat1622float2(h[e]);
-                  v[8 * j + 2 * e] += f.x;
-                  v[8 * j + 2 * e + 1] += f.y;
-                }
-              }
-            } else if constexpr (EPI == EPI_GELU) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (p.act_gelu == 2) {
-                  v[j] = relu_sq(v[j]);
-                } else {
-                  v[j] = p.act_gelu == 3 ? xielu(v[j], p.rope_theta, p.q_scale) : gelu_tanh(v[j]);
-                }
-              }
-            } else if constexpr (EPI == EPI_QKV_ROPE) {
-              const int f = n + half * 32;
-              const int sect = f < q_dim ? 0 : (f < q_dim + kv_dim ? 1 : 2);
-              if (sect < 2 && p.rope_theta > 0.f) {
-                const int j0 = ((f - (sect ? q_dim : 0)) % p.head_dim) >> 1;      // columns (2j, 2j+1) hold (x_j, x_{j+hd/2})
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                  float sn, cs;
-                  sincosf(pos * freq_s[j0 + j], &sn, &cs);
-                  const float a = v[2 * j], b = v[2 * j + 1];
-                  v[2 * j] = a * cs - b * sn;
-                  v[2 * j + 1] = b * cs + a * sn;
-                }
-              }
-              if (sect == 0) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] *= p.q_scale;
+              for (int e = 0; e < 4; ++e) {
+                const float2 f = __bfloat1622float2(h[e]);
+                v[8 * j + 2 * e] += f.x;
+                v[8 * j + 2 * e + 1] += f.y;
               }
             }
-            put(half, v);
+          } else if constexpr (EPI == EPI_GELU) {
+            if (p.act_gelu == 2) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = relu_sq(v[j]);
+            } else if (p.act_gelu == 3) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = xielu(v[j], p.rope_theta, p.q_scale);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
+            }
+          } else if constexpr (EPI == EPI_QKV_ROPE) {
+            const int sect = n < q_dim ? 0 : (n < q_dim + kv_dim ? 1 : 2);
+            if (sect < 2 && p.rope_theta > 0.f) {
+              const int j0 = ((n - (sect ? q_dim : 0)) % p.head_dim) >> 1;      // columns (2j, 2j+1) hold (x_j, x_{j+hd/2})
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                float sn, cs;
+                sincosf(pos * freq_s[j0 + j], &sn, &cs);
+                const float a = v[2 * j], b = v[2 * j + 1];
+                v[2 * j] = a * cs - b * sn;
+                v[2 * j + 1] = b * cs + a * sn;
+              }
+            }
+            if (sect == 0) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) v[j] *= p.q_scale;
+            }
           }
+          put(v);
           if constexpr (EPI == EPI_QKV_ROPE) {
             if (n < q_dim) {
               flush(reinterpret_cast<uint8_t*>(p.q_out + n), static_cast<size_t>(q_dim) * 2);
@@ -589,8 +599,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
               uint8_t* base = reinterpret_cast<uint8_t*>(key ? p.k_cache + (n - q_dim) : p.v_cache + (n - q_dim - kv_dim));
               __syncwarp();
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const int r = sr + 4 * i;
+              for (int i = 0; i < 4; ++i) {
+                const int r = sr + 8 * i;
                 const int sl = __shfl_sync(0xffffffffu, slot, r);
                 const uint4 w = *reinterpret_cast<const uint4*>(sbuf + r * EPI_PITCH + sc);
                 if (sl >= 0) *reinterpret_cast<uint4*>(base + static_cast<size_t>(sl) * kv_dim * 2 + sc) = w;
@@ -619,7 +629,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     for (; ok && plan.get(i, pair, it); ++i) {
       const uint32_t b = i & 1;
       const int m0 = it.t % plan.tok_tiles * (2 * WM) + (odd ? WM : 0), n0 = it.t / plan.tok_tiles * BN;
-      fetch_res(m0, n0 + (it.split && (crank >> 1) ? BN / 2 : 0));
+      fetch_res(m0, n0 + hw * 32 + (it.split && (crank >> 1) ? BN / 2 : 0));
       ok = __all_sync(0xffffffffu, ma_wait(&acc_full[b], i >> 1 & 1, abort));
       if (!ok) break;
       tc_fence_after();
@@ -628,9 +638,11 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         break;
       }
       if constexpr (Cfg::kShared) {
-        hold_c = b ? 0 : static_cast<int>(Cfg::kAccStride);
-        ma_ld32(lanes + Cfg::kAccStride, hold);
-        ma_ld_fence(hold);
+        if (hw == (b ? 0 : 1)) {                   // (columns 0.. of every 64 are the first warp's, 32.. the second's)
+          hold_c = b ? 0 : static_cast<int>(Cfg::kAccStride);
+          ma_ld32(lanes + Cfg::kAccStride, hold);
+          ma_ld_fence(hold);
+        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) arrive_cluster(mapa_smem(smem_u32(&acc_empty[b]), lead));
@@ -652,7 +664,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       if (tail) {
         const uint32_t zone = mapa_smem(smem_u32(smem), crank ^ 2u) + static_cast<uint32_t>(row * Cfg::kLandPitch * 4);
 #pragma unroll 1
-        for (int c = 0; c < BN / 2; c += 32) {
+        for (int c = hw * 32; c < BN / 2; c += 64) {
           uint32_t r[32];
           ma_ld32(acc + theirs + c, r);
           ma_ld_fence(r);
@@ -671,7 +683,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
     if (p.signal_flag != nullptr || p.bump_epoch != nullptr) {        // tail of a piece: the last CTA publishes the payload
       __threadfence_system();                      // my (possibly peer-directed) stores are performed
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      asm volatile("bar.sync 1, 256;" ::: "memory");
       if (threadIdx.x == 64) publish_handoff(p, gridDim.x, *abort != 0u);
     }
   }

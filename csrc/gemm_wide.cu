@@ -129,8 +129,10 @@ __device__ __forceinline__ void tma_load2(void* smem_dst, const CUtensorMap* m, 
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
-__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+// the accumulator has been read (tcgen05.fence orders that): nothing that was written goes with it, and a release to the cluster waits until the tile's stores have
+// arrived in L2
+__device__ __forceinline__ void arrive_cluster_read(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // One arrival per CTA; the last one releases the payload to the downstream piece and this piece's input slot to the upstream one -- unless a
@@ -645,14 +647,14 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster(mapa_smem(smem_u32(&acc_empty[b]), lead));
+        if (lane == 0) arrive_cluster_read(mapa_smem(smem_u32(&acc_empty[b]), lead));
         finish(lanes + b * Cfg::kAccStride, m0, n0, 0, BN, nullptr);
         hold_c = -1;
       } else {
         finish(lanes + b * BN, m0, n0, 0, BN, nullptr);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster(mapa_smem(smem_u32(&acc_empty[b]), lead));
+        if (lane == 0) arrive_cluster_read(mapa_smem(smem_u32(&acc_empty[b]), lead));
       }
     }
     if (plan.split) {
@@ -699,7 +701,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (*abort != 0u) __nanosleep(200000);           // copies in flight land before the shared memory is given back
   tc_fence_before();
   __syncthreads();
-  cluster_arrive_release();                        // no CTA leaves while another may still arrive on its barriers or read its operands
+  cluster_arrive_relaxed();                        // no CTA leaves while another may still arrive on its barriers or read its operands
   cluster_wait_acquire();
   if (warp == 1) {
     tc_fence_after();

@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                   }
                   if (end > first) {
                     if (!(ok = lc_wait_due(due_s, at - 1, abort))) break;
-                    fence_proxy_async_all();
+                    fence_proxy_async_global();
                     appended = true;
                   }
                 }
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
           if (at > 0) {                              // the operations so far are complete: this thread alone polls, the others of the CTA look at due_s
             if (!(ok = lc_wait_op(ctr + at - 1, ctas, p.polls, abort, p.ctl))) break;
             asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(due_s)), "r"(at) : "memory");
-            fence_proxy_async_all();
+            fence_proxy_async_global();
           }
           ++at;
           if (lc_weight(op) >= 0) {

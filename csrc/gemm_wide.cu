@@ -258,7 +258,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
-  cluster_arrive_release();                        // the other CTAs arrive on these barriers
+  cluster_arrive_relaxed();                        // the other CTAs arrive on these barriers (their initialisation is released by its own fence)
   cluster_wait_acquire();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
@@ -394,20 +394,28 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
       }
     };
+    // what belongs to this lane's token, in flight while the accumulator is awaited
+    float tok_scale = 1.f, tok_pos = 0.f;
+    int tok_slot = -1;
+    auto fetch_token = [&](int m0) {
+      const int tok = m0 + row;
+      const bool live = tok < p.m_tok;
+      tok_scale = (p.rstd != nullptr && live) ? p.rstd[tok] : 1.f;
+      if constexpr (MX)
+        if (p.sumsq != nullptr && live) tok_scale *= rsqrtf(p.sumsq[tok] / static_cast<float>(p.k) + p.eps);
+      if constexpr (EPI == EPI_QKV_ROPE) {
+        tok_slot = live ? p.slots[tok] : -1;
+        tok_pos = (p.positions != nullptr && live) ? static_cast<float>(p.positions[tok]) : 0.f;
+      }
+    };
     // columns [c0, c1) of the tile at (token m0, feature n0); `land`: the other pair's partial sums of this lane's row, from column c0 on
     auto finish = [&](uint32_t acc, int m0, int n0, int c0, int c1, const float* land) {
       const int tok = m0 + row;
       const bool live = tok < p.m_tok;
       if (m0 + q * 32 >= p.m_tok) return;          // no token of this warp (warp-uniform)
-      float rs = (p.rstd != nullptr && live) ? p.rstd[tok] : 1.f, ssq = 0.f;
-      if constexpr (MX)
-        if (p.sumsq != nullptr && live) rs *= rsqrtf(p.sumsq[tok] / static_cast<float>(p.k) + p.eps);
-      int slot = -1;
-      float pos = 0.f;
-      if constexpr (EPI == EPI_QKV_ROPE) {
-        slot = live ? p.slots[tok] : -1;
-        pos = (p.positions != nullptr && live) ? static_cast<float>(p.positions[tok]) : 0.f;
-      }
+      const float rs = tok_scale, pos = tok_pos;
+      const int slot = tok_slot;
+      float ssq = 0.f;
       auto load = [&](int c, float* v) {           // 32 accumulator columns, scaled
         uint32_t r[32];
         ma_ld32(acc + c, r);
@@ -631,6 +639,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     for (; ok && plan.get(i, pair, it); ++i) {
       const uint32_t b = i & 1;
       const int m0 = it.t % plan.tok_tiles * (2 * WM) + (odd ? WM : 0), n0 = it.t / plan.tok_tiles * BN;
+      fetch_token(m0);
       fetch_res(m0, n0 + hw * 32 + (it.split && (crank >> 1) ? BN / 2 : 0));
       ok = __all_sync(0xffffffffu, ma_wait(&acc_full[b], i >> 1 & 1, abort));
       if (!ok) break;
@@ -661,7 +670,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       // ------------------------------------- exchange of a split tile: pair 0 finishes columns [0, BN/2), pair 1 the others
       const uint32_t acc = lanes + (i & 1) * Cfg::kAccStride;
       const int mine = (crank >> 1) ? BN / 2 : 0, theirs = BN / 2 - mine;
-      cluster_arrive_release();                    // every MMA of the cluster has retired: the rings are free
+      cluster_arrive_relaxed();                    // every MMA of the cluster has retired: the rings are free
       cluster_wait_acquire();
       if (tail) {
         const uint32_t zone = mapa_smem(smem_u32(smem), crank ^ 2u) + static_cast<uint32_t>(row * Cfg::kLandPitch * 4);
@@ -693,7 +702,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __syncwarp();
     if (plan.split) {
       for (int k = 0; k < 2; ++k) {
-        cluster_arrive_release();
+        cluster_arrive_relaxed();
         cluster_wait_acquire();
       }
     }
@@ -826,7 +835,10 @@ bool gemm_wide_supported(const GemmParams& p) {
 int launch_gemm_wide(const GemmParams& p, const void* w, const void* x, int bn, int split, cudaStream_t stream) {
   if (!gemm_wide_supported(p)) return -2;
   const bool mx = p.fp8;
-  const bool can_split = p.k / (mx ? 128 : WK) >= 8;
+  // Two pairs on a tile save half of its blocks of K (0.17 us each) and exchange sums (1.6 us): 768 x 768, 240 tokens, whole 6.9 us, cut 7.4; 3072 x 768 7.4
+  // and 8.2; 768 x 3072 12.4 and 10.0.  (Where the call names it, from 8 blocks on: halves of four.)
+  const int blocks = p.k / (mx ? 128 : WK);
+  const bool can_split = blocks >= (split == 1 ? 8 : 20);
   WideChoice best{0, 0, false, 1e30};
   for (int b = 256; b >= 128; b -= 64) {
     if (bn >= 128 && bn <= 256 && b != bn) continue;

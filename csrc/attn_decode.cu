@@ -19,12 +19,15 @@
 // the partial sums through distributed shared memory -- no workspace and no second kernel.
 //
 // Bound: the cache stream.  Measured on B200 (attention_tc.cu -> here), 32 query / 8 key/value heads of 128, us: 32 sequences x 8100 keys
-// 252 -> 160 (6.6 TB/s), 32 x 500 22 -> 16, 8 x 4000 50 -> 26, one x 700 18 -> 7.6, one x 8000 26 -> 13; 8 / 4 heads of 256, 32 x 4000 91 -> 80.
+// 252 -> 160 (6.6 TB/s), 32 x 500 22 -> 16, 8 x 4000 50 -> 26, one x 700 18 -> 7.6, one x 8000 26 -> 13; 8 / 4 heads of 256, 32 x 4000 91 -> 80; 12 / 12 heads of 64
+// (in pairs), 8 x 8000 107 -> 36, 32 x 8000 214 -> 124, 32 x 2000 56 -> 34, 8 x 400 9.8 -> 7.6, error 0.00230 -> 0.00217 (8 x 3000).
 // Warp roles: 0 = TMA producer, 1 = TMEM owner + MMA issuer, 2..5 = softmax / correction / output.
 #include "kernels.h"
 
 #include <cuda.h>
 #include <cuda_fp8.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "launch.cuh"
@@ -58,15 +61,19 @@ struct DecodeParams {
   int q_bn;
 };
 
-template <int D>
+// PAIR: two neighbouring key/value heads of 64 channels as one of D = 128.  Their scores are products of their own (the halves of a key row, each into columns of
+// its own), so nothing of one head enters the other's; of O, every column holds its head's 64 channels and 64 that nobody reads.
+template <int D, bool PAIR>
 struct DecCfg {
   static constexpr int kTile = DKEYS * D * 2;                      // a K or V tile
   static constexpr int kQ = DHEADS * D * 2;
   static constexpr int kP = DHEADS * DKEYS * 2;
   static constexpr int kSmem = 1024 + DSLOTS * kTile + kQ + 2 * kP + 512;
   static constexpr int kMinCtas = D == 128 ? 2 : 1;
-  static constexpr uint32_t kCols = 64;                            // S twice, O for every 128 channels
-  static constexpr uint32_t kOCol = 2 * DHEADS;
+  static constexpr uint32_t kSCols = PAIR ? 2 * DHEADS : DHEADS;
+  static constexpr uint32_t kOCol = 2 * kSCols;                    // S twice, O for every 128 channels
+  static constexpr uint32_t kCols = PAIR ? 128 : 64;
+  static_assert(!PAIR || D == 128, "two heads of 64 channels");
 };
 
 template <int GP>
@@ -120,13 +127,15 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr) {
   return v;
 }
 
-// GP: query heads per key/value head rounded up to 4, 8 or 16.  grid (CTAs of the cluster, key/value heads, sequences)
-template <int D, int GP, bool SOFTCAP>
-__global__ void __launch_bounds__(DEC_THREADS, DecCfg<D>::kMinCtas)
+// GP: query heads per key/value head rounded up to 4, 8 or 16 (PAIR: to 4 or 8, twice).  grid (CTAs of the cluster, key/value heads or pairs of them, sequences)
+template <int D, int GP, bool SOFTCAP, bool PAIR>
+__global__ void __launch_bounds__(DEC_THREADS, (DecCfg<D, PAIR>::kMinCtas))
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const DecodeParams p, const int G) {
-  using Cfg = DecCfg<D>;
+  using Cfg = DecCfg<D, PAIR>;
   constexpr int DB = D / 64, MB = D / 128;         // 64-channel blocks of a row; 128-channel blocks of O
+  constexpr int GH = PAIR ? GP / 2 : GP;           // columns of a key/value head
+  const int hd = PAIR ? 64 : D, heads = PAIR ? 2 * G : G;          // channels of a head, query heads of this CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_s = smem + DSLOTS * Cfg::kTile;
@@ -188,7 +197,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (elect_one()) {
       mbar_arrive_expect_tx(q_full, Cfg::kQ);
 #pragma unroll
-      for (int c = 0; c < DB; ++c) tma_load_2d(q_s + c * (DHEADS * 128), &tm_q, q_full, c * 64, p.q_start[seq] * p.n_q + kvh * G);
+      for (int c = 0; c < DB; ++c)
+        tma_load_2d(q_s + c * (DHEADS * 128), &tm_q, q_full, PAIR ? 0 : c * 64, p.q_start[seq] * p.n_q + kvh * heads + (PAIR ? c * G : 0));
       const int* bt = p.block_table + static_cast<size_t>(seq) * p.max_pages;
       uint32_t i = 0;
       auto load = [&](const CUtensorMap* tm, int n) {                // K or V tile n of this CTA into the next slot
@@ -226,7 +236,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint64_t a = make_sw128_kmajor_desc(smem_u32(smem + s * Cfg::kTile + (kk / 4) * (DKEYS * 128))) + static_cast<uint64_t>((kk % 4) * 2);
           const uint64_t b = make_sw128_kmajor_desc(smem_u32(q_s + (kk / 4) * (DHEADS * 128))) + static_cast<uint64_t>((kk % 4) * 2);
-          umma_bf16(tmem + static_cast<uint32_t>(n & 1) * DHEADS, a, b, idesc_s, kk > 0 ? 1u : 0u);
+          umma_bf16(tmem + static_cast<uint32_t>(n & 1) * Cfg::kSCols + (PAIR ? kk / 4 * DHEADS : 0), a, b, idesc_s, (PAIR ? kk % 4 : kk) > 0 ? 1u : 0u);
         }
         umma_commit(&empty[s]);
         umma_commit(&s_full[n & 1]);
@@ -273,14 +283,17 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       ok = __all_sync(0xffffffffu, ma_wait(&s_full[b], n >> 1 & 1, abort)) && ok;
       tc_fence_after();
       float x[GP] = {};
-      if (ok) dec_ld<GP>(lanes + b * DHEADS, x);
+      if (ok) {
+        dec_ld<GH>(lanes + b * Cfg::kSCols, x);
+        if constexpr (PAIR) dec_ld<GH>(lanes + b * Cfg::kSCols + DHEADS, x + GH);
+      }
       const bool seen = key < kvlen && key >= kv_lo;
       bool up = false;
 #pragma unroll
       for (int g = 0; g < GP; ++g) {
         if constexpr (SOFTCAP) x[g] = p.softcap * tanh_exp(x[g] * inv_cap);
         x[g] = seen ? x[g] * DEC_LOG2E : -INFINITY;
-        up |= g < G && (x[g] > m_ref[g] + 8.f || (m_ref[g] == -INFINITY && x[g] > -INFINITY));
+        up |= g % GH < G && (x[g] > m_ref[g] + 8.f || (m_ref[g] == -INFINITY && x[g] > -INFINITY));
       }
       // P(n - 2) has been read; waited for in every tile so that no parity wait lags two phases behind
       if (ok && n > 1) ok = __all_sync(0xffffffffu, ma_wait(&pv_done[b], (n - 2) >> 1 & 1, abort));
@@ -297,7 +310,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 #pragma unroll
         for (int g = 0; g < GP; ++g) {
           const float m = fmaxf(m_ref[g], fmaxf(fmaxf(red_s[0][g], red_s[1][g]), fmaxf(red_s[2][g], red_s[3][g])));
-          alpha[g] = (m_ref[g] == -INFINITY || g >= G) ? 0.f : ex2(m_ref[g] - m);
+          alpha[g] = (m_ref[g] == -INFINITY || g % GH >= G) ? 0.f : ex2(m_ref[g] - m);
           m_ref[g] = m;
           l[g] *= alpha[g];
         }
@@ -320,7 +333,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       uint8_t* pt = p_s + b * Cfg::kP + (row >> 6) * (DHEADS * 128) + (row & 7) * 2;
 #pragma unroll
       for (int g = 0; g < GP; ++g) {
-        if (g < G) {
+        if (g % GH < G) {
           const float e = ex2(x[g] - (m_ref[g] == -INFINITY ? 0.f : m_ref[g]));
           const __nv_bfloat16 w = __float2bfloat16_rn(e);
           l[g] += __bfloat162float(w);             // the sum of what the product sees: the rounding of a dominant weight cancels
@@ -358,7 +371,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (warp >= 2 && active) {
 #pragma unroll
     for (int g = 0; g < GP; ++g) {
-      if (g < G) {
+      if (g % GH < G) {
 #pragma unroll
         for (int m = 0; m < MB; ++m) part[g * D + m * 128 + row] = o[m][g];
         if (row == 0) {
@@ -377,8 +390,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   if (warp >= 2 && active) {
     // ---------------------------------------------------------------- merge: this CTA finishes every parts-th run of 128 outputs
     const uint32_t mine = smem_u32(part);
-    for (int e = rank * 128 + row; e < G * D; e += parts * 128) {
-      const int g = e / D;
+    for (int e = rank * 128 + row; e < heads * hd; e += parts * 128) {
+      const int head = e / hd, g = PAIR ? head / G * GH + head % G : head;
+      const uint32_t from = mine + (PAIR ? g * D + head / G * 64 + e % 64 : e) * 4;
       float m = -INFINITY;
       for (int r = 0; r < parts; ++r) m = fmaxf(m, ld_dsmem_f32(mapa_smem(mine + (DHEADS * D + g) * 4, r)));
       float num = 0.f, den = 0.f;
@@ -386,10 +400,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         const float mr = ld_dsmem_f32(mapa_smem(mine + (DHEADS * D + g) * 4, r));
         const float w = mr == -INFINITY ? 0.f : ex2(mr - m);
         den += w * ld_dsmem_f32(mapa_smem(mine + (DHEADS * D + DHEADS + g) * 4, r));
-        num += w * ld_dsmem_f32(mapa_smem(mine + e * 4, r));
+        num += w * ld_dsmem_f32(mapa_smem(from, r));
       }
       const float v = den == 0.f ? 0.f : num / den;      // (no key: zero; a NaN among the scores stays one)
-      const int tok = p.q_start[seq], feat = kvh * G * D + e, ldq = p.n_q * D;
+      const int tok = p.q_start[seq], feat = kvh * heads * hd + e, ldq = p.n_q * hd;
       if (p.q_out8 == nullptr) {
         p.out[static_cast<size_t>(tok) * ldq + feat] = __float2bfloat16_rn(v);
       } else {                                     // e4m3 + scale of the warp's 32 features (what a separate quantiser would compute)
@@ -427,39 +441,83 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   }
 }
 
-template <int D, int GP, bool SOFTCAP>
-int launch_dec(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int G, int seqs, int parts,
-               cudaStream_t s) {
+// Clusters of 4 or 8 CTAs, one per SM, that fit the device at once: fewer than 37 or 18, because GPCs have 16 to 18 SMs.
+int dec_clusters(int size) {
+  static int known[2][64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 64 && known[size / 8][dev] > 0) return known[size / 8][dev];
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(144);
+  cfg.blockDim = dim3(DEC_THREADS);
+  cfg.dynamicSmemBytes = DecCfg<256, false>::kSmem;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeClusterDimension;
+  a[0].val.clusterDim.x = static_cast<unsigned>(size);
+  a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
+  cfg.attrs = a;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(attn_decode_kernel<256, 4, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecCfg<256, false>::kSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, attn_decode_kernel<256, 4, false, false>, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = 112 / size;
+  }
+  if (dev < 64) known[size / 8][dev] = n;
+  return n;
+}
+
+// CTAs of a cluster: they share the keys of a (sequence, key/value head) while that still adds resident CTAs (two per SM at 128 channels) and every CTA can have a
+// tile and all clusters fit at once.  256-wide heads, 4 sequences of 8000 / 2000 keys: 16 clusters of eight ran in two rounds (37.7 / 14.6 us), in clusters of four
+// 27.7 / 10.0.  With two CTAs on an SM 32 clusters of eight and 64 of four ran at once (4 and 8 sequences of 8 heads), 36 and 72 did not (6 and 12 sequences of 6 pairs, 2000
+// keys: 15.0 against 10.0 us in clusters of four, 23.9 against 17.4 in clusters of two).
+int dec_parts(int items, int tiles, bool one_per_sm) {
+  const int slots = one_per_sm ? 148 : 296;
+  int parts = 1;
+  while (parts < 8 && static_cast<long long>(items) * parts * 2 <= slots && parts * 2 <= tiles) parts *= 2;
+  while (parts > 2 && items > (one_per_sm ? dec_clusters(parts) : 256 / parts)) parts /= 2;
+  return parts;
+}
+
+template <int D, int GP, bool SOFTCAP, bool PAIR>
+int launch_dec(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int G, int seqs, int tiles, cudaStream_t s) {
   static bool set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64 || !set[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, GP, SOFTCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecCfg<D>::kSmem);
+    const cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D, GP, SOFTCAP, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecCfg<D, PAIR>::kSmem);
     if (e != cudaSuccess) return static_cast<int>(e);
     if (dev < 64) set[dev] = true;
   }
-  const dim3 grid(parts, p.n_kv, seqs);
+  const int kv = PAIR ? p.n_kv / 2 : p.n_kv, parts = dec_parts(seqs * kv, tiles, DecCfg<D, PAIR>::kMinCtas == 1);
+  const dim3 grid(parts, kv, seqs);
   if (parts > 1)
-    return static_cast<int>(launch_kernel_cx(attn_decode_kernel<D, GP, SOFTCAP>, grid, dim3(DEC_THREADS), DecCfg<D>::kSmem, s,
+    return static_cast<int>(launch_kernel_cx(attn_decode_kernel<D, GP, SOFTCAP, PAIR>, grid, dim3(DEC_THREADS), DecCfg<D, PAIR>::kSmem, s,
                                              static_cast<unsigned>(parts), tq, tk, tv, p, G));
-  return static_cast<int>(launch_kernel(attn_decode_kernel<D, GP, SOFTCAP>, grid, dim3(DEC_THREADS), DecCfg<D>::kSmem, s, 1u, tq, tk, tv, p, G));
+  return static_cast<int>(launch_kernel(attn_decode_kernel<D, GP, SOFTCAP, PAIR>, grid, dim3(DEC_THREADS), DecCfg<D, PAIR>::kSmem, s, 1u, tq, tk, tv, p, G));
 }
 
-template <int D>
-int launch_dec_g(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int G, int seqs, int parts,
+template <int D, bool PAIR>
+int launch_dec_g(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int G, int seqs, int tiles,
                  cudaStream_t s) {
 #define B2B_DEC(GP) \
-  (p.softcap > 0.f ? launch_dec<D, GP, true>(tq, tk, tv, p, G, seqs, parts, s) : launch_dec<D, GP, false>(tq, tk, tv, p, G, seqs, parts, s))
-  if (G <= 4) return B2B_DEC(4);
-  if (G <= 8) return B2B_DEC(8);
-  return B2B_DEC(16);
+  (p.softcap > 0.f ? launch_dec<D, GP, true, PAIR>(tq, tk, tv, p, G, seqs, tiles, s) : launch_dec<D, GP, false, PAIR>(tq, tk, tv, p, G, seqs, tiles, s))
+  if constexpr (PAIR) {
+    return G <= 4 ? B2B_DEC(8) : B2B_DEC(16);
+  } else {
+    if (G <= 4) return B2B_DEC(4);
+    if (G <= 8) return B2B_DEC(8);
+    return B2B_DEC(16);
+  }
 #undef B2B_DEC
 }
 
 }  // namespace
 
 bool attn_decode_supported(int n_q, int n_kv, int head_dim) {
-  return n_kv > 0 && n_q % n_kv == 0 && n_q / n_kv <= DHEADS && (head_dim == 128 || head_dim == 256);
+  if (n_kv <= 0 || n_q % n_kv != 0) return false;
+  if (head_dim == 64) return n_kv % 2 == 0 && n_q / n_kv <= DHEADS / 2;
+  return n_q / n_kv <= DHEADS && (head_dim == 128 || head_dim == 256);
 }
 
 int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table, const int* q_start,
@@ -479,11 +537,9 @@ int launch_attn_decode(const void* q, const void* k_cache, const void* v_cache, 
   p.q_out8 = static_cast<uint8_t*>(q_out8);
   p.q_sf = static_cast<uint8_t*>(q_sf);
   p.q_bn = q_bn > 0 ? q_bn : 32;
-  // a cluster shares the keys while that still adds resident CTAs (two per SM at D = 128) and every CTA can have a tile
-  const int slots = head_dim == 128 ? 296 : 148;
-  int parts = 1;
-  while (parts < 8 && static_cast<long long>(seqs) * n_kv * parts * 2 <= slots && parts * 2 * (DKEYS / DPAGE) <= max_pages) parts *= 2;
-  return head_dim == 128 ? launch_dec_g<128>(tq, tk, tv, p, n_q / n_kv, seqs, parts, s) : launch_dec_g<256>(tq, tk, tv, p, n_q / n_kv, seqs, parts, s);
+  const int g = n_q / n_kv, tiles = std::max(1, max_pages / (DKEYS / DPAGE));
+  if (head_dim == 64) return launch_dec_g<128, true>(tq, tk, tv, p, g, seqs, tiles, s);
+  return head_dim == 128 ? launch_dec_g<128, false>(tq, tk, tv, p, g, seqs, tiles, s) : launch_dec_g<256, false>(tq, tk, tv, p, g, seqs, tiles, s);
 }
 
 int set_wait_policy_decode(uint32_t* abort_word, unsigned long long limit_ns) {

@@ -134,3 +134,31 @@ def test_dominant_weight():
     ops.attention(q, k, v, out, table, i32(list(range(S))), i32([1] * S), i32([300] * S), max_q=1, n_q=nq, n_kv=nkv, head_dim=D)
     ref = reference(q, k, v, table, [300] * S, nq, nkv, D, 0, 0.0)
     assert float((out.double() - ref).norm() / ref.norm()) < 0.0019
+
+
+# Two neighbouring key/value heads of 64 channels are one of 128: one query head each and several (in columns 4 or 8 apart), one pair and many, few sequences
+# in clusters of 8, 4 and 2 and more of them than fit at once in the larger size (6 and 12 sequences of 6 pairs)
+@pytest.mark.parametrize("nq,nkv", [(12, 12), (2, 2), (8, 4), (20, 4), (16, 2)])
+@pytest.mark.parametrize("lens,spare", [([1], 0), ([128, 129, 127, 64, 63, 65], 0), ([1, 3000, 250, 17], 40), ([1100 + 31 * i for i in range(12)], 0),
+                                        ([90 * i + 1 for i in range(40)], 0)])
+@pytest.mark.parametrize("window,cap", [(0, 0.0), (100, 50.0)])
+def test_pairs_of_64(nq, nkv, lens, spare, window, cap):
+    test_decode(nq, nkv, 64, lens, spare, window, cap)
+
+
+def test_a_pair_stays_apart():
+    """keys and values of one head that are not finite reach its own query heads alone"""
+    lens, nq, nkv = [70, 300], 8, 4
+    q, k, v, table = setup(lens, nq, nkv, 64)
+    ref = reference(q, k, v, table, lens, nq, nkv, 64, 0, 0.0).view(2, nq, 64)
+    page = int(table[1][1])
+    k[page, 5, 1, 3] = float("inf")
+    v[page, 9, 2, 60] = float("nan")
+    out = torch.empty_like(q)
+    ops.attention(q, k, v, out, table, i32([0, 1]), i32([1, 1]), i32(lens), max_q=1, n_q=nq, n_kv=nkv, head_dim=64)
+    out = out.view(2, nq, 64)
+    assert torch.isnan(out[1, 4:6, 60]).all()
+    for s, h in ((0, slice(0, 8)), (1, slice(0, 2)), (1, slice(6, 8))):
+        assert float((out[s, h].double() - ref[s, h]).norm() / ref[s, h].norm()) < BOUND
+    other = torch.arange(64, device="cuda") != 60
+    assert float((out[1, 4:6, other].double() - ref[1, 4:6, other]).norm() / ref[1, 4:6, other].norm()) < BOUND

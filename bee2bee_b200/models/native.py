@@ -329,17 +329,19 @@ class NativePiece:
         return chain_key_limit(tokens, self.cfg.n_heads, self._chain.ctas)
 
     def _chain_pays(self, m: BatchMeta) -> bool:
-        """the persistent kernel is the faster one for as many keys as the tokens of ``m`` may see.  Per layer it gains (products and launches) 9.5 us on Llama and
-        Mistral shapes, 5 behind post norms, 11.5 from 33 tokens on; block-scaled fp8 5 up to 16 tokens and nothing beyond (measured as above, the smaller
-        ones of each)."""
+        """the persistent kernel is the faster one for as many keys as the tokens of ``m`` may see.  Per layer it gains (products and launches, the smallest of
+        500 to 4000 keys) 11.7 us on Llama and Mistral shapes up to 16 tokens, 16.3 up to 32, 18.5 beyond; behind post norms 11.2 up to 32 and 17.2 beyond;
+        block-scaled fp8 13.6 up to 16 tokens and 12.7 up to 32."""
         c = self.cfg
         keys = m.max_keys or m.block_table.shape[1] * ops.PAGE
         if self._chain_ln:                     # (their positions come from a table)
             return min(keys, c.max_position) <= self.span_keys(m.n_tokens)
         if self.mx_fuse:
-            gain = 5.0 if m.n_tokens <= 16 else 0.25
+            gain = 13.5 if m.n_tokens <= 16 else 12.5
+        elif c.post_norms:
+            gain = 11.0 if m.n_tokens <= 32 else 17.0
         else:
-            gain = 11.5 if m.n_tokens > 32 else (5.0 if c.post_norms else 9.5)
+            gain = 11.5 if m.n_tokens <= 16 else (16.0 if m.n_tokens <= 32 else 18.5)
         windows = [c.layer_window(l) for l in self.layers]
         lost = sum(windows.count(w) * chain_attention_us(m.n_seqs, c.n_kv_heads, c.head_dim, keys, w, self._chain.ctas) for w in set(windows))
         return lost <= gain * len(windows)

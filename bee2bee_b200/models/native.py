@@ -124,8 +124,8 @@ def chain_attention_us(seqs: int, n_kv: int, head_dim: int, keys: int, window: i
 def chain_key_limit(tokens: int, heads: int, ctas: int) -> int:
     """LayerNorm models: the most keys that a token may see for the persistent kernel to be the faster one.  Its attention reads all keys of a (token, head) for
     that one alone, on a warp up to 128 keys and on a CTA beyond; the kernel of its own reads them once for 16 tokens.  gpt2, us per layer gained, by
-    rounds of (token, head) over the CTAs: one round 3 to 9 at 900 keys; two 4 at 256 to 300, -4 to -23 at 500 to 900; three and four 3 to 7 at 128, 2 to
-    -1 at 170; more 4 at 115, 1 to -1 at 124."""
+    rounds of (token, head) over the CTAs: one round 1 at 900 keys; two 6 to 9 at 300, 5 to -2 at 500, -4 to -22 at 900; three (32 tokens) 5 at 120, 3 at
+    200, -1 at 300; more (64) 10 to 13 at 60, 0 at 120."""
     rounds = -(-tokens * heads // ctas)
     return 1024 if rounds <= 1 else (256 if rounds == 2 else (128 if rounds <= 4 else 112))
 

@@ -185,8 +185,8 @@ def use_wide(n_out: int, m_tok: int, mx: bool = False) -> bool:
     tokens: 17 against 40 us for 6144 x 4096, 55 against 84 for 28672 x 4096); at 65 .. 128 tokens, where both read the weights
     once, it is while gemm_tc.cu has no more than one tile per SM (128 tokens: 17 against 33 us for 6144 x 4096, 30 against 63 for
     4096 x 14336, 23 against 27 for 18432 x 2304, but 54 against 51 for 28672 x 4096).  Block-scaled fp8 (``mx``): for all of them from 65
-    tokens on (gate/up 28672 x 4096, gemm_tc.cu / CTA pairs: 96 tokens 79 / 47 us, 256 170 / 48, 1000 463 / 100, 4096 1718 / 335; 4096 x 14336:
-    59 / 31, 59 / 31, 120 / 58, 414 / 178; with cold caches and the latency of a launch)."""
+    tokens on (gate/up 28672 x 4096, gemm_tc.cu / CTA pairs, back to back with cold weights: 128 tokens 84 / 32 us, 512 286 / 50, 4096 1751 / 333;
+    4096 x 14336: 55 / 20, 77 / 29, 461 / 189)."""
     return m_tok > 128 or (m_tok > 64 and (mx or n_out <= 128 * NUM_SMS))
 
 

@@ -23,19 +23,18 @@
 //
 // Bound: tensor pipe (98 % active while a tile runs) and the power cap.  Measured on B200, Llama-3-8B layer shapes, us (TFLOP/s), back to
 // back with cold weights, gemm_tc.cu -> here:
-//   4096 tokens: QKV 218 (945) -> 131 (1573), O 157 (875) -> 96 (1436), gate/up 1041 (924) -> 595 (1616), down 404 (1191) -> 342 (1405)
-//    512 tokens: QKV 39 (656) -> 22 (1193),   O 27 (633) -> 18 (978),   gate/up 139 (866) -> 91 (1326),   down 59 (1019) -> 50 (1198)
-//    160 tokens: QKV 40 -> 17, O 33 -> 14, gate/up 84 -> 55, down 60 -> 30 (the weights alone: 8, 5, 36, 18)
+//   4096 tokens: QKV 218 (945) -> 132 (1556), O 157 (875) -> 97 (1422), gate/up 1041 (924) -> 581 (1656), down 404 (1191) -> 359 (1339)
+//    512 tokens: QKV 39 (656) -> 21 (1246),   O 27 (633) -> 16 (1062),  gate/up 139 (866) -> 87 (1384),   down 59 (1019) -> 48 (1244)
+//    160 tokens: QKV 40 -> 16, O 33 -> 13, gate/up 84 -> 52, down 60 -> 30 (the weights alone: 8, 5, 36, 18)
 //
 // Block-scaled fp8 (MX): the same tiles with 128 K per stage; the scale factors come through the ring in runs of 512 bytes and are copied to tensor
 // memory in front of their products.  The epilogue's lane has whole blocks of 32 features of its token, so the e4m3 copy that the next product reads
 // needs no exchange between lanes.  256-wide tiles leave no columns for scale factors beside two accumulators, so these overlap by 32 columns, which
 // the epilogue takes first (128-wide tiles have none of that, but twice the rounds: gate/up of 4096 tokens 384 us against 335).  gemm_tc.cu reads
-// 128 + 256 operand rows per 128 x 256 tile and has no second accumulator.  Llama-3-8B layer shapes, us, with cold caches and the latency of a launch,
-// gemm_tc.cu -> here:
-//   4096 tokens: QKV 349 -> 91, O 282 -> 74, gate/up 1718 -> 335 (2.9 PFLOP/s), down 414 -> 178
-//    512 tokens: QKV  78 -> 27, O  53 -> 23, gate/up  290 -> 66, down 88 -> 41
-//    128 tokens: QKV  41 -> 21, O  25 -> 21, gate/up   90 -> 48, down 62 -> 31
+// 128 + 256 operand rows per 128 x 256 tile and has no second accumulator.  Llama-3-8B layer shapes, us, back to back with cold weights, gemm_tc.cu -> here:
+//   4096 tokens: QKV 223 -> 76, O 264 -> 59, gate/up 1751 -> 333 (2.9 PFLOP/s), down 461 -> 189
+//    512 tokens: QKV  50 -> 17, O  44 -> 13, gate/up  286 -> 50, down 77 -> 29
+//    128 tokens: QKV  28 -> 11, O  17 -> 12, gate/up   84 -> 32, down 55 -> 20
 // Roles (320 threads): warp 0 = TMA producer (both CTAs), warp 1 = TMEM owner, MMA issuer in the pair's even CTA, warps 2..9 = epilogue.
 #include "gemm_tc.cuh"
 

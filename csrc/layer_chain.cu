@@ -20,11 +20,10 @@
 //     factors travel behind the operands' blocks and go through TMEM (tcgen05.cp) to kind::mxf8f6f4.block_scale.
 //   * the sums of squares for the next norm are left by the CTAs that write the rows, one number per CTA and token, added in a fixed order.
 //
-// Bound: the HBM stream and, between operations, the chain of last product, exchange, store, counter, poll and first activations (3 to 5 us, of
-// which the ring hides most).  Measured on B200, replayed back to back, two Llama-3-8B layers behind 500 keys, us (kernels one by one / here): one token 191 /
-// 173, 32 tokens 221 / 200, 64 tokens 280 / 243; two Gemma-2-2B layers: one token 125 / 110, 32 tokens 146 / 134; the layers of distilgpt2, 19 tokens 231 /
-// 182, of gpt2, 64 tokens 617 / 472 (42 and 84 operations of 3 to 5 us); block-scaled fp8, two Llama-3-8B layers: one token 142 / 126, 8 tokens 143 / 131,
-// 32 tokens 169 / 166 (a conversion behind each of three products).
+// Bound: the HBM stream and, between operations, the chain of last product, exchange, store, counter, poll and first activations (3 to 4.5 us, of
+// which the ring hides most).  Measured on B200, replayed back to back, two Llama-3-8B layers behind 500 keys, us (kernels one by one / here): one token 189 /
+// 164, 32 tokens 220 / 185, 64 tokens 274 / 225; two Gemma-2-2B layers: one token 121 / 95, 32 tokens 146 / 122; the layers of gpt2, 16 tokens 489 / 291, 64
+// tokens 622 / 430 (84 operations of 3 to 5 us); block-scaled fp8, two Llama-3-8B layers: one token 144 / 112, 16 tokens 150 / 119, 32 tokens 170 / 142.
 // Roles: warps 0 and 7 = weights and pages (TMA), 1 = MMA issuer, 2..5 = epilogues and softmax, 6 = activations (TMA).
 // All waits are bounded: one that runs out raises the abort word, every other wait then ends too, and the CTAs leave.
 #include "kernels.h"

@@ -1639,8 +1639,9 @@ int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
   return B2B_CHAIN64(launch_chain_one, m, p, s);
 }
 
-// Block-scaled fp8 steps of 33 tokens and more stay with the kernels one by one: half the bytes of bf16, and the conversions of 64 tokens' results, put
-// them behind (two layers of Zephyr-7B, 40 tokens: 193.5 us one by one, 195.0 here; 64 tokens: 194.0 and 196.0).
+// Block-scaled fp8 steps of 33 tokens and more stay with the kernels one by one.  That was measured when a tile's stores held up the next one (two layers of
+// Zephyr-7B, 40 tokens: 193.5 us one by one, 195.0 here); here they would now be the faster ones (Llama-3-8B behind 500 keys, one by one / here: 40 tokens 211 / 194, 64
+// tokens 228 / 214, but 34 tokens 193 / 192, and behind 4000 keys 335 / 373).
 int layer_chain_tokens(const ChainDims& d) { return d.mx ? 32 : 64; }
 
 // clusters that are resident at once (0: the kernel cannot run here); also sets the kernels' shared memory sizes, so that a first launch may

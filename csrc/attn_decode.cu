@@ -20,7 +20,7 @@
 //
 // Bound: the cache stream.  Measured on B200 (attention_tc.cu -> here), 32 query / 8 key/value heads of 128, us: 32 sequences x 8100 keys
 // 252 -> 160 (6.6 TB/s), 32 x 500 22 -> 16, 8 x 4000 50 -> 26, one x 700 18 -> 7.6, one x 8000 26 -> 13; 8 / 4 heads of 256, 32 x 4000 91 -> 80; 12 / 12 heads of 64
-// (in pairs), 8 x 8000 107 -> 36, 32 x 8000 214 -> 124, 32 x 2000 56 -> 34, 8 x 400 9.8 -> 7.6, error 0.00230 -> 0.00217 (8 x 3000).
+// (in pairs), 8 x 8000 107 -> 36, 32 x 8000 214 -> 124, 32 x 2000 56 -> 33, 8 x 400 9.8 -> 7.3, error 0.00230 -> 0.00217 (8 x 3000).
 // Warp roles: 0 = TMA producer, 1 = TMEM owner + MMA issuer, 2..5 = softmax / correction / output.
 #include "kernels.h"
 
@@ -424,8 +424,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
     }
   }
-  if (parts > 1) {                                 // no CTA leaves while another reads its sums
-    cluster_arrive_release();
+  if (parts > 1) {                                 // no CTA leaves while another reads its sums (which have gone into what was stored: nothing to release)
+    cluster_arrive_relaxed();
     cluster_wait_acquire();
   }
   if (*abort != 0u) __nanosleep(200000);           // copies in flight land before the shared memory is given back

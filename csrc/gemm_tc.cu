@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
   float* red = reinterpret_cast<float*>(smem);   // landing zone [splitk][128 rows][CW + 4]
   const int CWP = ncol + 4;                      // row pitch in floats (16-byte aligned rows, bank spread)
   if (splitk > 1) {
-    cluster_arrive_release();
+    cluster_arrive_relaxed();                    // (nothing has been written yet that a neighbour reads)
     cluster_wait_acquire();
     if (warp >= 2) {
       const uint32_t zone = smem_u32(red) + static_cast<uint32_t>(((krank * BM + row) * CWP) * 4);

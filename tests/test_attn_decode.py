@@ -162,3 +162,20 @@ def test_a_pair_stays_apart():
         assert float((out[s, h].double() - ref[s, h]).norm() / ref[s, h].norm()) < BOUND
     other = torch.arange(64, device="cuda") != 60
     assert float((out[1, 4:6, other].double() - ref[1, 4:6, other]).norm() / ref[1, 4:6, other].norm()) < BOUND
+
+
+def test_pairs_quantised_copy():
+    """the e4m3 copy of 64-wide heads is what quantising the output gives; with split keys it is refused"""
+    lens, nq, nkv = [70, 300, 129], 8, 4
+    q, k, v, table = setup(lens, nq, nkv, 64)
+    args = (q, k, v, torch.empty_like(q), table, i32([0, 1, 2]), i32([1, 1, 1]), i32(lens))
+    opts = dict(max_q=1, n_q=nq, n_kv=nkv, head_dim=64)
+    out = ops.attention(*args, **opts)
+    q8 = torch.zeros(3, nq * 64, device="cuda", dtype=torch.float8_e4m3fn)
+    sf = torch.full((nq * 64 // 128 * 512,), 127, device="cuda", dtype=torch.uint8)
+    ops.attention(*args, **opts, fq_out=q8, fq_sf=sf, fq_bn=32)
+    want, want_sf = ops.quant_mxfp8_rows(out, 32)
+    assert torch.equal(q8.view(torch.uint8), want.view(torch.uint8))
+    assert torch.equal(ops.mx_unchunk(sf, 3, nq * 64, 32), ops.mx_unchunk(want_sf, 3, nq * 64, 32))
+    with pytest.raises(RuntimeError):
+        ops.attention(*args, **opts, splits=2, ws=torch.zeros(1 << 20, device="cuda"), fq_out=q8, fq_sf=sf, fq_bn=32)

@@ -424,10 +424,10 @@ def add(a, b, out=None):
 def attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, *, max_q, n_q, n_kv, head_dim,
               window=0, softcap=0.0, splits=1, ws=None, use_tc=-1, fq_out=None, fq_sf=None, fq_bn=0):
     """Paged-KV attention.  Prefill chunks (max_q >= 2) run on the tcgen05 flash kernel (csrc/attention_tc.cu).  Decode steps (max_q == 1) of
-    128- and 256-wide heads, and of an even number of 64-wide key/value heads, run on csrc/attn_decode.cu, which spreads the keys of few sequences
-    over clusters by itself (``splits`` and ``ws`` are not used; 32 sequences x 8.1 k keys: 160 us against 252 on the flash kernel, one sequence x 700
-    keys: 7.6 against 17.6).  Other 64-wide heads: the flash kernel with one-token query blocks, ``splits`` parts of the keys merged by a second
-    kernel.  ``use_tc`` 0: the CUDA-core kernel."""
+    128- and 256-wide heads, and of an even number of 64-wide key/value heads with 1, 2, 4 or 8 query heads each, run on csrc/attn_decode.cu, which
+    spreads the keys of few sequences over clusters by itself (``splits`` and ``ws`` are not used; 32 sequences x 8.1 k keys: 160 us against 252 on the
+    flash kernel, one sequence x 700 keys: 7.6 against 17.6).  An odd number of 64-wide heads in such groups: the flash kernel with one-token query
+    blocks, ``splits`` parts of the keys merged by a second kernel.  64-wide heads in other groups, and ``use_tc`` 0: the CUDA-core kernel."""
     if use_tc < 0 and max_q == 1:
         use_tc = 1
     n = native().attention(q, k_cache, v_cache, out, block_table, q_start, q_len, kv_len, ws, max_q, n_q, n_kv, head_dim,

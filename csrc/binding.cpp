@@ -476,8 +476,7 @@ int64_t attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache,
   }
   if (want_tc && max_q == 1 && b2b::attn_decode_supported(static_cast<int>(n_q), static_cast<int>(n_kv), static_cast<int>(head_dim))) {
     // (64-wide heads: the e4m3 copy where the flash kernel, which takes an odd number of them, leaves one, too)
-    TORCH_CHECK(fq_out == 0 || head_dim != 64 || (splits <= 1 && b2b::attention_tc_supported(static_cast<int>(n_q), static_cast<int>(n_kv), 64)),
-                "fused output quantisation needs the tcgen05 attention kernel without split keys");
+    TORCH_CHECK(fq_out == 0 || head_dim != 64 || splits <= 1, "fused output quantisation needs the tcgen05 attention kernel without split keys");
     check(b2b::launch_attn_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(),
                                   reinterpret_cast<const int*>(block_table.data_ptr()), reinterpret_cast<const int*>(q_start.data_ptr()),
                                   reinterpret_cast<const int*>(q_len.data_ptr()), reinterpret_cast<const int*>(kv_len.data_ptr()), seqs,

@@ -179,3 +179,21 @@ def test_pairs_quantised_copy():
     assert torch.equal(ops.mx_unchunk(sf, 3, nq * 64, 32), ops.mx_unchunk(want_sf, 3, nq * 64, 32))
     with pytest.raises(RuntimeError):
         ops.attention(*args, **opts, splits=2, ws=torch.zeros(1 << 20, device="cuda"), fq_out=q8, fq_sf=sf, fq_bn=32)
+
+
+@pytest.mark.parametrize("nq,nkv", [(6, 2), (20, 4), (12, 2), (14, 2)])
+def test_other_groups_of_64_keep_fp32_weights(nq, nkv):
+    """64-wide heads in groups that the tensor-core kernels with bf16 weights did not take in pairs: the CUDA-core kernel's result, bit for bit, whole and with
+    split keys, and no e4m3 copy"""
+    lens = [70, 3000, 129, 1]
+    q, k, v, table = setup(lens, nq, nkv, 64)
+    args = (table, i32([0, 1, 2, 3]), i32([1] * 4), i32(lens))
+    opts = dict(max_q=1, n_q=nq, n_kv=nkv, head_dim=64)
+    for split in (dict(), dict(splits=4, ws=torch.zeros(1 << 20, device="cuda"))):
+        out, cuda_core = (ops.attention(q, k, v, torch.zeros_like(q), *args, **opts, **split, use_tc=tc) for tc in (-1, 0))
+        assert torch.equal(out, cuda_core)
+        ref = reference(q, k, v, table, lens, nq, nkv, 64, 0, 0.0)
+        assert float((out.double() - ref).norm() / ref.norm()) < 0.0019     # (the rounding of the result; bf16 weights add as much again)
+    with pytest.raises(RuntimeError):
+        ops.attention(q, k, v, torch.zeros_like(q), *args, **opts, fq_out=torch.zeros(4, nq * 64, device="cuda", dtype=torch.float8_e4m3fn),
+                      fq_sf=torch.zeros(1 << 14, device="cuda", dtype=torch.uint8), fq_bn=32)

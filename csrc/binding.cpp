@@ -29,6 +29,9 @@ inline T* ptr_or_null(const OptT& t) {
 template <typename T>
 inline T* as_ptr(int64_t addr) { return reinterpret_cast<T*>(static_cast<uintptr_t>(addr)); }
 
+// Scale factors of tokens come in tiles of up to 128 tokens with 512 bytes per 128 K, or of up to 256 with 1024: nothing holds more of them
+constexpr int64_t MX_MAX_TILE = 256;
+
 void check_bf16(const Tensor& t, const char* name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(), name,
               " must be a contiguous CUDA bf16 tensor");
@@ -58,7 +61,7 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
     TORCH_CHECK(mx == sfb.has_value(), "MX fp8 gemm needs both sfa and sfb");
     if (mx) {
       const int64_t nkc = w.size(1) / 128, chunk = bn > 128 ? 1024 : 512;
-      TORCH_CHECK(w.size(1) % 128 == 0 && bn >= 32, "MX fp8 gemm: K must be a multiple of 128 and bn >= 32");
+      TORCH_CHECK(w.size(1) % 128 == 0 && bn >= 32 && bn <= MX_MAX_TILE, "MX fp8 gemm: K must be a multiple of 128 and bn 32 to 256");
       TORCH_CHECK(sfa->scalar_type() == at::kByte && sfa->is_contiguous() && sfa->numel() >= (w.size(0) / 128) * nkc * 512,
                   "MX fp8 gemm: sfa too small");
       TORCH_CHECK(sfb->scalar_type() == at::kByte && sfb->is_contiguous() &&
@@ -96,8 +99,8 @@ void gemm(const Tensor& w, const Tensor& x, int64_t out_ptr, int64_t ld_out, int
   p.sumsq_out = as_ptr<float>(sumsq_out);
   p.zero_buf = as_ptr<float>(zero_buf);
   p.sumsq = as_ptr<const float>(sumsq);
-  TORCH_CHECK(!p.q_out8 || (p.q_sf && p.sfa && p.ld_q % 128 == 0 && (epi == b2b::EPI_RESIDUAL || epi == b2b::EPI_GLU)),
-              "fused output quantisation: MX GEMMs with residual / GLU epilogues, scale-factor buffer, row stride multiple of 128");
+  TORCH_CHECK(!p.q_out8 || (p.q_sf && p.sfa && p.ld_q % 128 == 0 && q_bn <= MX_MAX_TILE && (epi == b2b::EPI_RESIDUAL || epi == b2b::EPI_GLU)),
+              "fused output quantisation: MX GEMMs with residual / GLU epilogues, scale-factor buffer in tiles of up to 256, row stride multiple of 128");
   p.residual = as_ptr<const __nv_bfloat16>(residual_ptr);
   p.ld_res = static_cast<int>(ld_res);
   p.bias = ptr_or_null<const float>(bias);
@@ -237,6 +240,7 @@ void quant_mxfp8_rows(const Tensor& x, const Tensor& q, const Tensor& sf, int64_
   c10::cuda::CUDAGuard guard(x.device());
   const int h = static_cast<int>(x.size(-1));
   const int tokens = static_cast<int>(x.numel() / h);
+  TORCH_CHECK(bn > 0 && bn <= MX_MAX_TILE, "quant_mxfp8_rows: scale factors come in tiles of up to 256 tokens");
   TORCH_CHECK(sf.numel() >= ((tokens + bn - 1) / bn) * (h / 128) * (bn > 128 ? 1024 : 512), "quant_mxfp8_rows: sf too small");
   check(b2b::launch_quant_mxfp8_rows(x.data_ptr(), q.data_ptr(), sf.data_ptr(), tokens, h, static_cast<int>(bn),
                                      static_cast<float>(eps), static_cast<int>(with_rms), ptr_or_null<float>(sumsq_out),
@@ -465,6 +469,7 @@ int64_t attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_cache,
   check_bf16(q, "q");
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(block_table.scalar_type() == at::kInt && q_len.scalar_type() == at::kInt, "int32 metadata expected");
+  TORCH_CHECK(fq_out == 0 || fq_bn <= MX_MAX_TILE, "fused output quantisation: scale factors come in tiles of up to 256 tokens");
   const int seqs = static_cast<int>(q_len.size(0));
   // use_tc: -1 = by query-chunk length (prefill chunks), 1 = force the tcgen05 kernel (decode: one-token query blocks,
   // the GQA group stacked into the MMA rows), 0 = force the CUDA-core kernel (split-KV decode of few sequences)

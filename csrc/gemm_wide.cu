@@ -815,10 +815,10 @@ bool gemm_wide_supported(const GemmParams& p) {
   const int ke = mx ? 128 : WK;
   if (p.n_out % 128 != 0 || p.k % ke != 0 || p.k < 2 * ke || p.m_tok <= 0) return false;
   if (mx) {
-    if (p.epi == EPI_GELU || p.w_scale || p.sfb == nullptr || p.sf_bn < 128) return false;
+    if (p.epi == EPI_GELU || p.w_scale || p.sfb == nullptr || (p.sf_bn != 128 && p.sf_bn != 256)) return false;      // (runs of 128 tokens, alone or side by side)
     if ((reinterpret_cast<uintptr_t>(p.sfa) | reinterpret_cast<uintptr_t>(p.sfb)) & 15) return false;
     if (p.q_out8 && (((reinterpret_cast<uintptr_t>(p.q_out8) | static_cast<uintptr_t>(p.ld_q)) & 15) || (reinterpret_cast<uintptr_t>(p.q_sf) & 1))) return false;
-    if (p.q_out8 && p.q_bn < 128) return false;
+    if (p.q_out8 && p.q_bn != 128 && p.q_bn != 256) return false;
   }
   if (p.epi == EPI_GELU && p.act_gelu == 4) return false;
   if (p.bias && (reinterpret_cast<uintptr_t>(p.bias) & 15)) return false;

@@ -246,3 +246,22 @@ def test_block_scaled(tile, split, m, n, k):
         near(quantised(lambda **q: ops.gemm(wq, xq, epi=ops.EPI_GLU, sumsq=ss, eps=1e-5, out=torch.empty(m, n // 2, device="cuda", dtype=torch.bfloat16),
                                             **q, **sf), n // 2), (torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]).flatten(1))
     assert ops.native().gemm_wide_gave_up() == 0
+
+
+@pytest.mark.parametrize("bn", [192, 512, 65536 + 128])
+def test_unknown_token_tiles_are_refused(bn):
+    """scale factors of tokens are read in runs of 128, alone or two side by side; a call that names any other tile is refused by the host, with the kernel's
+    tile named or not, and so are copies that would be written in larger tiles"""
+    m, n, k = 300, 256, 1024
+    wq, sfa = ops.quantize_weight_mxfp8(bf(n, k))
+    xq = torch.zeros(m, k, device="cuda", dtype=torch.float8_e4m3fn)
+    sf = torch.full((((m + 127) // 128 + 1) * (k // 128) * 1024,), 127, device="cuda", dtype=torch.uint8)
+    for tile in (dict(wide_tile=256), dict(wide_tile=1), dict()):
+        with pytest.raises(RuntimeError):
+            ops.gemm(wq, xq, sfa=sfa, sfb=sf, bn=bn, **tile)
+    if bn > 256:
+        with pytest.raises(RuntimeError):
+            ops.quant_mxfp8_rows(bf(m, k), bn)
+        with pytest.raises(RuntimeError):
+            ops.gemm(wq, xq, sfa=sfa, sfb=sf, bn=128, epi=ops.EPI_RESIDUAL, residual=bf(m, n), fq_out=torch.zeros(m, n, device="cuda", dtype=torch.float8_e4m3fn),
+                     fq_sf=sf, fq_bn=bn)

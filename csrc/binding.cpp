@@ -8,6 +8,7 @@
 #include "kernels.h"
 #include "launch.cuh"
 #include "peer.h"
+#include "wide_plan.cuh"
 
 using at::Tensor;
 using OptT = c10::optional<Tensor>;
@@ -1225,6 +1226,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_decode_gave_up", &b2b::attn_decode_gave_up);
   m.def("gemm_max_splitk", &gemm_max_splitk);
   m.def("gemm_wide_gave_up", &b2b::gemm_wide_gave_up);
+  // per pair of CTAs and item: (tile, its accumulator's readers arrive for a later item)
+  m.def("gemm_wide_plan", [](int tok_tiles, int feature_tiles, int nkb, int pairs, bool may_split, bool overlap) {
+    const b2b::WidePlan plan(tok_tiles, feature_tiles, nkb, pairs, may_split);
+    std::vector<std::vector<std::pair<int, bool>>> items(pairs);
+    b2b::WideItem it;
+    for (int pair = 0; pair < pairs; ++pair)
+      for (int i = 0; plan.get(i, pair, it); ++i) items[pair].emplace_back(it.t, !it.split && plan.awaited(i, pair, b2b::wide_gap(overlap)));
+    return items;
+  });
   m.def("init_kernels", &init_kernels);
   m.def("set_pdl", &set_pdl);
   m.def("get_pdl", &get_pdl);

@@ -47,6 +47,7 @@
 #include "kernels.h"
 #include "launch.cuh"
 #include "tmem.cuh"
+#include "wide_plan.cuh"
 
 namespace b2b {
 
@@ -166,32 +167,6 @@ __device__ __forceinline__ void wait_downstream(const GemmParams& p) {
   if (p.free_flag != nullptr) wait_flag_ge(p.free_flag, *reinterpret_cast<const volatile uint32_t*>(p.signal_epoch) - p.free_lag);
 }
 
-// what a pair works on: tile `t`, k-blocks [kb0, kb1), `split`: the other pair of the cluster has the rest of K
-struct Item {
-  int t, kb0, kb1;
-  bool split;
-};
-struct Plan {
-  int tiles, tok_tiles, nkb, pairs, full, rest;
-  bool split;
-  __device__ __forceinline__ bool get(int i, int pair, Item& it) const {
-    const int t = pair + i * pairs;
-    if (t < full) {
-      it = {t, 0, nkb, false};
-      return true;
-    }
-    if (i != full / pairs) return false;
-    if (split) {
-      if ((pair >> 1) >= rest) return false;
-      const int half = nkb / 2;
-      it = {full + (pair >> 1), (pair & 1) ? half : 0, (pair & 1) ? nkb : half, true};
-      return true;
-    }
-    it = {t, 0, nkb, false};
-    return t < tiles;
-  }
-};
-
 struct NoMaps {};
 struct SfMaps {                            // scale factors as rows of 512 bytes
   CUtensorMap w, x;
@@ -222,14 +197,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   const uint32_t lead = crank & ~1u;
   const int pair = static_cast<int>(blockIdx.x >> 1);
 
-  Plan plan;
-  plan.tok_tiles = (p.m_tok + 2 * WM - 1) / (2 * WM);
-  plan.tiles = plan.tok_tiles * ((p.n_out + BN - 1) / BN);
-  plan.nkb = p.k / KE;
-  plan.pairs = static_cast<int>(gridDim.x >> 1);
-  plan.full = plan.tiles / plan.pairs * plan.pairs;
-  plan.rest = plan.tiles - plan.full;
-  plan.split = allow_split != 0 && plan.rest > 0 && plan.rest <= plan.pairs / 2;      // (clusters of four)
+  const WidePlan plan((p.m_tok + 2 * WM - 1) / (2 * WM), (p.n_out + BN - 1) / BN, p.k / KE, static_cast<int>(gridDim.x >> 1), allow_split != 0);
+  constexpr int GAP = wide_gap(Cfg::kShared);
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_w);
@@ -264,7 +233,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   pdl_launch_dependents();
 
   bool ok = true;
-  Item it;
+  WideItem it;
   auto fill = [&](uint32_t n, int kb, int n0, int m0, bool w, bool x) {       // stage n of this CTA
     const uint32_t s = n % STAGES;
     uint8_t* st = smem + s * Cfg::kStageBytes;
@@ -307,6 +276,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           fill(n, kb, n0, m0, true, true);
         }
       }
+      // the odd CTA hears of its stages from the even one's products: of the last ones, too, before it leaves
+      for (uint32_t j = n > STAGES ? n - STAGES : 0; ok && j < n; ++j) ok = ma_wait(&empty_bar[j % STAGES], j / STAGES & 1u, abort);
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------------------------------------------- MMA issuer
@@ -321,11 +292,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           wait_upstream(p);
         }
         if (i == (Cfg::kShared ? 1 : 2)) wait_downstream(p);
-        if constexpr (Cfg::kShared) {              // the tile before has left the shared columns, the one before that all of them
-          if (i > 0 && !(ok = ma_wait(&acc_empty[b ^ 1u], (i - 1) >> 1 & 1, abort))) break;
-        } else {
-          if (!(ok = ma_wait(&acc_empty[b], (i >> 1 & 1) ^ 1u, abort))) break;
-        }
+        // (overlapping accumulators: the tile before has left the shared columns, and the one before that all of them)
+        if (i >= GAP && !(ok = ma_wait(&acc_empty[(i - GAP) & 1], (i - GAP) >> 1 & 1, abort))) break;
         tc_fence_after();
         for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
           const uint32_t s = n % STAGES;
@@ -655,14 +623,14 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster_read(mapa_smem(smem_u32(&acc_empty[b]), lead));
+        if (lane == 0 && plan.awaited(i, pair, GAP)) arrive_cluster_read(mapa_smem(smem_u32(&acc_empty[b]), lead));
         finish(lanes + b * Cfg::kAccStride, m0, n0, 0, BN, nullptr);
         hold_c = -1;
       } else {
         finish(lanes + b * BN, m0, n0, 0, BN, nullptr);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster_read(mapa_smem(smem_u32(&acc_empty[b]), lead));
+        if (lane == 0 && plan.awaited(i, pair, GAP)) arrive_cluster_read(mapa_smem(smem_u32(&acc_empty[b]), lead));
       }
     }
     if (plan.split) {
@@ -709,7 +677,9 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (*abort != 0u) __nanosleep(200000);           // copies in flight land before the shared memory is given back
   tc_fence_before();
   __syncthreads();
-  cluster_arrive_relaxed();                        // no CTA leaves while another may still arrive on its barriers or read its operands
+  // No CTA leaves while another may still read its operands (these products have retired) or arrive on its barriers.  All arrivals from another CTA are waited for:
+  // acc_empty by the even CTA's products (WidePlan::awaited), stages and accumulators by the producer and the epilogue.  So there is nothing to release.
+  cluster_arrive_relaxed();
   cluster_wait_acquire();
   if (warp == 1) {
     tc_fence_after();

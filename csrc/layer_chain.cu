@@ -654,6 +654,10 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
                 if (++s == x_slots) { s = 0; ph ^= 1u; }
               }
           } else if (!LN && op == OP_ATT) {
+            // Queries land where the partial sums and the exchange of gate and up lay (plain loads and stores, complete with the operations in front), which is
+            // the only target of that kind: the other operations do without this fence (0.2 us each; here it hides, two layers of one token 165.3 us without
+            // and with it).
+            fence_proxy_async_smem();
 #pragma unroll 1
             for (int j = item0; ok && j < items; j += item_step) {
               const LcItem it = lc_item(p, kvlen_s, window, j, part);

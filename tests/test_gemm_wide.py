@@ -265,3 +265,117 @@ def test_unknown_token_tiles_are_refused(bn):
         with pytest.raises(RuntimeError):
             ops.gemm(wq, xq, sfa=sfa, sfb=sf, bn=128, epi=ops.EPI_RESIDUAL, residual=bf(m, n), fq_out=torch.zeros(m, n, device="cuda", dtype=torch.float8_e4m3fn),
                      fq_sf=sf, fq_bn=bn)
+
+
+def mx_operands(m, n, k):
+    """block-scaled weights and tokens with the tokens' sums of squares, and their exact product behind the norm"""
+    wq, sfa = ops.quantize_weight_mxfp8(spread(n, k, 1))
+    bn = ops.pick_bn_mx(m)
+    ss = torch.zeros(m, device="cuda")
+    xq, sfb = ops.quant_mxfp8_rows(spread(m, k, 2), bn, sumsq_out=ss)
+    ref = ops.mx_dequant(xq, ops.mx_unchunk(sfb, m, k, bn)).double() @ ops.mx_dequant(wq, ops.mx_unchunk(sfa, n, k)).double().t()
+    return wq, xq, dict(sfa=sfa, sfb=sfb, sumsq=ss, eps=1e-5), ref * (ss.double() / k + 1e-5).rsqrt()[:, None], bn
+
+
+def mx_copy(m, width, bn):
+    """room for an e4m3 copy and its scale factors"""
+    return (torch.zeros(m, width, device="cuda", dtype=torch.float8_e4m3fn),
+            torch.full(((m + bn - 1) // bn * (width // 128) * (bn // 128) * 512,), 127, device="cuda", dtype=torch.uint8))
+
+
+def is_copy(q8, q_sf, out, bn):
+    want, want_sf = ops.quant_mxfp8_rows(out, bn)
+    assert torch.equal(q8.view(torch.uint8), want.view(torch.uint8))
+    assert torch.equal(ops.mx_unchunk(q_sf, *out.shape, bn), ops.mx_unchunk(want_sf, *out.shape, bn))
+
+
+# rotary pairs, cache rows and the norm of block-scaled tokens: every prompt of more than 64 tokens goes through them.  k 1152: 9 stages, halves of 4 and 5;
+# 520 tokens: runs of scale factors in tiles of 256
+@pytest.mark.parametrize("tile,split", MX_TILES)
+@pytest.mark.parametrize("hd,nq,nkv,m", [(128, 3, 1, 300), (64, 6, 2, 129), (256, 3, 2, 520), (32, 20, 4, 65)])
+def test_block_scaled_qkv(tile, split, hd, nq, nkv, m):
+    theta, k, n = 10000.0, 1152, (nq + 2 * nkv) * hd
+    wq, xq, mx, ref, _ = mx_operands(m, n, k)
+    pages = m // ops.PAGE + 2
+    pos = torch.randperm(600, device="cuda")[:m].int()
+    slots = torch.randperm(pages * ops.PAGE, device="cuda")[:m].int()
+    slots[::5] = -1
+    kc = torch.zeros(pages, ops.PAGE, nkv, hd, device="cuda", dtype=torch.bfloat16)
+    vc, q = torch.zeros_like(kc), torch.zeros(m, nq * hd, device="cuda", dtype=torch.bfloat16)
+    ops.gemm(wq, xq, epi=ops.EPI_QKV_ROPE, q_out=q, k_cache=kc, v_cache=vc, positions=pos, slots=slots, n_q_heads=nq, n_kv_heads=nkv, head_dim=hd,
+             rope_theta=theta, q_scale=0.25, **mx, **(dict(wide_tile=tile, wide_split=split) if tile else {}))
+    y = ref.view(m, -1, hd)
+    ang = pos.double()[:, None] * theta ** (-torch.arange(0, hd, 2, device="cuda", dtype=torch.float64) / hd)
+    cos, sin = ang.cos()[:, None], ang.sin()[:, None]
+    a, b = y[..., 0::2], y[..., 1::2]
+    turned = torch.stack([a * cos - b * sin, b * cos + a * sin], -1).flatten(-2)
+    near(q.view(m, nq, hd), turned[:, :nq] * 0.25)
+    keep = slots >= 0
+    for cache, rows in ((kc, turned[:, nq:nq + nkv]), (vc, y[:, nq + nkv:])):
+        want = torch.zeros(pages * ops.PAGE, nkv, hd, device="cuda", dtype=torch.float64)
+        want[slots[keep].long()] = rows[keep]
+        got = cache.view(-1, nkv, hd)
+        near(got, want)
+        assert not got[want.flatten(1).norm(dim=1) == 0].any()
+    assert ops.native().gemm_wide_gave_up() == 0
+
+
+@pytest.mark.parametrize("gelu", [0, 1])
+@pytest.mark.parametrize("m,n,k,tile", [(70, 512, 256, 0), (300, 768, 1024, 256), (1000, 18944, 256, 256)])
+def test_block_scaled_gate_up_without_rows(m, n, k, tile, gelu):
+    """a product whose only reader takes the e4m3 copy writes no bf16 rows: the copy is that of the call which does"""
+    wq, xq, mx, ref, bn = mx_operands(m, n, k)
+    kw = dict(epi=ops.EPI_GLU, act_gelu=gelu, **mx, **(dict(wide_tile=tile, wide_split=0) if tile else {}))
+    out = ops.gemm(wq, xq, **kw)
+    g, u = (ref.view(m, n // 128, 2, 64)[:, :, i] for i in (0, 1))
+    act = torch.nn.functional.gelu(g, approximate="tanh") if gelu else torch.nn.functional.silu(g)
+    near(out, (act * u).flatten(1))
+    q8, q_sf = mx_copy(m, n // 2, bn)
+    ops.gemm(wq, xq, fq_out=q8, fq_sf=q_sf, fq_bn=bn, no_out=True, **kw)
+    is_copy(q8, q_sf, out, bn)
+    assert ops.native().gemm_wide_gave_up() == 0
+
+
+def _quantised_hop(m, n, k, flags):
+    """a product between two neighbours that hand over block-scaled rows: it waits for the upstream one's, and leaves its rows, their e4m3 copy and their sums
+    of squares in the downstream one's memory"""
+    wq, xq, mx, ref, bn = mx_operands(m, n, k)
+    res = bf(m, n)
+    word = torch.zeros(8, device="cuda", dtype=torch.int32)      # in epoch, out flag, out epoch, done, ack
+    at = [word.data_ptr() + 4 * i for i in range(8)]
+    out, (q8, q_sf) = torch.zeros(m, n, device="cuda", dtype=torch.bfloat16), mx_copy(m, n, bn)
+    sums, clear = torch.zeros(m, device="cuda"), torch.ones(m, device="cuda")
+    word[2] = 1                                                  # one payload is out already: the next one waits for its release
+    torch.cuda.synchronize()
+    ops.gemm(wq, xq, out=out, epi=ops.EPI_RESIDUAL, residual=res, wait_flag=flags.data_ptr(), wait_epoch=at[0], signal_flag=at[1], signal_epoch=at[2],
+             done_counter=at[3], bump_epoch=at[0], ack_flag=at[4], free_flag=flags.data_ptr() + 64, free_lag=0, fq_out=q8, fq_sf=q_sf, fq_bn=bn,
+             sumsq_out=sums, zero_buf=clear, wide_tile=256, wide_split=0, **mx)
+
+    def arrived():
+        near(out, ref + res.double())
+        is_copy(q8, q_sf, out, bn)
+        near(sums, out.double().pow(2).sum(1), 1e-5)
+        assert not clear.any()
+    return arrived, word
+
+
+@pytest.mark.parametrize("m,n", [(200, 512), (1000, 18944)])     # one tile per pair and four, whose accumulators overlap
+def test_quantised_hop(m, n, abort_word):
+    """both neighbours are there, and then both are late, each by more than a bounded wait of a kernel lasts"""
+    abort = abort_word(30000)
+    before = ops.native().gemm_wide_gave_up()
+    flags = torch.ones(32, dtype=torch.int32).pin_memory()
+    arrived, word = _quantised_hop(m, n, 256, flags)
+    torch.cuda.synchronize()
+    arrived()
+    assert word.tolist() == [1, 2, 2, 0, 1, 0, 0, 0]
+    flags.zero_()
+    arrived, word = _quantised_hop(m, n, 256, flags)
+    time.sleep(4.5)                                              # (2^24 polls last 1 to 4 s)
+    flags[0] = 1
+    time.sleep(4.5)
+    flags[16] = 1
+    torch.cuda.synchronize()
+    arrived()
+    assert word.tolist() == [1, 2, 2, 0, 1, 0, 0, 0]
+    assert ops.native().gemm_wide_gave_up() == before and int(abort[0]) == 0

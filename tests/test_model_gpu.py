@@ -7,6 +7,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+from bee2bee_b200 import ops  # noqa: E402
 from bee2bee_b200.engine.core import Engine, SamplingParams  # noqa: E402
 from bee2bee_b200.engine.runner import GpuRunner, SeqInit  # noqa: E402
 from bee2bee_b200.models.config import resolve_config  # noqa: E402
@@ -120,6 +121,39 @@ def test_piece_fp8_close_to_oracle(name, quant):
                 assert err < 0.2, f"{name} step {step} seq {b}: rel err {err}"
                 cos = torch.nn.functional.cosine_similarity(got[b].float(), ref.float(), dim=0).item()
                 assert cos > 0.98, cos
+    runner.close()
+
+
+@pytest.mark.parametrize("name", ["tiny-llama", "tiny-mistral"])
+def test_block_scaled_prompt_close_to_oracle(name, monkeypatch):
+    """block-scaled prompts of more than 64 tokens run on the CTA-pair products: the steps that read their keys and values stay within fp8 noise of the oracle"""
+    cfg = resolve_config(name)
+    wide, use = [], ops.use_wide
+    monkeypatch.setattr(ops, "use_wide", lambda n, t, mx=False: wide.append((t, mx)) or use(n, t, mx))
+    runner = GpuRunner(cfg, "", 0, 1, torch.device("cuda:0"), max_batch=4, groups=1, max_seq_len=512, max_prefill_tokens=512, seed=0, quant="mxfp8")
+    oracle = _oracle(cfg)
+    V = cfg.vocab_size
+    prompts = [[(7 * i + 5) % V for i in range(150)], [(11 * i + 3) % V for i in range(61)]]
+    seqs = [SeqInit(slot=i, prompt=p, pages=list(range(1 + 8 * i, 9 + 8 * i)), temperature=0.0, top_p=1.0, repetition_penalty=1.0, seed=i)
+            for i, p in enumerate(prompts)]
+    runner.prefill(seqs)
+    assert any(mx and t > 128 for t, mx in wide)
+    caches = [oracle.new_cache() for _ in seqs]
+    with torch.no_grad():
+        for s, c in zip(seqs, caches):
+            oracle.forward(torch.tensor([s.prompt], device="cuda"), torch.arange(len(s.prompt), device="cuda")[None], c)
+    for step in range(3):
+        fed = runner.tokens[:2].tolist()
+        runner.decode(1)
+        runner.sync()
+        got = runner.piece.logits[:2, :V]
+        with torch.no_grad():
+            for b in range(2):
+                ref = oracle.forward(torch.tensor([[fed[b]]], device="cuda"), torch.tensor([[len(seqs[b].prompt) + step]], device="cuda"), caches[b])[0, -1]
+                err = _rel_err(got[b], ref)
+                assert err < 0.2, f"{name} step {step} seq {b}: rel err {err}"
+                assert torch.nn.functional.cosine_similarity(got[b].float(), ref.float(), dim=0).item() > 0.98
+    assert ops.native().gemm_wide_gave_up() == 0
     runner.close()
 
 

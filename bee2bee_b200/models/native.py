@@ -103,7 +103,9 @@ def chain_attention_us(seqs: int, n_kv: int, head_dim: int, keys: int, window: i
 
     A (sequence, key/value head) is an item.  The persistent kernel has one CTA per SM on ``ctas`` SMs and shares an item among at most 4 of them; items that
     do not fill its last round leave most CTAs waiting for the few that walk one more (17 to 24 Llama-3-8B sequences behind 8000 keys: 20 to 37 us per layer
-    lost).  The other kernel shares an item among up to 8 CTAs and starts new ones as the first end."""
+    lost).  The other kernel shares an item among up to 8 CTAs and starts new ones as the first end.  (It takes smaller clusters where those of 8 or 4 do not
+    all fit at once, ``dec_parts``: 9 Llama-3-8B sequences have two CTAs each, not four, 4 Gemma-2-2B sequences four, not eight.  The model leaves that out.  It
+    would move steps of 9 sequences alone, behind more than 10 thousand keys, and the wrong way: 321 us one by one, 305 in the persistent kernel.)"""
     if window > 0:
         keys = min(keys, window + 127)
     items, unit, tiles = seqs * n_kv, head_dim / 128, (keys + 127) // 128
@@ -124,8 +126,10 @@ def chain_attention_us(seqs: int, n_kv: int, head_dim: int, keys: int, window: i
 def chain_key_limit(tokens: int, heads: int, ctas: int) -> int:
     """LayerNorm models: the most keys that a token may see for the persistent kernel to be the faster one.  Its attention reads all keys of a (token, head) for
     that one alone, on a warp up to 128 keys and on a CTA beyond; the kernel of its own reads them once for 16 tokens.  gpt2, us per layer gained, by
-    rounds of (token, head) over the CTAs: one round 1 at 900 keys; two 6 to 9 at 300, 5 to -2 at 500, -4 to -22 at 900; three (32 tokens) 5 at 120, 3 at
-    200, -1 at 300; more (64) 10 to 13 at 60, 0 at 120."""
+    rounds of (token, head) over the CTAs and keys: one round 1 at 900; two 6 to 9 at 260 to 300, 3 to -2 at 470 to 500, -3 to -22 at 900; three 7 at 128, 3 at
+    184 to 232, -1 to -2 at 300 to 330; four 10 at 148, 6 at 204, 4 at 264, -1 at 344; more (64 tokens) 16 at 64, 10 to 0 at 121 to 124, -1 at 184.  The limits of two to
+    four rounds are those of an earlier, slower form of the persistent kernel and lie below these crossings: a call between them goes one by one and loses what
+    is written here."""
     rounds = -(-tokens * heads // ctas)
     return 1024 if rounds <= 1 else (256 if rounds == 2 else (128 if rounds <= 4 else 112))
 

@@ -12,9 +12,9 @@
 // q is pre-scaled by 1/sqrt(d) and rotated by the QKV GEMM epilogue; K is rotated when appended.
 //
 // Bound: the softmax warps' issue slots and latencies beside the hardware exponential (64 per row and tile, 47 % of its rate at T = 4096).
-// Measured on B200, causal, 32 / 8 heads of 128: 4096 tokens 169 -> 135 us (1019 TFLOP/s) with the query blocks of all heads in one
+// Measured on B200, causal, 32 / 8 heads of 128: 4096 tokens 169 -> 135 us (1019 TFLOP/s; 127 at best, 136 for a long time) with the query blocks of all heads in one
 // longest-first order, packed multiply-adds for the exponents and sums, and four chains instead of one for the row maximum; 8 / 4 heads of 256 with
-// capped scores 110 -> 80 us.
+// capped scores 110 -> 80 us (77 at best, 82 for a long time).
 //
 // Layouts: q/out [tokens, n_q, D]; K/V cache [pages, 64, n_kv, D]; block_table [seqs, max_pages].
 // Reference parity: torch SDPA under `transformers.generate` (bee2bee/hf.py:42-43).
@@ -105,7 +105,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// EXPERIMENTAL (P_TMEM variant, not yet run on hardware): D[tmem] (+)= A[tmem] * B[smem] -- the A operand (P) is read
+// P_TMEM: D[tmem] (+)= A[tmem] * B[smem] -- the A operand (P) is read
 // from tensor memory: lane = row, 16-bit elements packed two per 32-bit column (element 2j in the low half).
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                              uint32_t accumulate) {
@@ -190,7 +190,7 @@ struct AtcCfg {
   static constexpr int kMinCtas = (D <= 128) ? 2 : 1;                  // two CTAs per SM: one's softmax hides the other's MMAs
 };
 
-// P_TMEM (EXPERIMENTAL, default false): P stays in tensor memory (written over the first BKV/2 columns of the S buffer
+// P_TMEM (the default): P stays in tensor memory (written over the first BKV/2 columns of the S buffer
 // it was computed from) and feeds the PV MMA as a TMEM A operand; no P tile in shared memory, no fence.proxy.async.
 // Q32: the options of the hybrid graphs (see AttnTcParams); P_TMEM only.
 template <int D, bool SOFTCAP, bool P_TMEM, bool Q32>

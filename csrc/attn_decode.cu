@@ -470,7 +470,8 @@ int dec_clusters(int size) {
 // CTAs of a cluster: they share the keys of a (sequence, key/value head) while that still adds resident CTAs (two per SM at 128 channels) and every CTA can have a
 // tile and all clusters fit at once.  256-wide heads, 4 sequences of 8000 / 2000 keys: 16 clusters of eight ran in two rounds (37.7 / 14.6 us), in clusters of four
 // 27.7 / 10.0.  With two CTAs on an SM 32 clusters of eight and 64 of four ran at once (4 and 8 sequences of 8 heads), 36 and 72 did not (6 and 12 sequences of 6 pairs, 2000
-// keys: 15.0 against 10.0 us in clusters of four, 23.9 against 17.4 in clusters of two).
+// keys: 15.0 against 10.0 us in clusters of four, 23.9 against 17.4 in clusters of two).  Those two numbers are of a B200's 148 SMs and not asked of the device:
+// cudaOccupancyMaxActiveClusters counts fewer of these clusters than run at once, and by it 16 of eight became fours (2 sequences of 8000 keys 16.7 -> 21.7 us).
 int dec_parts(int items, int tiles, bool one_per_sm) {
   const int slots = one_per_sm ? 148 : 296;
   int parts = 1;

@@ -254,6 +254,12 @@ __device__ __forceinline__ void cluster_arrive_release() {
 __device__ __forceinline__ void cluster_arrive_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
 }
+// An arrival on a barrier of a neighbour's (mapped address) which only says that memory has been READ.  A release to the cluster would wait until every earlier
+// store of the thread has arrived in L2 (1 to 2.5 us per tile of a decode product while the weights stream).  Stores into what the neighbour writes next have to be
+// complete by other means: read back behind a barrier of the CTA, as the exchange of gate and up in layer_chain.cu is.
+__device__ __forceinline__ void arrive_cluster_read(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void cluster_wait_acquire() {
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }

@@ -23,14 +23,15 @@
 //
 // Bound: tensor pipe (98 % active while a tile runs) and the power cap.  Measured on B200, Llama-3-8B layer shapes, us (TFLOP/s), back to
 // back with cold weights, gemm_tc.cu -> here:
-//   4096 tokens: QKV 218 (945) -> 132 (1556), O 157 (875) -> 97 (1422), gate/up 1041 (924) -> 581 (1656), down 404 (1191) -> 359 (1339)
+//   4096 tokens: QKV 218 (945) -> 130 (1586), O 157 (875) -> 95 (1447), gate/up 1041 (924) -> 581 (1656), down 404 (1191) -> 329 (1462)
 //    512 tokens: QKV 39 (656) -> 21 (1246),   O 27 (633) -> 16 (1062),  gate/up 139 (866) -> 87 (1384),   down 59 (1019) -> 48 (1244)
 //    160 tokens: QKV 40 -> 16, O 33 -> 13, gate/up 84 -> 52, down 60 -> 30 (the weights alone: 8, 5, 36, 18)
+// These are shortest times.  For seconds on end 4096 tokens are bound by the power cap (988 W, 1.21 to 1.24 GHz): down 398 us, O 111.
 //
 // Block-scaled fp8 (MX): the same tiles with 128 K per stage; the scale factors come through the ring in runs of 512 bytes and are copied to tensor
 // memory in front of their products.  The epilogue's lane has whole blocks of 32 features of its token, so the e4m3 copy that the next product reads
 // needs no exchange between lanes.  256-wide tiles leave no columns for scale factors beside two accumulators, so these overlap by 32 columns, which
-// the epilogue takes first (128-wide tiles have none of that, but twice the rounds: gate/up of 4096 tokens 384 us against 335).  gemm_tc.cu reads
+// the epilogue takes first (128-wide tiles have none of that, but twice the rounds: gate/up of 4096 tokens 384 us against 333).  gemm_tc.cu reads
 // 128 + 256 operand rows per 128 x 256 tile and has no second accumulator.  Llama-3-8B layer shapes, us, back to back with cold weights, gemm_tc.cu -> here:
 //   4096 tokens: QKV 223 -> 76, O 264 -> 59, gate/up 1751 -> 333 (2.9 PFLOP/s), down 461 -> 189
 //    512 tokens: QKV  50 -> 17, O  44 -> 13, gate/up  286 -> 50, down 77 -> 29
@@ -128,11 +129,6 @@ __device__ __forceinline__ void tma_load2(void* smem_dst, const CUtensorMap* m, 
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
-}
-// the accumulator has been read (tcgen05.fence orders that): nothing that was written goes with it, and a release to the cluster waits until the tile's stores have
-// arrived in L2
-__device__ __forceinline__ void arrive_cluster_read(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // One arrival per CTA; the last one releases the payload to the downstream piece and this piece's input slot to the upstream one -- unless a

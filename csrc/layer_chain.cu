@@ -125,11 +125,6 @@ __device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, float a
 __device__ __forceinline__ void arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// The same where the neighbour only has to know that this warp has READ its shared memory: nothing that was written goes with it, and a release to the cluster
-// waits until every earlier store of the thread has arrived in L2 (1 to 2.5 us per tile of a product while the weights stream).
-__device__ __forceinline__ void arrive_cluster_read(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ bool try_wait_cluster(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -967,7 +962,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) layer_chain_kernel(const __grid
               for (int i = 0; i < HB; ++i) c1[i] = from[i * 64];
             }
             __syncwarp();
-            if (lane < LC_CL && ok) arrive_cluster_read(mapa_smem(smem_u32(zone_free), lane));    // the sums have been read
+            if (lane < LC_CL && ok) arrive_cluster_read(mapa_smem(smem_u32(zone_free), lane));    // the sums have been read (and the halves, stored and read back)
             if (GLU && op == OP_GU) {
               const int t0 = up ? HB : 0;
               float h[HB];
@@ -1643,9 +1638,9 @@ int launch_layer_chain(const ChainDims& d, const ChainCall& c, cudaStream_t s) {
   return B2B_CHAIN64(launch_chain_one, m, p, s);
 }
 
-// Block-scaled fp8 steps of 33 tokens and more stay with the kernels one by one.  That was measured when a tile's stores held up the next one (two layers of
-// Zephyr-7B, 40 tokens: 193.5 us one by one, 195.0 here); here they would now be the faster ones (Llama-3-8B behind 500 keys, one by one / here: 40 tokens 211 / 194, 64
-// tokens 228 / 214, but 34 tokens 193 / 192, and behind 4000 keys 335 / 373).
+// Block-scaled fp8 steps of 33 tokens and more stay with the kernels one by one.  The line was drawn when a tile's stores held up the next one (two layers of
+// Zephyr-7B, 40 tokens: 193.5 us one by one, 195.0 here) and is now too low for few keys (Llama-3-8B behind 500 keys, one by one / here: 40 tokens 211 / 194, 64
+// tokens 228 / 214; but 34 tokens 193 / 192, and behind 4000 keys 335 / 373): beyond it what attention costs has not been measured.
 int layer_chain_tokens(const ChainDims& d) { return d.mx ? 32 : 64; }
 
 // clusters that are resident at once (0: the kernel cannot run here); also sets the kernels' shared memory sizes, so that a first launch may

@@ -23,7 +23,7 @@
 //
 // Bound: tensor pipe (98 % active while a tile runs) and the power cap.  Measured on B200, Llama-3-8B layer shapes, us (TFLOP/s), back to
 // back with cold weights, gemm_tc.cu -> here:
-//   4096 tokens: QKV 218 (945) -> 130 (1586), O 157 (875) -> 95 (1447), gate/up 1041 (924) -> 581 (1656), down 404 (1191) -> 329 (1462)
+//   4096 tokens: QKV 218 (945) -> 129 (1598), O 157 (875) -> 94 (1462), gate/up 1041 (924) -> 573 (1679), down 404 (1191) -> 329 (1462)
 //    512 tokens: QKV 39 (656) -> 21 (1246),   O 27 (633) -> 16 (1062),  gate/up 139 (866) -> 87 (1384),   down 59 (1019) -> 48 (1244)
 //    160 tokens: QKV 40 -> 16, O 33 -> 13, gate/up 84 -> 52, down 60 -> 30 (the weights alone: 8, 5, 36, 18)
 // These are shortest times.  For seconds on end 4096 tokens are bound by the power cap (988 W, 1.21 to 1.24 GHz): down 398 us, O 111.

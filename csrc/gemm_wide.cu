@@ -434,7 +434,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       // that product's operand, and the row's sum of squares.  A lane has the whole block of its token: no exchange.
       auto emit_q = [&](int feat) {
         uint32_t e8[8];
-        float r[32], most = 0.f;
+        float r[32];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const uint4 w = *reinterpret_cast<const uint4*>(srow + j * 16);
@@ -446,6 +446,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             r[8 * j + 2 * e + 1] = f.y;
           }
         }
+        float most = fabsf(r[0]);                  // (of nothing but NaNs: NaN, as in the other quantisers)
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           most = fmaxf(most, fabsf(r[j]));

@@ -336,6 +336,18 @@ def test_block_scaled_gate_up_without_rows(m, n, k, tile, gelu):
     assert ops.native().gemm_wide_gave_up() == 0
 
 
+def test_block_scaled_copy_of_nan():
+    """a token that is not a number leaves the copy that the quantiser would, its own rows alone"""
+    m, n, k = 200, 512, 256
+    wq, xq, mx, ref, bn = mx_operands(m, n, k)
+    res = bf(m, n)
+    res[7], res[9, 40] = float("nan"), float("inf")
+    q8, q_sf = mx_copy(m, n, bn)
+    out = ops.gemm(wq, xq, epi=ops.EPI_RESIDUAL, residual=res, fq_out=q8, fq_sf=q_sf, fq_bn=bn, **mx)
+    assert out[7].isnan().all() and out.isfinite().sum() == m * n - n - 1
+    is_copy(q8, q_sf, out, bn)
+
+
 def _quantised_hop(m, n, k, flags):
     """a product between two neighbours that hand over block-scaled rows: it waits for the upstream one's, and leaves its rows, their e4m3 copy and their sums
     of squares in the downstream one's memory"""

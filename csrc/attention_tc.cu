@@ -555,10 +555,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           o[e] = __bfloat162float(__float2bfloat16_rn(o[e] * inv));
           amax = fmaxf(amax, fabsf(o[e]));
         }
-        const uint32_t u = __float_as_uint(amax * (1.f / 448.f));
-        int ex = static_cast<int>(u >> 23) - 127 + ((u & 0x7FFFFFu) ? 1 : 0);
-        ex = max(-126, min(127, ex));
-        const float sc = __uint_as_float(static_cast<uint32_t>(127 - ex) << 23);
+        const int ex = mx_exponent(amax);
+        const float sc = mx_inverse(ex);
         const int tok = qtok0 + i, feat = (kvh * G + g) * D + c, ldq = p.n_q * D;
         uint32_t w8[8];
 #pragma unroll
@@ -572,9 +570,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         uint4* q4 = reinterpret_cast<uint4*>(p.q_out8 + static_cast<size_t>(tok) * ldq + feat);
         q4[0] = make_uint4(w8[0], w8[1], w8[2], w8[3]);
         q4[1] = make_uint4(w8[4], w8[5], w8[6], w8[7]);
-        const int tile = tok / p.q_bn, n = tok - tile * p.q_bn, rr = n & 127;
-        p.q_sf[(static_cast<size_t>(tile) * (ldq >> 7) + (feat >> 7)) * (p.q_bn > 128 ? 1024 : 512) + (n >> 7) * 512 +
-               (rr & 31) * 16 + (rr >> 5) * 4 + ((feat >> 5) & 3)] = static_cast<uint8_t>(ex + 127);
+        p.q_sf[mx_sf_at(tok, feat, p.q_bn, ldq >> 7)] = static_cast<uint8_t>(ex + 127);
       } else if (row_valid) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {

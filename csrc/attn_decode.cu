@@ -411,16 +411,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         float amax = fabsf(rv);
 #pragma unroll
         for (int sh = 16; sh > 0; sh >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, sh));
-        const uint32_t u = __float_as_uint(amax * (1.f / 448.f));
-        int ex = static_cast<int>(u >> 23) - 127 + ((u & 0x7FFFFFu) ? 1 : 0);
-        ex = max(-126, min(127, ex));
+        const int ex = mx_exponent(amax);
         p.q_out8[static_cast<size_t>(tok) * ldq + feat] = static_cast<uint8_t>(
-            __nv_cvt_float_to_fp8(rv * __uint_as_float(static_cast<uint32_t>(127 - ex) << 23), __NV_SATFINITE, __NV_E4M3));
-        if (lane == 0) {
-          const int tile = tok / p.q_bn, nn = tok - tile * p.q_bn, rr = nn & 127;
-          p.q_sf[(static_cast<size_t>(tile) * (ldq >> 7) + (feat >> 7)) * (p.q_bn > 128 ? 1024 : 512) + (nn >> 7) * 512 + (rr & 31) * 16 +
-                 (rr >> 5) * 4 + ((feat >> 5) & 3)] = static_cast<uint8_t>(ex + 127);
-        }
+            __nv_cvt_float_to_fp8(rv * mx_inverse(ex), __NV_SATFINITE, __NV_E4M3));
+        if (lane == 0) p.q_sf[mx_sf_at(tok, feat, p.q_bn, ldq >> 7)] = static_cast<uint8_t>(ex + 127);
       }
     }
   }

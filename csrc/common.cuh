@@ -254,6 +254,19 @@ __device__ __forceinline__ void cluster_arrive_release() {
 __device__ __forceinline__ void cluster_arrive_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
 }
+// Block-scaled fp8: the power of two, 2^e with e = ceil(log2(most / 448)) in the range of UE8M0, that brings a block's largest magnitude to at most 448 (e + 127 is
+// stored); 2^-e; and where the scale factor of (token, 32 features) lies for tokens in tiles of `bn` and a consumer with 128 * nkc features: the tcgen05.cp
+// layout, 512 bytes per 128 features and up to 128 tokens, twice that for tiles of up to 256.
+__device__ __forceinline__ int mx_exponent(float most) {
+  const uint32_t u = __float_as_uint(most * (1.f / 448.f));
+  return max(-126, min(127, static_cast<int>(u >> 23) - 127 + ((u & 0x7FFFFFu) ? 1 : 0)));
+}
+__device__ __forceinline__ float mx_inverse(int e) { return __uint_as_float(static_cast<uint32_t>(127 - e) << 23); }
+__device__ __forceinline__ size_t mx_sf_at(int tok, int feat, int bn, int nkc) {
+  const int tile = tok / bn, n = tok - tile * bn, r = n & 127;
+  return (static_cast<size_t>(tile) * nkc + (feat >> 7)) * (bn > 128 ? 1024 : 512) + (n >> 7) * 512 + (r & 31) * 16 + (r >> 5) * 4 + ((feat >> 5) & 3);
+}
+
 // An arrival on a barrier of a neighbour's (mapped address) which only says that memory has been READ.  A release to the cluster would wait until every earlier
 // store of the thread has arrived in L2 (1 to 2.5 us per tile of a decode product while the weights stream).  Stores into what the neighbour writes next have to be
 // complete by other means: read back behind a barrier of the CTA, as the exchange of gate and up in layer_chain.cu is.

@@ -345,11 +345,8 @@ __global__ void quant_mxfp8_rows_kernel(const __nv_bfloat16* __restrict__ x, uin
     float amax = fmaxf(fmaxf(fabsf(f0), fabsf(f1)), fmaxf(fabsf(f2), fabsf(f3)));
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    // e = ceil(log2(amax / 448)) clamped to the UE8M0 range; 2^e >= amax / 448 so |q| <= 448
-    const uint32_t u = __float_as_uint(amax * (1.f / 448.f));
-    int e = static_cast<int>(u >> 23) - 127 + ((u & 0x7FFFFFu) ? 1 : 0);
-    e = max(-126, min(127, e));
-    const float inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);      // 2^-e (e = 127 -> 2^-127 denormal -> 0; unreachable for bf16 inputs)
+    const int e = mx_exponent(amax);
+    const float inv = mx_inverse(e);               // (e = 127 -> 2^-127 denormal -> 0: infinities alone)
     uint8_t o8[4];
     o8[0] = __nv_cvt_float_to_fp8(f0 * inv, __NV_SATFINITE, __NV_E4M3);
     o8[1] = __nv_cvt_float_to_fp8(f1 * inv, __NV_SATFINITE, __NV_E4M3);

@@ -399,7 +399,6 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
     // computed with a transpose-reduce (8 + 4 + 2 + 1 + 1 shuffles for all 16 tokens instead of 5 dependent shuffles per
     // token): afterwards lanes 2t and 2t+1 hold the totals of token t.
     const int q_nkc = MX ? (p.ld_q >> 7) : 0;
-    const int q_chunk = (MX && p.q_bn > 128) ? 1024 : 512;
     auto emit_q_chunk = [&](const float* qv, int tok_base, int nvalid, int feat) {
       float r[16], am[16], ss[16];
 #pragma unroll
@@ -421,15 +420,12 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
       }
       am[0] = fmaxf(am[0], __shfl_xor_sync(0xffffffffu, am[0], 1));
       ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
-      // this lane's token: t = (lane >> 1) & 15; e = ceil(log2(amax / 448)) clamped to the UE8M0 range
-      const uint32_t u = __float_as_uint(am[0] * (1.f / 448.f));
-      int e_mine = static_cast<int>(u >> 23) - 127 + ((u & 0x7FFFFFu) ? 1 : 0);
-      e_mine = max(-126, min(127, e_mine));
+      const int e_mine = mx_exponent(am[0]);       // of this lane's token: t = (lane >> 1) & 15
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int e = __shfl_sync(0xffffffffu, e_mine, 2 * i);
         if (i < nvalid) {
-          const float inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+          const float inv = mx_inverse(e);
           p.q_out8[static_cast<size_t>(tok_base + i) * p.ld_q + feat] =
               static_cast<uint8_t>(__nv_cvt_float_to_fp8(r[i] * inv, __NV_SATFINITE, __NV_E4M3));
         }
@@ -437,9 +433,7 @@ __global__ void __launch_bounds__(192) gemm_tc_kernel(const __grid_constant__ CU
       const int t = lane >> 1;
       if ((lane & 1) == 0 && t < nvalid) {
         const int tok = tok_base + t;
-        const int tile = tok / p.q_bn, n = tok - tile * p.q_bn, rr = n & 127;
-        p.q_sf[(static_cast<size_t>(tile) * q_nkc + (feat >> 7)) * q_chunk + (n >> 7) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 +
-               ((feat >> 5) & 3)] = static_cast<uint8_t>(e_mine + 127);
+        p.q_sf[mx_sf_at(tok, feat, p.q_bn, q_nkc)] = static_cast<uint8_t>(e_mine + 127);
         if (p.sumsq_out != nullptr) {
           if (p.signal_flag != nullptr) atomicAdd_system(&p.sumsq_out[tok], ss[0]);   // tail GEMM: the counter lives in the peer's memory
           else atomicAdd(&p.sumsq_out[tok], ss[0]);

@@ -452,20 +452,15 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           most = fmaxf(most, fabsf(r[j]));
           ssq += r[j] * r[j];
         }
-        const uint32_t b = __float_as_uint(most * (1.f / 448.f));
-        const int ex = max(-126, min(127, static_cast<int>(b >> 23) - 127 + ((b & 0x7FFFFFu) ? 1 : 0)));
-        const float inv = __uint_as_float(static_cast<uint32_t>(127 - ex) << 23);
+        const int ex = mx_exponent(most);
+        const float inv = mx_inverse(ex);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j] * inv, r[4 * j + 1] * inv), __NV_SATFINITE, __NV_E4M3);
           const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(r[4 * j + 2] * inv, r[4 * j + 3] * inv), __NV_SATFINITE, __NV_E4M3);
           e8[j] = lo | (hi << 16);
         }
-        if (live) {
-          const int n = tok % p.q_bn, rr = n & 127, run = p.q_bn > 128 ? 1024 : 512;
-          p.q_sf[(static_cast<size_t>(tok / p.q_bn) * (p.ld_q >> 7) + (feat >> 7)) * run + (n >> 7) * 512 + (rr & 31) * 16 + (rr >> 5) * 4 +
-                 ((feat >> 5) & 3)] = static_cast<uint8_t>(ex + 127);
-        }
+        if (live) p.q_sf[mx_sf_at(tok, feat, p.q_bn, p.ld_q >> 7)] = static_cast<uint8_t>(ex + 127);
         __syncwarp();                              // the bf16 rows have been stored
         *reinterpret_cast<uint4*>(srow) = make_uint4(e8[0], e8[1], e8[2], e8[3]);
         *reinterpret_cast<uint4*>(srow + 16) = make_uint4(e8[4], e8[5], e8[6], e8[7]);

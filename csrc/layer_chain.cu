@@ -251,10 +251,8 @@ __device__ __forceinline__ void lc_st_heads(uint32_t taddr, const float* v) {
 // block-scaled copy of a value per lane, 32 consecutive features of a token: e4m3 and the power of two that brings the largest (`most`) to at most 448, in
 // the layout of the product that reads it
 __device__ __forceinline__ void lc_store_mx(float r, float most, int tok, int feat, int ld, uint8_t* to, uint8_t* sf, int lane) {
-  const uint32_t b = __float_as_uint(most * (1.f / 448.f));
-  const int e = max(-126, min(127, static_cast<int>(b >> 23) - 127 + ((b & 0x7FFFFFu) ? 1 : 0)));
-  to[static_cast<size_t>(tok) * ld + feat] =
-      static_cast<uint8_t>(__nv_cvt_float_to_fp8(r * __uint_as_float(static_cast<uint32_t>(127 - e) << 23), __NV_SATFINITE, __NV_E4M3));
+  const int e = mx_exponent(most);
+  to[static_cast<size_t>(tok) * ld + feat] = static_cast<uint8_t>(__nv_cvt_float_to_fp8(r * mx_inverse(e), __NV_SATFINITE, __NV_E4M3));
   if (lane == 0) sf[static_cast<size_t>(feat >> 7) * 512 + (tok & 31) * 16 + (tok >> 5) * 4 + ((feat >> 5) & 3)] = static_cast<uint8_t>(e + 127);
 }
 // the same for tokens tok0 .. tok0 + N, `n` of them wanted, of the values as bf16 (like a separate quantiser): the N chains of shuffles run side by side
